@@ -816,20 +816,6 @@ using namespace skv;
 // ---- tensor maps of the 8-bit bucket (host) -------------------------------------------------------------
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess) return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
-
 // rows [num_kv_heads * cap][128 B] of every (layer, sequence) arena, box = 128 rows
 bool encode_rows_map(CUtensorMap* map, const uint8_t* base, long long rows, long long arenas, long long arena_bytes) {
   EncodeTiledFn enc = encode_fn();

@@ -2,295 +2,782 @@
 // cache), with the per-key attention mass the importance tracker needs -- without ever writing the
 // [batch, heads, queries, keys] probability tensor to memory.
 //
-//   pass 1 (prefill_fwd_kernel):  per (64-query tile, query head, sequence) the usual streaming
-//       softmax: S = Q K^T, running max / sum, O += P V; writes O (fp16) and, per query row, the
-//       log-sum-exp in base-2 units.
-//   pass 2 (prefill_mass_kernel): per (64-key tile, KV head, sequence) the transposed product
-//       S^T = K Q^T over every query tile at or after the key tile and every query head of the group;
+//   pass 1 (prefill_fwd_kernel): streaming softmax, S = Q K^T, running max / sum, O += P V; writes O
+//       (fp16) and, per query row, the log-sum-exp in base-2 units.
+//   pass 2 (prefill_mass_kernel): the transposed product S^T = K Q^T per (128-key tile, KV head,
+//       sequence) over every query tile at or after the key tile and every query head of the group;
 //       with the row normalisers of pass 1, p = exp2(s - lse[q]) is final, and its sum over the
 //       queries, weighted by the head weight, is the key's mass.  One value per (sequence, KV head,
 //       key) is written; the caller adds the KV heads (a fixed order, so the result is reproducible).
 //
-// Both products are GEMM tiles on mma.sync m16n8k16 (fp16 in, fp32 accumulate): the prompt pass runs
-// once per sequence, reads O(n) bytes for O(n^2) arithmetic, and is a small part of a generation.
+// What bounds both: the exponentials.  A 128 x 128 tile has 16384 of them, 1024 cycles of an SM's 16-a-cycle
+// unit; its products take 1024 cycles (pass 1, head_dim 128), 512 (pass 1 at 64, pass 2 at 128) or 256 cycles of the
+// tensor core.  So the products run on tcgen05 (fp16 in, fp32 accumulators in tensor memory) from TMA-fetched
+// tiles, issued by one thread, and the threads are left with one query (pass 2: key) row each: no shuffle, no
+// shared-memory traffic for S or P.  P goes back to tensor memory as the A operand of P V (fp16, as everywhere
+// here), over the columns its S came from.
+//
+// Both kernels are persistent, one CTA per SM: two softmax warpgroups, one loading warp, one warp that issues the MMAs.
+// Pass 1 gives each warpgroup its own 128-query tile so that one computes exponentials while the tensor core works
+// for the other: two query heads of one KV head at the same positions where the group is even (they share every K
+// and V tile and have the same causal range), otherwise two neighbouring query tiles of one head.  Pass 2 hands the
+// query tiles of the stream to the two warpgroups in turn, through four accumulators.  Units of work are dealt
+// longest first, back and forth over the CTAs, because a causal unit's length is proportional to its position.
+//
+// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 1020 us (4315 us with 64 x 64 tiles on
+// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 72 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
+// head_dim 128: 77 us (289 us).
 #include <cuda_fp16.h>
 
-#include "common.cuh"
+#include "tc05.cuh"
 
 namespace skv {
 
-constexpr int kPfTile = 64;     // queries per CTA tile and keys per streamed tile
-constexpr int kPfThreads = 128;  // 4 warps x 16 rows
+constexpr int kPfTile = 128;                 // queries per tile and keys per streamed tile
+constexpr int kPfSoftmaxThreads = 256;       // two warpgroups
+constexpr int kPfThreads = kPfSoftmaxThreads + 64;  // + the loading warp and the MMA warp
+constexpr uint32_t kPfTmemCols = 512;
+
+struct PrefillTensor {
+  const __half* base;
+  long long sb, st, sh;  // element strides of batch, token, head (head_dim is contiguous)
+  int mul_h, mul_b;      // 0: the map has no such dimension (one entry, or the same data for all of them)
+  int by_rows;           // the map cannot express the strides: the loading warp copies row by row
+};
 
 struct PrefillParams {
-  const __half* q;
-  const __half* k;
-  const __half* v;
-  long long q_sb, q_st, q_sh;  // element strides of batch, token, head (head_dim is contiguous)
-  long long k_sb, k_st, k_sh;
-  long long v_sb, v_st, v_sh;
+  PrefillTensor q, k, v;
   __half* out;                 // [batch][tokens][q heads][head_dim]
   float* lse;                  // [batch][q heads][tokens], base-2
   const float* head_w;         // [batch][q heads] or null
   float* mass;                 // [batch][kv heads][tokens]
   int batch, tokens, num_q_heads, num_kv_heads;
+  int tiles;                   // 128-token tiles of a sequence
+  int units;
   float scale_log2;
 };
 
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t& r0, uint32_t& r1, const void* smem_row) {
-  const uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem_row);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-  __half2 h = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-__device__ __forceinline__ float fast_exp2(float x) {
+template <int D>
+struct PfCfg {
+  static constexpr int kTileBytes = kPfTile * D * 2;
+  static constexpr int kStages = D == 128 ? 4 : 6;
+  static constexpr uint32_t kFwdSmem = (kStages + 2) * kTileBytes + 1024 + 256;
+  static constexpr uint32_t kMassSmem = (kStages + 1) * kTileBytes + 1024 + 8 * 136 * 4 + 2 * kPfTile * 4 + 448;
+};
+
+__device__ __forceinline__ float pf_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ uint32_t pf_pack_half2(float lo, float hi) {
+  __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+// two fp32 operations per instruction
+__device__ __forceinline__ uint64_t pf_pair(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void pf_unpair(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t pf_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t pf_add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 
-// Copies rows [row0, row0 + 64) x D halves of a strided [tokens][D] matrix into shared memory with row
-// stride LD; rows at or beyond `tokens` are zero.
-template <int D, int LD>
-__device__ __forceinline__ void load_tile(__half* dst, const __half* src, long long token_stride, int row0, int tokens) {
+// Bounded wait: the thread is suspended inside try_wait; after two seconds' worth of clock cycles, or once another
+// role gave up, it returns false.  A CTA that gives up writes NaN to the rows it still owed.
+__device__ __noinline__ bool pf_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const long long t0 = clock64();
+  while (clock64() - t0 < 4000000000ll) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return mbar_try_wait(bar, parity) || pf_wait_slow(bar, parity, abort_flag);
+}
+
+// The unit a CTA takes in its `round`-th turn (-1: none left): back and forth, so that whoever got the longest unit of
+// one round gets the shortest of the next.
+__device__ __forceinline__ int pf_unit(int round, int units) {
+  const int grid = (int)gridDim.x, c = (int)blockIdx.x;
+  const long long u = (long long)round * grid + ((round & 1) ? grid - 1 - c : c);
+  return u < units ? (int)u : -1;
+}
+
+// One 128-row tile of a strided [tokens][D] matrix into shared memory as K-major 128-byte swizzled blocks of 64 columns
+// ([D / 64][128 rows][128 B], rows at or beyond `tokens` zero).  Whole warp; `bar` must have been armed for the bytes when
+// the tile goes through the map.
+template <int D>
+__device__ __forceinline__ void pf_load_tile(uint8_t* dst, const CUtensorMap* map, const PrefillTensor& t, int row0, int h, int b,
+                                             int tokens, uint64_t* bar, int lane) {
+  if (!t.by_rows) {
+    if (lane == 0) {
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c)
+        tma_load_4d(dst + c * (kPfTile * 128), map, c * 64, row0, h * t.mul_h, b * t.mul_b, bar);
+    }
+    return;
+  }
   constexpr int CH = D / 8;  // 16-byte chunks per row
-  for (int i = threadIdx.x; i < kPfTile * CH; i += kPfThreads) {
+  const __half* src = t.base + b * t.sb + h * t.sh;
+  for (int i = lane; i < kPfTile * CH; i += 32) {
     const int r = i / CH, c = i % CH;
     uint4 val = make_uint4(0u, 0u, 0u, 0u);
-    if (row0 + r < tokens) val = *reinterpret_cast<const uint4*>(src + (long long)(row0 + r) * token_stride + c * 8);
-    *reinterpret_cast<uint4*>(dst + r * LD + c * 8) = val;
+    if (row0 + r < tokens) val = *reinterpret_cast<const uint4*>(src + (long long)(row0 + r) * t.st + c * 8);
+    *reinterpret_cast<uint4*>(dst + (c >> 3) * (kPfTile * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
   }
+  fence_proxy_async();  // the MMAs read the tile through the async proxy
+  __syncwarp();
+}
+template <int D>
+__device__ __forceinline__ uint32_t pf_tile_tx(const PrefillTensor& t) {
+  return t.by_rows ? 0u : (uint32_t)PfCfg<D>::kTileBytes;
 }
 
-// A fragments (16 rows x D) of this warp's rows out of a shared tile [64][LD]
-template <int D, int LD>
-__device__ __forceinline__ void load_a_frags(const __half* tile, int warp, int lane, uint32_t (&a)[D / 16][4]) {
-  const int g = lane >> 2, t = lane & 3;
-  const __half* r0 = tile + (warp * 16 + g) * LD;
-  const __half* r1 = r0 + 8 * LD;
+// S = A B^T over head_dim, both K-major: one 16-column step per instruction
+template <int D>
+__device__ __forceinline__ void pf_issue_scores(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem) {
+  constexpr uint32_t idesc = idesc_f16(0, 0, 128, 128);
 #pragma unroll
   for (int kk = 0; kk < D / 16; ++kk) {
-    a[kk][0] = *reinterpret_cast<const uint32_t*>(r0 + kk * 16 + 2 * t);
-    a[kk][1] = *reinterpret_cast<const uint32_t*>(r1 + kk * 16 + 2 * t);
-    a[kk][2] = *reinterpret_cast<const uint32_t*>(r0 + kk * 16 + 2 * t + 8);
-    a[kk][3] = *reinterpret_cast<const uint32_t*>(r1 + kk * 16 + 2 * t + 8);
+    const uint32_t off = (kk / 4) * (kPfTile * 128) + (kk % 4) * 32;
+    mma_f16_ss(d_tmem, smem_desc(a_smem + off, 1, 64, 2), smem_desc(b_smem + off, 1, 64, 2), idesc, kk > 0);
   }
 }
 
-// c[j] (j = 0..7: eight 8-column tiles) = A (16 x D, registers) times the transpose of the shared tile [64][LD]
-template <int D, int LD>
-__device__ __forceinline__ void gemm_a_bt(const uint32_t (&a)[D / 16][4], const __half* tile, int lane, float (&c)[8][4]) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
-    const __half* row = tile + (j * 8 + g) * LD + 2 * t;
-#pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      const uint32_t b0 = *reinterpret_cast<const uint32_t*>(row + kk * 16);
-      const uint32_t b1 = *reinterpret_cast<const uint32_t*>(row + kk * 16 + 8);
-      mma_f16(c[j], a[kk], b0, b1);
-    }
-  }
-}
-
-template <int D>
-__global__ void __launch_bounds__(kPfThreads) prefill_fwd_kernel(const PrefillParams p) {
-  constexpr int LD = D + 8;
-  extern __shared__ __align__(16) uint8_t pf_smem[];
-  __half* ks = reinterpret_cast<__half*>(pf_smem);  // [64][LD], first used for the query tile
-  __half* vs = ks + kPfTile * LD;                   // [64][LD]
-  const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;  // the longest rows first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hk = h / (p.num_q_heads / p.num_kv_heads);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n = p.tokens, q0 = qt * kPfTile;
-
-  load_tile<D, LD>(ks, p.q + b * p.q_sb + h * p.q_sh, p.q_st, q0, n);
-  __syncthreads();
-  uint32_t qa[D / 16][4];
-  load_a_frags<D, LD>(ks, warp, lane, qa);
-  __syncthreads();
-
-  float o[D / 8][4];
-#pragma unroll
-  for (int j = 0; j < D / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // rows g and g + 8 of this warp
-  const int row0 = q0 + warp * 16 + g, row1 = row0 + 8;
-
-  const __half* kbase = p.k + b * p.k_sb + hk * p.k_sh;
-  const __half* vbase = p.v + b * p.v_sb + hk * p.v_sh;
-  for (int kt = 0; kt <= qt; ++kt) {
-    const int k0 = kt * kPfTile;
-    load_tile<D, LD>(ks, kbase, p.k_st, k0, n);
-    load_tile<D, LD>(vs, vbase, p.v_st, k0, n);
-    __syncthreads();
-    float s[8][4];
-    gemm_a_bt<D, LD>(qa, ks, lane, s);
-    // scale, causal mask (only the diagonal tile and the ragged end need it)
-    const bool edge = kt == qt || k0 + kPfTile > n;
-    float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float x = s[j][e] * p.scale_log2;
-        if (edge) {
-          const int key = k0 + j * 8 + 2 * t + (e & 1);
-          const int row = (e < 2) ? row0 : row1;
-          if (key > row || key >= n) x = -INFINITY;
-        }
-        s[j][e] = x;
-      }
-      mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
-      mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
-    }
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
-    const float a0 = (n0 == -INFINITY) ? 1.f : fast_exp2(m0 - n0), a1 = (n1 == -INFINITY) ? 1.f : fast_exp2(m1 - n1);
-    const float u0 = (n0 == -INFINITY) ? 0.f : n0, u1 = (n1 == -INFINITY) ? 0.f : n1;
-    m0 = n0;
-    m1 = n1;
-    l0 *= a0;
-    l1 *= a1;
-#pragma unroll
-    for (int j = 0; j < D / 8; ++j) {
-      o[j][0] *= a0;
-      o[j][1] *= a0;
-      o[j][2] *= a1;
-      o[j][3] *= a1;
-    }
-    uint32_t pa[4][4];  // P as A fragments: four 16-key steps
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float p0 = fast_exp2(s[j][0] - u0), p1 = fast_exp2(s[j][1] - u0);
-      const float p2 = fast_exp2(s[j][2] - u1), p3 = fast_exp2(s[j][3] - u1);
-      l0 += p0 + p1;
-      l1 += p2 + p3;
-      pa[j >> 1][(j & 1) * 2] = pack_half2(p0, p1);
-      pa[j >> 1][(j & 1) * 2 + 1] = pack_half2(p2, p3);
-    }
-    // O += P V : B fragments of V (keys x dims) through transposing matrix loads
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const __half* vrow = vs + (kk * 16 + (lane & 15)) * LD;
-#pragma unroll
-      for (int j = 0; j < D / 8; ++j) {
-        uint32_t b0, b1;
-        ldmatrix_x2_trans(b0, b1, vrow + j * 8);
-        mma_f16(o[j], pa[kk], b0, b1);
-      }
-    }
-    __syncthreads();
-  }
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  const float i0 = l0 > 0.f ? 1.f / l0 : 0.f, i1 = l1 > 0.f ? 1.f / l1 : 0.f;
-  if (t == 0) {
-    float* lse = p.lse + ((long long)b * p.num_q_heads + h) * n;
-    if (row0 < n) lse[row0] = m0 + log2f(l0);
-    if (row1 < n) lse[row1] = m1 + log2f(l1);
-  }
-  __half* ob = p.out + ((long long)b * n * p.num_q_heads + h) * D;
-#pragma unroll
-  for (int j = 0; j < D / 8; ++j) {
-    if (row0 < n)
-      *reinterpret_cast<__half2*>(ob + (long long)row0 * p.num_q_heads * D + j * 8 + 2 * t) =
-          __floats2half2_rn(o[j][0] * i0, o[j][1] * i0);
-    if (row1 < n)
-      *reinterpret_cast<__half2*>(ob + (long long)row1 * p.num_q_heads * D + j * 8 + 2 * t) =
-          __floats2half2_rn(o[j][2] * i1, o[j][3] * i1);
-  }
-}
-
-template <int D>
-__global__ void __launch_bounds__(kPfThreads) prefill_mass_kernel(const PrefillParams p) {
-  constexpr int LD = D + 8;
-  extern __shared__ __align__(16) uint8_t pf_smem[];
-  __half* qs = reinterpret_cast<__half*>(pf_smem);                  // [64][LD]: key tile first, then query tiles
-  float* lse_s = reinterpret_cast<float*>(qs + kPfTile * LD);       // [64]
-  const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+struct PfFwdUnit {
+  int tile[2], head[2], blocks[2];  // per warpgroup: query tile, query head, key tiles (0: nothing to do)
+  int hk, b;
+};
+__device__ __forceinline__ PfFwdUnit pf_fwd_unit(const PrefillParams& p, int u) {
+  PfFwdUnit r;
   const int G = p.num_q_heads / p.num_kv_heads;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n = p.tokens, k0 = kt * kPfTile;
-  const int nqt = (n + kPfTile - 1) / kPfTile;
+  if ((G & 1) == 0) {
+    const int pairs = p.num_q_heads >> 1, per = pairs * p.batch;
+    const int t = p.tiles - 1 - u / per, rest = u % per;
+    r.b = rest / pairs;
+    const int h = 2 * (rest % pairs);
+    r.tile[0] = r.tile[1] = t;
+    r.head[0] = h;
+    r.head[1] = h + 1;
+    r.blocks[0] = r.blocks[1] = t + 1;
+    r.hk = h / G;
+  } else {
+    const int per = p.num_q_heads * p.batch;
+    const int t = (p.tiles + 1) / 2 - 1 - u / per, rest = u % per;
+    r.b = rest / p.num_q_heads;
+    const int h = rest % p.num_q_heads;
+    r.tile[0] = 2 * t;
+    r.tile[1] = 2 * t + 1;
+    r.head[0] = r.head[1] = h;
+    r.blocks[0] = 2 * t + 1;
+    r.blocks[1] = 2 * t + 1 < p.tiles ? 2 * t + 2 : 0;
+    r.hk = h / G;
+  }
+  return r;
+}
 
-  load_tile<D, LD>(qs, p.k + b * p.k_sb + hk * p.k_sh, p.k_st, k0, n);
-  __syncthreads();
-  uint32_t ka[D / 16][4];
-  load_a_frags<D, LD>(qs, warp, lane, ka);
-  __syncthreads();
+struct PfFwdBars {
+  uint64_t full[6], empty[6];
+  uint64_t qfull, qempty;
+  uint64_t sfull[2], pready[2], oready[2];
+  uint64_t drain;
+  uint32_t tmem_base;
+  int abort_flag;
+};
 
-  const int key0 = k0 + warp * 16 + g, key1 = key0 + 8;
-  float acc0 = 0.f, acc1 = 0.f;
-  for (int hh = 0; hh < G; ++hh) {
-    const int h = hk * G + hh;
-    const float w = p.head_w != nullptr ? p.head_w[(long long)b * p.num_q_heads + h] : 1.f;
-    const float* lse = p.lse + ((long long)b * p.num_q_heads + h) * n;
-    float h0 = 0.f, h1 = 0.f;
-    for (int qt = kt; qt < nqt; ++qt) {
-      const int q0 = qt * kPfTile;
-      load_tile<D, LD>(qs, p.q + b * p.q_sb + h * p.q_sh, p.q_st, q0, n);
-      if (threadIdx.x < kPfTile) lse_s[threadIdx.x] = (q0 + threadIdx.x < n) ? lse[q0 + threadIdx.x] : INFINITY;
-      __syncthreads();
-      float s[8][4];
-      gemm_a_bt<D, LD>(ka, qs, lane, s);
-      const bool edge = qt == kt;
+template <int D>
+__global__ void __launch_bounds__(kPfThreads, 1)
+    prefill_fwd_kernel(const __grid_constant__ PrefillParams p, const __grid_constant__ CUtensorMap qmap,
+                       const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
+  using Cfg = PfCfg<D>;
+  constexpr int NS = Cfg::kStages, TB = Cfg::kTileBytes;
+  extern __shared__ uint8_t pf_smem_raw[];
+  uint8_t* smem = pf_smem_raw + ((1024u - (smem_u32(pf_smem_raw) & 1023u)) & 1023u);  // swizzle atoms are 1024 bytes
+  uint8_t* ring = smem;                    // [NS][TB]: K and V tiles in the order they are used
+  uint8_t* qs = ring + NS * TB;            // [2][TB]
+  PfFwdBars& br = *reinterpret_cast<PfFwdBars*>(qs + 2 * TB);
+  static_assert(sizeof(PfFwdBars) <= 256, "barrier block");
+  volatile int* abort_flag = &br.abort_flag;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  if (tid == 0) {
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(&br.full[s], 1);
+      mbar_init(&br.empty[s], 1);
+    }
+    mbar_init(&br.qfull, 1);
+    mbar_init(&br.qempty, 1);
+    for (int w = 0; w < 2; ++w) {
+      mbar_init(&br.sfull[w], 1);
+      mbar_init(&br.pready[w], 4);  // one arrival per warp
+      mbar_init(&br.oready[w], 1);
+    }
+    mbar_init(&br.drain, 1);
+    br.abort_flag = 0;
+    mbar_fence_init();
+  }
+  __syncwarp();
+  if (warp == 0) tmem_alloc(&br.tmem_base, kPfTmemCols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = br.tmem_base;  // columns: S_0 S_1 (128 each), O_0 O_1 (D each)
+
+  if (warp == 8) {
+    // ================================ loading warp ================================
+    int i = 0, last_unit = -1;
+    bool ok = true;
+    auto stage = [&](const CUtensorMap* map, const PrefillTensor& t, int row0, int h, int b) {
+      const int s = i % NS;
+      ok = pf_wait(&br.empty[s], ((i / NS) & 1) ^ 1u, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return;
+      const uint32_t tx = pf_tile_tx<D>(t);
+      if (tx && lane == 0) mbar_expect_tx(&br.full[s], tx);
+      pf_load_tile<D>(ring + s * TB, map, t, row0, h, b, p.tokens, &br.full[s], lane);
+      if (!tx && lane == 0) mbar_arrive(&br.full[s]);
+      ++i;
+    };
+    for (int round = 0; ok; ++round) {
+      const int u = pf_unit(round, p.units);
+      if (u < 0) break;
+      const PfFwdUnit un = pf_fwd_unit(p, u);
+      ok = __all_sync(0xffffffffu, pf_wait(&br.qempty, (round & 1) ^ 1u, abort_flag));
+      if (!ok) break;
+      const int nq = un.blocks[1] > 0 ? 2 : 1;
+      const uint32_t tx = pf_tile_tx<D>(p.q) * nq;
+      if (tx && lane == 0) mbar_expect_tx(&br.qfull, tx);
+      for (int w = 0; w < nq; ++w)
+        pf_load_tile<D>(qs + w * TB, &qmap, p.q, un.tile[w] * kPfTile, un.head[w], un.b, p.tokens, &br.qfull, lane);
+      if (!tx && lane == 0) mbar_arrive(&br.qfull);
+      last_unit = round;
+      const int blocks = max(un.blocks[0], un.blocks[1]);
+      for (int j = 0; ok && j < blocks; ++j) {
+        stage(&kmap, p.k, j * kPfTile, un.hk, un.b);
+        if (ok) stage(&vmap, p.v, j * kPfTile, un.hk, un.b);
+      }
+    }
+    if (!ok) {  // no copy in flight may outlive the shared memory it targets
+      for (int s = 0; s < NS; ++s) {
+        const int cnt = i > s ? (i - 1 - s) / NS + 1 : 0;
+        const long long t0 = clock64();
+        while (cnt > 0 && !mbar_try_wait(&br.full[s], (cnt - 1) & 1) && clock64() - t0 < 1000000000ll) {}
+      }
+      const long long t0 = clock64();
+      while (last_unit >= 0 && !mbar_try_wait(&br.qfull, last_unit & 1) && clock64() - t0 < 1000000000ll) {}
+    }
+  } else if (warp == 9) {
+    // ================================ MMA warp (one thread) ================================
+    if (lane == 0) {
+      int base = 0;                 // ring index of the unit's first K tile
+      int pc[2] = {0, 0};           // P blocks taken from each warpgroup so far
+      bool ok = true;
+      const uint32_t ring_a = smem_u32(ring), qs_a = smem_u32(qs);
+      constexpr uint32_t pv_idesc = idesc_f16(0, 1, 128, D);
+      for (int round = 0; ok; ++round) {
+        const int u = pf_unit(round, p.units);
+        if (u < 0) break;
+        const PfFwdUnit un = pf_fwd_unit(p, u);
+        const int blocks = max(un.blocks[0], un.blocks[1]);
+        ok = pf_wait(&br.qfull, round & 1, abort_flag);
+        // step j: P V of block j-1, then the scores of block j, for one warpgroup and then the other
+        for (int j = 0; ok && j <= blocks; ++j) {
+          const int ik = base + 2 * j, iv = ik - 1;
+          const int sk = ik % NS, sv = (iv + NS) % NS;
+          if (j < blocks) ok = pf_wait(&br.full[sk], (ik / NS) & 1, abort_flag);
+          if (ok && j > 0) ok = pf_wait(&br.full[sv], (iv / NS) & 1, abort_flag);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+          for (int w = 0; w < 2; ++w) {
+            if (ok && j > 0 && j - 1 < un.blocks[w]) {
+              ok = pf_wait(&br.pready[w], pc[w] & 1, abort_flag);
+              if (!ok) break;
+              ++pc[w];
+              tc_fence_after();
+              const uint32_t va = ring_a + sv * TB;
+#pragma unroll
+              for (int kk = 0; kk < kPfTile / 16; ++kk)  // V rows are the contraction: MN-major, 64-column blocks 16 KB apart
+                mma_f16_ts(tmem + 256 + w * D, tmem + w * 128 + kk * 8, smem_desc(va + kk * 2048, kPfTile * 128 / 16, 64, 2),
+                           pv_idesc, (j > 1 || kk > 0) ? 1u : 0u);
+              if (j == un.blocks[w]) mma_commit(&br.oready[w]);
+            }
+            if (ok && j < un.blocks[w]) {
+              // the S columns hold P of the block before; its P V was issued first by this thread, and MMAs run in order
+              pf_issue_scores<D>(tmem + w * 128, qs_a + w * TB, ring_a + sk * TB);
+              mma_commit(&br.sfull[w]);
+            }
+          }
+          if (!ok) break;
+          if (j > 0) mma_commit(&br.empty[sv]);
+          if (j < blocks) mma_commit(&br.empty[sk]);
+          if (j == blocks - 1) mma_commit(&br.qempty);
+        }
+        base += 2 * blocks;
+      }
+      mma_commit(&br.drain);
+      const long long t0 = clock64();
+      while (!mbar_try_wait(&br.drain, 0) && clock64() - t0 < 1000000000ll) {}
+    }
+    __syncwarp();
+  } else {
+    // ================================ softmax warpgroups: one query row per thread ================================
+    const int wg = warp >> 2, wq = warp & 3;
+    const uint32_t lanes = (uint32_t)(wq * 32) << 16;
+    const uint32_t ts = tmem + wg * 128 + lanes, to = tmem + 256 + wg * D + lanes;
+    const float sc = p.scale_log2, grow = 8.0f / sc;
+    const uint64_t sc2 = pf_pair(sc, sc);
+    const int n = p.tokens;
+    int sn = 0, on = 0;  // score tiles / outputs received so far
+    bool ok = true;
+    for (int round = 0;; ++round) {
+      const int u = pf_unit(round, p.units);
+      if (u < 0) break;
+      const PfFwdUnit un = pf_fwd_unit(p, u);
+      const int blocks = un.blocks[wg];
+      if (blocks == 0) continue;
+      const int row = un.tile[wg] * kPfTile + wq * 32 + lane;
+      float m = -INFINITY, l = 0.f;  // m: the maximum the row is scaled by; it lags the true one by at most 2^8
+      for (int j = 0; ok && j < blocks; ++j) {
+        ok = pf_wait(&br.sfull[wg], sn & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        ++sn;
+        tc_fence_after();
+        // The row is read twice, for its maximum and for the exponentials: 128 values held in between would leave the
+        // compiler no registers to overlap anything with.  In the diagonal block a warp's rows see nothing of the chunks
+        // after its own and, in its own, the keys up to the row's position (keys beyond the prompt lie behind those).
+        const int chunks = j == blocks - 1 ? wq + 1 : 4;
+        const bool diag = j == blocks - 1;
+        uint32_t s0[32], s1[32];
+        float b0 = -INFINITY, b1 = -INFINITY, b2 = -INFINITY, b3 = -INFINITY;
+        auto chunk_max = [&](uint32_t (&s)[32], bool masked) {
+          if (masked) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (e > lane) s[e] = 0xff800000u;
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            b0 = fmaxf(b0, __uint_as_float(s[e]));
+            b1 = fmaxf(b1, __uint_as_float(s[e + 1]));
+            b2 = fmaxf(b2, __uint_as_float(s[e + 2]));
+            b3 = fmaxf(b3, __uint_as_float(s[e + 3]));
+          }
+        };
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+          if (c < chunks) {
+            tmem_ld32(ts + c * 32, s0);
+            tmem_ld32(ts + c * 32 + 32, s1);
+            tmem_ld_wait(s0);
+            tmem_ld_wait(s1);
+            chunk_max(s0, diag && c == wq);
+            if (c + 1 < chunks) chunk_max(s1, diag && c + 1 == wq);
+          }
+        }
+        tmem_ld32(ts, s0);  // on its way while the maximum is settled
+        const float bm = fmaxf(fmaxf(b0, b1), fmaxf(b2, b3));
+        if (j == 0) {
+          m = bm;
+        } else {
+          // Rescaling costs a round trip of O through registers, so it waits until a row has outgrown its maximum by
+          // 2^8 (fp16 holds P up to there with the same relative precision).
+          const bool need = bm > m + grow;
+          if (__any_sync(0xffffffffu, need)) {
+            const float f = need ? pf_exp2((m - bm) * sc) : 1.f;
+            if (need) m = bm;
+            l *= f;
+#pragma unroll 1
+            for (int c = 0; c < D / 16; ++c) {  // P V of the block before is complete: this block's scores came after it
+              uint32_t o[16];
+              tmem_ld16(to + c * 16, o);
+              tmem_ld_wait(o);
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+              tmem_st16(to + c * 16, o);
+            }
+          }
+        }
+        const float msc = m == -INFINITY ? 0.f : m * sc;
+        const uint64_t nm2 = pf_pair(-msc, -msc);
+        uint64_t l2a = 0, l2b = 0;
+        auto chunk_exp = [&](int c, uint32_t (&s)[32], uint32_t (&next)[32]) {
+          uint32_t pk[16];
+          if (c < chunks) {
+            tmem_ld_wait(s);
+            if (c + 1 < chunks) tmem_ld32(ts + c * 32 + 32, next);
+            if (diag && c == wq) {
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (e > lane) s[e] = 0xff800000u;
+            }
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              float x0, x1;
+              pf_unpair(pf_fma2(pf_pair(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), sc2, nm2), x0, x1);
+              x0 = pf_exp2(x0);
+              x1 = pf_exp2(x1);
+              if (e & 1) l2b = pf_add2(l2b, pf_pair(x0, x1));
+              else l2a = pf_add2(l2a, pf_pair(x0, x1));
+              pk[e] = pf_pack_half2(x0, x1);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) pk[e] = 0u;
+          }
+          // P of chunk c lies over S columns 16c .. 16c+15, which have been read: chunk c/2 and those before it
+          tmem_st16(ts + c * 16, pk);
+        };
+        chunk_exp(0, s0, s1);
+        chunk_exp(1, s1, s0);
+        chunk_exp(2, s0, s1);
+        chunk_exp(3, s1, s0);
+        float la, lb;
+        pf_unpair(pf_add2(l2a, l2b), la, lb);
+        l += la + lb;
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&br.pready[wg]);
+      }
+      float inv = l > 0.f ? 1.f / l : 0.f, ls = m * sc + log2f(l);
+      if (ok) {
+        ok = pf_wait(&br.oready[wg], on & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        ++on;
+        tc_fence_after();
+      }
+      if (!ok) inv = ls = __int_as_float(0x7fffffff);
+      if (row < n) p.lse[((long long)un.b * p.num_q_heads + un.head[wg]) * n + row] = ls;
+      __half* ob = p.out + (((long long)un.b * n + row) * p.num_q_heads + un.head[wg]) * D;
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld32(to + c * 32, o);
+        tmem_ld_wait(o);
+        if (row < n) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint4 w4;
+            w4.x = pf_pack_half2(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
+            w4.y = pf_pack_half2(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
+            w4.z = pf_pack_half2(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
+            w4.w = pf_pack_half2(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
+            *reinterpret_cast<uint4*>(ob + c * 32 + e * 8) = w4;
+          }
+        }
+      }
+      tc_fence_before();  // O has been read: the arrival on the next unit's first P orders it before the next P V
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_free(tmem, kPfTmemCols);
+}
+
+constexpr int kPfLseSlots = 8;
+constexpr int kPfAcc = 4;  // score accumulators in tensor memory
+
+struct PfMassBars {
+  uint64_t full[6], empty[6];
+  uint64_t kfull, kempty;
+  uint64_t sfull[kPfAcc], sempty[kPfAcc];
+  uint64_t lfull[kPfLseSlots], lempty[kPfLseSlots];
+  uint64_t drain;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+struct PfMassUnit {
+  int kt, hk, b, count;  // key tile, KV head, sequence, query tiles in the stream
+};
+__device__ __forceinline__ PfMassUnit pf_mass_unit(const PrefillParams& p, int u) {
+  PfMassUnit r;
+  const int per = p.num_kv_heads * p.batch, rest = u % per;
+  r.kt = u / per;  // the first key tile sees the most queries
+  r.b = rest / p.num_kv_heads;
+  r.hk = rest % p.num_kv_heads;
+  r.count = (p.tiles - r.kt) * (p.num_q_heads / p.num_kv_heads);
+  return r;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kPfThreads, 1)
+    prefill_mass_kernel(const __grid_constant__ PrefillParams p, const __grid_constant__ CUtensorMap qmap,
+                        const __grid_constant__ CUtensorMap kmap) {
+  using Cfg = PfCfg<D>;
+  constexpr int NS = Cfg::kStages, TB = Cfg::kTileBytes, LS = 136;  // floats per lse slot: 128 + the head weight, 16-byte rows
+  extern __shared__ uint8_t pf_smem_raw[];
+  uint8_t* smem = pf_smem_raw + ((1024u - (smem_u32(pf_smem_raw) & 1023u)) & 1023u);
+  uint8_t* ring = smem;                                            // [NS][TB]: query tiles
+  uint8_t* ks = ring + NS * TB;                                    // the unit's key tile
+  float* lse_s = reinterpret_cast<float*>(ks + TB);                // [kPfLseSlots][LS], negated
+  float* red = lse_s + kPfLseSlots * LS;                           // [2][128]: the second warpgroup's sums
+  PfMassBars& br = *reinterpret_cast<PfMassBars*>(red + 2 * kPfTile);
+  static_assert(sizeof(PfMassBars) <= 448, "barrier block");
+  volatile int* abort_flag = &br.abort_flag;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = p.num_q_heads / p.num_kv_heads, n = p.tokens;
+
+  if (tid == 0) {
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(&br.full[s], 1);
+      mbar_init(&br.empty[s], 1);
+    }
+    mbar_init(&br.kfull, 1);
+    mbar_init(&br.kempty, 1);
+    for (int s = 0; s < kPfAcc; ++s) {
+      mbar_init(&br.sfull[s], 1);
+      mbar_init(&br.sempty[s], 4);  // one arrival per warp of the warpgroup that takes the tile
+    }
+    for (int s = 0; s < kPfLseSlots; ++s) {
+      mbar_init(&br.lfull[s], 1);
+      mbar_init(&br.lempty[s], 4);
+    }
+    mbar_init(&br.drain, 1);
+    br.abort_flag = 0;
+    mbar_fence_init();
+  }
+  __syncwarp();
+  if (warp == 0) tmem_alloc(&br.tmem_base, kPfTmemCols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = br.tmem_base;
+
+  if (warp == 8) {
+    // ================================ loading warp ================================
+    int i = 0, last_unit = -1;
+    bool ok = true;
+    for (int round = 0; ok; ++round) {
+      const int u = pf_unit(round, p.units);
+      if (u < 0) break;
+      const PfMassUnit un = pf_mass_unit(p, u);
+      ok = __all_sync(0xffffffffu, pf_wait(&br.kempty, (round & 1) ^ 1u, abort_flag));
+      if (!ok) break;
+      const uint32_t ktx = pf_tile_tx<D>(p.k), qtx = pf_tile_tx<D>(p.q);
+      if (ktx && lane == 0) mbar_expect_tx(&br.kfull, ktx);
+      pf_load_tile<D>(ks, &kmap, p.k, un.kt * kPfTile, un.hk, un.b, n, &br.kfull, lane);
+      if (!ktx && lane == 0) mbar_arrive(&br.kfull);
+      last_unit = round;
+      int qt = un.kt, h = un.hk * G;
+      for (int j = 0; j < un.count; ++j, ++i) {
+        const int s = i % NS, ls = i % kPfLseSlots;
+        // the row normalisers are on their way while the warp waits for a free stage; a query beyond the prompt gets
+        // -inf (negated lse), which makes its probability zero
+        const float* lse = p.lse + ((long long)un.b * p.num_q_heads + h) * n;
+        float nl[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int qi = j * 8 + 2 * t + (e & 1);
-          // a query beyond the prompt carries lse = +inf, which makes its probability zero
-          float pr = fast_exp2(s[j][e] * p.scale_log2 - lse_s[qi]);
-          if (edge && q0 + qi < ((e < 2) ? key0 : key1)) pr = 0.f;  // causal: the query precedes the key
-          if (e < 2) h0 += pr; else h1 += pr;
+          const int q = qt * kPfTile + e * 32 + lane;
+          nl[e] = q < n ? -lse[q] : -INFINITY;
+        }
+        const float w = p.head_w != nullptr ? p.head_w[(long long)un.b * p.num_q_heads + h] : 1.f;
+        ok = pf_wait(&br.empty[s], ((i / NS) & 1) ^ 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (qtx && lane == 0) mbar_expect_tx(&br.full[s], qtx);
+        pf_load_tile<D>(ring + s * TB, &qmap, p.q, qt * kPfTile, h, un.b, n, &br.full[s], lane);
+        if (!qtx && lane == 0) mbar_arrive(&br.full[s]);
+        ok = __all_sync(0xffffffffu, pf_wait(&br.lempty[ls], ((i / kPfLseSlots) & 1) ^ 1u, abort_flag));
+        if (!ok) {
+          ++i;  // this stage's copy is in flight
+          break;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) lse_s[ls * LS + e * 32 + lane] = nl[e];
+        if (lane == 0) lse_s[ls * LS + 128] = w;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&br.lfull[ls]);
+        if (++qt == p.tiles) {
+          qt = un.kt;
+          ++h;
         }
       }
-      __syncthreads();
     }
-    acc0 = fmaf(w, h0, acc0);
-    acc1 = fmaf(w, h1, acc1);
+    if (!ok) {  // no copy in flight may outlive the shared memory it targets
+      for (int s = 0; s < NS; ++s) {
+        const int cnt = i > s ? (i - 1 - s) / NS + 1 : 0;
+        const long long t0 = clock64();
+        while (cnt > 0 && !mbar_try_wait(&br.full[s], (cnt - 1) & 1) && clock64() - t0 < 1000000000ll) {}
+      }
+      const long long t0 = clock64();
+      while (last_unit >= 0 && !mbar_try_wait(&br.kfull, last_unit & 1) && clock64() - t0 < 1000000000ll) {}
+    }
+  } else if (warp == 9) {
+    // ================================ MMA warp (one thread) ================================
+    if (lane == 0) {
+      int i = 0;
+      bool ok = true;
+      const uint32_t ring_a = smem_u32(ring), ks_a = smem_u32(ks);
+      for (int round = 0; ok; ++round) {
+        const int u = pf_unit(round, p.units);
+        if (u < 0) break;
+        const PfMassUnit un = pf_mass_unit(p, u);
+        ok = pf_wait(&br.kfull, round & 1, abort_flag);
+        for (int j = 0; ok && j < un.count; ++j, ++i) {
+          const int s = i % NS, a = i % kPfAcc;
+          ok = pf_wait(&br.full[s], (i / NS) & 1, abort_flag) && pf_wait(&br.sempty[a], ((i / kPfAcc) & 1) ^ 1u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          pf_issue_scores<D>(tmem + a * 128, ks_a, ring_a + s * TB);
+          mma_commit(&br.sfull[a]);
+          mma_commit(&br.empty[s]);
+          if (j == un.count - 1) mma_commit(&br.kempty);
+        }
+      }
+      mma_commit(&br.drain);
+      const long long t0 = clock64();
+      while (!mbar_try_wait(&br.drain, 0) && clock64() - t0 < 1000000000ll) {}
+    }
+    __syncwarp();
+  } else {
+    // ================================ two warpgroups: one key row per thread ================================
+    const int wg = warp >> 2, wq = warp & 3, wt = tid & 127;
+    const uint32_t lanes = (uint32_t)(wq * 32) << 16;
+    const uint64_t sc2 = pf_pair(p.scale_log2, p.scale_log2);
+    int i0 = 0;  // stream index of the unit's first query tile
+    bool ok = true;
+    for (int round = 0;; ++round) {
+      const int u = pf_unit(round, p.units);
+      if (u < 0) break;
+      const PfMassUnit un = pf_mass_unit(p, u);
+      const int per_head = p.tiles - un.kt;
+      float acc = 0.f;
+      for (int j = (i0 & 1) == wg ? 0 : 1; ok && j < un.count; j += 2) {
+        const int i = i0 + j, a = i % kPfAcc, ls = i % kPfLseSlots;
+        const bool diag = j % per_head == 0;
+        ok = pf_wait(&br.sfull[a], (i / kPfAcc) & 1, abort_flag) && pf_wait(&br.lfull[ls], (i / kPfLseSlots) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const float* nl = lse_s + ls * LS;
+        uint64_t t0 = 0, t1 = 0;
+        const uint32_t ta0 = tmem + a * 128 + lanes;
+        auto chunk_sum = [&](int c, uint32_t (&s)[32]) {
+          if (diag) {  // queries before the row's key: all of the chunks before the warp's own, part of its own
+            if (c < wq) return;
+            if (c == wq) {
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (e < lane) s[e] = 0xff800000u;
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            const float4 q4 = *reinterpret_cast<const float4*>(nl + c * 32 + e);
+            float x0, x1, x2, x3;
+            pf_unpair(pf_fma2(pf_pair(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc2, pf_pair(q4.x, q4.y)), x0, x1);
+            pf_unpair(pf_fma2(pf_pair(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), sc2, pf_pair(q4.z, q4.w)), x2, x3);
+            t0 = pf_add2(t0, pf_pair(pf_exp2(x0), pf_exp2(x1)));
+            t1 = pf_add2(t1, pf_pair(pf_exp2(x2), pf_exp2(x3)));
+          }
+        };
+        uint32_t s0[32], s1[32];
+        tmem_ld32(ta0, s0);
+        tmem_ld_wait(s0);
+        tmem_ld32(ta0 + 32, s1);
+        chunk_sum(0, s0);
+        tmem_ld_wait(s1);
+        tmem_ld32(ta0 + 64, s0);
+        chunk_sum(1, s1);
+        tmem_ld_wait(s0);
+        tmem_ld32(ta0 + 96, s1);
+        chunk_sum(2, s0);
+        tmem_ld_wait(s1);
+        tc_fence_before();  // the accumulator has been read
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&br.sempty[a]);
+        chunk_sum(3, s1);
+        float ta, tb;
+        pf_unpair(pf_add2(t0, t1), ta, tb);
+        acc = fmaf(nl[128], ta + tb, acc);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&br.lempty[ls]);
+      }
+      i0 += un.count;
+      if (!ok) acc = __int_as_float(0x7fffffff);
+      // the second warpgroup hands its sums to the first; the buffer alternates, so the barrier of the next unit protects it
+      if (wg == 1) red[(round & 1) * kPfTile + wt] = acc;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (wg == 0) {
+        const int key = un.kt * kPfTile + wt;
+        if (key < n) p.mass[((long long)un.b * p.num_kv_heads + un.hk) * n + key] = acc + red[(round & 1) * kPfTile + wt];
+      }
+    }
   }
-  acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1);
-  acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
-  acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1);
-  acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
-  if (t == 0) {
-    float* m = p.mass + ((long long)b * p.num_kv_heads + hk) * n;
-    if (key0 < n) m[key0] = acc0;
-    if (key1 < n) m[key1] = acc1;
-  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_free(tmem, kPfTmemCols);
+}
+
+// ---- host ---------------------------------------------------------------------------------------------------
+// A map of {head_dim, token, head, batch}, box = 128 tokens x 64 columns.  A dimension with one entry, or one that repeats the
+// same data (stride 0), is left at extent 1 and its coordinate stays 0.  What no map can hold (every token the same row, or a
+// stride beyond 2^40 bytes) is copied row by row in the kernel.
+static bool make_map(CUtensorMap* map, PrefillTensor& t, int head_dim, int tokens, int heads, int batch) {
+  constexpr long long kMaxStride = 1ll << 39;  // elements; 2^40 bytes
+  t.mul_h = heads > 1 && t.sh != 0;
+  t.mul_b = batch > 1 && t.sb != 0;
+  auto fits = [](long long s) { return s > 0 && s < kMaxStride; };
+  t.by_rows = (tokens > 1 && !fits(t.st)) || (t.mul_h && !fits(t.sh)) || (t.mul_b && !fits(t.sb));
+  if (t.by_rows) return true;
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return false;
+  const cuuint64_t gdim[4] = {(cuuint64_t)head_dim, (cuuint64_t)tokens, (cuuint64_t)(t.mul_h ? heads : 1),
+                              (cuuint64_t)(t.mul_b ? batch : 1)};
+  const cuuint64_t row = (cuuint64_t)head_dim * 2;
+  const cuuint64_t gstr[3] = {tokens > 1 ? (cuuint64_t)t.st * 2 : row, t.mul_h ? (cuuint64_t)t.sh * 2 : row,
+                              t.mul_b ? (cuuint64_t)t.sb * 2 : row};
+  const cuuint32_t box[4] = {64, kPfTile, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half*>(t.base), gdim, gstr, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int D>
-static int launch_prefill(const PrefillParams& p, bool want_mass, cudaStream_t st) {
-  constexpr int LD = D + 8;
-  const int tiles = (p.tokens + kPfTile - 1) / kPfTile;
-  const size_t smem_fwd = 2 * (size_t)kPfTile * LD * sizeof(__half);
-  const size_t smem_mass = (size_t)kPfTile * LD * sizeof(__half) + kPfTile * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(prefill_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fwd) != cudaSuccess)
+static int launch_prefill(PrefillParams& p, bool want_mass, cudaStream_t st) {
+  using Cfg = PfCfg<D>;
+  CUtensorMap qmap = {}, kmap = {}, vmap = {};
+  if (!make_map(&qmap, p.q, D, p.tokens, p.num_q_heads, p.batch) || !make_map(&kmap, p.k, D, p.tokens, p.num_kv_heads, p.batch) ||
+      !make_map(&vmap, p.v, D, p.tokens, p.num_kv_heads, p.batch))
+    return SKV_ERR_CUDA;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return SKV_ERR_CUDA;
+  static bool configured[64] = {};  // the attribute belongs to the device's context
+  if (dev >= 64 || !configured[dev]) {
+    if (cudaFuncSetAttribute(prefill_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kFwdSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(prefill_mass_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kMassSmem) !=
+            cudaSuccess)
       return SKV_ERR_CUDA;
-    configured = true;
+    if (dev < 64) configured[dev] = true;
   }
-  prefill_fwd_kernel<D><<<dim3(tiles, p.num_q_heads, p.batch), kPfThreads, smem_fwd, st>>>(p);
-  if (want_mass)
-    prefill_mass_kernel<D><<<dim3(tiles, p.num_kv_heads, p.batch), kPfThreads, smem_mass, st>>>(p);
+  const int G = p.num_q_heads / p.num_kv_heads;
+  const long long fwd_units = (long long)p.batch * (G % 2 == 0 ? (long long)p.tiles * (p.num_q_heads / 2)
+                                                               : (long long)((p.tiles + 1) / 2) * p.num_q_heads);
+  const long long mass_units = (long long)p.batch * p.tiles * p.num_kv_heads;
+  if (fwd_units > 0x7fffffffll || mass_units > 0x7fffffffll) return SKV_ERR_UNSUPPORTED;
+  p.units = (int)fwd_units;
+  prefill_fwd_kernel<D><<<p.units < sms ? p.units : sms, kPfThreads, Cfg::kFwdSmem, st>>>(p, qmap, kmap, vmap);
+  if (want_mass) {
+    p.units = (int)mass_units;
+    prefill_mass_kernel<D><<<p.units < sms ? p.units : sms, kPfThreads, Cfg::kMassSmem, st>>>(p, qmap, kmap);
+  }
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }
 
@@ -307,16 +794,16 @@ extern "C" int skv_prefill_attention(const void* q, const void* k, const void* v
   if (head_dim != 64 && head_dim != 128) return SKV_ERR_UNSUPPORTED;
   if (batch <= 0 || tokens <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return SKV_ERR_INVALID;
   if (batch > 65535 || num_q_heads > 65535) return SKV_ERR_UNSUPPORTED;
-  for (int i = 0; i < 3; ++i)  // 16-byte vector loads of every row
+  for (int i = 0; i < 3; ++i)  // 16-byte pieces of every row
     if (q_strides[i] % 8 || k_strides[i] % 8 || v_strides[i] % 8) return SKV_ERR_INVALID;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) return SKV_ERR_INVALID;
-  PrefillParams p;
-  p.q = static_cast<const __half*>(q);
-  p.k = static_cast<const __half*>(k);
-  p.v = static_cast<const __half*>(v);
-  p.q_sb = q_strides[0]; p.q_st = q_strides[1]; p.q_sh = q_strides[2];
-  p.k_sb = k_strides[0]; p.k_st = k_strides[1]; p.k_sh = k_strides[2];
-  p.v_sb = v_strides[0]; p.v_st = v_strides[1]; p.v_sh = v_strides[2];
+  auto tensor = [](const void* base, const int64_t* s) {
+    return PrefillTensor{static_cast<const __half*>(base), s[0], s[1], s[2], 0, 0, 0};
+  };
+  PrefillParams p = {};
+  p.q = tensor(q, q_strides);
+  p.k = tensor(k, k_strides);
+  p.v = tensor(v, v_strides);
   p.out = static_cast<__half*>(out);
   p.lse = lse;
   p.head_w = head_weights;
@@ -325,6 +812,7 @@ extern "C" int skv_prefill_attention(const void* q, const void* k, const void* v
   p.tokens = tokens;
   p.num_q_heads = num_q_heads;
   p.num_kv_heads = num_kv_heads;
+  p.tiles = (tokens + kPfTile - 1) / kPfTile;
   p.scale_log2 = 1.4426950408889634f / sqrtf((float)head_dim);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return head_dim == 64 ? launch_prefill<64>(p, key_mass != nullptr, st) : launch_prefill<128>(p, key_mass != nullptr, st);

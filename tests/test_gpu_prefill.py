@@ -80,3 +80,50 @@ def test_prefill_rejects_what_it_cannot_run():
     h = torch.randn((1, 8, 4, 96), device="cuda").half()
     with pytest.raises(SmartKVLibraryError):
         causal_prefill_attention(h, h, h)                                   # head_dim 96
+
+
+def _dense64(q, k, v, w):
+    """fp64 (out [B, n, Hq, D], mass [B, n]) from the same fp16 numbers."""
+    B, n, hq, d = q.shape
+    qh, kh, vh = (x.transpose(1, 2).double() for x in (q, k, v))
+    kh, vh = (x.repeat_interleave(hq // x.shape[1], 1) for x in (kh, vh))
+    s = qh @ kh.transpose(2, 3) / d ** 0.5
+    s.masked_fill_(torch.ones((n, n), dtype=torch.bool, device=q.device).triu_(1), float("-inf"))
+    p = torch.softmax(s, -1)
+    return (p @ vh).transpose(1, 2), (p.sum(2) * w.double()[..., None]).sum(1)
+
+
+# The 128-token tiles: one token short, exact, one over; several tiles; heads in pairs (even groups) and query tiles in
+# pairs (odd groups, the second tile missing for an odd number of tiles); fewer and more units than SMs.
+@pytest.mark.parametrize("hq,hkv,d,n,B,layout", [
+    (4, 2, 128, 127, 1, "token"), (4, 2, 64, 128, 2, "head"), (8, 1, 128, 129, 1, "token"), (3, 1, 64, 256, 1, "token"),
+    (3, 3, 128, 257, 2, "head"), (6, 2, 64, 385, 1, "token"), (32, 8, 128, 700, 3, "head"), (32, 4, 64, 1024, 2, "token"),
+    (4, 2, 128, 300, 1, "rows"), (4, 2, 64, 300, 2, "expanded"), (4, 1, 64, 40, 1, "grow")])
+def test_prefill_tiles_pairs_and_strides(hq, hkv, d, n, B, layout):
+    """Against fp64.  Error bounds: P and the output are rounded to fp16 (2^-11 relative each, P's averaging out over the
+    keys), so 2e-3 of the result's magnitude leaves a factor of two; the mass is an fp32 sum of at most n * hq terms."""
+    from smartkv_b200.prefill import causal_prefill_attention
+    g = torch.Generator(device="cuda").manual_seed(n + hq)
+
+    def make(heads):
+        if layout == "head":
+            return torch.randn((B, heads, n, d), generator=g, device="cuda").half().transpose(1, 2)
+        return torch.randn((B, n, heads, d), generator=g, device="cuda").half()
+    q, k, v = make(hq), make(hkv), make(hkv)
+    if layout == "rows":          # every key token is the same row: stride 0, which no tensor map holds
+        k = k[:, :1].expand(B, n, hkv, d)
+    elif layout == "expanded":    # one head's and one sequence's data for all of them
+        k, v = k[:1, :, :1].expand(B, n, hkv, d), v[:1].expand(B, n, hkv, d)
+    elif layout == "grow":        # scores that outgrow the running maximum by far more than 2^8, tile after tile
+        n = 500
+        q = torch.randn((B, n, hq, d), generator=g, device="cuda").abs().half()
+        k = (torch.rand((B, n, hkv, d), generator=g, device="cuda") * torch.linspace(0, 8, n, device="cuda")[:, None, None]).half()
+        v = torch.randn((B, n, hkv, d), generator=g, device="cuda").half()
+    w = torch.rand((B, hq), generator=g, device="cuda") + 0.5
+    out, mass = causal_prefill_attention(q, k, v, w)
+    ref, ref_mass = _dense64(q, k, v, w)
+    err = (out.double() - ref).abs()
+    assert bool((err <= 2e-3 + 2e-3 * ref.abs()).all()), float(err.max())
+    assert torch.allclose(mass.double(), ref_mass, rtol=1e-3, atol=1e-5), float((mass.double() - ref_mass).abs().max())
+    alone, none = causal_prefill_attention(q, k, v, want_mass=False)
+    assert none is None and torch.equal(alone, out)
