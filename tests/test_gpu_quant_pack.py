@@ -155,3 +155,49 @@ def test_append_then_export_bit_exact(hkv, d):
                 want_v = orc.pack_rows(vq[sel], w).transpose(1, 0, 2)
                 assert np.array_equal(kr.cpu().numpy(), want_k)
                 assert np.array_equal(vr.cpu().numpy(), want_v)
+
+
+@pytest.mark.parametrize("hkv,d,n,dtype,offset", [
+    (1, 64, 37, "f16", 0), (3, 64, 41, "f32", 0), (3, 128, 43, "f16", 0), (1, 128, 5, "f32", 0), (8, 128, 9000, "f16", 0),
+    (3, 64, 23001, "f16", 0), (5, 128, 14000, "f32", 0), (4, 64, 50, "f16", 2), (2, 128, 50, "f32", 4)])
+def test_bulk_append_rows_of_every_kind(hkv, d, n, dtype, offset):
+    """Mixed widths in one call, odd head counts (two tokens meet in one warp at head_dim 64), both numbers of row groups
+    per warp and inputs off a 16-byte boundary, with rows of zeros, near-ties, tiny and infinite values: packed bytes
+    and scales against the oracle."""
+    from tests.gpu_util import make_store, oracle_quantized
+    rng = np.random.default_rng(hkv * n + d)
+    bits = rng.choice([2, 3, 4, 8], size=(1, n))
+    np_t = np.float16 if dtype == "f16" else np.float32
+    kv = []
+    for i in range(2):
+        x = rng.standard_normal((n, hkv, d)).astype(np_t)
+        x[0] = 0                                                   # scale 1
+        if n > 4:
+            lv = np.maximum(2.0 ** (bits[0, 1:4] - 1) - 1, 1)[:, None, None]
+            x[1:4] = ((rng.integers(-1, 1, size=(3, hkv, d)) + 0.5) / lv).astype(np_t)   # ties, exact and rounded
+            x[1:4, :, 7] = 1.0
+            x[4] = (x[4].astype(np.float32) * 1e-7).astype(np_t)   # subnormal halves
+            if i == 0:
+                x[2, :, 3] = np.inf
+        kv.append(x)
+
+    def device(x):
+        flat = torch.zeros(x.size + 8, dtype=torch.from_numpy(x).dtype, device="cuda")
+        flat[offset:offset + x.size] = torch.from_numpy(x).cuda().view(-1)
+        return flat[offset:offset + x.size].view(n, hkv, d)
+    store = make_store(1, 1, hkv, d, hkv, n)
+    dst = store.plan_bulk(torch.from_numpy(bits.astype(np.int64)).cuda())
+    store.append(0, device(kv[0]), device(kv[1]), *dst[:3])
+    torch.cuda.synchronize()
+    with np.errstate(all="ignore"):
+        kq, vq, ks, vs = oracle_quantized(kv[0].astype(np.float32), kv[1].astype(np.float32), bits[0])
+    for bi, w in enumerate((2, 3, 4, 8)):
+        sel = np.nonzero(bits[0] == w)[0]
+        sel = sel[sel != 2] if n > 4 else sel       # inf / inf has no code the two sides must agree on; its scale is checked
+        raw = np.nonzero(bits[0] == w)[0]
+        keep = np.isin(raw, sel)
+        kr, vr, ksc, vsc = (t.cpu().numpy() for t in store.bucket_rows(0, 0, bi))
+        assert np.array_equal(kr[:, keep], orc.pack_rows(kq[sel], w).transpose(1, 0, 2))
+        assert np.array_equal(vr[:, keep], orc.pack_rows(vq[sel], w).transpose(1, 0, 2))
+        assert np.array_equal(ksc.view(np.uint32), ks[raw].T.view(np.uint32))
+        assert np.array_equal(vsc.view(np.uint32), vs[raw].T.view(np.uint32))
