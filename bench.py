@@ -50,7 +50,7 @@ CONFIGS = {
 }
 CFG = CONFIGS[1]
 FALLBACK_HBM_GBS = 6650.0
-# staging of the graphed reallocation: 4 GiB lets one pair of row-move launches cover 14 of the 32 layers
+# staging of the graphed reallocation: enough for one row-move launch over all 32 layers
 REALLOC_STAGING_BYTES = 4 << 30
 
 
@@ -419,9 +419,9 @@ def run_ours(args):
     reallocate()
     torch.cuda.synchronize()
     store.check_errors()
-    realloc_chunks = -(-L // max(1, min(L, ((1 << 30) if args.no_graph else REALLOC_STAGING_BYTES) // max(1, int(store.lib.skv_requant_staging_bytes(
-        ctypes.byref(store.desc), store.appended_total if args.no_graph else store.num_seqs * store.slots, 1))))))
-    realloc_launches = 15 + (3 if B > 1 else 0) + 2 * realloc_chunks
+    realloc_chunk, _ = store.repack_chunk(store.appended_total if args.no_graph else store.num_seqs * store.slots,
+                                          (1 << 30) if args.no_graph else REALLOC_STAGING_BYTES)
+    realloc_launches = 6 + -(-L // realloc_chunk)      # allocator, move plan, four per-token launches; row moves
 
     # ---- per-step inputs (resident) -----------------------------------------------------------
     gen.manual_seed(rank + 99)

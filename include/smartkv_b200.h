@@ -385,7 +385,8 @@ int skv_repack_plan(const SkvStoreDesc* desc, const int32_t* counts, const uint8
  * A row whose destination bucket has another width is dequantised (code * scale, fp32) and
  * quantised again at the new width, from the stored codes as the reference does (cache.py:819-844);
  * other rows are copied.  Every moved row passes through `staging`
- * (skv_requant_staging_bytes(desc, upper bound of the moves of all sequences, layers per call));
+ * (skv_requant_staging_bytes(desc, upper bound of the moves of all sequences, layers per call): a place for
+ * every row, or one slot per concurrent worker for a sequence's moves, whichever is less);
  * if the staging buffer is too small for the moves found on the device nothing moves and
  * *err_flag = 6. */
 int64_t skv_requant_staging_bytes(const SkvStoreDesc* desc, int64_t max_moves, int num_layers);

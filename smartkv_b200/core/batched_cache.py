@@ -153,7 +153,7 @@ class BatchedSmartKVCache:
             # inside a captured decode step the launches become part of that graph; buffers sized for the capacity
             st.reallocate(self._cfg, max_moves=self.batch_size * st.slots, staging_budget=self._staging_budget)
         elif recency is None:
-            # allocator + repack are some seventy small launches; replayed as one CUDA graph after the first time
+            # allocator + repack are a handful of small launches; replayed as one CUDA graph after the first time
             st.reallocate_graphed(self._cfg, staging_budget=self._staging_budget)
         else:
             new_bits, _, _ = st.allocate_bits(self._cfg, recency=recency)

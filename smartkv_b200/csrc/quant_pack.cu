@@ -25,36 +25,10 @@ __global__ void quantize_pack_append_kernel(const AppendParams p) {
 // (token, KV head) go through the same instructions side by side, NPASS groups of them in flight per warp.
 //
 // What bounds it is issue slots: with a row per warp, 282 warp instructions a row, 16 x 8192 x 8 rows of head_dim 128
-// took 634 us for 0.72 GB; now 325 us.  Everything per element runs on two elements at once (fma.rn.f32x2; element i is
-// paired with i + 4): t = x / s rounded by the add of 1.5 * 2^23 inside the fused multiply-add, the distance to the tie
-// by a second one, and the codes are joined by a third, as a polynomial in 2^bits whose values stay below 2^17 and are
-// therefore exact.  A lane with a near-tie, a NaN or a scale outside the normal range redoes its values with the
-// division, as quantize_vals does.
-constexpr float kRoundMagic = 12582912.f;  // 1.5 * 2^23 = 0x4B400000
-
-__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 f32x2_parts(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
+// took 634 us for 0.72 GB; now 273 us (quantize8; 64 registers, so that 32 warps fit an SM: 303 us with 24).  One or two
+// groups in flight per warp instead of four: 285 us and more.
 template <int D, bool HALF, int NPASS>
-__global__ void __launch_bounds__(256) append_bulk_kernel(const AppendParams p) {
+__global__ void __launch_bounds__(256, 4) append_bulk_kernel(const AppendParams p) {
   constexpr int LPR = D / 8;               // lanes per row
   constexpr int PPP = 32 / (2 * LPR);      // (token, head) pairs per pass: 1 or 2
   const StoreGeom& g = p.g;
@@ -116,65 +90,16 @@ __global__ void __launch_bounds__(256) append_bulk_kernel(const AppendParams p) 
 #pragma unroll
       for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
     }
-#pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const bool valid = seq[u] >= 0 && seq[u] < g.num_seqs && bucket[u] >= 0 && bucket[u] < kNumBuckets && pos[u] >= 0 &&
                        pos[u] < g.cap[bucket[u] & 3];
-    const int bk = bucket[u] & 3, bits = bucket_bits(bk);
-    const int hi = (1 << (bits - 1)) - 1;
-    float scale = scale_of(amax, hi);
-    if (scale == 0.f) scale = 1.f;
-
-    bool exact = !(scale >= 1e-30f && scale <= 1e30f);
-    const float rc = rcp_approx(scale);
-    const uint64_t rc2 = f32x2(rc, rc), magic2 = f32x2(kRoundMagic, kRoundMagic), neg2 = f32x2(-1.f, -1.f);
-    uint64_t nq[4];  // the negated codes of elements i and i + 4, as floats
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint64_t x2 = f32x2(x[i], x[i + 4]);
-      nq[i] = f32x2_fma(f32x2_fma(x2, rc2, magic2), neg2, magic2);
-      const float2 d = f32x2_parts(f32x2_fma(x2, rc2, nq[i]));
-      exact |= !(fabsf(d.x) < 0.5f - 1.25e-4f) || !(fabsf(d.y) < 0.5f - 1.25e-4f);  // also true for a NaN
-    }
-    if (exact) {
-      const float flo = -(float)(1 << (bits - 1)), fhi = (float)hi;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        nq[i] = f32x2(-fminf(fmaxf(rintf(__fdiv_rn(x[i], scale)), flo), fhi),
-                      -fminf(fmaxf(rintf(__fdiv_rn(x[i + 4], scale)), flo), fhi));
-    }
+    const int bk = bucket[u] & 3;
+    uint32_t lo, up;
+    const float scale = quantize8<LPR>(x, amax, bk, lo, up);
     uint8_t* arena = arena_ptr(g, p.store, p.layer, valid ? seq[u] : 0);
     const long long row = (long long)head[u] * g.cap[bk] + pos[u];
-    uint32_t* out = reinterpret_cast<uint32_t*>(arena + (which ? g.v_off[bk] : g.k_off[bk]) + row * g.row_bytes[bk]);
-    // 2 to 4 bits: four codes each as a polynomial in 2^bits, made non-negative by the offset of every code, then joined
-    const float base = (float)(1 << bits);
-    const uint64_t base2 = f32x2(base, base);
-    const float2 poly = f32x2_parts(f32x2_add(
-        f32x2_fma(f32x2_fma(f32x2_fma(nq[3], base2, nq[2]), base2, nq[1]), base2, nq[0]), magic2));
-    const uint32_t ones = 1u + (1u << bits) + (1u << (2 * bits)) + (1u << (3 * bits));
-    const uint32_t off = (1u << (bits - 1)) * ones + 0x4B400000u;
-    const uint32_t f = (off - __float_as_uint(poly.x)) + ((off - __float_as_uint(poly.y)) << ((4 * bits) & 31));
-    const uint32_t next = __shfl_down_sync(0xffffffffu, f, 1);
+    const uint32_t next = __shfl_down_sync(0xffffffffu, lo, 1);
     if (valid) {
-      if (bits == 8) {  // two's complement bytes: the low byte of 1.5 * 2^23 + code
-        uint32_t lo[4], up[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 m = f32x2_parts(f32x2_fma(nq[i], neg2, magic2));
-          lo[i] = __float_as_uint(m.x);
-          up[i] = __float_as_uint(m.y);
-        }
-        reinterpret_cast<uint2*>(out)[l] = make_uint2(prmt(prmt(lo[0], lo[1], 0x0040), prmt(lo[2], lo[3], 0x0040), 0x5410),
-                                                      prmt(prmt(up[0], up[1], 0x0040), prmt(up[2], up[3], 0x0040), 0x5410));
-      } else if (bits == 4) {
-        out[l] = f;
-      } else if (bits == 2) {
-        reinterpret_cast<uint16_t*>(out)[l] = (uint16_t)f;
-      } else {  // 3 bits: four lanes' 24-bit fields make three words
-        const int q = l & 3;
-        const uint32_t word = q == 0 ? (f | (next << 24)) : q == 1 ? ((f >> 8) | (next << 16)) : ((f >> 16) | (next << 8));
-        if (q < 3) out[3 * (l >> 2) + q] = word;
-      }
+      store_field8(arena + (which ? g.v_off[bk] : g.k_off[bk]) + row * g.row_bytes[bk], bk, l, lo, up, next);
       if (l == 0) {
         reinterpret_cast<float*>(arena + g.sc_off[bk])[2 * row + which] = scale;
         if (which) note_v_scale(g, arena, scale);

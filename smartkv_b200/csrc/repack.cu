@@ -15,17 +15,23 @@
 //   skv_repack_plan     one block per sequence: the list of moves (source -> destination
 //                       storage index), the same for every layer
 //   skv_requant_repack  per layer range: all moved rows -> staging (requantised where the
-//                       width changed), then staging -> destination.  Two kernels, so every
-//                       read of the old layout precedes every write of the new one.
+//                       width changed), then staging -> destination, so that every read of the
+//                       old layout precedes every write of the new one.  Rows of different
+//                       (layer, sequence, KV head) never touch, so one cluster of CTAs takes one
+//                       of those at a time and its own barrier is the only order needed.
 //   skv_repack_meta     the per-token arrays kept in storage order follow the same moves.
+#include <cooperative_groups.h>
+
 #include <cub/block/block_scan.cuh>
 
 #include "quant_row.cuh"
 
 namespace skv {
 
+namespace cg = cooperative_groups;
+
 constexpr int kPlanThreads = 1024;
-constexpr int kStageRowBytes = 136;  // 128 packed bytes at most, the fp32 scale at offset 128, padding
+constexpr int kStageRowBytes = 136;  // 8 bytes for each of up to 16 lanes, the fp32 scale, padding
 constexpr int kMaxSeqsRepack = 1024;
 
 __device__ __forceinline__ int bucket_of_slot(const StoreGeom& g, int s) {
@@ -175,17 +181,21 @@ struct RowMoveParams {
   int32_t* err;
 };
 
-// prefix of the per-sequence move counts into shared memory; returns the total
+// prefix of the per-sequence move counts into shared memory (at least one warp per block); returns the total
 __device__ __forceinline__ int load_move_prefix(const int32_t* n_moves, int B, int* s_prefix) {
-  // all counts are fetched at once (one round trip to memory), then one thread adds them up
-  for (int b = threadIdx.x; b < B; b += blockDim.x) s_prefix[b + 1] = n_moves[b];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    s_prefix[0] = 0;
-    for (int b = 0; b < B; ++b) {
-      acc += s_prefix[b + 1];
-      s_prefix[b + 1] = acc;
+  if (threadIdx.x < 32) {
+    int carry = 0;
+    if (threadIdx.x == 0) s_prefix[0] = 0;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+      const int b = b0 + (int)threadIdx.x;
+      int v = b < B ? n_moves[b] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, v, o);
+        if ((int)threadIdx.x >= o) v += up;
+      }
+      if (b < B) s_prefix[b + 1] = carry + v;
+      carry += __shfl_sync(0xffffffffu, v, 31);
     }
   }
   __syncthreads();
@@ -200,269 +210,186 @@ __device__ __forceinline__ int find_seq(const int* s_prefix, int B, int m) {
   return lo;
 }
 
-// ---- head_dim 128: half a warp per row, 8 consecutive elements per lane --------------------------------
-// The K row and the V row of one (token, head) are handled by the two halves of a warp at once, which
-// halves the per-row cost of everything that is not per element (reductions, address arithmetic, packing).
+// Clusters that work at once at most, two CTAs of 512 threads per SM of a B200; the staging buffer is divided among them.
+constexpr int kRowThreads = 512;
+constexpr int kRowSlots = 296;
+constexpr int kRowBatch = 4;  // row groups whose loads a warp has in flight
 
-// this lane's 8 values code * scale (elements 8*l16 .. 8*l16+7) of a packed 128-element row, from the two
-// aligned words (w0 at word bitpos/32, w1 the next one or 0 past the row's end) that hold the lane's field.
-// The code goes into the significand of 2^23 and the offset comes off in the same subtraction, so no
-// int->float conversion is needed; 8-bit rows hold two's complement, which flipping the top bit turns
-// into the offset form of the other widths.
-__device__ __forceinline__ void dequant8(uint32_t w0, uint32_t w1, int l16, int bits, float scale, float (&x)[8]) {
-  const int sh = (l16 * 8 * bits) & 31;
-  // a lane's field is 8 * bits wide: 64 bits = two aligned words at 8 bits (sh == 0), else at most 32 bits
-  const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = w1;
-  const uint32_t fm = (1u << bits) - 1u, flip = bits == 8 ? 0x80u : 0u;
-  const float bias = bits == 8 ? 8388736.f : bits == 4 ? 8388616.f : bits == 3 ? 8388612.f : 8388610.f;  // 2^23 + 2^(bits-1)
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int at = bits * i;
-    const uint32_t u = (((at >= 32 ? hi : lo) >> (at & 31)) ^ flip) & fm;
-    x[i] = __fmul_rn(__fsub_rn(__uint_as_float(u | 0x4B000000u), bias), scale);  // codes.float() * scale
-  }
-}
-
-// packs this lane's 8 codes and stores the half-warp's 128-element row at dst (4-byte aligned)
-__device__ __forceinline__ void pack8_store(const int (&code)[8], int bits, uint8_t* dst, int l16) {
-  uint32_t* out = reinterpret_cast<uint32_t*>(dst);
-  if (bits == 8) {
-    uint32_t lo = 0, hi = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      lo |= ((uint32_t)code[i] & 0xffu) << (8 * i);
-      hi |= ((uint32_t)code[4 + i] & 0xffu) << (8 * i);
-    }
-    out[2 * l16] = lo;
-    out[2 * l16 + 1] = hi;
-    return;
-  }
-  const int off = 1 << (bits - 1);
-  const uint32_t fm = (1u << bits) - 1u;
-  uint32_t f = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) f |= (((uint32_t)(code[i] + off)) & fm) << (bits * i);  // 16, 24 or 32 bits
-  const uint32_t n = __shfl_down_sync(0xffffffffu, f, 1);  // the next lane's field (same half for the lanes that use it)
-  if (bits == 4) {
-    out[l16] = f;
-  } else if (bits == 2) {
-    if ((l16 & 1) == 0) out[l16 >> 1] = f | (n << 16);
-  } else {  // 3 bits: four 24-bit fields make three words
-    const int r = l16 & 3;
-    const uint32_t word = r == 0 ? (f | (n << 24)) : r == 1 ? ((f >> 8) | (n << 16)) : ((f >> 16) | (n << 8));
-    if (r < 3) out[3 * (l16 >> 2) + r] = word;
-  }
-}
-
-// quantises the half-warp's row x again at `bits`; returns the new scale (all 16 lanes of the row)
-__device__ __forceinline__ float requant8(const float (&x)[8], int bits, int (&q)[8]) {
-  float amax = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));  // stays inside the half
-  const int hi = (1 << (bits - 1)) - 1, lo = -(1 << (bits - 1));
-  float ns = scale_of(amax, hi);
-  if (ns == 0.f) ns = 1.f;
-  quantize_vals<8>(x, ns, lo, hi, q);
-  return ns;
-}
-
-// head_dim 64: the same with 4 consecutive elements per lane
-__device__ __forceinline__ float requant4(const int (&code)[4], float scale, int bits, int (&q)[4]) {
-  float x[4];
-  float amax = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    x[i] = __fmul_rn((float)code[i], scale);
-    amax = fmaxf(amax, fabsf(x[i]));
-  }
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  const int hi = (1 << (bits - 1)) - 1, lo = -(1 << (bits - 1));
-  float ns = scale_of(amax, hi);
-  if (ns == 0.f) ns = 1.f;
-  quantize_vals<4>(x, ns, lo, hi, q);
-  return ns;
-}
-
-// packs the half-warp's 64-element row (4 codes per lane) and stores its 2 * bits words at dst
-__device__ __forceinline__ void pack4_store(const int (&code)[4], int bits, uint8_t* dst, int l16) {
-  const int wb = 4 * bits;  // bits this lane contributes: 8, 12, 16 or 32
-  uint32_t mine = 0;
-  if (bits == 8) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) mine |= ((uint32_t)code[i] & 0xffu) << (8 * i);
-  } else {
-    const int off = 1 << (bits - 1);
-    const uint32_t fm = (1u << bits) - 1u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) mine |= (((uint32_t)(code[i] + off)) & fm) << (bits * i);
-  }
-  // lane l16 assembles word l16 of the row from the (at most four) lanes whose fields overlap it
-  const int base_lane = (threadIdx.x & 16), first = (32 * l16) / wb;
-  uint32_t word = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int sl = first + i;
-    const uint32_t f = __shfl_sync(0xffffffffu, mine, base_lane + (sl & 15));
-    const int pos = sl * wb - 32 * l16;
-    if (sl < 16 && pos < 32 && pos + wb > 0) word |= pos >= 0 ? (f << pos) : (f >> (-pos));
-  }
-  if (l16 < 2 * bits) reinterpret_cast<uint32_t*>(dst)[l16] = word;
-}
-
-// phase 0: source rows -> staging (requantised at the destination width); phase 1: staging -> destination.
-// Staging holds one row per (layer, KV head, K|V, move), moves innermost.
+// One item = the moves of one (layer, KV head, sequence).  Phase 0 reads the source rows, requantises where the width changes
+// and leaves every lane's packed field and the scale in staging; after the cluster's barrier phase 1 writes the
+// destinations.  Staging is written and read back by the same few CTAs, so it lives in L2.
 //
-// A row is a separate memory transaction of 32..128 bytes.  Two things keep the memory system busy with
-// such small pieces: a warp takes kRowBatch consecutive moves of one (layer, KV head) and issues all their
-// loads before it does anything with them; and because consecutive moves mostly have consecutive source
-// and destination positions (the planner lists them in ascending order), the warps of a block touch
-// neighbouring rows, scales and staging rows at about the same time, so that the 4- and 8-byte scale
-// accesses and the short rows of neighbouring tokens share sectors and DRAM pages.
-// Half a warp per row: the K row in lanes 0..15, the V row of the same (token, head) in lanes 16..31.
-constexpr int kRowBatch = 4;
+// What bounds it: the rows are scattered pieces of 32 to 128 bytes, so the memory system needs many of them in flight
+// (a warp issues the loads of kRowBatch groups of rows first), and the quantiser's instructions.  As two grid-wide kernels per
+// layer range, each with one row per half-warp and a staging buffer in HBM, 16 sequences of 8192 tokens, 32 layers, 8 heads
+// took 2330 us for 13,000 moves (2.9 GB of DRAM traffic: a row is two or three 32-byte sectors and its scale one); now 1360 us.
+// A row's place inside its (arena, KV head): bucket and position in one word, so that a warp passes it round in one shuffle.
+// Positions stay below 2^30 (a store has fewer than 2^31 / 3 storage indices), so all ones is no place.
+constexpr uint32_t kNoPlace = 0xffffffffu;
+__device__ __forceinline__ uint32_t row_place(const StoreGeom& g, int slot) {
+  const int b = bucket_of_slot(g, slot);
+  return ((uint32_t)b << 30) | (uint32_t)(slot - g.bucket_base[b]);
+}
 
-struct MoveInfo {
-  int src, dst, seq;
-};
-
-template <int EPL, int PHASE>
-__global__ void __launch_bounds__(256) repack_rows_kernel(const RowMoveParams p) {
+template <int D, int CS>
+__global__ void __launch_bounds__(kRowThreads, 2) repack_rows_kernel(const __grid_constant__ RowMoveParams p) {
+  constexpr int LPR = D / 8;              // lanes per row
+  constexpr int PPP = 32 / (2 * LPR);     // moves side by side in a warp: the K and the V row of each
+  constexpr int MB = kRowBatch * PPP;     // moves whose rows a warp has in flight
+  constexpr int MC = 8;                   // moves a warp looks up at a time: lanes 0-7 the sources, 8-15 the destinations
   const StoreGeom& g = p.g;
   __shared__ int s_prefix[kMaxSeqsRepack + 1];
-  const int total_moves = load_move_prefix(p.n_moves, g.num_seqs, s_prefix);
-  const int Hkv = g.num_kv_heads, nl = p.layer_end - p.layer_begin;
-  if ((long long)total_moves * nl * Hkv * 2 > p.staging_rows) {
+  __shared__ int s_max;
+  __shared__ uint8_t* s_base[3][kNumBuckets];  // of the item: K rows, V rows, scale pairs of every bucket
+  if (threadIdx.x == 0) s_max = 0;
+  const int B = g.num_seqs, total = load_move_prefix(p.n_moves, B, s_prefix);
+  for (int b = threadIdx.x; b < B; b += kRowThreads) atomicMax(&s_max, s_prefix[b + 1] - s_prefix[b]);
+  __syncthreads();
+  const int longest = s_max, Hkv = g.num_kv_heads, nl = p.layer_end - p.layer_begin;
+  if (longest == 0) return;
+  // staging: a slot of `longest` moves per cluster, or, if the buffer was sized for few moves, a place for every row
+  const bool slots = (long long)longest * 2 * kRowSlots <= p.staging_rows;
+  if (!slots && (long long)total * nl * Hkv * 2 > p.staging_rows) {
     if (threadIdx.x == 0 && blockIdx.x == 0 && p.err) atomicExch(p.err, 6);  // staging too small: nothing moves
     return;
   }
-  const int lane = threadIdx.x & 31;
-  const int which = lane >> 4, l16 = lane & 15;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  const int groups = (total_moves + kRowBatch - 1) / kRowBatch;
-  const long long items = (long long)groups * nl * Hkv;
-  for (long long it = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += nwarps) {
-    int lh, grp;
-    if (items >> 31) {  // 64-bit division is a long subroutine: only where the item count needs it
-      lh = (int)(it / groups);
-      grp = (int)(it - (long long)lh * groups);
-    } else {
-      lh = (int)it / groups;
-      grp = (int)it - lh * groups;
+  const int lane = threadIdx.x & 31, l = lane & (LPR - 1), which = (lane / LPR) & 1, sub = lane / (2 * LPR);
+  const int rank = CS == 1 ? 0 : (int)(blockIdx.x % CS), cluster = (int)blockIdx.x / CS, clusters = (int)gridDim.x / CS;
+  const int cw = rank * (kRowThreads / 32) + (threadIdx.x >> 5), cwarps = CS * (kRowThreads / 32);
+  const long long items = (long long)nl * Hkv * B;
+  auto sync = [&] {
+    if constexpr (CS == 1) __syncthreads();
+    else cg::this_cluster().sync();
+  };
+  for (long long it = cluster; it < items; it += clusters) {
+    const int seq = (int)(it % B), lh = (int)(it / B), li = lh / Hkv, h = lh - li * Hkv;
+    const int moves = s_prefix[seq + 1] - s_prefix[seq];
+    if (moves == 0) continue;  // the same for the whole cluster
+    uint8_t* arena = arena_ptr(g, p.store, p.layer_begin + li, seq);
+    const int32_t* msrc = p.move_src + (long long)seq * g.slots;
+    const int32_t* mdst = p.move_dst + (long long)seq * g.slots;
+    uint8_t* stage = p.staging + (slots ? (long long)cluster * longest * 2 : ((long long)lh * total + s_prefix[seq]) * 2) * kStageRowBytes +
+                     which * kStageRowBytes;
+    if (threadIdx.x < 3 * kNumBuckets) {
+      const int what = threadIdx.x / kNumBuckets, b = threadIdx.x % kNumBuckets;
+      const long long first = (long long)h * g.cap[b];
+      s_base[what][b] = arena + (what == 0   ? g.k_off[b] + first * g.row_bytes[b]
+                                 : what == 1 ? g.v_off[b] + first * g.row_bytes[b]
+                                             : g.sc_off[b] + first * 8);
     }
-    const int li = lh / Hkv, h = lh - li * Hkv;
-    const int m0 = grp * kRowBatch;
-    // lanes 0..kRowBatch-1 look one move up each
-    MoveInfo mine{-1, -1, 0};
-    if (lane < kRowBatch && m0 + lane < total_moves) {
-      mine.seq = find_seq(s_prefix, g.num_seqs, m0 + lane);
-      const long long at = (long long)mine.seq * g.slots + (m0 + lane - s_prefix[mine.seq]);
-      mine.src = p.move_src[at];
-      mine.dst = p.move_dst[at];
-    }
-    // rows of (layer li, head h, K|V): staging row index = ((lh * 2 + which) * total_moves + move)
-    uint8_t* stage = p.staging + (((long long)lh * 2 + which) * total_moves + m0) * kStageRowBytes;
-    uint32_t w0[kRowBatch], w1[kRowBatch];
-    float sc[kRowBatch];
-    if (PHASE == 0) {
+    __syncthreads();
+    auto look_up = [&](int c0) -> uint32_t {
+      const int m = c0 + (lane & (MC - 1));
+      return lane < 2 * MC && m < moves ? row_place(g, (lane < MC ? msrc : mdst)[m]) : kNoPlace;
+    };
+    auto row_ptr = [&](uint32_t place) -> uint8_t* {
+      const int b = (int)(place >> 30);
+      return s_base[which][b] + (long long)(place & 0x3fffffffu) * (D / 8 * kWidthConst[b].bits);
+    };
+    auto scale_ptr = [&](uint32_t place) -> float* {
+      return reinterpret_cast<float*>(s_base[2][place >> 30]) + 2ll * (place & 0x3fffffffu) + which;
+    };
+
+    for (int c0 = cw * MC; c0 < moves; c0 += cwarps * MC) {
+      const uint32_t mine = look_up(c0);
+#pragma unroll 1
+      for (int m0 = 0; m0 < MC && c0 + m0 < moves; m0 += MB) {
+        uint32_t w0[kRowBatch], w1[kRowBatch];
+        float sc[kRowBatch];
+        int bs[kRowBatch];
 #pragma unroll
-      for (int u = 0; u < kRowBatch; ++u) {
-        const int src = __shfl_sync(0xffffffffu, mine.src, u), seq = __shfl_sync(0xffffffffu, mine.seq, u);
-        const int dst = __shfl_sync(0xffffffffu, mine.dst, u);
-        w0[u] = w1[u] = 0u;
-        sc[u] = 0.f;
-        if (src < 0) continue;
-        const int wb_s = bucket_of_slot(g, src), bits_s = bucket_bits(wb_s), rb_s = g.row_bytes[wb_s];
-        const uint8_t* arena = arena_ptr(g, p.store, p.layer_begin + li, seq);
-        const long long row = (long long)h * g.cap[wb_s] + (src - g.bucket_base[wb_s]);
-        const uint32_t* rp =
-            reinterpret_cast<const uint32_t*>(arena + (which ? g.v_off[wb_s] : g.k_off[wb_s]) + row * rb_s);
-        const float2 t = reinterpret_cast<const float2*>(arena + g.sc_off[wb_s])[row];
-        sc[u] = which ? t.y : t.x;
-        if (bucket_of_slot(g, dst) == wb_s || EPL != 4) {
-          // the row only changes place (up to 32 words, two per lane), or head_dim 64: whole-row words
-          const int words = rb_s >> 2;
-          if (l16 < words) w0[u] = rp[l16];
-          if (l16 + 16 < words) w1[u] = rp[l16 + 16];
-        } else {
-          // head_dim 128: 8 consecutive elements per lane lie in at most two aligned words
-          const int wi = (l16 * 8 * bits_s) >> 5;
+        for (int u = 0; u < kRowBatch; ++u) {
+          const uint32_t at = __shfl_sync(0xffffffffu, mine, m0 + u * PPP + sub);
+          bs[u] = at == kNoPlace ? 0 : (int)(at >> 30);
+          w0[u] = w1[u] = 0u;
+          sc[u] = 0.f;
+          if (at == kNoPlace) continue;
+          const int bits = kWidthConst[bs[u]].bits;
+          const int wi = (l * bits) >> 2;  // a lane's 8 * bits bits lie in at most two aligned words
+          const uint32_t* rp = reinterpret_cast<const uint32_t*>(row_ptr(at));
           w0[u] = rp[wi];
-          if (wi + 1 < 4 * bits_s) w1[u] = rp[wi + 1];
+          if (wi + 1 < D / 32 * bits) w1[u] = rp[wi + 1];
+          sc[u] = *scale_ptr(at);
         }
-      }
 #pragma unroll
-      for (int u = 0; u < kRowBatch; ++u) {
-        const int src = __shfl_sync(0xffffffffu, mine.src, u), dst = __shfl_sync(0xffffffffu, mine.dst, u);
-        if (src < 0) continue;  // the same for the whole warp: the shuffles below see every lane
-        const int wb_s = bucket_of_slot(g, src), wb_d = bucket_of_slot(g, dst);
-        const int bits_s = bucket_bits(wb_s), bits_d = bucket_bits(wb_d);
-        uint8_t* st = stage + u * kStageRowBytes;
-        if (wb_s == wb_d) {
-          const int words = g.row_bytes[wb_s] >> 2;
-          if (l16 < words) reinterpret_cast<uint32_t*>(st)[l16] = w0[u];
-          if (l16 + 16 < words) reinterpret_cast<uint32_t*>(st)[l16 + 16] = w1[u];
-          if (l16 == 0) *reinterpret_cast<float*>(st + 128) = sc[u];
-        } else if constexpr (EPL == 4) {
-          float x[8];
-          int q[8];
-          dequant8(w0[u], w1[u], l16, bits_s, sc[u], x);
-          const float ns = requant8(x, bits_d, q);
-          pack8_store(q, bits_d, st, l16);
-          if (l16 == 0) *reinterpret_cast<float*>(st + 128) = ns;
-        } else {
-          // head_dim 64: 4 consecutive elements per lane, out of the row's words held by the half-warp
-          const int bitpos = l16 * 4 * bits_s, wi = bitpos >> 5, sh = bitpos & 31;
-          const int base_lane = lane & 16;
-          const uint32_t lo = __shfl_sync(0xffffffffu, w0[u], base_lane + (wi & 15));
-          const uint32_t hi = __shfl_sync(0xffffffffu, w0[u], base_lane + ((wi + 1) & 15));
-          const uint32_t field = __funnelshift_r(lo, hi, sh);
-          int code[4], q[4];
-          if (bits_s == 8) {
+        for (int u = 0; u < kRowBatch; ++u) {
+          const uint32_t to = __shfl_sync(0xffffffffu, mine, MC + m0 + u * PPP + sub);
+          if (__all_sync(0xffffffffu, to == kNoPlace)) break;
+          const int b_from = bs[u], b_to = to == kNoPlace ? 0 : (int)(to >> 30);
+          uint32_t lo = __funnelshift_r(w0[u], w1[u], (l * 8 * kWidthConst[b_from].bits) & 31), hi = w1[u];
+          float scale = sc[u];
+          if (__any_sync(0xffffffffu, b_from != b_to)) {
+            float x[8], amax = 0.f;
+            dequantize8(lo, hi, b_from, scale, x);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) code[i] = (int)(int8_t)((field >> (8 * i)) & 0xffu);
-          } else {
-            const uint32_t fm = (1u << bits_s) - 1u;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) code[i] = (int)((field >> (bits_s * i)) & fm) - (1 << (bits_s - 1));
+            for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
+            uint32_t nlo, nhi;
+            const float ns = quantize8<LPR>(x, amax, b_to, nlo, nhi);
+            if (b_from != b_to) {
+              lo = nlo;
+              hi = nhi;
+              scale = ns;
+            }
           }
-          const float ns = requant4(code, sc[u], bits_d, q);
-          pack4_store(q, bits_d, st, l16);
-          if (l16 == 0) *reinterpret_cast<float*>(st + 128) = ns;
-        }
-      }
-    } else {
-#pragma unroll
-      for (int u = 0; u < kRowBatch; ++u) {
-        const int dst = __shfl_sync(0xffffffffu, mine.dst, u);
-        w0[u] = w1[u] = 0u;
-        sc[u] = 0.f;
-        if (dst < 0) continue;
-        const int words = g.row_bytes[bucket_of_slot(g, dst)] >> 2;
-        const uint32_t* st = reinterpret_cast<const uint32_t*>(stage + u * kStageRowBytes);
-        if (l16 < words) w0[u] = st[l16];
-        if (l16 + 16 < words) w1[u] = st[l16 + 16];
-        if (l16 == 0) sc[u] = reinterpret_cast<const float*>(st)[32];
-      }
-#pragma unroll
-      for (int u = 0; u < kRowBatch; ++u) {
-        const int dst = __shfl_sync(0xffffffffu, mine.dst, u), seq = __shfl_sync(0xffffffffu, mine.seq, u);
-        if (dst < 0) continue;
-        const int wb_d = bucket_of_slot(g, dst), rb_d = g.row_bytes[wb_d], words = rb_d >> 2;
-        uint8_t* arena = arena_ptr(g, p.store, p.layer_begin + li, seq);
-        const long long row = (long long)h * g.cap[wb_d] + (dst - g.bucket_base[wb_d]);
-        uint32_t* rp = reinterpret_cast<uint32_t*>(arena + (which ? g.v_off[wb_d] : g.k_off[wb_d]) + row * rb_d);
-        if (l16 < words) rp[l16] = w0[u];
-        if (l16 + 16 < words) rp[l16 + 16] = w1[u];
-        if (l16 == 0) {
-          reinterpret_cast<float*>(arena + g.sc_off[wb_d])[2 * row + which] = sc[u];
-          if (which) note_v_scale(g, arena, sc[u]);
+          if (to != kNoPlace) {
+            uint8_t* st = stage + (long long)(c0 + m0 + u * PPP + sub) * 2 * kStageRowBytes;
+            reinterpret_cast<uint2*>(st)[l] = make_uint2(lo, hi);
+            if (l == 0) *reinterpret_cast<float*>(st + 8 * LPR) = scale;
+          }
         }
       }
     }
+    sync();
+    for (int c0 = cw * MC; c0 < moves; c0 += cwarps * MC) {
+      const uint32_t mine = look_up(c0);
+#pragma unroll 1
+      for (int m0 = 0; m0 < MC && c0 + m0 < moves; m0 += MB) {
+        uint2 f[kRowBatch];
+        float sc[kRowBatch];
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) {
+          f[u] = make_uint2(0u, 0u);
+          sc[u] = 0.f;
+          if (c0 + m0 + u * PPP + sub < moves) {
+            const uint8_t* st = stage + (long long)(c0 + m0 + u * PPP + sub) * 2 * kStageRowBytes;
+            f[u] = reinterpret_cast<const uint2*>(st)[l];
+            if (l == 0) sc[u] = *reinterpret_cast<const float*>(st + 8 * LPR);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) {
+          const uint32_t at = __shfl_sync(0xffffffffu, mine, MC + m0 + u * PPP + sub);
+          const int b = (int)(at >> 30);
+          // the fields of a 3-bit row moved unchanged carry their neighbours' bits above the lane's 24
+          const uint32_t lo = b == 1 ? f[u].x & 0x00ffffffu : f[u].x;
+          const uint32_t next = __shfl_down_sync(0xffffffffu, lo, 1);
+          if (at == kNoPlace) continue;
+          store_field8(row_ptr(at), b, l, lo, f[u].y, next);
+          if (l == 0) {
+            *scale_ptr(at) = sc[u];
+            if (which) note_v_scale(g, arena, sc[u]);
+          }
+        }
+      }
+    }
+    sync();  // the slot is free for the next item
   }
+}
+
+template <int D, int CS>
+static cudaError_t launch_rows(const RowMoveParams& p, long long items, cudaStream_t st) {
+  const long long clusters = items < kRowSlots / CS ? items : kRowSlots / CS;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * CS));
+  cfg.blockDim = dim3(kRowThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, repack_rows_kernel<D, CS>, p);
 }
 
 // ---- per-token arrays -----------------------------------------------------------------------------------
@@ -503,29 +430,34 @@ __global__ void repack_meta_kernel(const MetaParams p) {
   float* st_ema = reinterpret_cast<float*>(st_tok + p.staging_moves);             // [L][moves]
   uint8_t* st_tch = reinterpret_cast<uint8_t*>(st_ema + (long long)L * p.staging_moves);  // [L][moves]
   int8_t* st_str = reinterpret_cast<int8_t*>(st_tch + (long long)L * p.staging_moves);
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
-  for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < total; m += nthreads) {
-    const int b = find_seq(s_prefix, B, (int)m);
-    const int k = (int)m - s_prefix[b];
+  // one (move, layer) per thread, moves innermost; "layer" L stands for the arrays that have none
+  const long long nthreads = (long long)gridDim.x * blockDim.x, pairs = (long long)total * (L + 1);
+  for (long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x; it < pairs; it += nthreads) {
+    const int l = (int)(it / total), m = (int)(it - (long long)l * total);
+    const int b = find_seq(s_prefix, B, m);
+    const int k = m - s_prefix[b];
     const long long si = (long long)b * T + p.move_src[(long long)b * T + k];
     const long long di = (long long)b * T + p.move_dst[(long long)b * T + k];
+    const long long sl = (long long)l * p.staging_moves + m, la = (long long)l * B * T;
     if (PHASE == 0) {
-      st_cum[m] = p.cumulative[si];
-      st_pct[m] = p.rank_pct[si];
-      st_tok[m] = p.slot_token[si];
-      st_str[m] = p.rank_streak[si];
-      for (int l = 0; l < L; ++l) {
-        st_ema[(long long)l * p.staging_moves + m] = p.layer_ema[(long long)l * B * T + si];
-        st_tch[(long long)l * p.staging_moves + m] = p.touched[(long long)l * B * T + si];
+      if (l == L) {
+        st_cum[m] = p.cumulative[si];
+        st_pct[m] = p.rank_pct[si];
+        st_tok[m] = p.slot_token[si];
+        st_str[m] = p.rank_streak[si];
+      } else {
+        st_ema[sl] = p.layer_ema[la + si];
+        st_tch[sl] = p.touched[la + si];
       }
     } else {
-      p.cumulative[di] = st_cum[m];
-      p.rank_pct[di] = st_pct[m];
-      p.slot_token[di] = st_tok[m];
-      p.rank_streak[di] = st_str[m];
-      for (int l = 0; l < L; ++l) {
-        p.layer_ema[(long long)l * B * T + di] = st_ema[(long long)l * p.staging_moves + m];
-        p.touched[(long long)l * B * T + di] = st_tch[(long long)l * p.staging_moves + m];
+      if (l == L) {
+        p.cumulative[di] = st_cum[m];
+        p.rank_pct[di] = st_pct[m];
+        p.slot_token[di] = st_tok[m];
+        p.rank_streak[di] = st_str[m];
+      } else {
+        p.layer_ema[la + di] = st_ema[sl];
+        p.touched[la + di] = st_tch[sl];
       }
     }
   }
@@ -578,7 +510,10 @@ extern "C" int skv_repack_plan(const SkvStoreDesc* desc, const int32_t* counts, 
 
 extern "C" int64_t skv_requant_staging_bytes(const SkvStoreDesc* desc, int64_t max_moves, int num_layers) {
   if (!desc || max_moves < 0 || num_layers <= 0) return SKV_ERR_INVALID;
-  return max_moves * num_layers * desc->num_kv_heads * 2 * (int64_t)kStageRowBytes;
+  // a place for every row, or one slot per cluster for the moves of one sequence, whichever is less
+  const int64_t rows = max_moves * num_layers * desc->num_kv_heads * 2;
+  const int64_t slots = (max_moves < desc->slots ? max_moves : (int64_t)desc->slots) * 2 * kRowSlots;
+  return (rows < slots ? rows : slots) * (int64_t)kStageRowBytes;
 }
 
 extern "C" int skv_requant_repack(const SkvStoreDesc* desc, void* store, int layer_begin, int layer_end,
@@ -599,18 +534,17 @@ extern "C" int skv_requant_repack(const SkvStoreDesc* desc, void* store, int lay
   p.staging = static_cast<uint8_t*>(staging);
   p.staging_rows = staging_bytes / kStageRowBytes;
   p.err = err_flag;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = sms * 8, threads = 256;
+  if (desc->slots >= (1 << 30)) return SKV_ERR_UNSUPPORTED;  // row_place
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (desc->head_dim == 128) {
-    repack_rows_kernel<4, 0><<<grid, threads, 0, st>>>(p);
-    repack_rows_kernel<4, 1><<<grid, threads, 0, st>>>(p);
-  } else {
-    repack_rows_kernel<2, 0><<<grid, threads, 0, st>>>(p);
-    repack_rows_kernel<2, 1><<<grid, threads, 0, st>>>(p);
-  }
+  // Few items (a small store, one sequence): up to 8 CTAs, the portable cluster size, share each.
+  const long long items = (long long)(layer_end - layer_begin) * desc->num_kv_heads * desc->num_seqs;
+  const int cs = items * 2 > kRowSlots ? 1 : items * 4 > kRowSlots ? 2 : items * 8 > kRowSlots ? 4 : 8;
+  const bool d128 = desc->head_dim == 128;
+  const cudaError_t rc = cs == 1   ? (d128 ? launch_rows<128, 1>(p, items, st) : launch_rows<64, 1>(p, items, st))
+                         : cs == 2 ? (d128 ? launch_rows<128, 2>(p, items, st) : launch_rows<64, 2>(p, items, st))
+                         : cs == 4 ? (d128 ? launch_rows<128, 4>(p, items, st) : launch_rows<64, 4>(p, items, st))
+                                   : (d128 ? launch_rows<128, 8>(p, items, st) : launch_rows<64, 8>(p, items, st));
+  if (rc != cudaSuccess) return SKV_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }
 

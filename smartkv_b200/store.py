@@ -589,6 +589,16 @@ class PackedKVStore:
                                       self._stream()), "skv_alloc_bits")
         return r["new_bits"], r["new_counts"], r["changed"]
 
+    def repack_chunk(self, max_moves: int, staging_budget: int) -> Tuple[int, int]:
+        """(layers per row-move launch, staging bytes): all layers at once where the budget holds the staging for up
+        to ``max_moves`` moves, otherwise fewer at a time, at least one."""
+        chunk = self.num_layers
+        need = int(self.lib.skv_requant_staging_bytes(ctypes.byref(self.desc), max_moves, chunk))
+        while need > staging_budget and chunk > 1:
+            chunk = (chunk + 1) // 2
+            need = int(self.lib.skv_requant_staging_bytes(ctypes.byref(self.desc), max_moves, chunk))
+        return chunk, need
+
     def repack(self, new_bits: torch.Tensor, max_moves: Optional[int] = None, staging_budget: int = 1 << 30):
         """Moves every token to the bucket of its new width (requantising from the stored codes)
         in all layers and permutes the per-token arrays accordingly.  ``max_moves``: upper bound of
@@ -602,9 +612,7 @@ class PackedKVStore:
         if max_moves is None:
             max_moves = self.appended_total
         max_moves = max(int(max_moves), 1)
-        per_layer = int(self.lib.skv_requant_staging_bytes(d, max_moves, 1))
-        chunk = max(1, min(self.num_layers, staging_budget // max(per_layer, 1)))
-        need = per_layer * chunk
+        chunk, need = self.repack_chunk(max_moves, staging_budget)
         if r["staging"] is None or r["staging"].numel() < need:
             r["staging"] = torch.empty(need, dtype=torch.uint8, device=self.device)
         mneed = int(self.lib.skv_repack_meta_staging_bytes(d, max_moves + 8))
@@ -628,12 +636,11 @@ class PackedKVStore:
         self.repack(new_bits, max_moves=max_moves, staging_budget=staging_budget)
 
     def reallocate_graphed(self, cfg, staging_budget: int = 1 << 30):
-        """reallocate() as one CUDA graph launch: a reallocation is about 70 small launches, and issuing them
+        """reallocate() as one CUDA graph launch: a reallocation is a handful of small launches, and issuing them
         one by one costs more than running them once the allocation has settled.  The first call runs eagerly
         (it sizes every buffer for the store's whole capacity, so that the captured launches stay valid as the
         cache grows) and captures the graph; later calls replay it.  ``cfg`` must be the same at every call.
-        ``staging_budget`` bytes of staging decide how many layers one pair of row-move launches covers: every
-        pair costs tens of microseconds however few rows move, so a larger budget makes a quiet reallocation cheaper."""
+        ``staging_budget`` bytes of staging decide how many layers one row-move launch covers (repack_chunk)."""
         self.flush_importance()
         cap_moves = self.num_seqs * self.slots
         if getattr(self, "_realloc_graph", None) is None:
