@@ -148,8 +148,8 @@ def check(status, what=""):
 
 
 def ptr(t):
-    """Device (or host) address of a torch tensor / None."""
-    return None if t is None else c_void_p(t.data_ptr())
+    """Device (or host) address of a torch tensor / None (an int: what ctypes converts fastest to a pointer argument)."""
+    return None if t is None else t.data_ptr()
 
 
 def stream_ptr(device=None):

@@ -155,7 +155,7 @@ class PackedKVStore:
 
     # ------------------------------------------------------------------ helpers
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return torch.cuda.current_stream(self.device).cuda_stream
 
     @staticmethod
     def _dtype_code(t: torch.Tensor) -> int:
@@ -380,8 +380,9 @@ class PackedKVStore:
         dst_seq, dst_bucket, dst_pos, storage = step_plan if has_cur else (None, None, None, None)
         pend = pipe["pending"]
         pb = pipe["bufs"][pend["buf"]] if pend is not None else None
-        small = pipe["small"]                         # (max, sum, current-token probability) of every layer of the step
-        ps = {k2: v2[pend["layer"]] for k2, v2 in small.items()} if pend is not None else None
+        rows = pipe["rows"]                           # (max, sum, current-token probability) of every layer of the step
+        lse_max, lse_sum, cur_prob = rows[layer]
+        ps = rows[pend["layer"]] if pend is not None else (None, None, None)
         # Under stream capture the host scalars below would be baked into the graph: the importance blocks then
         # cover the store's token capacity (or every storage index, 0 = full grid, if nobody stated one) instead of
         # the capture-time token count, and the
@@ -397,11 +398,10 @@ class PackedKVStore:
                 ctypes.byref(self.desc), ptr(self.arena), layer, ptr(self.plan), ptr(q), self._dtype_code(q),
                 self.num_q_heads, ptr(partials), self.num_ctas, ptr(cur_k), ptr(cur_v),
                 self._dtype_code(cur_k) if has_cur else _lib.DTYPE_F32,
-                ptr(out), ptr(small["lse_max"][layer]), ptr(small["lse_sum"][layer]), ptr(small["cur_prob"][layer]),
+                ptr(out), ptr(lse_max), ptr(lse_sum), ptr(cur_prob),
                 ptr(self.counts),
                 pend["layer"] if pend is not None else 0, ptr(pb["logits"]) if pend is not None else None,
-                ptr(ps["lse_max"]) if pend is not None else None, ptr(ps["lse_sum"]) if pend is not None else None,
-                ptr(ps["cur_prob"]) if pend is not None else None,
+                ptr(ps[0]), ptr(ps[1]), ptr(ps[2]),
                 ptr(pend["storage"]) if pend is not None and pend["storage"] is not None else None,
                 ptr(self.head_state), self.head_parity, ptr(self.cumulative), ptr(self.layer_ema), ptr(self.touched),
                 self.decay, self.head_decay, ptr(dst_seq), ptr(dst_bucket), ptr(dst_pos), max_tokens_arg,
@@ -428,7 +428,7 @@ class PackedKVStore:
                 self._capture_updates = getattr(self, "_capture_updates", 0) + 1
         pipe["pending"] = {"layer": layer, "buf": lslot, "storage": storage} if want_logits else None
         pipe["calls"] = m + 1
-        self.lse_max, self.lse_sum, self.cur_prob = small["lse_max"][layer], small["lse_sum"][layer], small["cur_prob"][layer]
+        self.lse_max, self.lse_sum, self.cur_prob = lse_max, lse_sum, cur_prob
         return out
 
     def _pipe_buffers(self):
@@ -446,7 +446,9 @@ class PackedKVStore:
             # all layers' (max, sum, out) at once)
             small = {k: torch.empty((self.num_layers, B, Hq), dtype=torch.float32, device=dev)
                      for k in ("lse_max", "lse_sum", "cur_prob")}
-            self._pipe = {"bufs": bufs, "small": small, "partials": [self.partials, torch.empty_like(self.partials)],
+            # one view per layer, made once: an index expression costs more host time than the launch it feeds
+            rows = list(zip(*(small[k].unbind(0) for k in ("lse_max", "lse_sum", "cur_prob"))))
+            self._pipe = {"bufs": bufs, "small": small, "rows": rows, "partials": [self.partials, torch.empty_like(self.partials)],
                           "calls": 0, "pending": None, "side": torch.cuda.Stream(device=dev), "post_events": [],
                           "forked": False}
         return self._pipe
@@ -470,9 +472,7 @@ class PackedKVStore:
         self.join()
         pend = pipe["pending"]
         pipe["pending"] = None
-        sm = pipe["small"]
-        return (pipe["bufs"][pend["buf"]]["logits"], sm["lse_max"][pend["layer"]], sm["lse_sum"][pend["layer"]],
-                sm["cur_prob"][pend["layer"]])
+        return (pipe["bufs"][pend["buf"]]["logits"], *pipe["rows"][pend["layer"]])
 
     def flush_importance(self):
         """Runs the importance update still owed by the last decode_layer call (no-op otherwise)."""
@@ -484,12 +484,12 @@ class PackedKVStore:
         if pend is None:
             return
         pb = pipe["bufs"][pend["buf"]]
-        sm = {k: v[pend["layer"]] for k, v in pipe["small"].items()}
+        lse_max, lse_sum, cur_prob = pipe["rows"][pend["layer"]]
         if torch.cuda.is_current_stream_capturing():
             self._capture_updates = getattr(self, "_capture_updates", 0) + 1
         check(self.lib.skv_importance_update(ctypes.byref(self.desc), pend["layer"], ptr(self.counts), self.num_q_heads,
-                                             ptr(pb["logits"]), ptr(sm["lse_max"]), ptr(sm["lse_sum"]),
-                                             ptr(sm["cur_prob"]) if pend["storage"] is not None else None,
+                                             ptr(pb["logits"]), ptr(lse_max), ptr(lse_sum),
+                                             ptr(cur_prob) if pend["storage"] is not None else None,
                                              ptr(pend["storage"]) if pend["storage"] is not None else None, ptr(self.head_state),
                                              self.head_parity, ptr(self.cumulative), ptr(self.layer_ema),
                                              ptr(self.touched), self.decay, self.head_decay, self._stream()),
