@@ -321,6 +321,20 @@ int skv_importance_update(const SkvStoreDesc* desc, int layer, const int32_t* co
                           const int32_t* cur_slot, float* head_state, int parity, double* cumulative,
                           float* layer_ema, uint8_t* touched, float decay, float head_decay, void* stream);
 
+/* The importance update of one layer of a prompt pass (smartkv/core/cache.py:232-259, importance.py:44-101):
+ * key_mass fp32 [num_seqs][n], the head-weighted attention mass on the tokens with ids 0 .. n-1, is added to the
+ * cumulative importance of each (or, with `assign`, becomes it) and folded into the layer's EMA. */
+int skv_prompt_importance(const SkvStoreDesc* desc, int layer, const int32_t* counts, const int32_t* slot_token,
+                          const float* key_mass, int n, int assign, double decay, double* cumulative,
+                          float* layer_ema, uint8_t* touched, void* stream);
+
+/* Where the tokens with ids first .. first + n - 1 lie (first_token: device int64, NULL = 0): dst_seq / dst_bucket /
+ * dst_pos int32 [num_seqs][n] as skv_quantize_pack_append takes them, and the storage index.  A token that the store
+ * does not hold gets dst_seq and storage -1. */
+int skv_token_places(const SkvStoreDesc* desc, const int32_t* counts, const int32_t* slot_token,
+                     const int64_t* first_token, int n, int32_t* dst_seq, int32_t* dst_bucket, int32_t* dst_pos,
+                     int32_t* storage, void* stream);
+
 /* ---- reallocation: bit allocation ------------------------------------------- */
 
 #define SKV_ALLOC_MAX_PROTECTED 16

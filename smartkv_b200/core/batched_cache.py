@@ -129,13 +129,6 @@ class BatchedSmartKVCache:
         where[:, dump] = -1
         return where[:, : self.max_tokens]
 
-    def _plan_for(self, storage: torch.Tensor):
-        storage = storage.to(torch.int32)
-        flat = storage.reshape(-1).long()
-        n = storage.numel() // self.batch_size
-        seq = self.store._seq_ids[:, None].expand(self.batch_size, n).contiguous().view(-1)
-        return seq, self._slot_bucket[flat].contiguous(), self._slot_pos[flat].contiguous(), storage.contiguous()
-
     def _trigger(self, layer: int, new_tokens: int) -> bool:
         total = self.num_known + new_tokens
         adaptive = max(self.realloc_freq * (1 + layer // 4), max(32, total // 8))
@@ -199,28 +192,20 @@ class BatchedSmartKVCache:
             if n + 1 > self.max_tokens:
                 raise _lib.SmartKVLibraryError(f"{n} prompt tokens exceed the cache capacity of {self.max_tokens - 1}")
         if key_mass is not None:
-            mass = key_mass.double()
+            mass = key_mass
+            if tuple(mass.shape) != (B, n):
+                raise ValueError(f"key_mass must be [{B}, {n}]; got {list(mass.shape)}")
         else:
             w = self._weights(probs.float().mean(dim=(2, 3)))
-            mass = (probs.float() * w[:, :, None, None]).sum(dim=(1, 2)).double()      # [B, n] per key
-        ids = torch.arange(n, device=self._dev)
+            mass = (probs.float() * w[:, :, None, None]).sum(dim=(1, 2))      # [B, n] per key
+        places = None
         if layer == 0:
-            bits = torch.full((B, n), 4, dtype=torch.int32, device=self._dev)
-            storage = st.plan_bulk(bits)[3].long()
-            st.cumulative.scatter_(1, storage, mass)
+            places = st.plan_bulk(torch.full((B, n), 4, dtype=torch.int32, device=self._dev))[:3]
             self.num_known = n
-            first_known = 0
-        else:
-            storage = self._token_storage()[:, :n]
-            st.cumulative.scatter_add_(1, storage, mass)
-            first_known = n
-        old = st.layer_ema[layer].gather(1, storage)
-        seen = st.touched[layer].gather(1, storage).bool()
-        st.layer_ema[layer].scatter_(1, storage, torch.where(seen, self.decay * old + (1 - self.decay) * mass.float(),
-                                                             mass.float()))
-        st.touched[layer].scatter_(1, storage, torch.ones_like(storage, dtype=torch.uint8))
+        first_known = 0 if layer == 0 else n
+        st.prompt_importance(layer, mass, assign=layer == 0)
         self.global_step += 1
-        self.last_seen[ids] = float(self.global_step)
+        self.last_seen[:n] = float(self.global_step)
         # the reference counts len(precision_map) + len(token_ids); at layer 0 the map is still empty
         known = self.num_known
         self.num_known = first_known
@@ -228,10 +213,9 @@ class BatchedSmartKVCache:
         self.num_known = known
         if fire:
             self._reallocate()
-            storage = self._token_storage()[:, :n]
-        seq, bucket, pos, _ = self._plan_for(storage)
-        st.append(layer, k.reshape(B * n, self.num_heads, self.head_dim), v.reshape(B * n, self.num_heads, self.head_dim),
-                  seq, bucket, pos)
+        if fire or places is None:
+            places = st.token_places(n)[:3]
+        st.append(layer, k.reshape(B * n, self.num_heads, self.head_dim), v.reshape(B * n, self.num_heads, self.head_dim), *places)
         self.token_counter += n
         if layer == self.num_layers - 1:
             self.num_cached = n
@@ -277,9 +261,8 @@ class BatchedSmartKVCache:
                 step["early"] = True
                 self._mask.index_fill_(1, self._tok_dev, -1e30)   # ... but stays out of the cached keys of this step
             self._reallocate()
-            where = self._token_storage()
-            step["plan"] = self._plan_for(where.index_select(1, self._tok_dev)[:, 0])
-            step["token0"] = where[:, 0]
+            step["plan"] = st.token_places(1, self._tok_dev)
+            step["token0"] = None            # looked up again by whoever needs it
             # this layer's row at the width just decided, from the full-precision values (cache.py:1214)
             st.append(layer, k, v, *step["plan"][:3])
         self.num_known = self.num_cached + 1

@@ -202,6 +202,24 @@ class PackedKVStore:
         dst_seq = self._seq_ids[:, None].expand(B, n).contiguous().view(-1)
         return dst_seq, bucket.contiguous().view(-1), pos.contiguous().view(-1), storage
 
+    def token_places(self, n: int, first: Optional[torch.Tensor] = None):
+        """Where the tokens with ids first .. first + n - 1 of every sequence lie (``first``: int64 device scalar, default 0):
+        (dst_seq, dst_bucket, dst_pos, storage), int32 [num_seqs * n] each; sequence and storage are -1 for a token the
+        store does not hold."""
+        seq, bucket, pos, storage = torch.empty((4, self.num_seqs * n), dtype=torch.int32, device=self.device).unbind(0)
+        check(self.lib.skv_token_places(ctypes.byref(self.desc), ptr(self.counts), ptr(self.slot_token), ptr(first), n, ptr(seq),
+                                        ptr(bucket), ptr(pos), ptr(storage), self._stream()), "skv_token_places")
+        return seq, bucket, pos, storage
+
+    def prompt_importance(self, layer: int, key_mass: torch.Tensor, assign: bool):
+        """Adds the attention mass fp32 [num_seqs, n] of a prompt pass to the importance of the tokens 0 .. n-1
+        (``assign``: it becomes their cumulative importance) and folds it into the layer's EMA."""
+        mass = key_mass.to(torch.float32).contiguous()
+        assert mass.dim() == 2 and mass.shape[0] == self.num_seqs
+        check(self.lib.skv_prompt_importance(ctypes.byref(self.desc), layer, ptr(self.counts), ptr(self.slot_token), ptr(mass),
+                                             int(mass.shape[1]), int(assign), self.decay, ptr(self.cumulative),
+                                             ptr(self.layer_ema), ptr(self.touched), self._stream()), "skv_prompt_importance")
+
     def plan_step(self, bits: Optional[torch.Tensor] = None):
         """Destination of the token each sequence appends this decode step (same bucket position in every
         layer); does not commit.  Returns (dst_seq, dst_bucket, dst_pos, storage), int32 [num_seqs] each,

@@ -64,3 +64,29 @@ def test_importance_over_steps_and_layers():
         assert np.array_equal(wb.cpu().numpy()[n0:], np.full(steps, 4))
         assert np.array_equal(kc.cpu().numpy(), cache[b][1][0])
         assert np.array_equal(vs.cpu().numpy(), cache[b][1][3])
+
+
+@pytest.mark.parametrize("B,n,first", [(1, 1, 0), (3, 130, 0), (2, 300, 299), (5, 257, 100)])
+def test_token_places_and_prompt_importance(B, n, first):
+    """Against index expressions over the store's own bookkeeping, tokens spread over all buckets, one more asked for than
+    there are; the fp32 arithmetic is the same operation by operation, so the results are equal."""
+    from tests.gpu_util import make_store
+    g = torch.Generator(device="cuda").manual_seed(n)
+    store = make_store(2, B, 2, 64, 4, n + 1)
+    bits = torch.tensor([2, 3, 4, 8], device="cuda")[torch.randint(0, 4, (B, n), generator=g, device="cuda")]
+    seq, bucket, pos, storage = store.plan_bulk(bits)
+    count = n - first
+    got = store.token_places(count + 1, torch.tensor([first], device="cuda"))
+    for have, want in zip(got, (seq, bucket, pos, storage.to(torch.int32).view(-1))):
+        assert torch.equal(have.view(B, -1)[:, :count], want.view(B, n)[:, first:])
+    assert bool((got[0].view(B, -1)[:, count] == -1).all()) and bool((got[3].view(B, -1)[:, count] == -1).all())
+    mass = [torch.rand((B, n), generator=g, device="cuda") for _ in range(3)]
+    at = storage.long()
+    store.cumulative.fill_(7.0)
+    store.prompt_importance(0, mass[0], assign=True)
+    store.prompt_importance(1, mass[1], assign=False)
+    store.prompt_importance(1, mass[2], assign=False)
+    assert torch.equal(store.cumulative.gather(1, at), (mass[0].double() + mass[1].double()) + mass[2].double())
+    assert torch.equal(store.layer_ema[0].gather(1, at), mass[0])
+    assert torch.equal(store.layer_ema[1].gather(1, at), store.decay * mass[1] + (1 - store.decay) * mass[2])
+    assert int(store.touched.sum()) == 2 * B * n and int((store.cumulative != 7.0).sum()) == B * n
