@@ -13,20 +13,26 @@
 // What bounds both: the exponentials.  A 128 x 128 tile has 16384 of them, 1024 cycles of an SM's 16-a-cycle
 // unit; its products take 1024 cycles (pass 1, head_dim 128), 512 (pass 1 at 64, pass 2 at 128) or 256 cycles of the
 // tensor core.  So the products run on tcgen05 (fp16 in, fp32 accumulators in tensor memory) from TMA-fetched
-// tiles, issued by one thread, and the threads are left with one query (pass 2: key) row each: no shuffle, no
+// tiles, issued by one lane, and a thread is left with half a query row (pass 2: a key row): no shuffle, no
 // shared-memory traffic for S or P.  P goes back to tensor memory as the A operand of P V (fp16, as everywhere
 // here), over the columns its S came from.
 //
-// Both kernels are persistent, one CTA per SM: two softmax warpgroups, one loading warp, one warp that issues the MMAs.
-// Pass 1 gives each warpgroup its own 128-query tile so that one computes exponentials while the tensor core works
-// for the other: two query heads of one KV head at the same positions where the group is even (they share every K
-// and V tile and have the same causal range), otherwise two neighbouring query tiles of one head.  Pass 2 hands the
-// query tiles of the stream to the two warpgroups in turn, through four accumulators.  Units of work are dealt
-// longest first, back and forth over the CTAs, because a causal unit's length is proportional to its position.
+// Both kernels are persistent, one CTA per SM: four softmax warpgroups, one loading warp, one warp that issues the MMAs.
+// A warp's own work is a chain (wait, read S, maximum, exponentials, write P), so it takes four warps per scheduler to
+// keep the exponential unit busy: with two, each thread owning a whole row, it was 44 % busy in pass 1 (651 us at 8192 tokens,
+// 577 us now, 51 %) and 76 % in pass 2 (389 and 357 us, 86 %).  One warp issues the MMAs of both tiles in turn; with
+// one per tile both wait for the tensor core and then both for the exponential unit (792 us), and 64-key blocks with
+// scores two blocks ahead end up in the same lockstep (770 us).  Part of the exponentials as a polynomial on the
+// multiply-add pipe costs more issue time than it saves (10 to 20 % slower).
+// Pass 1 gives each pair of warpgroups its own 128-query tile, 64 keys to a thread, so that one pair computes exponentials
+// while the tensor core works for the other: two query heads of one KV head at the same positions where the group is
+// even (they share every K and V tile and have the same causal range), otherwise two neighbouring query tiles of one
+// head.  Pass 2 hands the query tiles of the stream to the warpgroups in turn, each with its own accumulator.  Units of
+// work are dealt longest first, back and forth over the CTAs, because a causal unit's length is proportional to its position.
 //
-// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 1020 us (4315 us with 64 x 64 tiles on
-// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 72 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
-// head_dim 128: 77 us (289 us).
+// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 953 us (4315 us with 64 x 64 tiles on
+// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 67 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
+// head_dim 128: 75 us (289 us).
 #include <cuda_fp16.h>
 
 #include "tc05.cuh"
@@ -34,7 +40,8 @@
 namespace skv {
 
 constexpr int kPfTile = 128;                 // queries per tile and keys per streamed tile
-constexpr int kPfSoftmaxThreads = 256;       // two warpgroups
+constexpr int kPfSoftmaxThreads = 512;       // four warpgroups
+constexpr int kPfLoadWarp = kPfSoftmaxThreads / 32, kPfMmaWarp = kPfLoadWarp + 1;
 constexpr int kPfThreads = kPfSoftmaxThreads + 64;  // + the loading warp and the MMA warp
 constexpr uint32_t kPfTmemCols = 512;
 
@@ -61,8 +68,8 @@ template <int D>
 struct PfCfg {
   static constexpr int kTileBytes = kPfTile * D * 2;
   static constexpr int kStages = D == 128 ? 4 : 6;
-  static constexpr uint32_t kFwdSmem = (kStages + 2) * kTileBytes + 1024 + 256;
-  static constexpr uint32_t kMassSmem = (kStages + 1) * kTileBytes + 1024 + 8 * 136 * 4 + 2 * kPfTile * 4 + 448;
+  static constexpr uint32_t kFwdSmem = (kStages + 2) * kTileBytes + 1024 + 2 * 2 * 2 * kPfTile * 4 + 256;
+  static constexpr uint32_t kMassSmem = (kStages + 1) * kTileBytes + 1024 + 8 * 136 * 4 + 2 * 3 * kPfTile * 4 + 448;
 };
 
 __device__ __forceinline__ float pf_exp2(float x) {
@@ -92,6 +99,18 @@ __device__ __forceinline__ uint64_t pf_add2(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+
+// max(a, b, c); a NaN loses against a number, as in fmaxf
+__device__ __forceinline__ float pf_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t pf_exp2_pair(uint64_t x2) {
+  float x0, x1;
+  pf_unpair(x2, x0, x1);
+  return pf_pair(pf_exp2(x0), pf_exp2(x1));
 }
 
 // Bounded wait: the thread is suspended inside try_wait; after two seconds' worth of clock cycles, or once another
@@ -147,14 +166,20 @@ __device__ __forceinline__ uint32_t pf_tile_tx(const PrefillTensor& t) {
   return t.by_rows ? 0u : (uint32_t)PfCfg<D>::kTileBytes;
 }
 
+// Low words of the matrix descriptors: start address in 16-byte units, below the leading byte offset (unused by K-major
+// swizzled tiles; between the 64-column blocks of a V tile).  The high word is the same for all tiles here.
+__device__ __forceinline__ uint32_t pf_desc_k(uint32_t smem_addr) { return (smem_addr >> 4) | (1u << 16); }
+__device__ __forceinline__ uint32_t pf_desc_v(uint32_t smem_addr) { return (smem_addr >> 4) | ((uint32_t)(kPfTile * 128 / 16) << 16); }
+
 // S = A B^T over head_dim, both K-major: one 16-column step per instruction
 template <int D>
-__device__ __forceinline__ void pf_issue_scores(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem) {
+__device__ __forceinline__ void pf_issue_scores(uint32_t d_tmem, uint32_t a_desc, uint32_t b_desc) {
   constexpr uint32_t idesc = idesc_f16(0, 0, 128, 128);
 #pragma unroll
   for (int kk = 0; kk < D / 16; ++kk) {
-    const uint32_t off = (kk / 4) * (kPfTile * 128) + (kk % 4) * 32;
-    mma_f16_ss(d_tmem, smem_desc(a_smem + off, 1, 64, 2), smem_desc(b_smem + off, 1, 64, 2), idesc, kk > 0);
+    const uint32_t off = ((kk / 4) * (kPfTile * 128) + (kk % 4) * 32) >> 4;
+    if (kk == 0) mma_f16_ss_sw128<false>(d_tmem, a_desc + off, b_desc + off, idesc);
+    else mma_f16_ss_sw128<true>(d_tmem, a_desc + off, b_desc + off, idesc);
   }
 }
 
@@ -209,10 +234,11 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   uint8_t* smem = pf_smem_raw + ((1024u - (smem_u32(pf_smem_raw) & 1023u)) & 1023u);  // swizzle atoms are 1024 bytes
   uint8_t* ring = smem;                    // [NS][TB]: K and V tiles in the order they are used
   uint8_t* qs = ring + NS * TB;            // [2][TB]
-  PfFwdBars& br = *reinterpret_cast<PfFwdBars*>(qs + 2 * TB);
+  float* xch = reinterpret_cast<float*>(qs + 2 * TB);  // [2 (step)][2 (tile)][2 (half)][128]: what the halves of a row tell each other
+  PfFwdBars& br = *reinterpret_cast<PfFwdBars*>(xch + 8 * kPfTile);
   static_assert(sizeof(PfFwdBars) <= 256, "barrier block");
   volatile int* abort_flag = &br.abort_flag;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) {
@@ -223,7 +249,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     mbar_init(&br.qempty, 1);
     for (int w = 0; w < 2; ++w) {
       mbar_init(&br.sfull[w], 1);
-      mbar_init(&br.pready[w], 4);  // one arrival per warp
+      mbar_init(&br.pready[w], 8);  // one arrival per warp
       mbar_init(&br.oready[w], 1);
     }
     mbar_init(&br.drain, 1);
@@ -235,9 +261,9 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = br.tmem_base;  // columns: S_0 S_1 (128 each), O_0 O_1 (D each)
+  const uint32_t tmem = __shfl_sync(0xffffffffu, br.tmem_base, 0);  // columns: S_0 S_1 (128 each), O_0 O_1 (D each)
 
-  if (warp == 8) {
+  if (warp == kPfLoadWarp) {
     // ================================ loading warp ================================
     int i = 0, last_unit = -1;
     bool ok = true;
@@ -280,128 +306,187 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const long long t0 = clock64();
       while (last_unit >= 0 && !mbar_try_wait(&br.qfull, last_unit & 1) && clock64() - t0 < 1000000000ll) {}
     }
-  } else if (warp == 9) {
-    // ================================ MMA warp (one thread) ================================
-    if (lane == 0) {
-      int base = 0;                 // ring index of the unit's first K tile
-      int pc[2] = {0, 0};           // P blocks taken from each warpgroup so far
-      bool ok = true;
-      const uint32_t ring_a = smem_u32(ring), qs_a = smem_u32(qs);
-      constexpr uint32_t pv_idesc = idesc_f16(0, 1, 128, D);
-      for (int round = 0; ok; ++round) {
-        const int u = pf_unit(round, p.units);
-        if (u < 0) break;
-        const PfFwdUnit un = pf_fwd_unit(p, u);
-        const int blocks = max(un.blocks[0], un.blocks[1]);
-        ok = pf_wait(&br.qfull, round & 1, abort_flag);
-        // step j: P V of block j-1, then the scores of block j, for one warpgroup and then the other
-        for (int j = 0; ok && j <= blocks; ++j) {
-          const int ik = base + 2 * j, iv = ik - 1;
-          const int sk = ik % NS, sv = (iv + NS) % NS;
-          if (j < blocks) ok = pf_wait(&br.full[sk], (ik / NS) & 1, abort_flag);
-          if (ok && j > 0) ok = pf_wait(&br.full[sv], (iv / NS) & 1, abort_flag);
+  } else if (warp == kPfMmaWarp) {
+    // ================================ MMA warp ================================
+    // The whole warp walks the loop and one elected lane issues, so that addresses and descriptors are warp-uniform values:
+    // computed by a single lane they cost the issuing thread more than the instruction itself.
+    int base = 0;                 // ring index of the unit's first K tile
+    int pc[2] = {0, 0};           // P blocks taken from each tile so far
+    bool ok = true;
+    const uint32_t ring_d = smem_u32(ring) >> 4, qs_a = smem_u32(qs);
+    constexpr uint32_t pv_idesc = idesc_f16(0, 1, 128, D);
+    for (int round = 0; ok; ++round) {
+      const int u = pf_unit(round, p.units);
+      if (u < 0) break;
+      const PfFwdUnit un = pf_fwd_unit(p, u);
+      const int blocks = max(un.blocks[0], un.blocks[1]);
+      ok = __all_sync(0xffffffffu, pf_wait(&br.qfull, round & 1, abort_flag));
+      // step j: P V of block j-1, then the scores of block j, for one tile and then the other
+      for (int j = 0; ok && j <= blocks; ++j) {
+        const int ik = base + 2 * j, iv = ik - 1;
+        const int sk = ik % NS, sv = (iv + NS) % NS;
+        if (j < blocks) ok = pf_wait(&br.full[sk], (ik / NS) & 1, abort_flag);
+        if (ok && j > 0) ok = pf_wait(&br.full[sv], (iv / NS) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            if (ok && j > 0 && j - 1 < un.blocks[w]) {
-              ok = pf_wait(&br.pready[w], pc[w] & 1, abort_flag);
-              if (!ok) break;
-              ++pc[w];
-              tc_fence_after();
-              const uint32_t va = ring_a + sv * TB;
+        for (int w = 0; w < 2; ++w) {
+          if (ok && j > 0 && j - 1 < un.blocks[w]) {
+            ok = __all_sync(0xffffffffu, pf_wait(&br.pready[w], pc[w] & 1, abort_flag));
+            if (!ok) break;
+            ++pc[w];
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t vd = pf_desc_v((ring_d << 4) + sv * TB);
 #pragma unroll
-              for (int kk = 0; kk < kPfTile / 16; ++kk)  // V rows are the contraction: MN-major, 64-column blocks 16 KB apart
-                mma_f16_ts(tmem + 256 + w * D, tmem + w * 128 + kk * 8, smem_desc(va + kk * 2048, kPfTile * 128 / 16, 64, 2),
-                           pv_idesc, (j > 1 || kk > 0) ? 1u : 0u);
+              for (int kk = 0; kk < kPfTile / 16; ++kk) {  // V rows are the contraction: MN-major, 64-column blocks 16 KB apart
+                const uint32_t pa = tmem + w * 128 + (kk / 4) * 64 + (kk % 4) * 8;
+                if (kk > 0) mma_f16_ts_sw128<true>(tmem + 256 + w * D, pa, vd + kk * 128, pv_idesc);
+                else if (j > 1) mma_f16_ts_sw128<true>(tmem + 256 + w * D, pa, vd, pv_idesc);
+                else mma_f16_ts_sw128<false>(tmem + 256 + w * D, pa, vd, pv_idesc);
+              }
               if (j == un.blocks[w]) mma_commit(&br.oready[w]);
             }
-            if (ok && j < un.blocks[w]) {
-              // the S columns hold P of the block before; its P V was issued first by this thread, and MMAs run in order
-              pf_issue_scores<D>(tmem + w * 128, qs_a + w * TB, ring_a + sk * TB);
+            __syncwarp();
+          }
+          if (ok && j < un.blocks[w]) {
+            // the S columns hold P of the block before; its P V was issued first by this warp's one lane, and MMAs run in order
+            if (elect_one()) {
+              pf_issue_scores<D>(tmem + w * 128, pf_desc_k(qs_a + w * TB), pf_desc_k((ring_d << 4) + sk * TB));
               mma_commit(&br.sfull[w]);
             }
+            __syncwarp();
           }
-          if (!ok) break;
+        }
+        if (!ok) break;
+        if (elect_one()) {
           if (j > 0) mma_commit(&br.empty[sv]);
           if (j < blocks) mma_commit(&br.empty[sk]);
           if (j == blocks - 1) mma_commit(&br.qempty);
         }
-        base += 2 * blocks;
+        __syncwarp();
       }
+      base += 2 * blocks;
+    }
+    if (elect_one()) {
       mma_commit(&br.drain);
       const long long t0 = clock64();
       while (!mbar_try_wait(&br.drain, 0) && clock64() - t0 < 1000000000ll) {}
     }
     __syncwarp();
   } else {
-    // ================================ softmax warpgroups: one query row per thread ================================
-    const int wg = warp >> 2, wq = warp & 3;
+    // ================================ softmax warpgroups: half a query row per thread ================================
+    const int wg = warp >> 3, half = (warp >> 2) & 1, wq = warp & 3;  // tile, half of the keys, lane quarter of tensor memory
     const uint32_t lanes = (uint32_t)(wq * 32) << 16;
-    const uint32_t ts = tmem + wg * 128 + lanes, to = tmem + 256 + wg * D + lanes;
+    const uint32_t ts = tmem + wg * 128 + lanes, to = tmem + 256 + wg * D + half * (D / 2) + lanes;
     const float sc = p.scale_log2, grow = 8.0f / sc;
     const uint64_t sc2 = pf_pair(sc, sc);
     const int n = p.tokens;
-    int sn = 0, on = 0;  // score tiles / outputs received so far
+    int sn = 0, on = 0, xp = 0;  // score tiles / outputs received so far; parity of the exchange buffer
     bool ok = true;
+    // the other half's value of the same row (all 256 threads of the tile)
+    auto exchange = [&](float v) -> float {
+      float* x = xch + ((xp * 2 + wg) * 2) * kPfTile + wq * 32 + lane;
+      x[half * kPfTile] = v;
+      if (wg == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+      else asm volatile("bar.sync 2, 256;" ::: "memory");
+      xp ^= 1;
+      return x[(half ^ 1) * kPfTile];
+    };
+    // The two tiles compute their exponentials in turn (tile 0 first): left alone they drift into step, both at the
+    // exponential unit and then both waiting for the tensor core (both passes 899 us at 8192 tokens, 866 us with the turns).
+    // Each turn is one pass of both through two named barriers, the same number for both tiles whatever they have to do.
+    auto turn_wait = [&] {
+      if (wg == 0) asm volatile("bar.sync 3, 512;" ::: "memory");
+      else asm volatile("bar.sync 4, 512;" ::: "memory");
+    };
+    auto turn_pass = [&] {
+      if (wg == 0) asm volatile("bar.arrive 4, 512;" ::: "memory");
+      else asm volatile("bar.arrive 3, 512;" ::: "memory");
+    };
+    if (wg == 1) turn_pass();
     for (int round = 0;; ++round) {
       const int u = pf_unit(round, p.units);
       if (u < 0) break;
       const PfFwdUnit un = pf_fwd_unit(p, u);
-      const int blocks = un.blocks[wg];
-      if (blocks == 0) continue;
+      const int blocks = un.blocks[wg], turns = max(un.blocks[0], un.blocks[1]);
       const int row = un.tile[wg] * kPfTile + wq * 32 + lane;
       float m = -INFINITY, l = 0.f;  // m: the maximum the row is scaled by; it lags the true one by at most 2^8
-      for (int j = 0; ok && j < blocks; ++j) {
-        ok = pf_wait(&br.sfull[wg], sn & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+      for (int j = 0; j < turns; ++j) {
+        if (j >= blocks) {  // the other tile's longer unit
+          turn_wait();
+          turn_pass();
+          continue;
+        }
+        if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.sfull[wg], sn & 1, abort_flag));
         ++sn;
-        tc_fence_after();
-        // The row is read twice, for its maximum and for the exponentials: 128 values held in between would leave the
-        // compiler no registers to overlap anything with.  In the diagonal block a warp's rows see nothing of the chunks
-        // after its own and, in its own, the keys up to the row's position (keys beyond the prompt lie behind those).
-        const int chunks = j == blocks - 1 ? wq + 1 : 4;
+        // In the diagonal block a warp's rows see nothing of the 32-key chunks after its own and, in its own, the keys up to
+        // the row's position (keys beyond the prompt lie behind those).
         const bool diag = j == blocks - 1;
-        uint32_t s0[32], s1[32];
-        float b0 = -INFINITY, b1 = -INFINITY, b2 = -INFINITY, b3 = -INFINITY;
-        auto chunk_max = [&](uint32_t (&s)[32], bool masked) {
-          if (masked) {
+        const int own = diag ? wq - 2 * half : 2;  // chunks of this half before it are visible in full, the one at it in part
+        tc_fence_after();
+        // 64 values would not fit beside everything else in the 96 registers a thread has, so the second 32 are read twice, 16 at a
+        // time: for the maximum, and again for the exponentials.
+        uint32_t s0[16], s1[16], t[16];
+        float bm = -INFINITY;
+        auto mask_own = [&](uint32_t (&s)[16], int first) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (e > lane) s[e] = 0xff800000u;
-          }
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            b0 = fmaxf(b0, __uint_as_float(s[e]));
-            b1 = fmaxf(b1, __uint_as_float(s[e + 1]));
-            b2 = fmaxf(b2, __uint_as_float(s[e + 2]));
-            b3 = fmaxf(b3, __uint_as_float(s[e + 3]));
-          }
+          for (int e = 0; e < 16; ++e)
+            if (first + e > lane) s[e] = 0xff800000u;
         };
+        auto piece_max = [&](const uint32_t (&s)[16]) {
+          float b0 = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 4; c += 2) {
-          if (c < chunks) {
-            tmem_ld32(ts + c * 32, s0);
-            tmem_ld32(ts + c * 32 + 32, s1);
-            tmem_ld_wait(s0);
-            tmem_ld_wait(s1);
-            chunk_max(s0, diag && c == wq);
-            if (c + 1 < chunks) chunk_max(s1, diag && c + 1 == wq);
+          for (int e = 0; e < 16; e += 4) {
+            b0 = pf_max3(b0, __uint_as_float(s[e]), __uint_as_float(s[e + 1]));
+            bm = pf_max3(bm, __uint_as_float(s[e + 2]), __uint_as_float(s[e + 3]));
+          }
+          bm = fmaxf(bm, b0);
+        };
+        const uint32_t th = ts + half * 64;
+        if (ok) {
+          tmem_ld16(th + 32, t);
+          tmem_ld16(th, s0);
+          tmem_ld16(th + 16, s1);
+          tmem_ld_wait(t);
+          tmem_ld_wait(s0);
+          tmem_ld_wait(s1);
+          if (own >= 1) {
+            if (own == 1) mask_own(t, 0);
+            piece_max(t);
+          }
+          tmem_ld16(th + 48, t);
+          if (own >= 0) {
+            if (own == 0) {
+              mask_own(s0, 0);
+              mask_own(s1, 16);
+            }
+            piece_max(s0);
+            piece_max(s1);
+          }
+          tmem_ld_wait(t);
+          if (own >= 1) {
+            if (own == 1) mask_own(t, 16);
+            piece_max(t);
           }
         }
-        tmem_ld32(ts, s0);  // on its way while the maximum is settled
-        const float bm = fmaxf(fmaxf(b0, b1), fmaxf(b2, b3));
+        bm = fmaxf(bm, exchange(bm));
+        if (!ok) {  // the other warps still need this one at the barriers
+          turn_wait();
+          turn_pass();
+          continue;
+        }
         if (j == 0) {
           m = bm;
         } else {
           // Rescaling costs a round trip of O through registers, so it waits until a row has outgrown its maximum by
-          // 2^8 (fp16 holds P up to there with the same relative precision).
+          // 2^8 (fp16 holds P up to there with the same relative precision).  Both halves of a row decide alike.
           const bool need = bm > m + grow;
           if (__any_sync(0xffffffffu, need)) {
             const float f = need ? pf_exp2((m - bm) * sc) : 1.f;
             if (need) m = bm;
             l *= f;
 #pragma unroll 1
-            for (int c = 0; c < D / 16; ++c) {  // P V of the block before is complete: this block's scores came after it
+            for (int c = 0; c < D / 32; ++c) {  // P V of the block before is complete: this block's scores came after it
               uint32_t o[16];
               tmem_ld16(to + c * 16, o);
               tmem_ld_wait(o);
@@ -411,40 +496,40 @@ __global__ void __launch_bounds__(kPfThreads, 1)
             }
           }
         }
+        turn_wait();
         const float msc = m == -INFINITY ? 0.f : m * sc;
         const uint64_t nm2 = pf_pair(-msc, -msc);
         uint64_t l2a = 0, l2b = 0;
-        auto chunk_exp = [&](int c, uint32_t (&s)[32], uint32_t (&next)[32]) {
-          uint32_t pk[16];
-          if (c < chunks) {
-            tmem_ld_wait(s);
-            if (c + 1 < chunks) tmem_ld32(ts + c * 32 + 32, next);
-            if (diag && c == wq) {
+        // P of a half lies over that half's own S columns, of which the ones written have been read.
+        auto piece_exp = [&](const uint32_t (&s)[16], bool seen, uint32_t to_col) {
+          uint32_t pk[8];
 #pragma unroll
-              for (int e = 0; e < 32; ++e)
-                if (e > lane) s[e] = 0xff800000u;
+          for (int e = 0; e < 8; ++e) {
+            if (!seen) {  // this warp's rows see none of these keys
+              pk[e] = 0u;
+              continue;
             }
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              float x0, x1;
-              pf_unpair(pf_fma2(pf_pair(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), sc2, nm2), x0, x1);
-              x0 = pf_exp2(x0);
-              x1 = pf_exp2(x1);
-              if (e & 1) l2b = pf_add2(l2b, pf_pair(x0, x1));
-              else l2a = pf_add2(l2a, pf_pair(x0, x1));
-              pk[e] = pf_pack_half2(x0, x1);
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) pk[e] = 0u;
+            const uint64_t x2 = pf_fma2(pf_pair(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), sc2, nm2);
+            const uint64_t p2 = pf_exp2_pair(x2);
+            if (e & 1) l2b = pf_add2(l2b, p2);
+            else l2a = pf_add2(l2a, p2);
+            float x0, x1;
+            pf_unpair(p2, x0, x1);
+            pk[e] = pf_pack_half2(x0, x1);
           }
-          // P of chunk c lies over S columns 16c .. 16c+15, which have been read: chunk c/2 and those before it
-          tmem_st16(ts + c * 16, pk);
+          tmem_st8(to_col, pk);
         };
-        chunk_exp(0, s0, s1);
-        chunk_exp(1, s1, s0);
-        chunk_exp(2, s0, s1);
-        chunk_exp(3, s1, s0);
+        tmem_ld16(th + 32, t);
+        piece_exp(s0, own >= 0, th);
+        tmem_ld_wait(t);
+        if (own == 1) mask_own(t, 0);
+        tmem_ld16(th + 48, s0);
+        piece_exp(s1, own >= 0, th + 8);
+        piece_exp(t, own >= 1, th + 16);
+        tmem_ld_wait(s0);
+        if (own == 1) mask_own(s0, 16);
+        piece_exp(s0, own >= 1, th + 24);
+        turn_pass();
         float la, lb;
         pf_unpair(pf_add2(l2a, l2b), la, lb);
         l += la + lb;
@@ -453,18 +538,17 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&br.pready[wg]);
       }
+      if (blocks == 0) continue;
+      l += exchange(l);
       float inv = l > 0.f ? 1.f / l : 0.f, ls = m * sc + log2f(l);
-      if (ok) {
-        ok = pf_wait(&br.oready[wg], on & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        ++on;
-        tc_fence_after();
-      }
+      if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.oready[wg], on & 1, abort_flag));
+      ++on;
+      tc_fence_after();
       if (!ok) inv = ls = __int_as_float(0x7fffffff);
-      if (row < n) p.lse[((long long)un.b * p.num_q_heads + un.head[wg]) * n + row] = ls;
-      __half* ob = p.out + (((long long)un.b * n + row) * p.num_q_heads + un.head[wg]) * D;
+      if (row < n && half == 0) p.lse[((long long)un.b * p.num_q_heads + un.head[wg]) * n + row] = ls;
+      __half* ob = p.out + (((long long)un.b * n + row) * p.num_q_heads + un.head[wg]) * D + half * (D / 2);
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
+      for (int c = 0; c < D / 64; ++c) {
         uint32_t o[32];
         tmem_ld32(to + c * 32, o);
         tmem_ld_wait(o);
@@ -482,6 +566,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       }
       tc_fence_before();  // O has been read: the arrival on the next unit's first P orders it before the next P V
     }
+    if (wg == 0) turn_wait();  // the last turn handed back
   }
   tc_fence_before();
   __syncthreads();
@@ -489,7 +574,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 }
 
 constexpr int kPfLseSlots = 8;
-constexpr int kPfAcc = 4;  // score accumulators in tensor memory
+constexpr int kPfAcc = 4;  // score accumulators in tensor memory, one per warpgroup
 
 struct PfMassBars {
   uint64_t full[6], empty[6];
@@ -525,11 +610,11 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   uint8_t* ring = smem;                                            // [NS][TB]: query tiles
   uint8_t* ks = ring + NS * TB;                                    // the unit's key tile
   float* lse_s = reinterpret_cast<float*>(ks + TB);                // [kPfLseSlots][LS], negated
-  float* red = lse_s + kPfLseSlots * LS;                           // [2][128]: the second warpgroup's sums
-  PfMassBars& br = *reinterpret_cast<PfMassBars*>(red + 2 * kPfTile);
+  float* red = lse_s + kPfLseSlots * LS;                           // [2][3][128]: the sums of the warpgroups but the first
+  PfMassBars& br = *reinterpret_cast<PfMassBars*>(red + 2 * 3 * kPfTile);
   static_assert(sizeof(PfMassBars) <= 448, "barrier block");
   volatile int* abort_flag = &br.abort_flag;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int G = p.num_q_heads / p.num_kv_heads, n = p.tokens;
 
   if (tid == 0) {
@@ -556,9 +641,9 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = br.tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, br.tmem_base, 0);
 
-  if (warp == 8) {
+  if (warp == kPfLoadWarp) {
     // ================================ loading warp ================================
     int i = 0, last_unit = -1;
     bool ok = true;
@@ -617,35 +702,39 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const long long t0 = clock64();
       while (last_unit >= 0 && !mbar_try_wait(&br.kfull, last_unit & 1) && clock64() - t0 < 1000000000ll) {}
     }
-  } else if (warp == 9) {
-    // ================================ MMA warp (one thread) ================================
-    if (lane == 0) {
-      int i = 0;
-      bool ok = true;
-      const uint32_t ring_a = smem_u32(ring), ks_a = smem_u32(ks);
-      for (int round = 0; ok; ++round) {
-        const int u = pf_unit(round, p.units);
-        if (u < 0) break;
-        const PfMassUnit un = pf_mass_unit(p, u);
-        ok = pf_wait(&br.kfull, round & 1, abort_flag);
-        for (int j = 0; ok && j < un.count; ++j, ++i) {
-          const int s = i % NS, a = i % kPfAcc;
-          ok = pf_wait(&br.full[s], (i / NS) & 1, abort_flag) && pf_wait(&br.sempty[a], ((i / kPfAcc) & 1) ^ 1u, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          pf_issue_scores<D>(tmem + a * 128, ks_a, ring_a + s * TB);
+  } else if (warp == kPfMmaWarp) {
+    // ================================ MMA warp ================================
+    int i = 0;
+    bool ok = true;
+    const uint32_t ring_d = smem_u32(ring), ks_d = pf_desc_k(smem_u32(ks));
+    for (int round = 0; ok; ++round) {
+      const int u = pf_unit(round, p.units);
+      if (u < 0) break;
+      const PfMassUnit un = pf_mass_unit(p, u);
+      ok = __all_sync(0xffffffffu, pf_wait(&br.kfull, round & 1, abort_flag));
+      for (int j = 0; ok && j < un.count; ++j, ++i) {
+        const int s = i % NS, a = i % kPfAcc;
+        ok = pf_wait(&br.full[s], (i / NS) & 1, abort_flag) && pf_wait(&br.sempty[a], ((i / kPfAcc) & 1) ^ 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          pf_issue_scores<D>(tmem + a * 128, ks_d, pf_desc_k(ring_d + s * TB));
           mma_commit(&br.sfull[a]);
           mma_commit(&br.empty[s]);
           if (j == un.count - 1) mma_commit(&br.kempty);
         }
+        __syncwarp();
       }
+    }
+    if (elect_one()) {
       mma_commit(&br.drain);
       const long long t0 = clock64();
       while (!mbar_try_wait(&br.drain, 0) && clock64() - t0 < 1000000000ll) {}
     }
     __syncwarp();
   } else {
-    // ================================ two warpgroups: one key row per thread ================================
+    // ================================ four warpgroups: one key row per thread ================================
     const int wg = warp >> 2, wq = warp & 3, wt = tid & 127;
     const uint32_t lanes = (uint32_t)(wq * 32) << 16;
     const uint64_t sc2 = pf_pair(p.scale_log2, p.scale_log2);
@@ -657,7 +746,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const PfMassUnit un = pf_mass_unit(p, u);
       const int per_head = p.tiles - un.kt;
       float acc = 0.f;
-      for (int j = (i0 & 1) == wg ? 0 : 1; ok && j < un.count; j += 2) {
+      for (int j = (wg - i0) & 3; ok && j < un.count; j += kPfAcc) {
         const int i = i0 + j, a = i % kPfAcc, ls = i % kPfLseSlots;
         const bool diag = j % per_head == 0;
         ok = pf_wait(&br.sfull[a], (i / kPfAcc) & 1, abort_flag) && pf_wait(&br.lfull[ls], (i / kPfLseSlots) & 1, abort_flag);
@@ -679,11 +768,10 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const float4 q4 = *reinterpret_cast<const float4*>(nl + c * 32 + e);
-            float x0, x1, x2, x3;
-            pf_unpair(pf_fma2(pf_pair(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc2, pf_pair(q4.x, q4.y)), x0, x1);
-            pf_unpair(pf_fma2(pf_pair(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), sc2, pf_pair(q4.z, q4.w)), x2, x3);
-            t0 = pf_add2(t0, pf_pair(pf_exp2(x0), pf_exp2(x1)));
-            t1 = pf_add2(t1, pf_pair(pf_exp2(x2), pf_exp2(x3)));
+            const uint64_t xa = pf_fma2(pf_pair(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc2, pf_pair(q4.x, q4.y));
+            const uint64_t xb = pf_fma2(pf_pair(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), sc2, pf_pair(q4.z, q4.w));
+            t0 = pf_add2(t0, pf_exp2_pair(xa));
+            t1 = pf_add2(t1, pf_exp2_pair(xb));
           }
         };
         uint32_t s0[32], s1[32];
@@ -710,12 +798,14 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       }
       i0 += un.count;
       if (!ok) acc = __int_as_float(0x7fffffff);
-      // the second warpgroup hands its sums to the first; the buffer alternates, so the barrier of the next unit protects it
-      if (wg == 1) red[(round & 1) * kPfTile + wt] = acc;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      // the warpgroups hand their sums to the first; the buffer alternates, so the barrier of the next unit protects it
+      float* rd = red + (round & 1) * 3 * kPfTile + wt;
+      if (wg != 0) rd[(wg - 1) * kPfTile] = acc;
+      asm volatile("bar.sync 1, 512;" ::: "memory");
       if (wg == 0) {
         const int key = un.kt * kPfTile + wt;
-        if (key < n) p.mass[((long long)un.b * p.num_kv_heads + un.hk) * n + key] = acc + red[(round & 1) * kPfTile + wt];
+        if (key < n)
+          p.mass[((long long)un.b * p.num_kv_heads + un.hk) * n + key] = ((acc + rd[0]) + rd[kPfTile]) + rd[2 * kPfTile];
       }
     }
   }
