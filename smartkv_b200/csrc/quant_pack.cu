@@ -7,6 +7,7 @@
 // this file: codes and scales are bit-exact with the CPU path.
 // Packed format: smartkv/csrc/bit_packing.cu:20-43, 69-95, 128-151.
 #include "post_attention.cuh"
+#include "quant_bulk.cuh"
 
 namespace skv {
 

@@ -24,7 +24,7 @@
 
 #include <cub/block/block_scan.cuh>
 
-#include "quant_row.cuh"
+#include "quant_bulk.cuh"
 
 namespace skv {
 

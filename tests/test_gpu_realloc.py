@@ -256,3 +256,66 @@ def test_reallocate_graphed_equals_eager():
         assert torch.equal(a.cumulative, g.cumulative) and torch.equal(a.rank_streak, g.rank_streak), it
     q = torch.from_numpy(rng.standard_normal((B, hq, d)).astype(np.float32)).cuda()
     assert torch.equal(stores[0].attention(0, q), stores[1].attention(0, q))
+
+
+@pytest.mark.parametrize("n_list", [[1100, 3], [9000], [2100, 1, 2000]])
+def test_allocator_clusters_of_every_size(n_list):
+    """Capacities that give a sequence clusters of 2, 8 and 4 CTAs (the other tests: 1 and 4), three calls with state."""
+    rng = np.random.default_rng(n_list[0])
+    h, d, beta = 8, 128, 0.35
+    store = _alloc_store(n_list, h, d, init_bits_seed=3)
+    cfg, ocfg = store.make_alloc_config(beta), _oracle_cfg(h, d, beta, (2, 3, 4, 8))
+    states = [dict() for _ in n_list]
+    for call in range(3):
+        imps = [_random_importance(rng, n, call) for n in n_list]
+        for b in range(len(n_list)):
+            _scatter_scores(store, b, imps[b])
+        new_bits, new_counts, _ = store.allocate_bits(cfg)
+        for b, n in enumerate(n_list):
+            a = orc.solve_allocation(ocfg, range(n), {t: (float("inf") if t < 4 else float(imps[b][t])) for t in range(n)}, states[b])
+            want = np.array([a[t] for t in range(n)], np.uint8)
+            assert np.array_equal(_device_bits(store, b, n, new_bits), want), (call, b)
+            assert new_counts[b].tolist() == [int((want == w).sum()) for w in (2, 3, 4, 8)]
+
+
+# (layer, head, sequence) items that give clusters of 1, 1, 2, 4 and 8 CTAs; the second case stages in per-cluster slots
+@pytest.mark.parametrize("L,hkv,B,d,n", [(4, 8, 5, 128, 70), (4, 4, 20, 64, 90), (4, 4, 5, 128, 33), (2, 4, 5, 64, 150), (1, 1, 3, 64, 700)])
+def test_row_moves_for_every_cluster_size(L, hkv, B, d, n):
+    """Random new widths, so that every (source, destination) width occurs, with moves inside a bucket: codes and scales of all
+    layers against the oracle's requantisation of the stored codes.  A staging buffer too small moves nothing."""
+    import ctypes
+    from smartkv_b200 import _lib
+    rng = np.random.default_rng(L * hkv * B)
+    store = make_store(L, B, hkv, d, hkv, n)
+    kvs = [tuple(x.reshape(B, n, hkv, d) for x in orc.synth_kv(B * n, hkv, d, seed=40 + l)) for l in range(L)]
+    bits0 = rng.choice((2, 3, 4, 8), size=(B, n))
+    fill_store(store, kvs, bits0)
+    bits1 = np.where(rng.random((B, n)) < 0.4, rng.choice((2, 3, 4, 8), size=(B, n)), bits0)
+    tok = store.slot_token.long()
+    new_bits = torch.where(tok >= 0, torch.from_numpy(bits1).cuda().gather(1, tok.clamp(min=0)), torch.zeros_like(tok)).to(torch.uint8)
+
+    r, before = store._realloc_buffers(), store.arena.clone()
+    lib, desc, st = store.lib, ctypes.byref(store.desc), store._stream()
+    _lib.check(lib.skv_repack_plan(desc, _lib.ptr(store.counts), _lib.ptr(new_bits), _lib.ptr(r["move_src"]), _lib.ptr(r["move_dst"]),
+                                   _lib.ptr(r["n_moves"]), _lib.ptr(r["counts_new"]), _lib.ptr(r["plan_ws"]), _lib.ptr(store.err), st))
+    small = torch.empty(136, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.skv_requant_repack(desc, _lib.ptr(store.arena), 0, L, _lib.ptr(r["move_src"]), _lib.ptr(r["move_dst"]),
+                                      _lib.ptr(r["n_moves"]), _lib.ptr(small), 136, _lib.ptr(store.err), st))
+    with pytest.raises(_lib.SmartKVLibraryError):
+        store.check_errors()
+    assert torch.equal(store.arena, before)
+
+    store.repack(new_bits)
+    store.check_errors()
+    for b in range(B):
+        assert np.array_equal(store.token_bits(b).cpu().numpy(), bits1[b])
+        for l in range(L):
+            _, _, kc, vc, ksc, vsc = (t.cpu().numpy() for t in store.export_sequence(l, b))
+            for w0 in (2, 3, 4, 8):
+                for w1 in (2, 3, 4, 8):
+                    sel = (bits0[b] == w0) & (bits1[b] == w1)
+                    for src, codes, scales in ((kvs[l][0][b], kc, ksc), (kvs[l][1][b], vc, vsc)):
+                        c, s = orc.quantize_rows(src[sel], w0)
+                        if w1 != w0:
+                            c, s = orc.requantize_rows(c, s, w1)
+                        assert np.array_equal(codes[sel], c) and np.array_equal(scales[sel].view(np.uint32), s.view(np.uint32)), (b, l, w0, w1)
