@@ -30,9 +30,9 @@
 // head.  Pass 2 hands the query tiles of the stream to the warpgroups in turn, each with its own accumulator.  Units of
 // work are dealt longest first, back and forth over the CTAs, because a causal unit's length is proportional to its position.
 //
-// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 953 us (4315 us with 64 x 64 tiles on
-// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 67 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
-// head_dim 128: 75 us (289 us).
+// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 991 us (4315 us with 64 x 64 tiles on
+// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 65 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
+// head_dim 128: 77 us (289 us).
 #include <cuda_fp16.h>
 
 #include "tc05.cuh"
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     const int wg = warp >> 3, half = (warp >> 2) & 1, wq = warp & 3;  // tile, half of the keys, lane quarter of tensor memory
     const uint32_t lanes = (uint32_t)(wq * 32) << 16;
     const uint32_t ts = tmem + wg * 128 + lanes, to = tmem + 256 + wg * D + half * (D / 2) + lanes;
-    const float sc = p.scale_log2, grow = 8.0f / sc;
+    const float sc = p.scale_log2;
     const uint64_t sc2 = pf_pair(sc, sc);
     const int n = p.tokens;
     int sn = 0, on = 0, xp = 0;  // score tiles / outputs received so far; parity of the exchange buffer
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const PfFwdUnit un = pf_fwd_unit(p, u);
       const int blocks = un.blocks[wg], turns = max(un.blocks[0], un.blocks[1]);
       const int row = un.tile[wg] * kPfTile + wq * 32 + lane;
-      float m = -INFINITY, l = 0.f;  // m: the maximum the row is scaled by; it lags the true one by at most 2^8
+      float m = -INFINITY, l = 0.f;  // the row's maximum and sum so far
       for (int j = 0; j < turns; ++j) {
         if (j >= blocks) {  // the other tile's longer unit
           turn_wait();
@@ -478,21 +478,23 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         if (j == 0) {
           m = bm;
         } else {
-          // Rescaling costs a round trip of O through registers, so it waits until a row has outgrown its maximum by
-          // 2^8 (fp16 holds P up to there with the same relative precision).  Both halves of a row decide alike.
-          const bool need = bm > m + grow;
+          // O is rescaled whenever a row's maximum grows, however little.  Waiting until it has grown by 2^8 is 4 % faster (949 against
+          // 991 us, both passes at 8192 tokens), but           // then the row's largest P is no longer exactly 1, and its rounding to fp16 (it is the weight that counts) makes
+          // the output's error against 64 bits 10 % larger.  Both halves of a row decide alike; the round trip of O
+          // mostly fits in the wait for the turn.
+          const bool need = bm > m;
           if (__any_sync(0xffffffffu, need)) {
             const float f = need ? pf_exp2((m - bm) * sc) : 1.f;
             if (need) m = bm;
             l *= f;
 #pragma unroll 1
-            for (int c = 0; c < D / 32; ++c) {  // P V of the block before is complete: this block's scores came after it
-              uint32_t o[16];
-              tmem_ld16(to + c * 16, o);
+            for (int c = 0; c < D / 64; ++c) {  // P V of the block before is complete: this block's scores came after it
+              uint32_t o[32];
+              tmem_ld32(to + c * 32, o);
               tmem_ld_wait(o);
 #pragma unroll
-              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-              tmem_st16(to + c * 16, o);
+              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+              tmem_st32(to + c * 32, o);
             }
           }
         }
