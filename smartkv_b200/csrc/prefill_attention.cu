@@ -478,10 +478,10 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         if (j == 0) {
           m = bm;
         } else {
-          // O is rescaled whenever a row's maximum grows, however little.  Waiting until it has grown by 2^8 is 4 % faster (949 against
-          // 991 us, both passes at 8192 tokens), but           // then the row's largest P is no longer exactly 1, and its rounding to fp16 (it is the weight that counts) makes
-          // the output's error against 64 bits 10 % larger.  Both halves of a row decide alike; the round trip of O
-          // mostly fits in the wait for the turn.
+          // O is rescaled whenever a row's maximum grows, however little.  Waiting until it has grown by 2^8 is 4 % faster
+          // (949 against 991 us, both passes at 8192 tokens), but then the row's largest P is no longer exactly 1, and its
+          // rounding to fp16 (it is the weight that counts) makes the output's error against 64 bits 10 % larger.  Both
+          // halves of a row decide alike; the round trip of O mostly fits in the wait for the turn.
           const bool need = bm > m;
           if (__any_sync(0xffffffffu, need)) {
             const float f = need ? pf_exp2((m - bm) * sc) : 1.f;
