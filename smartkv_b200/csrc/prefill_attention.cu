@@ -758,22 +758,32 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         const float* nl = lse_s + ls * LS;
         uint64_t t0 = 0, t1 = 0;
         const uint32_t ta0 = tmem + a * 128 + lanes;
+        auto add4 = [&](float4 q4, uint32_t sa, uint32_t sb, uint32_t sc, uint32_t sd) {
+          const uint64_t xa = pf_fma2(pf_pair(__uint_as_float(sa), __uint_as_float(sb)), sc2, pf_pair(q4.x, q4.y));
+          const uint64_t xb = pf_fma2(pf_pair(__uint_as_float(sc), __uint_as_float(sd)), sc2, pf_pair(q4.z, q4.w));
+          t0 = pf_add2(t0, pf_exp2_pair(xa));
+          t1 = pf_add2(t1, pf_exp2_pair(xb));
+        };
         auto chunk_sum = [&](int c, uint32_t (&s)[32]) {
-          if (diag) {  // queries before the row's key: all of the chunks before the warp's own, part of its own
-            if (c < wq) return;
-            if (c == wq) {
+          if (!diag || c > wq) {
 #pragma unroll
-              for (int e = 0; e < 32; ++e)
-                if (e < lane) s[e] = 0xff800000u;
+            for (int e = 0; e < 32; e += 4)
+              add4(*reinterpret_cast<const float4*>(nl + c * 32 + e), s[e], s[e + 1], s[e + 2], s[e + 3]);
+          } else if (c == wq) {
+            // Queries before the row's key do not see it: all of the chunks before the warp's own, and here the first `lane`.  Their
+            // normalisers become -inf too: the negated one of a query without a finite score is +inf or NaN, which a score of -inf
+            // does not absorb.
+            const uint32_t none = 0xff800000u;
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+              float4 q4 = *reinterpret_cast<const float4*>(nl + c * 32 + e);
+              q4.x = e < lane ? -INFINITY : q4.x;
+              q4.y = e + 1 < lane ? -INFINITY : q4.y;
+              q4.z = e + 2 < lane ? -INFINITY : q4.z;
+              q4.w = e + 3 < lane ? -INFINITY : q4.w;
+              add4(q4, e < lane ? none : s[e], e + 1 < lane ? none : s[e + 1], e + 2 < lane ? none : s[e + 2],
+                   e + 3 < lane ? none : s[e + 3]);
             }
-          }
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const float4 q4 = *reinterpret_cast<const float4*>(nl + c * 32 + e);
-            const uint64_t xa = pf_fma2(pf_pair(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc2, pf_pair(q4.x, q4.y));
-            const uint64_t xb = pf_fma2(pf_pair(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), sc2, pf_pair(q4.z, q4.w));
-            t0 = pf_add2(t0, pf_exp2_pair(xa));
-            t1 = pf_add2(t1, pf_exp2_pair(xb));
           }
         };
         uint32_t s0[32], s1[32];

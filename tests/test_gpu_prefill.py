@@ -127,3 +127,37 @@ def test_prefill_tiles_pairs_and_strides(hq, hkv, d, n, B, layout):
     assert torch.allclose(mass.double(), ref_mass, rtol=1e-3, atol=1e-5), float((mass.double() - ref_mass).abs().max())
     alone, none = causal_prefill_attention(q, k, v, want_mass=False)
     assert none is None and torch.equal(alone, out)
+
+def _expand64(q, k, v):
+    """q, k, v as [B, Hq, n, D] fp64."""
+    qh, kh, vh = (x.transpose(1, 2).double() for x in (q, k, v))
+    return qh, *(x.repeat_interleave(q.shape[2] // k.shape[2], 1) for x in (kh, vh))
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,at", [(4, 2, 64, 300, 70), (8, 2, 128, 200, 133), (3, 1, 128, 260, 0), (3, 3, 64, 129, 127)])
+@pytest.mark.parametrize("what", ["nan", "no_score"])
+def test_prefill_mass_of_keys_a_query_cannot_see(hq, hkv, d, n, at, what):
+    """A query whose row is NaN, or that has no finite score, spoils the mass of the keys it sees and of no other; the output of
+    every other query stays what it is.  Same bounds as above."""
+    from smartkv_b200.prefill import causal_prefill_attention
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn((1, n, h, d), generator=g, device="cuda").half() for h in (hq, hkv, hkv))
+    if what == "nan":
+        q[0, at, hq - 1] = float("nan")
+    else:
+        k[..., 0] = -k[..., 0].abs() - 0.5
+        q[0, at, hq - 1, 0] = float("inf")           # -inf against every key
+    w = torch.rand((1, hq), generator=g, device="cuda") + 0.5
+    out, mass = causal_prefill_attention(q, k, v, w)
+    qh, kh, vh = _expand64(q, k, v)
+    s = (qh @ kh.transpose(2, 3) / d ** 0.5).masked_fill_(torch.ones((n, n), dtype=torch.bool, device="cuda").triu_(1), float("-inf"))
+    p = torch.softmax(s, -1)
+    ref = (p @ vh).transpose(1, 2)
+    p[:, hq - 1, at] = 0
+    ref_mass = (p.sum(2) * w.double()[..., None]).sum(1)
+    assert torch.allclose(mass[:, at + 1:].double(), ref_mass[:, at + 1:], rtol=1e-3, atol=1e-5), mass[:, at + 1:]
+    assert not bool(mass[:, :at + 1].isfinite().any())
+    others = torch.ones((n, hq), dtype=torch.bool, device="cuda")
+    others[at, hq - 1] = False
+    err = (out[0].double() - ref[0]).abs()[others]
+    assert bool((err <= 2e-3 + 2e-3 * ref[0].abs()[others]).all())
