@@ -183,6 +183,11 @@ __device__ __forceinline__ void pf_issue_scores(uint32_t d_tmem, uint32_t a_desc
   }
 }
 
+// Of the tile's rows 32 g .. 32 g + 31, those before row 16 kk, as a bit mask.
+__device__ __forceinline__ constexpr uint32_t pf_rows_before(int kk, int g) {
+  return kk >= 2 * g + 2 ? 0xffffffffu : kk == 2 * g + 1 ? 0x0000ffffu : 0u;
+}
+
 struct PfFwdUnit {
   int tile[2], head[2], blocks[2];  // per warpgroup: query tile, query head, key tiles (0: nothing to do)
   int hk, b;
@@ -337,14 +342,23 @@ __global__ void __launch_bounds__(kPfThreads, 1)
             tc_fence_after();
             if (elect_one()) {
               const uint32_t vd = pf_desc_v((ring_d << 4) + sv * TB);
+              const uint32_t od = tmem + 256 + w * D, pd = tmem + w * 128;
+              auto p_at = [&](int kk) { return pd + (kk / 4) * 64 + (kk % 4) * 8; };
+              // V rows are the contraction: MN-major, 64-column blocks 16 KB apart
+              if (j > 1) mma_f16_ts_sw128<true>(od, pd, vd, pv_idesc);
+              else mma_f16_ts_sw128<false>(od, pd, vd, pv_idesc);
+              if (j < un.blocks[w]) {
 #pragma unroll
-              for (int kk = 0; kk < kPfTile / 16; ++kk) {  // V rows are the contraction: MN-major, 64-column blocks 16 KB apart
-                const uint32_t pa = tmem + w * 128 + (kk / 4) * 64 + (kk % 4) * 8;
-                if (kk > 0) mma_f16_ts_sw128<true>(tmem + 256 + w * D, pa, vd + kk * 128, pv_idesc);
-                else if (j > 1) mma_f16_ts_sw128<true>(tmem + 256 + w * D, pa, vd, pv_idesc);
-                else mma_f16_ts_sw128<false>(tmem + 256 + w * D, pa, vd, pv_idesc);
+                for (int kk = 1; kk < kPfTile / 16; ++kk) mma_f16_ts_sw128<true>(od, p_at(kk), vd + kk * 128, pv_idesc);
+              } else {
+                // In the diagonal block the queries before a step's 16 keys leave it out: their P there is zero, but zero times an
+                // infinite or NaN value is not.
+#pragma unroll
+                for (int kk = 1; kk < kPfTile / 16; ++kk)
+                  mma_f16_ts_sw128_lanes(od, p_at(kk), vd + kk * 128, pv_idesc, pf_rows_before(kk, 0), pf_rows_before(kk, 1),
+                                         pf_rows_before(kk, 2), pf_rows_before(kk, 3));
+                mma_commit(&br.oready[w]);
               }
-              if (j == un.blocks[w]) mma_commit(&br.oready[w]);
             }
             __syncwarp();
           }

@@ -124,6 +124,15 @@ __device__ __forceinline__ void mma_f16_ts_sw128(uint32_t d_tmem, uint32_t a_tme
       "r"(a_tmem), "r"(b_lo), "r"(idesc), "n"(kDescHiSw128), "n"((int)ACC)
       : "memory");
 }
+// the same, leaving the accumulator's lanes alone whose bit is set in (m0, m1, m2, m3), lane 0 in the lowest bit of m0
+__device__ __forceinline__ void mma_f16_ts_sw128_lanes(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t m0,
+                                                       uint32_t m1, uint32_t m2, uint32_t m3) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, 1, 0;\n\tmov.b64 db, {%2, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(idesc), "n"(kDescHiSw128), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
+      : "memory");
+}
 // one lane of a converged warp (the same at every call)
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;

@@ -161,3 +161,22 @@ def test_prefill_mass_of_keys_a_query_cannot_see(hq, hkv, d, n, at, what):
     others[at, hq - 1] = False
     err = (out[0].double() - ref[0]).abs()[others]
     assert bool((err <= 2e-3 + 2e-3 * ref[0].abs()[others]).all())
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,at", [(4, 2, 64, 300, 112), (8, 2, 128, 256, 255), (3, 1, 128, 260, 16), (2, 2, 64, 140, 129)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_prefill_output_of_queries_before_a_non_finite_value_row(hq, hkv, d, n, at, value):
+    """A value row that is not finite reaches the queries that see it, and of the ones before it at most those of its own group
+    of 16 positions (their weight for it is zero, and zero times infinity is not).  Same bounds as above."""
+    from smartkv_b200.prefill import causal_prefill_attention
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn((1, n, h, d), generator=g, device="cuda").half() for h in (hq, hkv, hkv))
+    v[0, at, hkv - 1] = value
+    out, _ = causal_prefill_attention(q, k, v, want_mass=False)
+    first = at // 16 * 16
+    ref, _ = _dense64(q[:, :first], k[:, :first], v[:, :first], torch.ones((1, hq), device="cuda"))
+    err = (out[:, :first].double() - ref).abs()
+    assert bool((err <= 2e-3 + 2e-3 * ref.abs()).all())
+    assert not bool(out[0, at:, hq - 1].isfinite().any())
+    if hkv > 1:
+        assert bool(out[0, :, 0].isfinite().all())
