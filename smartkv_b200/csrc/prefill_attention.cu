@@ -498,7 +498,9 @@ __global__ void __launch_bounds__(kPfThreads, 1)
           // halves of a row decide alike; the round trip of O mostly fits in the wait for the turn.
           const bool need = bm > m;
           if (__any_sync(0xffffffffu, need)) {
-            const float f = need ? pf_exp2((m - bm) * sc) : 1.f;
+            // the exponentials are taken against the maximum times the scale rounded to fp32, so the factor is that of the rounded
+            // numbers (and the log-sum-exp below uses it): otherwise the key mass is off by up to 2^-24 of the logit
+            const float f = need ? pf_exp2(__fmul_rn(m, sc) - __fmul_rn(bm, sc)) : 1.f;
             if (need) m = bm;
             l *= f;
 #pragma unroll 1
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
           }
         }
         turn_wait();
-        const float msc = m == -INFINITY ? 0.f : m * sc;
+        const float msc = m == -INFINITY ? 0.f : __fmul_rn(m, sc);
         const uint64_t nm2 = pf_pair(-msc, -msc);
         uint64_t l2a = 0, l2b = 0;
         // P of a half lies over that half's own S columns, of which the ones written have been read.
@@ -556,7 +558,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       }
       if (blocks == 0) continue;
       l += exchange(l);
-      float inv = l > 0.f ? 1.f / l : 0.f, ls = m * sc + log2f(l);
+      float inv = l > 0.f ? 1.f / l : 0.f, ls = __fadd_rn(__fmul_rn(m, sc), log2f(l));
       if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.oready[wg], on & 1, abort_flag));
       ++on;
       tc_fence_after();

@@ -180,3 +180,31 @@ def test_prefill_output_of_queries_before_a_non_finite_value_row(hq, hkv, d, n, 
     assert not bool(out[0, at:, hq - 1].isfinite().any())
     if hkv > 1:
         assert bool(out[0, :, 0].isfinite().all())
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,B", [(4, 2, 128, 700, 2), (3, 1, 64, 520, 1)])
+def test_prefill_log_sum_exp_at_large_logits(hq, hkv, d, n, B):
+    """The row normalisers against 64 bits.  Queries and keys are small whole numbers, so that the scores, in the thousands, are
+    exact in fp32; what is left is the rounding of the result, half a unit in its last place, and 2^-21 for the exponentials
+    and the sum.  A normaliser that does not belong to the maximum the sum was taken against is off by up to another half unit."""
+    import ctypes
+    from smartkv_b200 import _lib
+    from smartkv_b200.prefill import _strides
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k = (torch.randint(-24, 25, (B, n, h, d), generator=g, device="cuda").half() for h in (hq, hkv))
+    k *= torch.linspace(0.25, 1, n, device="cuda").mul(4).round().div(4).half()[None, :, None, None]      # maxima that grow
+    v = torch.zeros_like(k)
+    out, lse = torch.empty_like(q), torch.empty((B, hq, n), device="cuda")
+    _lib.check(_lib.lib().skv_prefill_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.DTYPE_F16, B, n, hq, hkv, d, _strides(q),
+                                                _strides(k), _strides(v), None, out.data_ptr(), lse.data_ptr(), None,
+                                                torch.cuda.current_stream().cuda_stream))
+    qh, kh, _ = _expand64(q, k, v)
+    scale = np.float32(1.4426950408889634) / np.sqrt(np.float32(d))
+    s = qh @ kh.transpose(2, 3) * float(scale)
+    s.masked_fill_(torch.ones((n, n), dtype=torch.bool, device="cuda").triu_(1), float("-inf"))
+    m = s.max(-1, keepdim=True).values
+    ref = (m + torch.log2(torch.exp2(s - m).sum(-1, keepdim=True)))[..., 0]
+    ulp = torch.exp2(torch.floor(torch.log2(ref.abs().clamp(min=1e-3))) - 23)
+    assert float(ref.abs().max()) > 256
+    worst = ((lse.double() - ref).abs() - 2.0 ** -21) / ulp
+    assert float(worst.max()) <= 0.5, float(worst.max())
