@@ -206,6 +206,8 @@ class PackedKVStore:
         """Where the tokens with ids first .. first + n - 1 of every sequence lie (``first``: int64 device scalar, default 0):
         (dst_seq, dst_bucket, dst_pos, storage), int32 [num_seqs * n] each; sequence and storage are -1 for a token the
         store does not hold."""
+        if first is not None and (first.dtype != torch.int64 or first.numel() != 1 or first.device != self.counts.device):
+            raise ValueError(f"first must be one int64 on {self.counts.device}; got {first.dtype} {list(first.shape)} on {first.device}")
         seq, bucket, pos, storage = torch.empty((4, self.num_seqs * n), dtype=torch.int32, device=self.device).unbind(0)
         check(self.lib.skv_token_places(ctypes.byref(self.desc), ptr(self.counts), ptr(self.slot_token), ptr(first), n, ptr(seq),
                                         ptr(bucket), ptr(pos), ptr(storage), self._stream()), "skv_token_places")
@@ -214,8 +216,10 @@ class PackedKVStore:
     def prompt_importance(self, layer: int, key_mass: torch.Tensor, assign: bool):
         """Adds the attention mass fp32 [num_seqs, n] of a prompt pass to the importance of the tokens 0 .. n-1
         (``assign``: it becomes their cumulative importance) and folds it into the layer's EMA."""
+        if key_mass.dim() != 2 or key_mass.shape[0] != self.num_seqs or key_mass.device != self.counts.device:
+            raise ValueError(f"key_mass must be [{self.num_seqs}, n] on {self.counts.device}; got {list(key_mass.shape)} on "
+                             f"{key_mass.device}")
         mass = key_mass.to(torch.float32).contiguous()
-        assert mass.dim() == 2 and mass.shape[0] == self.num_seqs
         check(self.lib.skv_prompt_importance(ctypes.byref(self.desc), layer, ptr(self.counts), ptr(self.slot_token), ptr(mass),
                                              int(mass.shape[1]), int(assign), self.decay, ptr(self.cumulative),
                                              ptr(self.layer_ema), ptr(self.touched), self._stream()), "skv_prompt_importance")

@@ -154,3 +154,27 @@ def test_graph_replayed_steps_are_bit_identical_to_eager_steps():
     assert b[7] >= 3 and a[5] == b[5] and a[6] == b[6]
     assert torch.equal(a[0], b[0]), float((a[0] - b[0]).abs().max())
     assert torch.equal(a[1], b[1]) and torch.equal(a[2], b[2]) and torch.equal(a[3], b[3]) and torch.equal(a[4], b[4])
+
+
+def _prompted(B=2, n=70, L=2):
+    """A cache for B sequences, keys and values of an n-token prompt, and the generator they came from."""
+    from smartkv_b200 import BatchedSmartKVCache
+    cache = BatchedSmartKVCache(L, 2, 64, 4, B, max_tokens=256, memory_budget=0.5)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    k, v = (torch.randn((B, n, 2, 64), generator=g, device="cuda") for _ in range(2))
+    return cache, k, v, g
+
+
+def test_prompt_importance_refuses_what_is_not_on_its_device():
+    """The kernels get raw addresses: a mass, or a first token id, that lies elsewhere is refused before any launch."""
+    cache, k, v, _ = _prompted()
+    with pytest.raises(ValueError):
+        cache.prefill_layer(0, k, v, key_mass=torch.rand((2, 70)))
+    with pytest.raises(ValueError):
+        cache.store.prompt_importance(0, torch.rand((2, 70)), assign=True)
+    with pytest.raises(ValueError):
+        cache.store.prompt_importance(0, torch.rand((3, 70), device="cuda"), assign=True)
+    for first in (torch.tensor([0]), torch.tensor([0], device="cuda", dtype=torch.int32), torch.tensor([0, 1], device="cuda")):
+        with pytest.raises(ValueError):
+            cache.store.token_places(1, first)
+    cache.check_errors()
