@@ -191,11 +191,15 @@ class BatchedSmartKVCache:
                 raise NotImplementedError("a second multi-token call on a non-empty batched cache (chunked prefill)")
             if n + 1 > self.max_tokens:
                 raise _lib.SmartKVLibraryError(f"{n} prompt tokens exceed the cache capacity of {self.max_tokens - 1}")
+        elif n > self.num_known:
+            raise ValueError(f"{n} prompt tokens in layer {layer}; the cache holds {self.num_known} per sequence")
         if key_mass is not None:
             mass = key_mass
-            if tuple(mass.shape) != (B, n):
-                raise ValueError(f"key_mass must be [{B}, {n}]; got {list(mass.shape)}")
+            if tuple(mass.shape) != (B, n) or mass.device != st.counts.device:
+                raise ValueError(f"key_mass must be [{B}, {n}] on {st.counts.device}; got {list(mass.shape)} on {mass.device}")
         else:
+            if probs.shape[-1] != n:
+                raise ValueError(f"probs must be over {n} keys; got {list(probs.shape)}")
             w = self._weights(probs.float().mean(dim=(2, 3)))
             mass = (probs.float() * w[:, :, None, None]).sum(dim=(1, 2))      # [B, n] per key
         places = None

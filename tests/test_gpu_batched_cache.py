@@ -178,3 +178,19 @@ def test_prompt_importance_refuses_what_is_not_on_its_device():
         with pytest.raises(ValueError):
             cache.store.token_places(1, first)
     cache.check_errors()
+
+
+def test_prefill_layer_refuses_tokens_the_cache_does_not_hold():
+    """A later layer can bring no more prompt tokens than layer 0 did, and the probabilities are over these tokens."""
+    cache, k, v, g = _prompted()
+    cache.prefill_layer(0, k, v, key_mass=torch.rand((2, 70), generator=g, device="cuda"))
+    before = [t.clone() for t in (cache.store.cumulative, cache.store.layer_ema, cache.store.arena, cache.last_seen)]
+    more = torch.randn((2, 71, 2, 64), generator=g, device="cuda")
+    with pytest.raises(ValueError):
+        cache.prefill_layer(1, more, more, key_mass=torch.rand((2, 71), device="cuda"))
+    with pytest.raises(ValueError):
+        cache.prefill_layer(1, k, v, probs=torch.rand((2, 4, 70, 71), device="cuda"))
+    for t, b in zip((cache.store.cumulative, cache.store.layer_ema, cache.store.arena, cache.last_seen), before):
+        assert torch.equal(t, b)
+    cache.prefill_layer(1, k, v, key_mass=torch.rand((2, 70), device="cuda"))
+    cache.check_errors()
