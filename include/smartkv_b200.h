@@ -327,6 +327,10 @@ int skv_importance_update(const SkvStoreDesc* desc, int layer, const int32_t* co
 int skv_prompt_importance(const SkvStoreDesc* desc, int layer, const int32_t* counts, const int32_t* slot_token,
                           const float* key_mass, int n, int assign, double decay, double* cumulative,
                           float* layer_ema, uint8_t* touched, void* stream);
+/* The same for a key mass in fp64, which is accumulated as it is. */
+int skv_prompt_importance_f64(const SkvStoreDesc* desc, int layer, const int32_t* counts, const int32_t* slot_token,
+                              const double* key_mass, int n, int assign, double decay, double* cumulative,
+                              float* layer_ema, uint8_t* touched, void* stream);
 
 /* Where the tokens with ids first .. first + n - 1 lie (first_token: device int64, NULL = 0): dst_seq / dst_bucket /
  * dst_pos int32 [num_seqs][n] as skv_quantize_pack_append takes them, and the storage index.  A token that the store

@@ -116,6 +116,8 @@ _SIGNATURES = {
                                       c_float, c_void_p]),
     "skv_prompt_importance": (c_int, [POINTER(StoreDesc), c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_double,
                                       c_void_p, c_void_p, c_void_p, c_void_p]),
+    "skv_prompt_importance_f64": (c_int, [POINTER(StoreDesc), c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_double,
+                                          c_void_p, c_void_p, c_void_p, c_void_p]),
     "skv_token_places": (c_int, [POINTER(StoreDesc), c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_void_p]),
     "skv_read_error_flag": (c_int, [c_void_p, POINTER(c_int32), c_void_p]),

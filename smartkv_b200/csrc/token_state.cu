@@ -36,27 +36,30 @@ __global__ void __launch_bounds__(kTokenThreads)
   storage[at] = s;
 }
 
+template <typename Mass>
 struct PromptParams {
   StoreGeom g;
   int layer;
   const int32_t* counts;
   const int32_t* slot_token;
-  const float* mass;  // [num_seqs][n]
+  const Mass* mass;  // [num_seqs][n]
   int n, assign;
   float decay, fresh;
   double* cumulative;
   float* layer_ema;
   uint8_t* touched;
 };
-__global__ void __launch_bounds__(kTokenThreads) prompt_importance_kernel(const PromptParams p) {
+template <typename Mass>
+__global__ void __launch_bounds__(kTokenThreads) prompt_importance_kernel(const PromptParams<Mass> p) {
   const int b = blockIdx.y, s = blockIdx.x * kTokenThreads + threadIdx.x;
   if (s >= p.g.slots) return;
   int bucket, pos;
   const int id = live_token(p.g, p.counts, p.slot_token, b, s, bucket, pos);
   if (id < 0 || id >= p.n) return;
-  const float m = p.mass[(long long)b * p.n + id];
+  const Mass mass = p.mass[(long long)b * p.n + id];
+  const float m = (float)mass;  // the layer's average is fp32 whatever the mass comes in
   const long long ci = (long long)b * p.g.slots + s;
-  p.cumulative[ci] = p.assign ? (double)m : p.cumulative[ci] + (double)m;
+  p.cumulative[ci] = p.assign ? (double)mass : p.cumulative[ci] + (double)mass;
   const long long li = ((long long)p.layer * p.g.num_seqs + b) * p.g.slots + s;
   if (p.touched[li]) {
     p.layer_ema[li] = __fadd_rn(__fmul_rn(p.decay, p.layer_ema[li]), __fmul_rn(p.fresh, m));
@@ -64,6 +67,20 @@ __global__ void __launch_bounds__(kTokenThreads) prompt_importance_kernel(const 
     p.layer_ema[li] = m;
     p.touched[li] = 1;
   }
+}
+
+template <typename Mass>
+static int prompt_importance(const SkvStoreDesc* desc, int layer, const int32_t* counts, const int32_t* slot_token,
+                             const Mass* key_mass, int n, int assign, double decay, double* cumulative, float* layer_ema,
+                             uint8_t* touched, void* stream) {
+  if (!desc || !counts || !slot_token || !key_mass || n <= 0 || !cumulative || !layer_ema || !touched) return SKV_ERR_INVALID;
+  if (layer < 0 || layer >= desc->num_layers) return SKV_ERR_INVALID;
+  if (desc->num_seqs > 65535) return SKV_ERR_UNSUPPORTED;
+  PromptParams<Mass> p = {make_geom(*desc), layer, counts, slot_token, key_mass, n, assign, (float)decay, (float)(1.0 - decay),
+                          cumulative, layer_ema, touched};
+  const dim3 grid((desc->slots + kTokenThreads - 1) / kTokenThreads, desc->num_seqs);
+  prompt_importance_kernel<<<grid, kTokenThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }
 
 }  // namespace skv
@@ -89,12 +106,11 @@ extern "C" int skv_token_places(const SkvStoreDesc* desc, const int32_t* counts,
 extern "C" int skv_prompt_importance(const SkvStoreDesc* desc, int layer, const int32_t* counts, const int32_t* slot_token,
                                      const float* key_mass, int n, int assign, double decay, double* cumulative,
                                      float* layer_ema, uint8_t* touched, void* stream) {
-  if (!desc || !counts || !slot_token || !key_mass || n <= 0 || !cumulative || !layer_ema || !touched) return SKV_ERR_INVALID;
-  if (layer < 0 || layer >= desc->num_layers) return SKV_ERR_INVALID;
-  if (desc->num_seqs > 65535) return SKV_ERR_UNSUPPORTED;
-  PromptParams p = {make_geom(*desc), layer, counts, slot_token, key_mass, n, assign, (float)decay, (float)(1.0 - decay),
-                    cumulative, layer_ema, touched};
-  const dim3 grid((desc->slots + kTokenThreads - 1) / kTokenThreads, desc->num_seqs);
-  prompt_importance_kernel<<<grid, kTokenThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
+  return prompt_importance(desc, layer, counts, slot_token, key_mass, n, assign, decay, cumulative, layer_ema, touched, stream);
+}
+
+extern "C" int skv_prompt_importance_f64(const SkvStoreDesc* desc, int layer, const int32_t* counts, const int32_t* slot_token,
+                                         const double* key_mass, int n, int assign, double decay, double* cumulative,
+                                         float* layer_ema, uint8_t* touched, void* stream) {
+  return prompt_importance(desc, layer, counts, slot_token, key_mass, n, assign, decay, cumulative, layer_ema, touched, stream);
 }

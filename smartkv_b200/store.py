@@ -214,15 +214,18 @@ class PackedKVStore:
         return seq, bucket, pos, storage
 
     def prompt_importance(self, layer: int, key_mass: torch.Tensor, assign: bool):
-        """Adds the attention mass fp32 [num_seqs, n] of a prompt pass to the importance of the tokens 0 .. n-1
-        (``assign``: it becomes their cumulative importance) and folds it into the layer's EMA."""
+        """Adds the attention mass [num_seqs, n] of a prompt pass to the importance of the tokens 0 .. n-1
+        (``assign``: it becomes their cumulative importance) and folds it into the layer's EMA.  fp16, bf16 and fp32 masses
+        are taken as fp32, every other type as fp64."""
         if key_mass.dim() != 2 or key_mass.shape[0] != self.num_seqs or key_mass.device != self.counts.device:
             raise ValueError(f"key_mass must be [{self.num_seqs}, n] on {self.counts.device}; got {list(key_mass.shape)} on "
                              f"{key_mass.device}")
-        mass = key_mass.to(torch.float32).contiguous()
-        check(self.lib.skv_prompt_importance(ctypes.byref(self.desc), layer, ptr(self.counts), ptr(self.slot_token), ptr(mass),
-                                             int(mass.shape[1]), int(assign), self.decay, ptr(self.cumulative),
-                                             ptr(self.layer_ema), ptr(self.touched), self._stream()), "skv_prompt_importance")
+        single = key_mass.dtype in (torch.float16, torch.bfloat16, torch.float32)
+        mass = key_mass.to(torch.float32 if single else torch.float64).contiguous()
+        update = self.lib.skv_prompt_importance if single else self.lib.skv_prompt_importance_f64
+        check(update(ctypes.byref(self.desc), layer, ptr(self.counts), ptr(self.slot_token), ptr(mass), int(mass.shape[1]),
+                     int(assign), self.decay, ptr(self.cumulative), ptr(self.layer_ema), ptr(self.touched), self._stream()),
+              "skv_prompt_importance")
 
     def plan_step(self, bits: Optional[torch.Tensor] = None):
         """Destination of the token each sequence appends this decode step (same bucket position in every

@@ -194,3 +194,16 @@ def test_prefill_layer_refuses_tokens_the_cache_does_not_hold():
         assert torch.equal(t, b)
     cache.prefill_layer(1, k, v, key_mass=torch.rand((2, 70), device="cuda"))
     cache.check_errors()
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.int64, torch.float16])
+def test_prefill_layer_accumulates_a_mass_as_it_comes(dtype):
+    """A key mass in 64 bits is accumulated in 64 bits; the layer average is fp32 as ever."""
+    cache, k, v, g = _prompted()
+    mass = [torch.rand((2, 70), generator=g, device="cuda", dtype=torch.float64) for _ in range(2)]
+    mass = [(m * 2 ** 40 if dtype == torch.int64 else m).to(dtype) for m in mass]
+    for layer in range(2):
+        cache.prefill_layer(layer, k, v, key_mass=mass[layer])
+    at = cache._token_storage()[:, :70]
+    assert torch.equal(cache.store.cumulative.gather(1, at), mass[0].double() + mass[1].double())
+    assert torch.equal(cache.store.layer_ema[1].gather(1, at), mass[1].float())
