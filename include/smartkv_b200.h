@@ -209,8 +209,9 @@ int skv_get_attention_path(void);
 /* Limit of every bounded device-side wait of the attention kernels, in polls of about 50 ns (default
  * 2^24, about one second).  When a wait runs out the kernel sets *err_flag, waits (bounded) for its own
  * copies still in flight and returns; nothing faults and the context stays usable.  The fragment kernel
- * honours any limit; the tensor-memory kernel never uses fewer than 2^20 polls.  No counterpart in the
- * reference. */
+ * honours any limit; the tensor-memory kernel never uses fewer than 2^20 polls; the prompt pass counts 128
+ * clock cycles a poll, up to 2^24 polls, and below 16 gives up on the first tile that is not there at once.
+ * No counterpart in the reference. */
 int skv_set_wait_limit(unsigned polls);
 
 /* Combines the partials with the newest token, which takes part in full precision
@@ -304,6 +305,13 @@ int skv_prefill_attention(const void* q, const void* k, const void* v, int dtype
                           int num_q_heads, int num_kv_heads, int head_dim, const int64_t* q_strides,
                           const int64_t* k_strides, const int64_t* v_strides, const float* head_weights, void* out,
                           float* lse, float* key_mass, void* stream);
+/* The same with an error flag (device, may be NULL).  The kernels' waits are bounded (skv_set_wait_limit); when one runs out
+ * *err_flag becomes 1, which skv_read_error_flag reports as SKV_ERR_TIMEOUT, and the output rows, log-sum-exps and masses
+ * still owed are NaN.  Without a flag the NaNs are the only sign. */
+int skv_prefill_attention_checked(const void* q, const void* k, const void* v, int dtype, int batch, int tokens,
+                                  int num_q_heads, int num_kv_heads, int head_dim, const int64_t* q_strides,
+                                  const int64_t* k_strides, const int64_t* v_strides, const float* head_weights, void* out,
+                                  float* lse, float* key_mass, int32_t* err_flag, void* stream);
 
 /* ---- importance ----------------------------------------------------------- */
 

@@ -9,6 +9,9 @@
 
 namespace skv {
 
+// The process's limit of device-side waits (skv_set_wait_limit), in polls of about 50 ns.
+unsigned wait_polls();
+
 constexpr int kNumBuckets = SKV_NUM_BUCKETS;
 
 __host__ __device__ constexpr int bucket_bits(int bucket) {

@@ -801,6 +801,7 @@ static int launch_attn(AttnParams& p, cudaStream_t st) {
 
 // Limit of every bounded device-side wait, in polls of about 50 ns (default 2^24, about a second).
 static std::atomic<unsigned> g_wait_polls{1u << 24};
+unsigned skv::wait_polls() { return g_wait_polls.load(); }
 extern "C" int skv_set_wait_limit(unsigned polls) {
   if (polls == 0) return SKV_ERR_INVALID;
   g_wait_polls.store(polls);
@@ -837,7 +838,7 @@ extern "C" int skv_decode_attention_masked(const SkvStoreDesc* desc, const void*
   p.mask_stride = mask_stride;
   p.err = err_flag;
   p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)desc->head_dim));
-  p.wait_polls = g_wait_polls.load();
+  p.wait_polls = wait_polls();
   p.dependent = (flags & SKV_ATTN_DEPENDENT_LAUNCH) ? 1 : 0;
   if (use_tc_path(desc, query_dtype)) return launch_attn_tc(p, *desc, as_stream(stream));
   const bool precise = !p.q_is_half;

@@ -62,6 +62,8 @@ struct PrefillParams {
   int tiles;                   // 128-token tiles of a sequence
   int units;
   float scale_log2;
+  unsigned wait_cycles;        // limit of every wait, at most 2^31
+  int32_t* err;                // set to 1 when a wait runs out (may be null)
 };
 
 template <int D>
@@ -113,19 +115,37 @@ __device__ __forceinline__ uint64_t pf_exp2_pair(uint64_t x2) {
   return pf_pair(pf_exp2(x0), pf_exp2(x1));
 }
 
-// Bounded wait: the thread is suspended inside try_wait; after two seconds' worth of clock cycles, or once another
-// role gave up, it returns false.  A CTA that gives up writes NaN to the rows it still owed.
-__device__ __noinline__ bool pf_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  const long long t0 = clock64();
-  while (clock64() - t0 < 4000000000ll) {
+// Bounded wait: the thread is suspended inside try_wait; after the limit, or once another role gave up, it returns false.  A CTA that
+// gives up sets the error flag, writes NaN to the rows it still owed, waits for its copies and MMAs in flight, frees its tensor
+// memory and ends.  With a limit of no cycles the MMA warp does so on the first tile that is not there at once.
+struct PfGiveUp {  // in shared memory, so that the call takes no registers from the callers
+  int32_t* err;
+  unsigned cycles;
+  int flag;
+};
+__device__ __noinline__ bool pf_wait_slow(uint64_t* bar, uint32_t parity, PfGiveUp* give_up) {
+  if (mbar_test_wait(bar, parity)) return true;
+  volatile int* flag = &give_up->flag;
+  const unsigned t0 = (unsigned)clock();
+  while ((unsigned)clock() - t0 < give_up->cycles) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
+    if (*flag) return false;
   }
-  *abort_flag = 1;
+  *flag = 1;
+  if (give_up->err) atomicExch(give_up->err, 1);
   return false;
 }
-__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  return mbar_try_wait(bar, parity) || pf_wait_slow(bar, parity, abort_flag);
+__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, PfGiveUp* give_up) {
+  return mbar_try_wait(bar, parity) || pf_wait_slow(bar, parity, give_up);
+}
+__device__ __forceinline__ bool pf_wait_unit(uint64_t* bar, uint32_t parity, PfGiveUp* give_up, unsigned cycles) {
+  return (cycles > 0 && mbar_try_wait(bar, parity)) || pf_wait_slow(bar, parity, give_up);
+}
+
+// Waits, bounded, for what this CTA itself has in flight, whatever the limit of the other waits.
+__device__ __forceinline__ void pf_drain(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity) && clock64() - t0 < 1000000000ll) {}
 }
 
 // The unit a CTA takes in its `round`-th turn (-1: none left): back and forth, so that whoever got the longest unit of
@@ -226,7 +246,7 @@ struct PfFwdBars {
   uint64_t sfull[2], pready[2], oready[2];
   uint64_t drain;
   uint32_t tmem_base;
-  int abort_flag;
+  PfGiveUp give_up;
 };
 
 template <int D>
@@ -242,7 +262,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   float* xch = reinterpret_cast<float*>(qs + 2 * TB);  // [2 (step)][2 (tile)][2 (half)][128]: what the halves of a row tell each other
   PfFwdBars& br = *reinterpret_cast<PfFwdBars*>(xch + 8 * kPfTile);
   static_assert(sizeof(PfFwdBars) <= 256, "barrier block");
-  volatile int* abort_flag = &br.abort_flag;
+  PfGiveUp* give_up = &br.give_up;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
   if (tid == 0) {
@@ -258,7 +278,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       mbar_init(&br.oready[w], 1);
     }
     mbar_init(&br.drain, 1);
-    br.abort_flag = 0;
+    br.give_up = {p.err, p.wait_cycles, 0};
     mbar_fence_init();
   }
   __syncwarp();
@@ -274,7 +294,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     bool ok = true;
     auto stage = [&](const CUtensorMap* map, const PrefillTensor& t, int row0, int h, int b) {
       const int s = i % NS;
-      ok = pf_wait(&br.empty[s], ((i / NS) & 1) ^ 1u, abort_flag);
+      ok = pf_wait(&br.empty[s], ((i / NS) & 1) ^ 1u, give_up);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) return;
       const uint32_t tx = pf_tile_tx<D>(t);
@@ -287,7 +307,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const int u = pf_unit(round, p.units);
       if (u < 0) break;
       const PfFwdUnit un = pf_fwd_unit(p, u);
-      ok = __all_sync(0xffffffffu, pf_wait(&br.qempty, (round & 1) ^ 1u, abort_flag));
+      ok = __all_sync(0xffffffffu, pf_wait(&br.qempty, (round & 1) ^ 1u, give_up));
       if (!ok) break;
       const int nq = un.blocks[1] > 0 ? 2 : 1;
       const uint32_t tx = pf_tile_tx<D>(p.q) * nq;
@@ -302,15 +322,13 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         if (ok) stage(&vmap, p.v, j * kPfTile, un.hk, un.b);
       }
     }
-    if (!ok) {  // no copy in flight may outlive the shared memory it targets
-      for (int s = 0; s < NS; ++s) {
-        const int cnt = i > s ? (i - 1 - s) / NS + 1 : 0;
-        const long long t0 = clock64();
-        while (cnt > 0 && !mbar_try_wait(&br.full[s], (cnt - 1) & 1) && clock64() - t0 < 1000000000ll) {}
-      }
-      const long long t0 = clock64();
-      while (last_unit >= 0 && !mbar_try_wait(&br.qfull, last_unit & 1) && clock64() - t0 < 1000000000ll) {}
+    // No copy in flight may outlive the shared memory it targets.  Usually every copy has been waited for by whoever uses it, but
+    // another role may have given up after this one issued its last.
+    for (int s = 0; s < NS; ++s) {
+      const int cnt = i > s ? (i - 1 - s) / NS + 1 : 0;
+      if (cnt > 0) pf_drain(&br.full[s], (cnt - 1) & 1);
     }
+    if (last_unit >= 0) pf_drain(&br.qfull, last_unit & 1);
   } else if (warp == kPfMmaWarp) {
     // ================================ MMA warp ================================
     // The whole warp walks the loop and one elected lane issues, so that addresses and descriptors are warp-uniform values:
@@ -325,18 +343,18 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       if (u < 0) break;
       const PfFwdUnit un = pf_fwd_unit(p, u);
       const int blocks = max(un.blocks[0], un.blocks[1]);
-      ok = __all_sync(0xffffffffu, pf_wait(&br.qfull, round & 1, abort_flag));
+      ok = __all_sync(0xffffffffu, pf_wait_unit(&br.qfull, round & 1, give_up, p.wait_cycles));
       // step j: P V of block j-1, then the scores of block j, for one tile and then the other
       for (int j = 0; ok && j <= blocks; ++j) {
         const int ik = base + 2 * j, iv = ik - 1;
         const int sk = ik % NS, sv = (iv + NS) % NS;
-        if (j < blocks) ok = pf_wait(&br.full[sk], (ik / NS) & 1, abort_flag);
-        if (ok && j > 0) ok = pf_wait(&br.full[sv], (iv / NS) & 1, abort_flag);
+        if (j < blocks) ok = pf_wait(&br.full[sk], (ik / NS) & 1, give_up);
+        if (ok && j > 0) ok = pf_wait(&br.full[sv], (iv / NS) & 1, give_up);
         ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
           if (ok && j > 0 && j - 1 < un.blocks[w]) {
-            ok = __all_sync(0xffffffffu, pf_wait(&br.pready[w], pc[w] & 1, abort_flag));
+            ok = __all_sync(0xffffffffu, pf_wait(&br.pready[w], pc[w] & 1, give_up));
             if (!ok) break;
             ++pc[w];
             tc_fence_after();
@@ -383,8 +401,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     }
     if (elect_one()) {
       mma_commit(&br.drain);
-      const long long t0 = clock64();
-      while (!mbar_try_wait(&br.drain, 0) && clock64() - t0 < 1000000000ll) {}
+      pf_drain(&br.drain, 0);
     }
     __syncwarp();
   } else {
@@ -431,7 +448,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
           turn_pass();
           continue;
         }
-        if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.sfull[wg], sn & 1, abort_flag));
+        if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.sfull[wg], sn & 1, give_up));
         ++sn;
         // In the diagonal block a warp's rows see nothing of the 32-key chunks after its own and, in its own, the keys up to
         // the row's position (keys beyond the prompt lie behind those).
@@ -559,7 +576,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       if (blocks == 0) continue;
       l += exchange(l);
       float inv = l > 0.f ? 1.f / l : 0.f, ls = __fadd_rn(__fmul_rn(m, sc), log2f(l));
-      if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.oready[wg], on & 1, abort_flag));
+      if (ok) ok = __all_sync(0xffffffffu, pf_wait(&br.oready[wg], on & 1, give_up));
       ++on;
       tc_fence_after();
       if (!ok) inv = ls = __int_as_float(0x7fffffff);
@@ -601,7 +618,7 @@ struct PfMassBars {
   uint64_t lfull[kPfLseSlots], lempty[kPfLseSlots];
   uint64_t drain;
   uint32_t tmem_base;
-  int abort_flag;
+  PfGiveUp give_up;
 };
 
 struct PfMassUnit {
@@ -631,7 +648,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   float* red = lse_s + kPfLseSlots * LS;                           // [2][3][128]: the sums of the warpgroups but the first
   PfMassBars& br = *reinterpret_cast<PfMassBars*>(red + 2 * 3 * kPfTile);
   static_assert(sizeof(PfMassBars) <= 448, "barrier block");
-  volatile int* abort_flag = &br.abort_flag;
+  PfGiveUp* give_up = &br.give_up;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int G = p.num_q_heads / p.num_kv_heads, n = p.tokens;
 
@@ -651,7 +668,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       mbar_init(&br.lempty[s], 4);
     }
     mbar_init(&br.drain, 1);
-    br.abort_flag = 0;
+    br.give_up = {p.err, p.wait_cycles, 0};
     mbar_fence_init();
   }
   __syncwarp();
@@ -669,7 +686,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const int u = pf_unit(round, p.units);
       if (u < 0) break;
       const PfMassUnit un = pf_mass_unit(p, u);
-      ok = __all_sync(0xffffffffu, pf_wait(&br.kempty, (round & 1) ^ 1u, abort_flag));
+      ok = __all_sync(0xffffffffu, pf_wait(&br.kempty, (round & 1) ^ 1u, give_up));
       if (!ok) break;
       const uint32_t ktx = pf_tile_tx<D>(p.k), qtx = pf_tile_tx<D>(p.q);
       if (ktx && lane == 0) mbar_expect_tx(&br.kfull, ktx);
@@ -689,13 +706,13 @@ __global__ void __launch_bounds__(kPfThreads, 1)
           nl[e] = q < n ? -lse[q] : -INFINITY;
         }
         const float w = p.head_w != nullptr ? p.head_w[(long long)un.b * p.num_q_heads + h] : 1.f;
-        ok = pf_wait(&br.empty[s], ((i / NS) & 1) ^ 1u, abort_flag);
+        ok = pf_wait(&br.empty[s], ((i / NS) & 1) ^ 1u, give_up);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (qtx && lane == 0) mbar_expect_tx(&br.full[s], qtx);
         pf_load_tile<D>(ring + s * TB, &qmap, p.q, qt * kPfTile, h, un.b, n, &br.full[s], lane);
         if (!qtx && lane == 0) mbar_arrive(&br.full[s]);
-        ok = __all_sync(0xffffffffu, pf_wait(&br.lempty[ls], ((i / kPfLseSlots) & 1) ^ 1u, abort_flag));
+        ok = __all_sync(0xffffffffu, pf_wait(&br.lempty[ls], ((i / kPfLseSlots) & 1) ^ 1u, give_up));
         if (!ok) {
           ++i;  // this stage's copy is in flight
           break;
@@ -711,15 +728,13 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         }
       }
     }
-    if (!ok) {  // no copy in flight may outlive the shared memory it targets
-      for (int s = 0; s < NS; ++s) {
-        const int cnt = i > s ? (i - 1 - s) / NS + 1 : 0;
-        const long long t0 = clock64();
-        while (cnt > 0 && !mbar_try_wait(&br.full[s], (cnt - 1) & 1) && clock64() - t0 < 1000000000ll) {}
-      }
-      const long long t0 = clock64();
-      while (last_unit >= 0 && !mbar_try_wait(&br.kfull, last_unit & 1) && clock64() - t0 < 1000000000ll) {}
+    // No copy in flight may outlive the shared memory it targets.  Usually every copy has been waited for by whoever uses it, but
+    // another role may have given up after this one issued its last.
+    for (int s = 0; s < NS; ++s) {
+      const int cnt = i > s ? (i - 1 - s) / NS + 1 : 0;
+      if (cnt > 0) pf_drain(&br.full[s], (cnt - 1) & 1);
     }
+    if (last_unit >= 0) pf_drain(&br.kfull, last_unit & 1);
   } else if (warp == kPfMmaWarp) {
     // ================================ MMA warp ================================
     int i = 0;
@@ -729,10 +744,10 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const int u = pf_unit(round, p.units);
       if (u < 0) break;
       const PfMassUnit un = pf_mass_unit(p, u);
-      ok = __all_sync(0xffffffffu, pf_wait(&br.kfull, round & 1, abort_flag));
+      ok = __all_sync(0xffffffffu, pf_wait_unit(&br.kfull, round & 1, give_up, p.wait_cycles));
       for (int j = 0; ok && j < un.count; ++j, ++i) {
         const int s = i % NS, a = i % kPfAcc;
-        ok = pf_wait(&br.full[s], (i / NS) & 1, abort_flag) && pf_wait(&br.sempty[a], ((i / kPfAcc) & 1) ^ 1u, abort_flag);
+        ok = pf_wait(&br.full[s], (i / NS) & 1, give_up) && pf_wait(&br.sempty[a], ((i / kPfAcc) & 1) ^ 1u, give_up);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -747,8 +762,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     }
     if (elect_one()) {
       mma_commit(&br.drain);
-      const long long t0 = clock64();
-      while (!mbar_try_wait(&br.drain, 0) && clock64() - t0 < 1000000000ll) {}
+      pf_drain(&br.drain, 0);
     }
     __syncwarp();
   } else {
@@ -767,7 +781,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       for (int j = (wg - i0) & 3; ok && j < un.count; j += kPfAcc) {
         const int i = i0 + j, a = i % kPfAcc, ls = i % kPfLseSlots;
         const bool diag = j % per_head == 0;
-        ok = pf_wait(&br.sfull[a], (i / kPfAcc) & 1, abort_flag) && pf_wait(&br.lfull[ls], (i / kPfLseSlots) & 1, abort_flag);
+        ok = pf_wait(&br.sfull[a], (i / kPfAcc) & 1, give_up) && pf_wait(&br.lfull[ls], (i / kPfLseSlots) & 1, give_up);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -903,10 +917,10 @@ static int launch_prefill(PrefillParams& p, bool want_mass, cudaStream_t st) {
 
 using namespace skv;
 
-extern "C" int skv_prefill_attention(const void* q, const void* k, const void* v, int dtype, int batch, int tokens,
-                                     int num_q_heads, int num_kv_heads, int head_dim, const int64_t* q_strides,
-                                     const int64_t* k_strides, const int64_t* v_strides, const float* head_weights,
-                                     void* out, float* lse, float* key_mass, void* stream) {
+extern "C" int skv_prefill_attention_checked(const void* q, const void* k, const void* v, int dtype, int batch, int tokens,
+                                             int num_q_heads, int num_kv_heads, int head_dim, const int64_t* q_strides,
+                                             const int64_t* k_strides, const int64_t* v_strides, const float* head_weights,
+                                             void* out, float* lse, float* key_mass, int32_t* err_flag, void* stream) {
   if (!q || !k || !v || !out || !lse || !q_strides || !k_strides || !v_strides) return SKV_ERR_INVALID;
   if (dtype != SKV_DTYPE_F16) return SKV_ERR_UNSUPPORTED;
   if (head_dim != 64 && head_dim != 128) return SKV_ERR_UNSUPPORTED;
@@ -932,6 +946,17 @@ extern "C" int skv_prefill_attention(const void* q, const void* k, const void* v
   p.num_kv_heads = num_kv_heads;
   p.tiles = (tokens + kPfTile - 1) / kPfTile;
   p.scale_log2 = 1.4426950408889634f / sqrtf((float)head_dim);
+  const unsigned polls = wait_polls();
+  p.wait_cycles = polls >= 1u << 24 ? 1u << 31 : polls >> 4 << 11;  // 128 cycles a poll, none below 16 polls
+  p.err = err_flag;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return head_dim == 64 ? launch_prefill<64>(p, key_mass != nullptr, st) : launch_prefill<128>(p, key_mass != nullptr, st);
+}
+
+extern "C" int skv_prefill_attention(const void* q, const void* k, const void* v, int dtype, int batch, int tokens,
+                                     int num_q_heads, int num_kv_heads, int head_dim, const int64_t* q_strides,
+                                     const int64_t* k_strides, const int64_t* v_strides, const float* head_weights,
+                                     void* out, float* lse, float* key_mass, void* stream) {
+  return skv_prefill_attention_checked(q, k, v, dtype, batch, tokens, num_q_heads, num_kv_heads, head_dim, q_strides, k_strides,
+                                       v_strides, head_weights, out, lse, key_mass, nullptr, stream);
 }

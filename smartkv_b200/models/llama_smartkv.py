@@ -189,7 +189,8 @@ class LlamaSmartKVAttention(nn.Module):
             # the prompt-pass kernel: attention output and per-key mass without the [B, Hq, n, n] probabilities
             from ..prefill import causal_prefill_attention
             w = cache.prefill_head_weights(q_len)
-            out, mass = causal_prefill_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), w)
+            out, mass = causal_prefill_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), w,
+                                                 error_flag=cache.store.err)
             attn_output = out.reshape(bsz, q_len, H * D)
             cache.prefill_layer(self.layer_idx, k.transpose(1, 2), v.transpose(1, 2), key_mass=mass)
         else:

@@ -208,3 +208,33 @@ def test_prefill_log_sum_exp_at_large_logits(hq, hkv, d, n, B):
     assert float(ref.abs().max()) > 256
     worst = ((lse.double() - ref).abs() - 2.0 ** -21) / ulp
     assert float(worst.max()) <= 0.5, float(worst.max())
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,B,layout", [(32, 8, 128, 700, 3, "token"), (3, 1, 64, 385, 2, "token"), (4, 2, 128, 300, 1, "rows")])
+def test_prefill_wait_that_runs_out_sets_the_error_flag(hq, hkv, d, n, B, layout):
+    """With the limit below one poll every role gives up on the first thing that is not ready yet: the launches return, the flag
+    is 1, what was owed is NaN, and the very next call in the stream, on the same shared and tensor memory, is right again."""
+    import ctypes
+    from smartkv_b200 import _lib
+    from smartkv_b200.prefill import causal_prefill_attention
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn((B, n, h, d), generator=g, device="cuda").half() for h in (hq, hkv, hkv))
+    if layout == "rows":
+        k = k[:, :1].expand(B, n, hkv, d)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    good = causal_prefill_attention(q, k, v, error_flag=err)
+    assert int(err) == 0
+    lib, value = _lib.lib(), ctypes.c_int32(0)
+    try:
+        assert lib.skv_set_wait_limit(1) == 0
+        out, mass = causal_prefill_attention(q, k, v, error_flag=err)
+        plain, _ = causal_prefill_attention(q, k, v)
+    finally:
+        assert lib.skv_set_wait_limit(1 << 24) == 0
+    again = causal_prefill_attention(q, k, v)
+    rc = lib.skv_read_error_flag(err.data_ptr(), ctypes.byref(value), torch.cuda.current_stream().cuda_stream)
+    assert value.value == 1 and b"timed out" in lib.skv_status_string(rc)
+    assert bool(out.isnan().any()) and bool(mass.isnan().any()) and bool(plain.isnan().any())
+    assert torch.equal(again[0], good[0]) and torch.equal(again[1], good[1])
+    with pytest.raises(ValueError):
+        causal_prefill_attention(q, k, v, error_flag=torch.zeros(1, dtype=torch.int32))
