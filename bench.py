@@ -50,7 +50,7 @@ CONFIGS = {
 }
 CFG = CONFIGS[1]
 FALLBACK_HBM_GBS = 6650.0
-# staging of the graphed reallocation: enough for one row-move launch over all 32 layers
+# staging of the graphed reallocation: a slot for every CTA of the row moves
 REALLOC_STAGING_BYTES = 4 << 30
 
 
@@ -419,9 +419,7 @@ def run_ours(args):
     reallocate()
     torch.cuda.synchronize()
     store.check_errors()
-    realloc_chunk, _ = store.repack_chunk(store.appended_total if args.no_graph else store.num_seqs * store.slots,
-                                          (1 << 30) if args.no_graph else REALLOC_STAGING_BYTES)
-    realloc_launches = 6 + -(-L // realloc_chunk)      # allocator, move plan, four per-token launches; row moves
+    realloc_launches = 7      # allocator, move plan, row moves, four per-token launches
 
     # ---- per-step inputs (resident) -----------------------------------------------------------
     gen.manual_seed(rank + 99)

@@ -412,10 +412,11 @@ int skv_repack_plan(const SkvStoreDesc* desc, const int32_t* counts, const uint8
  * quantised again at the new width, from the stored codes as the reference does (cache.py:819-844);
  * other rows are copied.  Every moved row passes through `staging`
  * (skv_requant_staging_bytes(desc, upper bound of the moves of all sequences, layers per call): a place for
- * every row, or one slot per concurrent worker for a sequence's moves, whichever is less);
- * if the staging buffer is too small for the moves found on the device nothing moves and
- * *err_flag = 6. */
+ * every row, or one slot per concurrent worker for a sequence's moves, whichever is less).  With less, down to one
+ * slot (skv_requant_min_staging_bytes), fewer rows are on their way at a time; if there is no room for the moves that
+ * one sequence has on the device nothing moves and *err_flag = 6. */
 int64_t skv_requant_staging_bytes(const SkvStoreDesc* desc, int64_t max_moves, int num_layers);
+int64_t skv_requant_min_staging_bytes(const SkvStoreDesc* desc, int64_t max_moves);
 int skv_requant_repack(const SkvStoreDesc* desc, void* store, int layer_begin, int layer_end,
                        const int32_t* move_src, const int32_t* move_dst, const int32_t* n_moves, void* staging,
                        int64_t staging_bytes, int32_t* err_flag, void* stream);

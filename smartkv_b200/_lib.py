@@ -108,6 +108,7 @@ _SIGNATURES = {
     "skv_repack_plan": (c_int, [POINTER(StoreDesc), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_void_p]),
     "skv_requant_staging_bytes": (c_int64, [POINTER(StoreDesc), c_int64, c_int]),
+    "skv_requant_min_staging_bytes": (c_int64, [POINTER(StoreDesc), c_int64]),
     "skv_requant_repack": (c_int, [POINTER(StoreDesc), c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_int64, c_void_p, c_void_p]),
     "skv_repack_meta_staging_bytes": (c_int64, [POINTER(StoreDesc), c_int64]),

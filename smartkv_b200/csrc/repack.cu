@@ -17,7 +17,7 @@
 //   skv_requant_repack  per layer range: all moved rows -> staging (requantised where the
 //                       width changed), then staging -> destination, so that every read of the
 //                       old layout precedes every write of the new one.  Rows of different
-//                       (layer, sequence, KV head) never touch, so one cluster of CTAs takes one
+//                       (layer, sequence, KV head) never touch, so one CTA or a cluster takes one
 //                       of those at a time and its own barrier is the only order needed.
 //   skv_repack_meta     the per-token arrays kept in storage order follow the same moves.
 #include <cooperative_groups.h>
@@ -210,14 +210,19 @@ __device__ __forceinline__ int find_seq(const int* s_prefix, int B, int m) {
   return lo;
 }
 
-// Clusters that work at once at most, two CTAs of 512 threads per SM of a B200; the staging buffer is divided among them.
+// CTAs that work at once, two of 512 threads per SM of a B200.
 constexpr int kRowThreads = 512;
-constexpr int kRowSlots = 296;
+constexpr int kRowCtas = 296;
 constexpr int kRowBatch = 4;  // row groups whose loads a warp has in flight
 
 // One item = the moves of one (layer, KV head, sequence).  Phase 0 reads the source rows, requantises where the width changes
 // and leaves every lane's packed field and the scale in staging; after the cluster's barrier phase 1 writes the
 // destinations.  Staging is written and read back by the same few CTAs, so it lives in L2.
+//
+// The staging buffer is divided among the workers that have an item in hand, by the moves there are and not by the moves there could be.
+// A worker is a single CTA, or a cluster where that ends sooner: where there are fewer items than CTAs, or room for few slots.  So a
+// buffer sized by a budget serves all layers in one launch: what it limits is how many items are in hand at once.  With a launch per as many layers as the worst case allows, 1 x 131072 tokens, 32 layers, 8 heads with 1 GiB
+// took 4377 us a reallocation, now 2720 us.
 //
 // What bounds it: the rows are scattered pieces of 32 to 128 bytes, so the memory system needs many of them in flight
 // (a warp issues the loads of kRowBatch groups of rows first), and the quantiser's instructions.  As two grid-wide kernels per
@@ -247,28 +252,37 @@ __global__ void __launch_bounds__(kRowThreads, 2) repack_rows_kernel(const __gri
   __syncthreads();
   const int longest = s_max, Hkv = g.num_kv_heads, nl = p.layer_end - p.layer_begin;
   if (longest == 0) return;
-  // staging: a slot of `longest` moves per cluster, or, if the buffer was sized for few moves, a place for every row
-  const bool slots = (long long)longest * 2 * kRowSlots <= p.staging_rows;
-  if (!slots && (long long)total * nl * Hkv * 2 > p.staging_rows) {
+  const int items = nl * Hkv * B;  // the host has checked that it fits
+  // a place for every row, or else a slot of `longest` moves for each worker; the same decisions in every CTA
+  const bool places = (long long)total * nl * Hkv * 2 <= p.staging_rows;
+  const long long room = p.staging_rows / (2ll * longest);
+  if (!places && room == 0) {
     if (threadIdx.x == 0 && blockIdx.x == 0 && p.err) atomicExch(p.err, 6);  // staging too small: nothing moves
     return;
   }
+  auto workers_of = [&](int n) -> int {
+    const int w = items < n ? items : n;
+    return places || w < room ? w : (int)room;
+  };
+  auto turns_of = [&](int n) -> int { return (items - 1) / n + 1; };
+  const bool share = CS > 1 && turns_of(workers_of((int)gridDim.x / CS)) < CS * turns_of(workers_of((int)gridDim.x));
+  const int per = share ? CS : 1, workers = workers_of((int)gridDim.x / per), worker = (int)blockIdx.x / per;
+  if (worker >= workers) return;  // the whole cluster, where one shares
+  const bool slots = room >= workers;
   const int lane = threadIdx.x & 31, l = lane & (LPR - 1), which = (lane / LPR) & 1, sub = lane / (2 * LPR);
-  const int rank = CS == 1 ? 0 : (int)(blockIdx.x % CS), cluster = (int)blockIdx.x / CS, clusters = (int)gridDim.x / CS;
-  const int cw = rank * (kRowThreads / 32) + (threadIdx.x >> 5), cwarps = CS * (kRowThreads / 32);
-  const long long items = (long long)nl * Hkv * B;
+  const int cw = ((int)blockIdx.x % per) * (kRowThreads / 32) + (threadIdx.x >> 5), cwarps = per * (kRowThreads / 32);
   auto sync = [&] {
-    if constexpr (CS == 1) __syncthreads();
+    if (CS == 1 || !share) __syncthreads();
     else cg::this_cluster().sync();
   };
-  for (long long it = cluster; it < items; it += clusters) {
-    const int seq = (int)(it % B), lh = (int)(it / B), li = lh / Hkv, h = lh - li * Hkv;
+  for (int it = worker; it < items; it += workers) {
+    const int lh = it / B, seq = it - lh * B, li = lh / Hkv, h = lh - li * Hkv;
     const int moves = s_prefix[seq + 1] - s_prefix[seq];
-    if (moves == 0) continue;  // the same for the whole cluster
+    if (moves == 0) continue;  // the same for the whole worker
     uint8_t* arena = arena_ptr(g, p.store, p.layer_begin + li, seq);
     const int32_t* msrc = p.move_src + (long long)seq * g.slots;
     const int32_t* mdst = p.move_dst + (long long)seq * g.slots;
-    uint8_t* stage = p.staging + (slots ? (long long)cluster * longest * 2 : ((long long)lh * total + s_prefix[seq]) * 2) * kStageRowBytes +
+    uint8_t* stage = p.staging + (slots ? (long long)worker * longest * 2 : ((long long)lh * total + s_prefix[seq]) * 2) * kStageRowBytes +
                      which * kStageRowBytes;
     if (threadIdx.x < 3 * kNumBuckets) {
       const int what = threadIdx.x / kNumBuckets, b = threadIdx.x % kNumBuckets;
@@ -376,9 +390,20 @@ __global__ void __launch_bounds__(kRowThreads, 2) repack_rows_kernel(const __gri
   }
 }
 
+// CTAs that share an item (up to 8, the portable cluster size): enough to keep them all busy when there are few items, or when the
+// staging buffer has room for few slots of the most moves there can be.
+static int row_cluster(long long items, long long room) {
+  int cs = items * 2 > kRowCtas ? 1 : items * 4 > kRowCtas ? 2 : items * 8 > kRowCtas ? 4 : 8;
+  while (cs < 8 && room < (items < kRowCtas / cs ? items : kRowCtas / cs)) cs *= 2;
+  return cs;
+}
+
 template <int D, int CS>
 static cudaError_t launch_rows(const RowMoveParams& p, long long items, cudaStream_t st) {
-  const long long clusters = items < kRowSlots / CS ? items : kRowSlots / CS;
+  // No more clusters than run at once (items are dealt in advance, so a second wave would wait for the first: 1554 instead of 1162 us
+  // for the rows of 1 x 131072 tokens in 32 layers): a cluster lies in one GPC, so 71 of 4 CTAs and 33 of 8 do.
+  constexpr long long fit = CS <= 2 ? kRowCtas / CS : 256 / CS;
+  const long long clusters = items < fit ? items : fit;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clusters * CS));
   cfg.blockDim = dim3(kRowThreads);
@@ -510,10 +535,15 @@ extern "C" int skv_repack_plan(const SkvStoreDesc* desc, const int32_t* counts, 
 
 extern "C" int64_t skv_requant_staging_bytes(const SkvStoreDesc* desc, int64_t max_moves, int num_layers) {
   if (!desc || max_moves < 0 || num_layers <= 0) return SKV_ERR_INVALID;
-  // a place for every row, or one slot per cluster for the moves of one sequence, whichever is less
+  // a place for every row, or one slot per CTA for the moves of one sequence, whichever is less
   const int64_t rows = max_moves * num_layers * desc->num_kv_heads * 2;
-  const int64_t slots = (max_moves < desc->slots ? max_moves : (int64_t)desc->slots) * 2 * kRowSlots;
+  const int64_t slots = (max_moves < desc->slots ? max_moves : (int64_t)desc->slots) * 2 * kRowCtas;
   return (rows < slots ? rows : slots) * (int64_t)kStageRowBytes;
+}
+
+extern "C" int64_t skv_requant_min_staging_bytes(const SkvStoreDesc* desc, int64_t max_moves) {
+  if (!desc || max_moves < 0) return SKV_ERR_INVALID;
+  return (max_moves < desc->slots ? max_moves : (int64_t)desc->slots) * 2 * kStageRowBytes;
 }
 
 extern "C" int skv_requant_repack(const SkvStoreDesc* desc, void* store, int layer_begin, int layer_end,
@@ -536,9 +566,9 @@ extern "C" int skv_requant_repack(const SkvStoreDesc* desc, void* store, int lay
   p.err = err_flag;
   if (desc->slots >= (1 << 30)) return SKV_ERR_UNSUPPORTED;  // row_place
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Few items (a small store, one sequence): up to 8 CTAs, the portable cluster size, share each.
   const long long items = (long long)(layer_end - layer_begin) * desc->num_kv_heads * desc->num_seqs;
-  const int cs = items * 2 > kRowSlots ? 1 : items * 4 > kRowSlots ? 2 : items * 8 > kRowSlots ? 4 : 8;
+  if (items > (1 << 30)) return SKV_ERR_UNSUPPORTED;
+  const int cs = row_cluster(items, p.staging_rows / (2ll * desc->slots));
   const bool d128 = desc->head_dim == 128;
   const cudaError_t rc = cs == 1   ? (d128 ? launch_rows<128, 1>(p, items, st) : launch_rows<64, 1>(p, items, st))
                          : cs == 2 ? (d128 ? launch_rows<128, 2>(p, items, st) : launch_rows<64, 2>(p, items, st))

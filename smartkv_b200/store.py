@@ -614,15 +614,12 @@ class PackedKVStore:
                                       self._stream()), "skv_alloc_bits")
         return r["new_bits"], r["new_counts"], r["changed"]
 
-    def repack_chunk(self, max_moves: int, staging_budget: int) -> Tuple[int, int]:
-        """(layers per row-move launch, staging bytes): all layers at once where the budget holds the staging for up
-        to ``max_moves`` moves, otherwise fewer at a time, at least one."""
-        chunk = self.num_layers
-        need = int(self.lib.skv_requant_staging_bytes(ctypes.byref(self.desc), max_moves, chunk))
-        while need > staging_budget and chunk > 1:
-            chunk = (chunk + 1) // 2
-            need = int(self.lib.skv_requant_staging_bytes(ctypes.byref(self.desc), max_moves, chunk))
-        return chunk, need
+    def repack_staging_bytes(self, max_moves: int, staging_budget: int) -> int:
+        """Staging for up to ``max_moves`` moved rows per layer and head: within the budget, but never less than the moves of
+        one sequence need."""
+        d = ctypes.byref(self.desc)
+        return max(min(int(self.lib.skv_requant_staging_bytes(d, max_moves, self.num_layers)), int(staging_budget)),
+                   int(self.lib.skv_requant_min_staging_bytes(d, max_moves)))
 
     def repack(self, new_bits: torch.Tensor, max_moves: Optional[int] = None, staging_budget: int = 1 << 30):
         """Moves every token to the bucket of its new width (requantising from the stored codes)
@@ -637,17 +634,15 @@ class PackedKVStore:
         if max_moves is None:
             max_moves = self.appended_total
         max_moves = max(int(max_moves), 1)
-        chunk, need = self.repack_chunk(max_moves, staging_budget)
+        need = self.repack_staging_bytes(max_moves, staging_budget)
         if r["staging"] is None or r["staging"].numel() < need:
             r["staging"] = torch.empty(need, dtype=torch.uint8, device=self.device)
         mneed = int(self.lib.skv_repack_meta_staging_bytes(d, max_moves + 8))
         if r["meta_staging"] is None or r["meta_staging"].numel() < mneed:
             r["meta_staging"] = torch.empty(mneed, dtype=torch.uint8, device=self.device)
-        for l0 in range(0, self.num_layers, chunk):
-            l1 = min(self.num_layers, l0 + chunk)
-            check(self.lib.skv_requant_repack(d, ptr(self.arena), l0, l1, ptr(r["move_src"]), ptr(r["move_dst"]),
-                                              ptr(r["n_moves"]), ptr(r["staging"]), r["staging"].numel(), ptr(self.err),
-                                              st), "skv_requant_repack")
+        check(self.lib.skv_requant_repack(d, ptr(self.arena), 0, self.num_layers, ptr(r["move_src"]), ptr(r["move_dst"]),
+                                          ptr(r["n_moves"]), ptr(r["staging"]), r["staging"].numel(), ptr(self.err), st),
+              "skv_requant_repack")
         check(self.lib.skv_repack_meta(d, ptr(r["move_src"]), ptr(r["move_dst"]), ptr(r["n_moves"]), ptr(self.counts),
                                        ptr(r["counts_new"]), ptr(self.slot_token), ptr(self.cumulative),
                                        ptr(self.rank_pct), ptr(self.rank_streak), ptr(self.layer_ema), ptr(self.touched),
@@ -665,7 +660,7 @@ class PackedKVStore:
         one by one costs more than running them once the allocation has settled.  The first call runs eagerly
         (it sizes every buffer for the store's whole capacity, so that the captured launches stay valid as the
         cache grows) and captures the graph; later calls replay it.  ``cfg`` must be the same at every call.
-        ``staging_budget`` bytes of staging decide how many layers one row-move launch covers (repack_chunk)."""
+        ``staging_budget`` bytes of staging decide how many rows are moved at a time (repack_staging_bytes)."""
         self.flush_importance()
         cap_moves = self.num_seqs * self.slots
         if getattr(self, "_realloc_graph", None) is None:

@@ -319,3 +319,60 @@ def test_row_moves_for_every_cluster_size(L, hkv, B, d, n):
                         if w1 != w0:
                             c, s = orc.requantize_rows(c, s, w1)
                         assert np.array_equal(codes[sel], c) and np.array_equal(scales[sel].view(np.uint32), s.view(np.uint32)), (b, l, w0, w1)
+
+
+# one slot, three, and one for every CTA but not a place for every row; items that make single CTAs and clusters the workers
+@pytest.mark.parametrize("L,hkv,B,d,n,slots", [(4, 8, 5, 128, 70, 1), (4, 8, 12, 64, 90, 3), (2, 4, 5, 64, 150, 3), (1, 1, 3, 128, 700, 1),
+                                               (4, 8, 12, 64, 40, 296), (1, 4, 2, 128, 300, 5)])
+def test_row_moves_with_little_staging(L, hkv, B, d, n, slots):
+    """Staging for a few slots of the moves there are, many fewer than there could be: the arenas end as with staging for
+    everything.  A byte less than one slot and nothing moves."""
+    import ctypes
+    from smartkv_b200 import _lib
+    rng = np.random.default_rng(L * hkv * B + slots)
+    kvs = [tuple(x.reshape(B, n, hkv, d) for x in orc.synth_kv(B * n, hkv, d, seed=70 + l)) for l in range(L)]
+    bits0 = rng.choice((2, 3, 4, 8), size=(B, n))
+    bits1 = np.where(rng.random((B, n)) < 0.3, rng.choice((2, 3, 4, 8), size=(B, n)), bits0)
+    stores = [make_store(L, B, hkv, d, hkv, n) for _ in range(2)]
+    for s in stores:
+        fill_store(s, kvs, bits0)
+    tok = stores[0].slot_token.long()
+    new_bits = torch.where(tok >= 0, torch.from_numpy(bits1).cuda().gather(1, tok.clamp(min=0)), torch.zeros_like(tok)).to(torch.uint8)
+    stores[0].repack(new_bits)
+    stores[0].check_errors()
+    store, before = stores[1], stores[1].arena.clone()
+    r, lib, desc, p = store._realloc_buffers(), store.lib, ctypes.byref(store.desc), _lib.ptr
+    _lib.check(lib.skv_repack_plan(desc, p(store.counts), p(new_bits), p(r["move_src"]), p(r["move_dst"]), p(r["n_moves"]), p(r["counts_new"]),
+                                   p(r["plan_ws"]), p(store.err), store._stream()))
+    slot = int(lib.skv_requant_min_staging_bytes(desc, int(r["n_moves"].max())))
+    staging = torch.empty(slots * slot, dtype=torch.uint8, device="cuda")
+    move = lambda size: _lib.check(lib.skv_requant_repack(desc, p(store.arena), 0, L, p(r["move_src"]), p(r["move_dst"]), p(r["n_moves"]),
+                                                          p(staging), size, p(store.err), store._stream()))
+    move(slot - 1)
+    with pytest.raises(_lib.SmartKVLibraryError):
+        store.check_errors()
+    assert torch.equal(store.arena, before)
+    move(slots * slot)
+    store.check_errors()
+    assert torch.equal(store.arena, stores[0].arena)
+
+
+def test_reallocation_within_a_staging_budget():
+    """A budget far below the worst case holds; the state is that of a reallocation with staging for everything."""
+    rng = np.random.default_rng(4)
+    B, hq, hkv, d, n, L = 2, 8, 2, 64, 900, 3
+    stores = [make_store(L, B, hkv, d, hq, n) for _ in range(2)]
+    kvs = [tuple(x.reshape(B, n, hkv, d) for x in orc.synth_kv(B * n, hkv, d, seed=500 + l)) for l in range(L)]
+    bits0 = rng.choice((2, 3, 4, 8), size=(B, n))
+    imp = [_random_importance(rng, n, b) for b in range(B)]
+    budget = 1 << 20
+    for s, size in zip(stores, (1 << 30, budget)):
+        fill_store(s, kvs, bits0)
+        for b in range(B):
+            _scatter_scores(s, b, imp[b])
+        s.reallocate_graphed(s.make_alloc_config(0.35), staging_budget=size)
+        s.check_errors()
+    a, b = stores
+    least = int(b.lib.skv_requant_min_staging_bytes(b.desc, B * b.slots))
+    assert b._realloc["staging"].numel() == max(budget, least) < a._realloc["staging"].numel()
+    assert torch.equal(a.arena, b.arena) and torch.equal(a.counts, b.counts) and torch.equal(a.slot_token, b.slot_token)
