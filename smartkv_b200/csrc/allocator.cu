@@ -689,13 +689,20 @@ extern "C" int skv_alloc_bits(const SkvStoreDesc* desc, const SkvAllocConfig* cf
   p.changed = changed;
   carve(p.w, workspace, NT);
 
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return SKV_ERR_CUDA;
-  // CTAs per sequence: one per 4096 storage indices (about a thousand live tokens: a couple per thread) as long as all
-  // sequences' clusters run at once, and at most 8, the portable cluster size.
+  // CTAs per sequence: one per 4096 storage indices (about a thousand live tokens: a couple per thread) as long as all sequences'
+  // clusters run at once.  A cluster lies in one GPC and a CTA fills an SM's registers, so 74 clusters of 2, 33 of 4, 15 of 8 and
+  // 7 of 16 do: 16 x 8192 tokens take 403 us with clusters of 8, in two waves, and 290 with clusters of 4.  Beyond 8, the portable
+  // size, one sequence of 131072 tokens takes 864 instead of 1548 us (1425 with the device-wide sorts before the clusters).
   int cs = 1;
-  while (cs < 8 && (long long)cs * 4096 < T && 2LL * cs * B <= sms) cs *= 2;
+  if (T > 4096 && B <= 74) cs = 2;
+  if (T > 2 * 4096 && B <= 33) cs = 4;
+  if (T > 4 * 4096 && B <= 15) cs = 8;
+  if (T > 8 * 4096 && B <= 7) {
+    if (cudaFuncSetAttribute(alloc_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        launch_alloc<16>(p, B, st) == SKV_OK)
+      return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
+    cudaGetLastError();  // such clusters are not to be had here
+  }
   const int rc = cs == 1 ? launch_alloc<1>(p, B, st) : cs == 2 ? launch_alloc<2>(p, B, st)
                : cs == 4 ? launch_alloc<4>(p, B, st) : launch_alloc<8>(p, B, st);
   if (rc != SKV_OK) return rc;

@@ -260,7 +260,7 @@ def test_reallocate_graphed_equals_eager():
 
 @pytest.mark.parametrize("n_list", [[1100, 3], [9000], [2100, 1, 2000]])
 def test_allocator_clusters_of_every_size(n_list):
-    """Capacities that give a sequence clusters of 2, 8 and 4 CTAs (the other tests: 1 and 4), three calls with state."""
+    """Capacities that give a sequence clusters of 2, 16 and 4 CTAs (the other tests: 1 and 4), three calls with state."""
     rng = np.random.default_rng(n_list[0])
     h, d, beta = 8, 128, 0.35
     store = _alloc_store(n_list, h, d, init_bits_seed=3)
@@ -376,3 +376,15 @@ def test_reallocation_within_a_staging_budget():
     least = int(b.lib.skv_requant_min_staging_bytes(b.desc, B * b.slots))
     assert b._realloc["staging"].numel() == max(budget, least) < a._realloc["staging"].numel()
     assert torch.equal(a.arena, b.arena) and torch.equal(a.counts, b.counts) and torch.equal(a.slot_token, b.slot_token)
+
+
+# clusters of 8 and 16 by capacity; then, from two capacities, one sequence more than the clusters of 16 (8), 8 (4) and 4 (2) there is room for
+@pytest.mark.parametrize("n_list", [[5000], [9000, 8500], [8300] + [40] * 6, [8300] + [40] * 7, [4300] + [30] * 15, [2100] + [20] * 33])
+def test_allocator_clusters_by_the_number_of_sequences(n_list):
+    test_allocator_clusters_of_every_size(n_list)
+
+
+def test_allocator_of_a_long_sequence():
+    """One sequence of 40000 tokens: every thread of the largest cluster has several items, the digits of the token ids reach three
+    bytes."""
+    test_allocator_clusters_of_every_size([40000])
