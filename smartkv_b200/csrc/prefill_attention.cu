@@ -19,22 +19,24 @@
 //
 // Both kernels are persistent, one CTA per SM: four softmax warpgroups, one loading warp, one warp that issues the MMAs.
 // A warp's own work is a chain (wait, read S, maximum, exponentials, write P), so it takes four warps per scheduler to
-// keep the exponential unit busy: with two, each thread owning a whole row, it was 44 % busy in pass 1 (651 us at 8192 tokens,
-// 577 us now, 51 %) and 76 % in pass 2 (389 and 357 us, 86 %).  One warp issues the MMAs of both tiles in turn; with
-// one per tile both wait for the tensor core and then both for the exponential unit (792 us), and 64-key blocks with
-// scores two blocks ahead end up in the same lockstep (770 us).  Part of the exponentials as a polynomial on the
-// multiply-add pipe costs more issue time than it saves (10 to 20 % slower).
+// keep the exponential unit busy.  While O was still rescaled only when a maximum had grown by 2^8, at 8192 tokens: with two warps,
+// each thread owning a whole row, the unit was 44 % busy in pass 1 (651 us) and 76 % in pass 2 (389 us), with four 51 %
+// (577 us) and 86 % (357 us).  One warp issues the MMAs of both tiles in turn; in those
+// builds, with one per tile both waited for the tensor core and then both for the exponential unit (pass 1 792 us), and 64-key
+// blocks with scores two blocks ahead ended up in the same lockstep (770 us).  Part of the exponentials as a polynomial on
+// the multiply-add pipe costs more issue time than it saves (10 to 20 % slower).
 // Pass 1 gives each pair of warpgroups its own 128-query tile, 64 keys to a thread, so that one pair computes exponentials
 // while the tensor core works for the other: two query heads of one KV head at the same positions where the group is
 // even (they share every K and V tile and have the same causal range), otherwise two neighbouring query tiles of one
 // head.  Pass 2 hands the query tiles of the stream to the warpgroups in turn, each with its own accumulator.  Units of
 // work are dealt longest first, back and forth over the CTAs, because a causal unit's length is proportional to its position.
 //
-// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 991 us (4315 us with 64 x 64 tiles on
-// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 65 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
-// head_dim 128: 77 us (289 us).
+// Both passes together, B200: one sequence of 8192 tokens, 32 / 8 heads, head_dim 128: 1004 us (4315 us with 64 x 64 tiles on
+// mma.sync); 8 x 512 tokens, 32 / 4 heads, head_dim 64: 64 us (223 us).  Pass 1 alone, 3 x 1391 tokens, 32 / 8 heads,
+// head_dim 128: 78 us (289 us).
 #include <cuda_fp16.h>
 
+#include "f32x2.cuh"
 #include "tc05.cuh"
 
 namespace skv {
@@ -83,26 +85,6 @@ __device__ __forceinline__ uint32_t pf_pack_half2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// two fp32 operations per instruction
-__device__ __forceinline__ uint64_t pf_pair(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void pf_unpair(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t pf_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t pf_add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // max(a, b, c); a NaN loses against a number, as in fmaxf
 __device__ __forceinline__ float pf_max3(float a, float b, float c) {
   float r;
@@ -110,9 +92,8 @@ __device__ __forceinline__ float pf_max3(float a, float b, float c) {
   return r;
 }
 __device__ __forceinline__ uint64_t pf_exp2_pair(uint64_t x2) {
-  float x0, x1;
-  pf_unpair(x2, x0, x1);
-  return pf_pair(pf_exp2(x0), pf_exp2(x1));
+  const float2 x = f32x2_parts(x2);
+  return f32x2(pf_exp2(x.x), pf_exp2(x.y));
 }
 
 // Bounded wait: the thread is suspended inside try_wait; after the limit, or once another role gave up, it returns false.  A CTA that
@@ -410,7 +391,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     const uint32_t lanes = (uint32_t)(wq * 32) << 16;
     const uint32_t ts = tmem + wg * 128 + lanes, to = tmem + 256 + wg * D + half * (D / 2) + lanes;
     const float sc = p.scale_log2;
-    const uint64_t sc2 = pf_pair(sc, sc);
+    const uint64_t sc2 = f32x2(sc, sc);
     const int n = p.tokens;
     int sn = 0, on = 0, xp = 0;  // score tiles / outputs received so far; parity of the exchange buffer
     bool ok = true;
@@ -424,7 +405,8 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       return x[(half ^ 1) * kPfTile];
     };
     // The two tiles compute their exponentials in turn (tile 0 first): left alone they drift into step, both at the
-    // exponential unit and then both waiting for the tensor core (both passes 899 us at 8192 tokens, 866 us with the turns).
+    // exponential unit and then both waiting for the tensor core (both passes at 8192 tokens, together with the MMA warp's uniform
+    // addresses and while O was rescaled at 2^8: 985 us, 949 with the turns).
     // Each turn is one pass of both through two named barriers, the same number for both tiles whatever they have to do.
     auto turn_wait = [&] {
       if (wg == 0) asm volatile("bar.sync 3, 512;" ::: "memory");
@@ -510,7 +492,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
           m = bm;
         } else {
           // O is rescaled whenever a row's maximum grows, however little.  Waiting until it has grown by 2^8 is 4 % faster
-          // (949 against 991 us, both passes at 8192 tokens), but then the row's largest P is no longer exactly 1, and its
+          // (949 against 991 us when it was changed, both passes at 8192 tokens), but then the row's largest P is no longer exactly 1, and its
           // rounding to fp16 (it is the weight that counts) makes the output's error against 64 bits 10 % larger.  Both
           // halves of a row decide alike; the round trip of O mostly fits in the wait for the turn.
           const bool need = bm > m;
@@ -533,7 +515,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         }
         turn_wait();
         const float msc = m == -INFINITY ? 0.f : __fmul_rn(m, sc);
-        const uint64_t nm2 = pf_pair(-msc, -msc);
+        const uint64_t nm2 = f32x2(-msc, -msc);
         uint64_t l2a = 0, l2b = 0;
         // P of a half lies over that half's own S columns, of which the ones written have been read.
         auto piece_exp = [&](const uint32_t (&s)[16], bool seen, uint32_t to_col) {
@@ -544,13 +526,12 @@ __global__ void __launch_bounds__(kPfThreads, 1)
               pk[e] = 0u;
               continue;
             }
-            const uint64_t x2 = pf_fma2(pf_pair(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), sc2, nm2);
+            const uint64_t x2 = f32x2_fma(f32x2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), sc2, nm2);
             const uint64_t p2 = pf_exp2_pair(x2);
-            if (e & 1) l2b = pf_add2(l2b, p2);
-            else l2a = pf_add2(l2a, p2);
-            float x0, x1;
-            pf_unpair(p2, x0, x1);
-            pk[e] = pf_pack_half2(x0, x1);
+            if (e & 1) l2b = f32x2_add(l2b, p2);
+            else l2a = f32x2_add(l2a, p2);
+            const float2 x = f32x2_parts(p2);
+            pk[e] = pf_pack_half2(x.x, x.y);
           }
           tmem_st8(to_col, pk);
         };
@@ -565,9 +546,8 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         if (own == 1) mask_own(s0, 16);
         piece_exp(s0, own >= 1, th + 24);
         turn_pass();
-        float la, lb;
-        pf_unpair(pf_add2(l2a, l2b), la, lb);
-        l += la + lb;
+        const float2 l2 = f32x2_parts(f32x2_add(l2a, l2b));
+        l += l2.x + l2.y;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -769,7 +749,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     // ================================ four warpgroups: one key row per thread ================================
     const int wg = warp >> 2, wq = warp & 3, wt = tid & 127;
     const uint32_t lanes = (uint32_t)(wq * 32) << 16;
-    const uint64_t sc2 = pf_pair(p.scale_log2, p.scale_log2);
+    const uint64_t sc2 = f32x2(p.scale_log2, p.scale_log2);
     int i0 = 0;  // stream index of the unit's first query tile
     bool ok = true;
     for (int round = 0;; ++round) {
@@ -789,10 +769,10 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         uint64_t t0 = 0, t1 = 0;
         const uint32_t ta0 = tmem + a * 128 + lanes;
         auto add4 = [&](float4 q4, uint32_t sa, uint32_t sb, uint32_t sc, uint32_t sd) {
-          const uint64_t xa = pf_fma2(pf_pair(__uint_as_float(sa), __uint_as_float(sb)), sc2, pf_pair(q4.x, q4.y));
-          const uint64_t xb = pf_fma2(pf_pair(__uint_as_float(sc), __uint_as_float(sd)), sc2, pf_pair(q4.z, q4.w));
-          t0 = pf_add2(t0, pf_exp2_pair(xa));
-          t1 = pf_add2(t1, pf_exp2_pair(xb));
+          const uint64_t xa = f32x2_fma(f32x2(__uint_as_float(sa), __uint_as_float(sb)), sc2, f32x2(q4.x, q4.y));
+          const uint64_t xb = f32x2_fma(f32x2(__uint_as_float(sc), __uint_as_float(sd)), sc2, f32x2(q4.z, q4.w));
+          t0 = f32x2_add(t0, pf_exp2_pair(xa));
+          t1 = f32x2_add(t1, pf_exp2_pair(xb));
         };
         auto chunk_sum = [&](int c, uint32_t (&s)[32]) {
           if (!diag || c > wq) {
@@ -832,9 +812,8 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&br.sempty[a]);
         chunk_sum(3, s1);
-        float ta, tb;
-        pf_unpair(pf_add2(t0, t1), ta, tb);
-        acc = fmaf(nl[128], ta + tb, acc);
+        const float2 t2 = f32x2_parts(f32x2_add(t0, t1));
+        acc = fmaf(nl[128], t2.x + t2.y, acc);
         __syncwarp();
         if (lane == 0) mbar_arrive(&br.lempty[ls]);
       }

@@ -3,6 +3,7 @@
 // slower (22 layers of a small model: 429 against 417 us) without any of them using it.
 #pragma once
 
+#include "f32x2.cuh"
 #include "quant_row.cuh"
 
 namespace skv {
@@ -18,32 +19,6 @@ namespace skv {
 //     per lane (a NaN does not pass either).
 //   * codes are joined as a polynomial in 2^bits, whose values stay below 2^17 and are therefore exact.
 constexpr float kRoundMagic = 12582912.f;  // 1.5 * 2^23 = 0x4B400000
-
-__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 f32x2_parts(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 
 // What the arithmetic needs to know about a bucket's width, one constant load each instead of a chain of selects.
 struct WidthConst {

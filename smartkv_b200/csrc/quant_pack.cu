@@ -26,8 +26,8 @@ __global__ void quantize_pack_append_kernel(const AppendParams p) {
 // (token, KV head) go through the same instructions side by side, NPASS groups of them in flight per warp.
 //
 // What bounds it is issue slots: with a row per warp, 282 warp instructions a row, 16 x 8192 x 8 rows of head_dim 128
-// took 634 us for 0.72 GB; now 273 us (quantize8; 64 registers, so that 32 warps fit an SM: 303 us with 24).  One or two
-// groups in flight per warp instead of four: 285 us and more.
+// took 638 us for 0.72 GB; now 260 us (quantize8; 64 registers, so that 32 warps fit an SM: a ninth slower with 24).  One or two
+// groups in flight per warp instead of four: a twentieth slower and more.
 template <int D, bool HALF, int NPASS>
 __global__ void __launch_bounds__(256, 4) append_bulk_kernel(const AppendParams p) {
   constexpr int LPR = D / 8;               // lanes per row

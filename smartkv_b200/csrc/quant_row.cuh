@@ -155,21 +155,4 @@ __device__ __forceinline__ void pack_store_row(const int (&code)[EPL], int bits,
   }
 }
 
-// Reads this lane's EPL codes (element index = lane*EPL + i) out of a packed row.
-template <int EPL>
-__device__ __forceinline__ void unpack_row(const uint8_t* src, int bits, int lane, int (&code)[EPL]) {
-#pragma unroll
-  for (int i = 0; i < EPL; ++i) {
-    const int e = lane * EPL + i;
-    if (bits == 8) {
-      code[i] = (int)(int8_t)src[e];
-    } else {
-      const int bitpos = e * bits, byte = bitpos >> 3, sh = bitpos & 7;
-      uint32_t win = src[byte];
-      if (sh + bits > 8) win |= (uint32_t)src[byte + 1] << 8;
-      code[i] = (int)((win >> sh) & ((1u << bits) - 1u)) - (1 << (bits - 1));
-    }
-  }
-}
-
 }  // namespace skv

@@ -210,7 +210,7 @@ __device__ __forceinline__ int find_seq(const int* s_prefix, int B, int m) {
   return lo;
 }
 
-// CTAs that work at once, two of 512 threads per SM of a B200.
+// CTAs of 512 threads that work at once: two per SM of a B200 (the staging size depends on it, so it is no question to a device).
 constexpr int kRowThreads = 512;
 constexpr int kRowCtas = 296;
 constexpr int kRowBatch = 4;  // row groups whose loads a warp has in flight
@@ -436,6 +436,8 @@ struct MetaParams {
   int32_t* err;
 };
 
+constexpr int kMetaCtas = 296;  // two per SM: a move and layer per thread, a few turns at most in a settled store
+
 __host__ __device__ inline long long meta_move_bytes(int num_layers) { return 24 + 8LL * num_layers; }
 
 template <int PHASE>
@@ -611,8 +613,8 @@ extern "C" int skv_repack_meta(const SkvStoreDesc* desc, const int32_t* move_src
   p.err = err_flag;
   if (p.staging_moves <= 0) return SKV_ERR_CAPACITY;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  repack_meta_kernel<0><<<296, 256, 0, st>>>(p);
-  repack_meta_kernel<1><<<296, 256, 0, st>>>(p);
+  repack_meta_kernel<0><<<kMetaCtas, 256, 0, st>>>(p);
+  repack_meta_kernel<1><<<kMetaCtas, 256, 0, st>>>(p);
   repack_meta_clear_kernel<<<dim3(8, desc->num_seqs), 256, 0, st>>>(p);
   repack_commit_counts_kernel<<<(desc->num_seqs * kNumBuckets + 255) / 256, 256, 0, st>>>(counts, counts_new,
                                                                                         desc->num_seqs * kNumBuckets);
