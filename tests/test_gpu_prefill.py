@@ -94,7 +94,7 @@ def _dense64(q, k, v, w):
 
 
 # The 128-token tiles: one token short, exact, one over; several tiles; heads in pairs (even groups) and query tiles in
-# pairs (odd groups, the second tile missing for an odd number of tiles); fewer and more units than SMs.
+# pairs (odd groups, the second tile missing for an odd number of tiles).  All but two have fewer units than SMs.
 @pytest.mark.parametrize("hq,hkv,d,n,B,layout", [
     (4, 2, 128, 127, 1, "token"), (4, 2, 64, 128, 2, "head"), (8, 1, 128, 129, 1, "token"), (3, 1, 64, 256, 1, "token"),
     (3, 3, 128, 257, 2, "head"), (6, 2, 64, 385, 1, "token"), (32, 8, 128, 700, 3, "head"), (32, 4, 64, 1024, 2, "token"),
@@ -238,3 +238,32 @@ def test_prefill_wait_that_runs_out_sets_the_error_flag(hq, hkv, d, n, B, layout
     assert torch.equal(again[0], good[0]) and torch.equal(again[1], good[1])
     with pytest.raises(ValueError):
         causal_prefill_attention(q, k, v, error_flag=torch.zeros(1, dtype=torch.int32))
+
+
+def _check64(q, k, v, w):
+    """Against fp64, the bounds of test_prefill_tiles_pairs_and_strides."""
+    from smartkv_b200.prefill import causal_prefill_attention
+    out, mass = causal_prefill_attention(q, k, v, w)
+    ref, ref_mass = _dense64(q, k, v, w)
+    err = (out.double() - ref).abs()
+    assert bool((err <= 2e-3 + 2e-3 * ref.abs()).all()), float(err.max())
+    assert torch.allclose(mass.double(), ref_mass, rtol=1e-3, atol=1e-5), float((mass.double() - ref_mass).abs().max())
+
+
+# On 148 SMs: three to six units a CTA in pass 1 and two to six in pass 2, which carry barrier phases, accumulators and buffers from
+# one unit to the next; even groups, odd groups whose second query tile is missing in every other unit, one head per group.
+@pytest.mark.parametrize("hq,hkv,d,n,B", [(32, 8, 128, 700, 10), (32, 4, 64, 515, 24), (12, 4, 64, 300, 24), (9, 9, 128, 257, 30),
+                                          (24, 8, 128, 385, 16)])
+def test_prefill_many_units_a_cta(hq, hkv, d, n, B):
+    g = torch.Generator(device="cuda").manual_seed(n + hq)
+    q, k, v = (torch.randn((B, n, h, d), generator=g, device="cuda").half() for h in (hq, hkv, hkv))
+    _check64(q, k, v, torch.rand((B, hq), generator=g, device="cuda") + 0.5)
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,B", [(4, 2, 128, 300, 1), (3, 1, 64, 260, 2), (5, 5, 128, 140, 40)])
+@pytest.mark.parametrize("rows", ["q", "v", "qk", "kv", "qkv"])
+def test_prefill_tensors_copied_row_by_row(hq, hkv, d, n, B, rows):
+    """Every token of the named tensors is the same row: stride 0, which no tensor map holds, so the loading warp copies the tiles."""
+    g = torch.Generator(device="cuda").manual_seed(n + d)
+    make = lambda name, h: (torch.randn((B, 1 if name in rows else n, h, d), generator=g, device="cuda").half().expand(B, n, h, d))
+    _check64(make("q", hq), make("k", hkv), make("v", hkv), torch.rand((B, hq), generator=g, device="cuda") + 0.5)
