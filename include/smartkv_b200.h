@@ -143,8 +143,8 @@ int skv_import_rows(const SkvStoreDesc* desc, void* store, int layer, int rows, 
 int skv_attn_num_ctas(int device);                       /* persistent CTAs the kernel launches */
 int64_t skv_attn_partials_bytes(const SkvStoreDesc* desc, int num_q_heads, int num_ctas);
 int64_t skv_attn_plan_bytes(const SkvStoreDesc* desc, int num_ctas);
-/* Partials every run writes (one per consumer warp of the attention launch for that query dtype);
- * skv_lse_combine folds runs * this many partials per (sequence, KV head). */
+/* Partials a run has room for in `partials` for that query dtype.  Partials a launch has no use for are marked empty
+ * (max -inf, sum 0): the fp16-query kernel fills the first two of a run. */
 int skv_attn_partials_per_run(const SkvStoreDesc* desc, int query_dtype);
 
 /* Builds the work partition of one decode step: which tiles of which (sequence, KV head) every
@@ -167,7 +167,7 @@ int skv_attn_plan(const SkvStoreDesc* desc, const int32_t* counts, int num_ctas,
  * logits[seq][q_head][storage index].
  *   query    [num_seqs][num_q_heads][head_dim] fp32 or fp16
  * num_q_heads must be a multiple of num_kv_heads with group size <= 8.
- * Two kernels can serve the call (skv_set_attention_path): the mma.sync fragment kernel (any shape) and,
+ * Two kernels can serve the call (skv_set_attention_path): the mma.sync kernel of the query's dtype (any shape) and,
  * for head_dim 128 with fp16 queries, a kernel on the tcgen05 tensor cores with the keys as the M operand,
  * accumulators in tensor memory and the 8-bit rows landed by tiled TMA loads.  Both read the same store.
  * err_flag: device int32, set non-zero if a bounded wait inside the kernel gave up. */

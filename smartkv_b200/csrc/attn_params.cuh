@@ -52,6 +52,11 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// fp16 queries (decode_attention_f16.cu).  A run has room for eleven partials, of which the kernel fills the first two --
+// what its warps merged, and the piece of a warp that went on to the next run -- and marks the rest empty.
+constexpr int kF16PartialsPerRun = 11, kF16LivePartials = 2;
+int launch_attn_f16(const AttnParams& p, cudaStream_t stream);
+
 // The tensor-memory kernel (decode_attention_tc.cu): head_dim 128, fp16 queries, group <= 8.
 int launch_attn_tc(const AttnParams& p, const SkvStoreDesc& desc, cudaStream_t stream);
 int attn_tc_partials_per_run();

@@ -2,9 +2,7 @@
 // persistent CTA owns.
 //
 // Two kernels consume a plan and each has its own cost model (`model`):
-//   model 0  mma.sync fragment kernel: tiles of 16 keys; the cost of a tile is the time one CTA needs
-//            for it (measured with every token at that width: narrow tiles are bound by their
-//            arithmetic, 8-bit tiles by their bytes)
+//   model 0  mma.sync kernels: tiles of 16 keys; the cost of a tile is the time it takes in a mixed cache
 //   model 1  tensor-memory (tcgen05) kernel: tiles of 128 keys = one MMA block; the cost is the block's
 //            bytes plus a fixed term for the per-block arithmetic and hand-offs
 // Every segment is a string of cost units: for each bucket in turn, ceil(count / tile_keys) tiles of
@@ -31,13 +29,14 @@ constexpr int kPlanModelFrag = 0;  // 16-key tiles, mma.sync fragment kernel
 constexpr int kPlanModelTc = 1;    // 128-key tiles, tensor-memory kernel
 __host__ __device__ constexpr int plan_tile_keys(int model) { return model == kPlanModelTc ? 128 : 16; }
 
-// Relative cost of one tile.  Model 0: nanoseconds one CTA spends per 16-key tile of each width at
-// head_dim 128 (B200, all tokens at one width: 46.5 / 51.6 / 48.9 / 63.3 us per launch of 65,536 tiles
-// on 148 CTAs).  Model 1: the block's bytes in units of 256 B plus a fixed per-block term.  Only the
-// ratios matter.
+// Relative cost of one tile.  Model 0: what a warp of the fp16-query kernel spends on a 16-key tile of each width while its
+// SM works on all of them (B200, head_dim 128, cycles per tile at 2 / 3 / 4 / 8 bits: 16 x 8192 keys at a budget of 0.35
+// 1770 / 1810 / 1890 / 2070, one sequence of 131072 at 0.25 1400 / 1720 / 1540 / 1730); the costs it replaces, 105 / 116 / 110 /
+// 143, had been measured width by width on whole launches (one sequence of 131072: 37.6 us a launch with those, 35.6 with
+// these).  Model 1: the block's bytes in units of 256 B plus a fixed per-block term.  Only the ratios matter.
 __host__ __device__ constexpr int tile_cost_for(int head_dim, int bits, int model) {
   if (model == kPlanModelTc) return 128 * (2 * row_bytes_for(head_dim, bits) + 8) / 256 + 24;
-  return bits == 2 ? 105 : bits == 3 ? 116 : bits == 4 ? 110 : 143;
+  return bits == 2 ? 95 : bits == 3 ? 107 : bits == 4 ? 100 : 115;
 }
 
 struct SegLayout {
@@ -103,8 +102,9 @@ static_assert(sizeof(RunDesc) == 64, "RunDesc is one 64-byte record");
 //   seg_begin[nseg]      first run of every segment (undefined when seg_count is 0)
 //   seg_count[nseg]      runs of every segment
 //   (padding to 16 words)  RunDesc runs[C + nseg]
-//   RunDesc first[C]     copy of every CTA's first run, so that a CTA reaches it with one load
+//   RunDesc first[C][kPlanFirstRuns]   copies of every CTA's first runs, so that a CTA reaches them with one load
 //                        instead of two dependent ones (cta_begin, then runs[])
+constexpr int kPlanFirstRuns = 8;
 struct PlanView {
   int* header;
   int* cta_begin;
@@ -116,7 +116,7 @@ struct PlanView {
 __host__ __device__ inline long long plan_words(int num_ctas, int nseg) {
   long long head = 4 + (num_ctas + 1) + 2LL * nseg;
   head = (head + 15) / 16 * 16;
-  return head + 16LL * (num_ctas + nseg) + 16LL * num_ctas;
+  return head + 16LL * (num_ctas + nseg) + 16LL * kPlanFirstRuns * num_ctas;
 }
 __host__ __device__ inline PlanView plan_view(int* base, int num_ctas, int nseg) {
   PlanView v;

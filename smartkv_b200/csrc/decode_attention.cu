@@ -1,4 +1,5 @@
-// Fused packed-KV decode attention for sm_100a (q_len == 1, GQA group <= 8).
+// Fused packed-KV decode attention for fp32 queries (q_len == 1, GQA group <= 8), the plan and the combine of all decode
+// attention, and the C entries that choose a kernel.  fp16 queries: decode_attention_f16.cu.
 //
 // Persistent CTAs (one per SM).  The packed buckets of every (sequence, KV head)
 // segment form one string of 16-key tiles; the global string is split into ranges of
@@ -36,9 +37,8 @@ template <int NCONS_, int STAGES_, int STAGE_BYTES_>
 struct AttnCfg {
   static constexpr int NCONS = NCONS_, STAGES = STAGES_, STAGE_BYTES = STAGE_BYTES_;
 };
-constexpr int kMaxPartialsPerRun = 11;  // consumer warps of the widest configuration
-using AttnCfgFast = AttnCfg<11, 3, 63360>;  // fp16 queries: 11 consumer warps x 145 registers (12 were no faster, 13 and 15 at 128 registers slower); 15 8-bit tiles per stage
-using AttnCfgPrecise = AttnCfg<7, 3, 42240>;   // fp32 queries (hi/lo split): 8 warps, more registers per thread
+constexpr int kMaxPartialsPerRun = kF16PartialsPerRun;
+using AttnCfgPrecise = AttnCfg<7, 3, 42240>;   // three query limbs and P in two halves: 8 warps, up to 255 registers a thread
 
 // tiles per block for a bit-width: as many 16-key tiles as fit one stage
 __host__ __device__ constexpr int block_tiles(int stage_bytes, int head_dim, int bits) {
@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(StoreGeom g, const int3
   for (int c = tid; c <= C; c += NT) pv.cta_begin[c] = nruns_of[c];
   for (int c = tid; c < C; c += NT) {
     if (total > 0) walk(c, pv.runs, nruns_of[c]);
-    if (nruns_of[c + 1] > nruns_of[c]) pv.first[c] = pv.runs[nruns_of[c]];  // written by this thread just above
+    for (int i = 0; i < kPlanFirstRuns && nruns_of[c] + i < nruns_of[c + 1]; ++i)
+      pv.first[c * kPlanFirstRuns + i] = pv.runs[nruns_of[c] + i];  // written by this thread just above
   }
 }
 
@@ -151,42 +152,42 @@ struct LaneState {
 constexpr float kLazyTau = 8.0f;
 
 // Per-run query data the producer warp prepares in shared memory.
-template <int D, bool PRECISE>
+template <int D>
 struct QSlot {
-  static constexpr int NLIMB = PRECISE ? 3 : 2;
-  static constexpr int QROWS = PRECISE ? 16 : 8;
+  static constexpr int NLIMB = 3;
+  static constexpr int QROWS = 16;
   __half qh[QROWS][D];       // fp16 rows (rows 8.. = fp16 residuals), for 3-bit keys
   int8_t limb[NLIMB][8][D];  // int8 limbs (radix 128), most significant first
   float sq[8];               // limb step per head: q = sq * sum_l limb_l * 128^(NLIMB-1-l)
   int sumA[8];               // 128*sum(limb0) + sum(limb1)
-  int sumB[8];               // sum(limb2) (precise mode)
+  int sumB[8];               // sum(limb2)
   RunDesc desc;
   int guard;                 // the run's arena holds a V scale above kVScaleGuard (see process_tile)
 };
 
 // Query of one run as a lane sees it, specialised per bit-width of the keys it meets.
-template <int D, int BITS, bool PRECISE>
+template <int D, int BITS>
 struct QFrags {
   static constexpr bool INT8 = BITS != 3 || D == 128;  // 3-bit rows of head_dim 64 keep the fp16 score path
   uint32_t qa[INT8 ? D / 32 : D / 16][4];   // A fragments: int8 limbs 0/1, or fp16 query/residual
-  uint32_t qa2[(INT8 && PRECISE) ? D / 32 : 1][4];  // precise mode: limb 2
+  uint32_t qa2[INT8 ? D / 32 : 1][4];       // int8 limb 2
   float sq;     // limb step of head g
   int initA;    // -offset * (128*sum(limb0) + sum(limb1)) of head g (offset-binary codes)
   int initB;    // -offset * sum(limb2)
 };
 
-template <int D, int BITS, bool PRECISE>
-__device__ __forceinline__ void load_qfrags(const QSlot<D, PRECISE>& q, int lane, QFrags<D, BITS, PRECISE>& f) {
+template <int D, int BITS>
+__device__ __forceinline__ void load_qfrags(const QSlot<D>& q, int lane, QFrags<D, BITS>& f) {
   const int g = lane >> 2;
   constexpr int off = BITS == 8 ? 0 : (1 << (BITS - 1));  // 8-bit rows are two's complement
-  if constexpr (QFrags<D, BITS, PRECISE>::INT8) {
+  if constexpr (QFrags<D, BITS>::INT8) {
     gather_qa_i8<D, BITS>(&q.limb[0][0][0], &q.limb[1][0][0], lane, f.qa);
-    if constexpr (PRECISE) gather_qa_i8<D, BITS>(&q.limb[2][0][0], nullptr, lane, f.qa2);
+    gather_qa_i8<D, BITS>(&q.limb[2][0][0], nullptr, lane, f.qa2);
     f.sq = q.sq[g];
     f.initA = -off * q.sumA[g];
     f.initB = -off * q.sumB[g];
   } else {
-    gather_qa_f16<D, BITS>(&q.qh[0][0], PRECISE, lane, f.qa);
+    gather_qa_f16<D, BITS>(&q.qh[0][0], true, lane, f.qa);
   }
 }
 
@@ -195,9 +196,9 @@ __device__ __forceinline__ void load_qfrags(const QSlot<D, PRECISE>& q, int lane
 // WRITE_LOGITS: lrow = logits row of head g (first key of the tile), written as two float2.
 // MASKED: the launch carries an additive mask (tok / mrow are only read then).  GUARD: the (layer, sequence) arena
 // holds a V scale above kVScaleGuard somewhere, so p * v_scale has to be checked against the fp16 range.
-template <int D, int BITS, bool PRECISE, bool WRITE_LOGITS, bool MASKED, bool GUARD>
+template <int D, int BITS, bool WRITE_LOGITS, bool MASKED, bool GUARD>
 __device__ __forceinline__ void process_tile(const uint8_t* ktile, const uint8_t* vtile, const float4* sc, int nvalid,
-                                             int lane, const QFrags<D, BITS, PRECISE>& qf, LaneState& st,
+                                             int lane, const QFrags<D, BITS>& qf, LaneState& st,
                                              float (&o)[D / 16][4], float scale_log2, float* lrow,
                                              const int32_t* tok, const float* mrow) {
   const int g = lane >> 2, t = lane & 3;
@@ -214,13 +215,13 @@ __device__ __forceinline__ void process_tile(const uint8_t* ktile, const uint8_t
   const float4 scA = sc[t], scB = sc[t + 4];  // (ks, vs) of keys 2t, 2t+1 and of keys 2t+8, 2t+9
   // ---- scores of head g (log2 units): x0, x1 = keys 2t, 2t+1; x2, x3 = keys 2t+8, 2t+9 ----
   float x0, x1, x2, x3;
-  if constexpr (QFrags<D, BITS, PRECISE>::INT8) {
+  if constexpr (QFrags<D, BITS>::INT8) {
     int c0[4] = {0, 0, qf.initA, qf.initA}, c1[4] = {0, 0, qf.initA, qf.initA};
     qk_ntile_i8<D, BITS>(kr0, qf.qa, c0);
     qk_ntile_i8<D, BITS>(kr1, qf.qa, c1);
     float f0 = (float)(c0[0] * 128 + c0[2]), f1 = (float)(c0[1] * 128 + c0[3]);
     float f2 = (float)(c1[0] * 128 + c1[2]), f3 = (float)(c1[1] * 128 + c1[3]);
-    if constexpr (PRECISE) {
+    {
       int e0[4] = {qf.initB, qf.initB, 0, 0}, e1[4] = {qf.initB, qf.initB, 0, 0};
       qk_ntile_i8<D, BITS>(kr0, qf.qa2, e0);
       qk_ntile_i8<D, BITS>(kr1, qf.qa2, e1);
@@ -304,24 +305,21 @@ __device__ __forceinline__ void process_tile(const uint8_t* ktile, const uint8_t
   const float a0 = p0 * vs0, a1 = p1 * vs1, a2 = p2 * vs2, a3 = p3 * vs3;
   // P^T B fragments: (keys 2t, 2t+1 ; head g) and (keys 2t+8, 2t+9 ; head g) -- already in place
   const uint32_t pb0 = pack_h2(a0, a1), pb1 = pack_h2(a2, a3);
-  uint32_t pl0 = 0u, pl1 = 0u;
-  if (PRECISE) {
-    const __half2 h0 = bits_h2(pb0), h1 = bits_h2(pb1);
-    pl0 = pack_h2(a0 - __low2float(h0), a1 - __high2float(h0));
-    pl1 = pack_h2(a2 - __low2float(h1), a3 - __high2float(h1));
-  }
+  const __half2 h0 = bits_h2(pb0), h1 = bits_h2(pb1);
+  const uint32_t pl0 = pack_h2(a0 - __low2float(h0), a1 - __high2float(h0));
+  const uint32_t pl1 = pack_h2(a2 - __low2float(h1), a3 - __high2float(h1));
   uint32_t v0[D / 8], v1[D / 8];
   unpack_vpair<D, BITS>(vr0, vr1, g, v0);
   unpack_vpair<D, BITS>(vr2, vr3, g, v1);
-  pv_tile<D, PRECISE>(v0, v1, pb0, pb1, pl0, pl1, o);
+  pv_tile<D, true>(v0, v1, pb0, pb1, pl0, pl1, o);
 }
 
 // One block = up to KBKEYS keys of one bucket, staged at `sb`: [K rows][V rows][float2 scales].
 // This warp owns tiles first, first + NCONS, ... of it.  lrow: logits row of head g at the
 // block's first key (null in lanes whose head does not exist).
-template <int D, int BITS, bool PRECISE, int KBKEYS, int NCONS, bool MASKED>
+template <int D, int BITS, int KBKEYS, int NCONS, bool MASKED>
 __device__ __forceinline__ void process_block(const uint8_t* sb, int nkeys, int first, int lane,
-                                              const QFrags<D, BITS, PRECISE>& qf, LaneState& st,
+                                              const QFrags<D, BITS>& qf, LaneState& st,
                                               float (&o)[D / 16][4], float scale_log2, bool write_logits, bool guard,
                                               float* lrow, const int32_t* tok, const float* mrow) {
   constexpr int PD = D * BITS / 8;
@@ -332,7 +330,7 @@ __device__ __forceinline__ void process_block(const uint8_t* sb, int nkeys, int 
   auto tiles = [&](auto wl_tag, auto gd_tag) {
     constexpr bool WL = decltype(wl_tag)::value, GD = decltype(gd_tag)::value;
     for (int tile = first; tile < ntl; tile += NCONS)
-      process_tile<D, BITS, PRECISE, WL, MASKED, GD>(kbase + tile * 16 * PD, vbase + tile * 16 * PD, sc + tile * 8,
+      process_tile<D, BITS, WL, MASKED, GD>(kbase + tile * 16 * PD, vbase + tile * 16 * PD, sc + tile * 8,
                                                      nkeys - tile * 16, lane, qf, st, o, scale_log2,
                                                      (WL && lrow) ? lrow + tile * 16 : nullptr,
                                                      MASKED ? tok + tile * 16 : nullptr, mrow);
@@ -345,13 +343,13 @@ __device__ __forceinline__ void process_block(const uint8_t* sb, int nkeys, int 
   }
 }
 
-// The query rows of a run: fp16 copy (plus a residual row in the precise mode) and radix-128 int8
+// The query rows of a run: fp16 copy plus a residual row, and radix-128 int8
 // limbs with their row sums.  One warp per call, heads [gq0, gq1) (at most 8); every head's elements are
 // fetched before any is processed, so the call costs one round trip to memory, not one per head.
-template <int D, bool PRECISE>
-__device__ __forceinline__ void prep_query_heads(QSlot<D, PRECISE>& slot, const AttnParams& p, int seq, int head,
+template <int D>
+__device__ __forceinline__ void prep_query_heads(QSlot<D>& slot, const AttnParams& p, int seq, int head,
                                                  int G, int gq0, int gq1, int lane) {
-  constexpr int NL = QSlot<D, PRECISE>::NLIMB;
+  constexpr int NL = QSlot<D>::NLIMB;
   constexpr int EPL = D / 32;  // query elements per lane and head
   const long long q_off = ((long long)seq * p.num_q_heads + (long long)head * G) * D;
   float q[8][EPL];
@@ -362,8 +360,7 @@ __device__ __forceinline__ void prep_query_heads(QSlot<D, PRECISE>& slot, const 
 #pragma unroll
       for (int e = 0; e < EPL; ++e) {
         const long long idx = q_off + (long long)gq * D + lane * EPL + e;
-        q[i][e] = p.q_is_half ? __half2float(static_cast<const __half*>(p.query)[idx])
-                              : static_cast<const float*>(p.query)[idx];
+        q[i][e] = static_cast<const float*>(p.query)[idx];
       }
     }
   }
@@ -388,7 +385,7 @@ __device__ __forceinline__ void prep_query_heads(QSlot<D, PRECISE>& slot, const 
       const int d_idx = lane * EPL + e;
       const __half qh = __float2half_rn(q[i][e]);
       slot.qh[gq][d_idx] = qh;
-      if (PRECISE) slot.qh[gq + 8][d_idx] = __float2half_rn(q[i][e] - __half2float(qh));
+      slot.qh[gq + 8][d_idx] = __float2half_rn(q[i][e] - __half2float(qh));
       float rem = fminf(fmaxf(rintf(q[i][e] * inv), -range), range);  // integer in [-range, range]
 #pragma unroll
       for (int l = NL - 1; l >= 1; --l) {
@@ -414,14 +411,14 @@ __device__ __forceinline__ void prep_query_heads(QSlot<D, PRECISE>& slot, const 
   }
 }
 
-template <int D, bool PRECISE, class CFG, bool MASKED>
+template <int D, class CFG, bool MASKED>
 __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(const AttnParams p) {
   constexpr int NCONS = CFG::NCONS, STAGES = CFG::STAGES, STAGE_BYTES = CFG::STAGE_BYTES;
   constexpr int NTC = NCONS * 32;  // consumer threads
   constexpr int KBT0 = block_tiles(STAGE_BYTES, D, 2), KBT1 = block_tiles(STAGE_BYTES, D, 3),
                 KBT2 = block_tiles(STAGE_BYTES, D, 4), KBT3 = block_tiles(STAGE_BYTES, D, 8);
   static_assert(KBT3 >= 1, "stage too small for one tile");
-  using Slot = QSlot<D, PRECISE>;
+  using Slot = QSlot<D>;
   extern __shared__ __align__(128) uint8_t smem[];
   const StoreGeom& g = p.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -523,7 +520,7 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
         slot.guard = *arena_flags(g, arena_ptr(g, p.store, p.layer, d.seq));
       }
       if (r != run_begin) {
-        prep_query_heads<D, PRECISE>(slot, p, d.seq, d.head, G, 0, G, lane);
+        prep_query_heads<D>(slot, p, d.seq, d.head, G, 0, G, lane);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&qfull[qi]);
@@ -546,7 +543,7 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
       }
       return x;
     };
-    RunDesc d = in_16_key_tiles(pv.first[blockIdx.x]);  // meaningful when the CTA has a run
+    RunDesc d = in_16_key_tiles(pv.first[blockIdx.x * kPlanFirstRuns]);  // meaningful when the CTA has a run
     bool ok = run_begin < run_end;
     for (int r = run_begin; ok && r < run_end; ++r) {
       int ci = 0, ct0 = -1;
@@ -599,7 +596,7 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
     const bool guard = slot.guard != 0;
     if (r == run_begin) {
       pdl_wait();
-      for (int gq = warp; gq < G; gq += NCONS) prep_query_heads<D, PRECISE>(qslots[qi], p, d.seq, d.head, G, gq, gq + 1, lane);
+      for (int gq = warp; gq < G; gq += NCONS) prep_query_heads<D>(qslots[qi], p, d.seq, d.head, G, gq, gq + 1, lane);
       named_bar_sync(1, NCONS * 32);
     }
     const int b = d.seq, h = d.head;
@@ -620,8 +617,8 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
       constexpr int BITS = decltype(bits_tag)::value;
       constexpr int KBT = decltype(kbt_tag)::value;
       if (d.ka[bucket] >= d.kb[bucket]) return;
-      QFrags<D, BITS, PRECISE> qf;
-      load_qfrags<D, BITS, PRECISE>(slot, lane, qf);
+      QFrags<D, BITS> qf;
+      load_qfrags<D, BITS>(slot, lane, qf);
       for (int t0 = d.ka[bucket], step = 0; t0 < d.kb[bucket]; t0 += step) {
         step = (first_block && KBT > NCONS) ? NCONS : KBT;  // as the producer issued it
         first_block = false;
@@ -634,7 +631,7 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
         if (!aborted && first < ntl) {
           float* lrow = lbase != nullptr ? lbase + g.bucket_base[bucket] + key0 : nullptr;
           const int32_t* tok = MASKED ? p.slot_token + (long long)b * g.slots + g.bucket_base[bucket] + key0 : nullptr;
-          process_block<D, BITS, PRECISE, KBT * 16, NCONS, MASKED>(
+          process_block<D, BITS, KBT * 16, NCONS, MASKED>(
               stages + (long long)stg * STAGE_BYTES, nkeys, first, lane, qf, st, o, p.scale_log2, write_logits, guard,
               lrow, tok, MASKED ? p.mask + (long long)b * p.mask_stride : nullptr);
         }
@@ -695,15 +692,15 @@ using namespace skv;
 
 static inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 
-template <int D, class CFG, bool PRECISE>
+template <int D, class CFG>
 static size_t attn_smem_bytes() {
-  return (size_t)CFG::STAGES * CFG::STAGE_BYTES + (size_t)kQBufs * sizeof(QSlot<D, PRECISE>) +
+  return (size_t)CFG::STAGES * CFG::STAGE_BYTES + (size_t)kQBufs * sizeof(QSlot<D>) +
          (2 * CFG::STAGES + 2 * kQBufs) * sizeof(uint64_t) + 64;
 }
 
 // ---- which kernel serves a launch -----------------------------------------------------------------
-// 0 = default: the mma.sync fragment kernel (measured faster on mixed-width caches: its narrow tiles cost less),
-// 1 = always the fragment kernel, 2 = the tensor-memory kernel wherever it applies (head_dim 128, fp16 queries;
+// 0 = default: the mma.sync kernels (measured faster on mixed-width caches: their narrow tiles cost less),
+// 1 = always those, 2 = the tensor-memory kernel wherever it applies (head_dim 128, fp16 queries;
 // measured faster once most cached tokens sit in the 8-bit bucket).  PackedKVStore.autotune_attention times both
 // on the live cache and sets this.
 static std::atomic<int> g_attn_path{0};
@@ -740,8 +737,11 @@ extern "C" int64_t skv_attn_partials_bytes(const SkvStoreDesc* desc, int num_q_h
 extern "C" int skv_attn_partials_per_run(const SkvStoreDesc* desc, int query_dtype) {
   if (!desc) return SKV_ERR_INVALID;
   if (use_tc_path(desc, query_dtype)) return attn_tc_partials_per_run();
-  int n = query_dtype == SKV_DTYPE_F16 ? AttnCfgFast::NCONS : AttnCfgPrecise::NCONS;
-  return n;
+  return query_dtype == SKV_DTYPE_F16 ? kF16PartialsPerRun : AttnCfgPrecise::NCONS;
+}
+int skv::attn_live_partials(const SkvStoreDesc* desc, int query_dtype) {
+  if (query_dtype == SKV_DTYPE_F16 && !use_tc_path(desc, query_dtype)) return kF16LivePartials;
+  return skv_attn_partials_per_run(desc, query_dtype);
 }
 
 extern "C" int64_t skv_attn_plan_bytes(const SkvStoreDesc* desc, int num_ctas) {
@@ -768,14 +768,14 @@ extern "C" int skv_set_dependent_launch(int on) {
   return SKV_OK;
 }
 
-template <int D, bool PRECISE, class CFG, bool MASKED>
+template <int D, class CFG, bool MASKED>
 static int launch_attn_inst(AttnParams& p, cudaStream_t st) {
   static bool configured[64] = {};  // per template instance and device: the attribute belongs to the device's context
-  const size_t smem = attn_smem_bytes<D, CFG, PRECISE>();
+  const size_t smem = attn_smem_bytes<D, CFG>();
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return SKV_ERR_CUDA;
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    const cudaError_t rc = cudaFuncSetAttribute(decode_attn_kernel<D, PRECISE, CFG, MASKED>,
+    const cudaError_t rc = cudaFuncSetAttribute(decode_attn_kernel<D, CFG, MASKED>,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (rc != cudaSuccess) {
       fprintf(stderr, "skv_decode_attention: cannot reserve %zu bytes of shared memory: %s\n", smem, cudaGetErrorString(rc));
@@ -783,7 +783,7 @@ static int launch_attn_inst(AttnParams& p, cudaStream_t st) {
     }
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  launch_maybe_dependent(decode_attn_kernel<D, PRECISE, CFG, MASKED>, dim3(p.num_ctas), dim3((CFG::NCONS + 1) * 32), smem, st, p,
+  launch_maybe_dependent(decode_attn_kernel<D, CFG, MASKED>, dim3(p.num_ctas), dim3((CFG::NCONS + 1) * 32), smem, st, p,
                          p.dependent != 0 && (g_dependent_launch.load() == 1 || g_dependent_launch.load() == 2));
   const cudaError_t rc = cudaGetLastError();
   if (rc != cudaSuccess) {
@@ -794,9 +794,9 @@ static int launch_attn_inst(AttnParams& p, cudaStream_t st) {
 }
 
 // A launch with an additive mask runs its own instantiation, so that launches without one carry none of its cost.
-template <int D, bool PRECISE, class CFG>
+template <int D, class CFG>
 static int launch_attn(AttnParams& p, cudaStream_t st) {
-  return p.mask != nullptr ? launch_attn_inst<D, PRECISE, CFG, true>(p, st) : launch_attn_inst<D, PRECISE, CFG, false>(p, st);
+  return p.mask != nullptr ? launch_attn_inst<D, CFG, true>(p, st) : launch_attn_inst<D, CFG, false>(p, st);
 }
 
 // Limit of every bounded device-side wait, in polls of about 50 ns (default 2^24, about a second).
@@ -841,12 +841,9 @@ extern "C" int skv_decode_attention_masked(const SkvStoreDesc* desc, const void*
   p.wait_polls = wait_polls();
   p.dependent = (flags & SKV_ATTN_DEPENDENT_LAUNCH) ? 1 : 0;
   if (use_tc_path(desc, query_dtype)) return launch_attn_tc(p, *desc, as_stream(stream));
-  const bool precise = !p.q_is_half;
-  if (desc->head_dim == 128)
-    return precise ? launch_attn<128, true, AttnCfgPrecise>(p, as_stream(stream))
-                   : launch_attn<128, false, AttnCfgFast>(p, as_stream(stream));
-  return precise ? launch_attn<64, true, AttnCfgPrecise>(p, as_stream(stream))
-                 : launch_attn<64, false, AttnCfgFast>(p, as_stream(stream));
+  if (p.q_is_half) return launch_attn_f16(p, as_stream(stream));
+  return desc->head_dim == 128 ? launch_attn<128, AttnCfgPrecise>(p, as_stream(stream))
+                               : launch_attn<64, AttnCfgPrecise>(p, as_stream(stream));
 }
 
 extern "C" int skv_decode_attention(const SkvStoreDesc* desc, const void* store, int layer, const void* plan,
@@ -885,6 +882,7 @@ extern "C" int skv_lse_combine_masked(const SkvStoreDesc* desc, const void* plan
   p.cur_prob = cur_prob;
   p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)desc->head_dim));
   p.per_run = skv_attn_partials_per_run(desc, query_dtype);
+  p.live = skv::attn_live_partials(desc, query_dtype);
   lse_combine_kernel<<<combine_units(p.g, group), kPostThreads, 0, as_stream(stream)>>>(p);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

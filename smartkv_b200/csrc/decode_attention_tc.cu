@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(TcCfg<GP>::THREADS, 1)
   const unsigned polls = p.wait_polls < (1u << 20) ? (1u << 20) : p.wait_polls;
 
   if (warp < G && run_begin < run_end) {  // warps 0..G-1 are consumer warps (G <= 8 < WGS * 4)
-    const RunDesc d0 = pv.first[blockIdx.x];
+    const RunDesc d0 = pv.first[blockIdx.x * kPlanFirstRuns];
     tc_prep_query_head<GP>(qbufs, mt.q[0], p, d0.seq, d0.head, G, warp, lane);
     fence_proxy_async();
     __syncwarp();
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(TcCfg<GP>::THREADS, 1)
     bool ok = run_begin < run_end;
     const uint64_t stream_policy = l2_evict_first_policy();  // the cache is read once per step
     for (int r = run_begin; ok && r < run_end; ++r) {
-      const RunDesc d = r == run_begin ? pv.first[blockIdx.x] : pv.runs[r];
+      const RunDesc d = r == run_begin ? pv.first[blockIdx.x * kPlanFirstRuns] : pv.runs[r];
       const TcRun run = tc_run(d);
       const uint8_t* arena = arena_ptr(g, p.store, p.layer, d.seq);
       for (int i = 0; ok && i < run.total; ++i, ++gi) {
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(TcCfg<GP>::THREADS, 1)
       bool ok = true;
       const uint32_t idesc = idesc_i8(1, 0, 1, 1, 128, PN);
       for (int r = run_begin; ok && r < run_end; ++r) {
-        const RunDesc d = r == run_begin ? pv.first[blockIdx.x] : pv.runs[r];
+        const RunDesc d = r == run_begin ? pv.first[blockIdx.x * kPlanFirstRuns] : pv.runs[r];
         const int nblocks = tc_run(d).total;
         for (int bi = 0; ok && bi < nblocks; ++bi, ++i) {
           const int w = i % WGS, j = i / WGS, slot = i % NS;
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(TcCfg<GP>::THREADS, 1)
     };
 
     for (int r = run_begin; r < run_end; ++r) {
-      const RunDesc d = r == run_begin ? pv.first[blockIdx.x] : pv.runs[r];
+      const RunDesc d = r == run_begin ? pv.first[blockIdx.x * kPlanFirstRuns] : pv.runs[r];
       if (!aborted && !tc_wait(&mt.qfull[qi], qfpar, abort_flag, p.err, polls)) aborted = true;
       const TcQMeta& qm = mt.q[qi];  // limb steps and limb sums of the run's query heads
       const int b = d.seq, hkv = d.head;

@@ -118,6 +118,7 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
   c.group = group;
   c.partials = static_cast<const float*>(partials);
   c.per_run = skv_attn_partials_per_run(desc, query_dtype);
+  c.live = attn_live_partials(desc, query_dtype);
   c.num_ctas = num_ctas;
   c.cur_k = cur_k;
   c.cur_v = cur_v;

@@ -19,6 +19,8 @@ constexpr int kPostThreads = 256;
 constexpr int kCombineChunk = 256;
 constexpr int kMaxQHeads = 128;
 
+int attn_live_partials(const SkvStoreDesc* desc, int query_dtype);  // decode_attention.cu
+
 __host__ __device__ inline int partial_stride(int group, int head_dim) { return group * (head_dim + 2); }
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -36,7 +38,8 @@ struct CombineParams {
   int num_q_heads;
   int group;
   const float* partials;
-  int per_run;  // partials per run = consumer warps of the attention launch
+  int per_run;  // partials a run has room for
+  int live;     // the first of them, which the attention launch fills (per_run or 2)
   int num_ctas;
   const void* cur_k;
   const void* cur_v;
@@ -86,9 +89,11 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
   const bool valid = gq < G;
   const int gqc = valid ? gq : G - 1;  // threads of a missing head go through the motions of the last one
   const PlanView pv = plan_view(const_cast<int*>(p.plan), p.num_ctas, g.num_seqs * Hkv);
-  const int nsplit = pv.seg_count[seg] * p.per_run;
+  const int nsplit = pv.seg_count[seg] * p.live;
   const int r0 = nsplit > 0 ? pv.seg_begin[seg] * p.per_run : 0;
   const int pstride = partial_stride(G, D);
+  const bool two = p.live == 2;
+  auto at = [&](int k) { return (long long)(two ? (k >> 1) * p.per_run + (k & 1) : k) * pstride; };  // k-th filled partial
   const float* base = p.partials + (long long)r0 * pstride + gqc * (D + 2);
   const bool has_cur = p.cur_k != nullptr && p.cur_v != nullptr;
   const long long hq = (long long)b * p.num_q_heads + h * G + gqc;
@@ -113,11 +118,11 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
 #pragma unroll
     for (int j = 0; j < kHdrRegs; ++j) {
       const int k = d + j * D;
-      hdr[j] = k < nsplit ? *reinterpret_cast<const float2*>(base + (long long)k * pstride) : make_float2(-INFINITY, 0.f);
+      hdr[j] = k < nsplit ? *reinterpret_cast<const float2*>(base + at(k)) : make_float2(-INFINITY, 0.f);
       mloc = fmaxf(mloc, hdr[j].x);
     }
   } else {
-    for (int k = d; k < nsplit; k += D) mloc = fmaxf(mloc, base[(long long)k * pstride]);
+    for (int k = d; k < nsplit; k += D) mloc = fmaxf(mloc, base[at(k)]);
   }
   float s_cur = head_dot(prod, sub, d, D, sh.red, 0) * p.scale_log2;
   if (has_cur && p.cur_mask != nullptr) s_cur = fmaf(p.cur_mask[b], 1.4426950408889634f, s_cur);
@@ -150,7 +155,7 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
       }
     } else {
       for (int k = d; k < cn; k += D) {
-        const float* row = base + (long long)(c0 + k) * pstride;
+        const float* row = base + at(c0 + k);
         const float mw = row[0];
         const float f = mw == -INFINITY ? 0.f : ex2f(mw - M);
         sh.f[sub][k] = f;
@@ -158,11 +163,11 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
       }
     }
     __syncthreads();
-    const float* col = base + (long long)c0 * pstride + 2 + d;
+    const float* col = base + 2 + d;
 #pragma unroll 16
     for (int k = 0; k < cn; ++k) {
       const float f = sh.f[sub][k];
-      const float x = col[(long long)k * pstride];  // a partial without keys holds stale bytes: select, not multiply
+      const float x = col[at(c0 + k)];  // a partial without keys holds stale bytes: select, not multiply
       acc += f == 0.f ? 0.f : x * f;
       L += sh.lf[sub][k];
     }

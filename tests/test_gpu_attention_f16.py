@@ -1,0 +1,58 @@
+"""The fp16-query decode-attention kernel against 64-bit arithmetic over the rows the store holds: group sizes on both sides of
+the halved softmax, tile and bucket edges, widths alone and mixed, and more runs than a CTA handles between two merges."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import smartkv_oracle as orc
+from tests.gpu_util import fill_store, make_store
+
+pytestmark = pytest.mark.gpu
+
+
+def check(hq, hkv, d, n, batch, widths, seed, sequences=None):
+    rng = np.random.default_rng(seed)
+    k, v = orc.synth_kv(batch * n, hkv, d, seed=seed)
+    bits = rng.choice(widths, size=(batch, n))
+    store = make_store(1, batch, hkv, d, hq, n)
+    fill_store(store, [(k.reshape(batch, n, hkv, d), v.reshape(batch, n, hkv, d))], bits)
+    q = torch.from_numpy(rng.standard_normal((batch, hq, d)).astype(np.float16)).cuda()
+    out = store.attention(0, q).double()
+    store.check_errors()
+    group = hq // hkv
+    for b in sequences or range(batch):
+        _, _, kc, vc, ks, vs = store.export_sequence(0, b)
+        for h in range(hkv):
+            kd, vd = kc[:, h].double() * ks[:, h, None].double(), vc[:, h].double() * vs[:, h, None].double()
+            qd = q[b, h * group:(h + 1) * group].double()
+            p = torch.softmax(qd @ kd.T / math.sqrt(d), -1)
+            # p * v_scale is rounded to fp16 (2^-11 of each term); the query to 2^-15 of its row's largest element, which moves
+            # a logit by at most that times sum |k| / sqrt(d) and a probability by twice as much of itself
+            logit = qd.abs().amax(1, keepdim=True) * 2.0 ** -15 * kd.abs().sum(1).max() / math.sqrt(d)
+            bound = (2.0 ** -11 + 2 * logit) * (p @ vd.abs()) + 1e-6
+            err = (out[b, h * group:(h + 1) * group] - p @ vd).abs()
+            assert bool((err <= bound).all()), (b, h, float((err / bound).max()))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("group", [1, 3, 4, 5, 8])
+def test_group_sizes(d, group):
+    check(2 * group, 2, d, 203, 2, (2, 3, 4, 8), seed=group + d)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("width", [2, 3, 4, 8])
+@pytest.mark.parametrize("n", [1, 17, 4096 + 5])
+def test_one_width(d, width, n):
+    check(8, 2, d, n, 1, (width,), seed=n + width)
+
+
+def test_one_long_segment_over_all_ctas():
+    check(8, 1, 128, 40007, 1, (2, 3, 4, 8), seed=5)
+
+
+def test_more_runs_than_a_merge_holds():
+    # 1600 segments: eleven or so in each of 148 CTAs, eight between two merges
+    check(32, 8, 128, 21, 200, (2, 3, 4, 8), seed=6, sequences=(0, 1, 73, 199))
