@@ -471,8 +471,6 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
     bool first_block = true;
     uint32_t armed = 0, armed_par = 0;  // stages with a copy issued, and the parity of their last full phase
     const uint64_t stream_policy = l2_evict_first_policy();  // the cache is read once per step
-    constexpr int NL = Slot::NLIMB;
-    constexpr int EPL = D / 32;  // query elements per lane and head
     // issues up to `limit` further blocks of run d, resuming at (bucket ci, tile ct0)
     auto issue_blocks = [&](const RunDesc& d, int& ci, int& ct0, int limit) -> bool {
       const uint8_t* arena = arena_ptr(g, p.store, p.layer, d.seq);

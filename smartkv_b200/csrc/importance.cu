@@ -15,10 +15,11 @@
 
 namespace skv {
 
-// grid = (ceil(slots / 256), num_seqs)
+// grid = (ceil(slots / kImpChunk), num_seqs)
+template <bool FEW, bool VEC>
 __global__ void __launch_bounds__(kPostThreads) importance_update_kernel(const ImportanceParams p) {
   __shared__ ImportanceShared sh;
-  importance_unit(p, blockIdx.x, blockIdx.y, blockIdx.x == 0, sh);
+  importance_block<imp_heads(FEW), VEC>(p, blockIdx.x, blockIdx.y, blockIdx.x == 0, sh);
 }
 
 }  // namespace skv
@@ -51,7 +52,10 @@ extern "C" int skv_importance_update(const SkvStoreDesc* desc, int layer, const 
   p.touched = touched;
   p.decay = decay;
   p.head_decay = head_decay;
-  dim3 grid((desc->slots + kPostThreads - 1) / kPostThreads, desc->num_seqs);
-  importance_update_kernel<<<grid, kPostThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  const dim3 grid((desc->slots + kImpChunk - 1) / kImpChunk, desc->num_seqs);
+  const bool few = num_q_heads <= imp_heads(true), vec = importance_aligned(p);
+  auto* k = few ? (vec ? importance_update_kernel<true, true> : importance_update_kernel<true, false>)
+                : (vec ? importance_update_kernel<false, true> : importance_update_kernel<false, false>);
+  k<<<grid, kPostThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

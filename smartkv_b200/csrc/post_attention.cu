@@ -10,8 +10,6 @@ extern std::atomic<int> g_dependent_launch;  // decode_attention.cu
 
 namespace skv {
 
-constexpr int kImpWide = 4;  // chunks per importance block once the grid would exceed two waves
-
 struct PostParams {
   CombineParams c;
   ImportanceParams imp;
@@ -19,7 +17,6 @@ struct PostParams {
   int combine_blocks;
   int imp_chunks;      // importance blocks = imp_chunks * num_seqs (0: no importance update)
   int imp_compact;     // 1: block j of a sequence takes that sequence's j-th live chunk
-  int imp_kpt;         // chunks per importance block (1 or kImpWide): one storage index of each per thread
   int append_blocks;   // 8 rows-of-a-head per block (0: no append)
 };
 
@@ -28,9 +25,7 @@ union PostShared {
   ImportanceShared i;
 };
 
-// WIDE: importance blocks of kImpWide chunks (large batches); its own instantiation, so that the common kernel's
-// register allocation is not touched by it
-template <int EPL, bool WIDE>
+template <int EPL, bool FEW, bool VEC>
 __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const PostParams p) {
   __shared__ PostShared sh;
   // dependent launch: the next layer's attention kernel may be scheduled as soon as every block here has started (it
@@ -38,43 +33,31 @@ __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const Post
   // before it complete
   pdl_launch_dependents();
   pdl_wait();
+  // the importance blocks, the longest, first
   int blk = blockIdx.x;
+  const int imp_blocks = p.imp_chunks * p.c.g.num_seqs;
+  if (blk < imp_blocks) {
+    const int b = blk / p.imp_chunks, j = blk - b * p.imp_chunks;
+    // a compact grid walks the live chunks only; the full grid visits every chunk
+    const int chunk = p.imp_compact ? live_chunk(p.c.g, p.imp.counts + b * kNumBuckets, j) : j;
+    if (chunk >= 0) importance_block<imp_heads(FEW), VEC>(p.imp, chunk, b, j == 0, sh.i);
+    return;
+  }
+  blk -= imp_blocks;
   if (blk < p.combine_blocks) {
     combine_unit(p.c, blk, sh.c);
     return;
   }
   blk -= p.combine_blocks;
-  const int per_seq = (p.imp_chunks + p.imp_kpt - 1) / p.imp_kpt;
-  const int imp_blocks = per_seq * p.c.g.num_seqs;
-  if (blk < imp_blocks) {
-    const int b = blk / per_seq, j = blk - b * per_seq;
-    if constexpr (!WIDE) {
-      // a compact grid walks the live chunks only; the full grid visits every chunk
-      const int chunk = p.imp_compact ? live_chunk(p.c.g, p.imp.counts + b * kNumBuckets, j) : j;
-      if (chunk >= 0) importance_unit(p.imp, chunk, b, j == 0, sh.i);
-      return;
-    } else {
-    // wide blocks (large batches): kImpWide chunks per block
-    const ImportanceSeq q = importance_seq(p.imp, b);
-    int chunks[kImpWide];
-    bool any = j == 0;  // the first block of a sequence publishes the head-importance EMA whatever it holds
-#pragma unroll
-    for (int k = 0; k < kImpWide; ++k) {
-      const int jj = j * kImpWide + k;
-      int c = jj < p.imp_chunks ? (p.imp_compact ? live_chunk(p.c.g, p.imp.counts + b * kNumBuckets, jj) : jj) : -1;
-      if (c >= 0 && !importance_chunk_live(p.c.g, q, c)) c = -1;
-      chunks[k] = c;
-      any |= c >= 0;
-    }
-    if (!any) return;
-    importance_prologue(p.imp, b, q, j == 0, sh.i);
-    importance_chunks<kImpWide>(p.imp, chunks, b, q, sh.i);
-    return;
-    }
-  }
-  blk -= imp_blocks;
   const long long warp = (long long)blk * (kPostThreads / 32) + (threadIdx.x >> 5);
   if (warp < (long long)p.app.rows * p.app.g.num_kv_heads * 2) append_row<EPL>(p.app, warp, threadIdx.x & 31);
+}
+
+template <int EPL>
+static cudaError_t launch_post(const PostParams& p, bool few, bool vec, int grid, cudaStream_t st, bool dep) {
+  auto* k = few ? (vec ? post_attention_kernel<EPL, true, true> : post_attention_kernel<EPL, true, false>)
+                : (vec ? post_attention_kernel<EPL, false, true> : post_attention_kernel<EPL, false, false>);
+  return launch_maybe_dependent(k, dim3(grid), dim3(kPostThreads), 0, st, p, dep);
 }
 
 }  // namespace skv
@@ -147,10 +130,11 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
     i.touched = touched;
     i.decay = decay;
     i.head_decay = head_decay;
-    p.imp_chunks = (desc->slots + kPostThreads - 1) / kPostThreads;
+    p.imp_chunks = (desc->slots + kImpChunk - 1) / kImpChunk;
     if (max_seq_tokens > 0) {
-      // live chunks of a sequence: its tokens spread over the buckets, every bucket may begin and end inside a chunk
-      const int compact = (max_seq_tokens + 1 + kPostThreads - 1) / kPostThreads + 2 * kNumBuckets + 2;
+      // live chunks of a sequence: its tokens (and a place behind them) spread over the buckets, every bucket may begin and
+      // end inside a chunk
+      const int compact = (max_seq_tokens + kNumBuckets + kImpChunk - 1) / kImpChunk + 2 * kNumBuckets;
       if (compact < p.imp_chunks) {
         p.imp_chunks = compact;
         p.imp_compact = 1;
@@ -173,18 +157,11 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
     const long long warps = (long long)a.rows * desc->num_kv_heads * 2;
     p.append_blocks = (int)((warps + kPostThreads / 32 - 1) / (kPostThreads / 32));
   }
-  p.imp_kpt = 1;
-  if (with_importance && (long long)p.imp_chunks * desc->num_seqs > 2LL * num_ctas * 4) p.imp_kpt = kImpWide;
-  const int imp_grid = with_importance ? ((p.imp_chunks + p.imp_kpt - 1) / p.imp_kpt) * desc->num_seqs : 0;
-  const int grid = p.combine_blocks + imp_grid + p.append_blocks;
+  const int grid = p.combine_blocks + p.imp_chunks * desc->num_seqs + p.append_blocks;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool dep = g_dependent_launch.load() == 1 || g_dependent_launch.load() == 3;
-  const bool wide = p.imp_kpt != 1;
-  if (desc->head_dim == 128)
-    launch_maybe_dependent(wide ? post_attention_kernel<4, true> : post_attention_kernel<4, false>, dim3(grid),
-                           dim3(kPostThreads), 0, st, p, dep);
-  else
-    launch_maybe_dependent(wide ? post_attention_kernel<2, true> : post_attention_kernel<2, false>, dim3(grid),
-                           dim3(kPostThreads), 0, st, p, dep);
+  const bool few = importance_few(num_q_heads, grid, num_ctas), vec = !with_importance || importance_aligned(p.imp);
+  if (desc->head_dim == 128) launch_post<4>(p, few, vec, grid, st, dep);
+  else launch_post<2>(p, few, vec, grid, st, dep);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

@@ -99,6 +99,16 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
   const long long hq = (long long)b * p.num_q_heads + h * G + gqc;
   const long long kv = ((long long)b * Hkv + h) * D + d;
 
+  // kRowsAhead rows at a time, their loads in flight together and the first of them beside the headers: a segment has two
+  // partials a run, and a loop over as many rows with a load each waits for every one (segments of 12 and of 40 partials: the
+  // last block ended 7.0 and 14.2 us after the attention launch, 4.5 and 9.3 with the rows in flight)
+  constexpr int kRowsAhead = 16;
+  float x[kRowsAhead];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int k = 0; k < kRowsAhead; ++k) x[k] = k0 + k < nsplit ? base[at(k0 + k) + 2 + d] : 0.f;
+  };
+  fetch(0);
   float prod = 0.f;
   if (has_cur) {
     const float q = p.q_is_half ? __half2float(static_cast<const __half*>(p.query)[hq * D + d])
@@ -163,13 +173,16 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
       }
     }
     __syncthreads();
-    const float* col = base + 2 + d;
-#pragma unroll 16
-    for (int k = 0; k < cn; ++k) {
-      const float f = sh.f[sub][k];
-      const float x = col[at(c0 + k)];  // a partial without keys holds stale bytes: select, not multiply
-      acc += f == 0.f ? 0.f : x * f;
-      L += sh.lf[sub][k];
+    for (int k0 = 0; k0 < cn; k0 += kRowsAhead) {
+      if (c0 + k0 > 0) fetch(c0 + k0);  // the first rows are on their way since the headers
+#pragma unroll
+      for (int k = 0; k < kRowsAhead; ++k) {
+        if (k0 + k < cn) {
+          const float f = sh.f[sub][k0 + k];
+          acc = f == 0.f ? acc : fmaf(x[k], f, acc);  // a partial without keys holds stale bytes: select, not multiply
+          L += sh.lf[sub][k0 + k];
+        }
+      }
     }
   }
   float pc = 0.f;
@@ -215,7 +228,10 @@ struct ImportanceShared {
   float cprob[kMaxQHeads];  // pc (unnormalised probability of the current token)
 };
 
-// Maps the j-th *live* chunk of sequence b (chunks of kPostThreads storage indices that hold a cached
+// An importance block updates kImpChunk consecutive storage indices of a sequence, four per thread.
+constexpr int kImpChunk = 4 * kPostThreads;
+
+// Maps the j-th *live* chunk of sequence b (chunks of kImpChunk storage indices that hold a cached
 // key or the slot the current token will take) to its chunk index; -1 when j is past the last one.
 // Buckets lie at increasing storage indices, so their chunk ranges are increasing and only neighbours can
 // share a chunk.  j == 0 always maps to a chunk (chunk 0 if nothing is live): that block publishes the
@@ -226,8 +242,8 @@ __device__ __forceinline__ int live_chunk(const StoreGeom& g, const int32_t* cou
   for (int i = 0; i < kNumBuckets; ++i) {
     const int cnt = counts4[i] + 1;  // + the slot a token appended this step would take
     if (g.cap[i] == 0) continue;
-    int first = g.bucket_base[i] / kPostThreads;
-    const int last = (g.bucket_base[i] + cnt - 1) / kPostThreads;
+    int first = g.bucket_base[i] / kImpChunk;
+    const int last = (g.bucket_base[i] + cnt - 1) / kImpChunk;
     if (first <= prev_last) first = prev_last + 1;
     if (last >= first) {
       const int n = last - first + 1;
@@ -255,42 +271,104 @@ __device__ __forceinline__ ImportanceSeq importance_seq(const ImportanceParams& 
   return q;
 }
 
-// True if the 256 storage indices of `chunk` hold a cached key or the slot of the current token.
-__device__ __forceinline__ bool importance_chunk_live(const StoreGeom& g, const ImportanceSeq& q, int chunk) {
-  const int s_lo = chunk * kPostThreads, s_hi = s_lo + kPostThreads;
-  bool live = q.has_cur && q.cur_slot >= s_lo && q.cur_slot < s_hi;
+// `VEC` loads and stores of the four consecutive elements of a thread (the arrays are aligned for it), or one by one.
+template <bool VEC>
+__device__ __forceinline__ void load4(const float* p, float (&x)[4]) {
+  if constexpr (VEC) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+  } else {
 #pragma unroll
-  for (int i = 0; i < kNumBuckets; ++i)
-    live |= q.cnt[i] > 0 && g.bucket_base[i] < s_hi && g.bucket_base[i] + q.cnt[i] > s_lo;
-  return live;
+    for (int i = 0; i < 4; ++i) x[i] = p[i];
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
+  if constexpr (VEC) {
+    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = p[i];
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void load4(const uint8_t* p, uint8_t (&x)[4]) {
+  if constexpr (VEC) {
+    const uchar4 v = *reinterpret_cast<const uchar4*>(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = p[i];
+  }
 }
 
-// Head weights of sequence b into shared memory: w = weight / final sum, mx = final max, cprob = unnormalised
-// probability of the current token (all threads of the block; ends with a barrier).  `publish` marks the one block
-// per sequence that writes the new head-importance EMA.
-__device__ __forceinline__ void importance_prologue(const ImportanceParams& p, int b, const ImportanceSeq& q, bool publish,
-                                                    ImportanceShared& sh) {
+// One chunk of sequence b; blockDim.x == kPostThreads.  `publish` marks the one block per sequence that writes the new
+// head-importance EMA.  HEADS: logits rows in flight per thread.
+//
+// Bound: round trips to memory, three one after the other (counts; state, (max, sum) and the first logits; the other logits)
+// for few bytes a thread.  So a thread takes four consecutive keys with 16-byte loads, every load that needs no weight is
+// issued before the weights are worked out, and the grid is one wave where a key a thread took several.  64 x 16384 keys, 8
+// heads: from the end of the attention launch to the last block's 29 us -> 19; 8 x 770, 32 heads 5.4 -> 5 (latency).
+template <int HEADS, bool VEC>
+__device__ __forceinline__ void importance_block(const ImportanceParams& p, int chunk, int b, bool publish, ImportanceShared& sh) {
+  const StoreGeom& g = p.g;
   const int tid = threadIdx.x, Hq = p.num_q_heads;
-  int nkeys = 0;
+  const ImportanceSeq q = importance_seq(p, b);
+  int total_keys = q.has_cur ? 1 : 0;
 #pragma unroll
-  for (int i = 0; i < kNumBuckets; ++i) nkeys += q.cnt[i];
-  const int total_keys = nkeys + (q.has_cur ? 1 : 0);
+  for (int i = 0; i < kNumBuckets; ++i) total_keys += q.cnt[i];
+
+  // The thread's four storage indices s .. s + 3 lie in one bucket (capacities are multiples of 128): those before `live` hold
+  // cached keys, `cur` is the one the current token will lie at.
+  const int s = chunk * kImpChunk + 4 * tid;
+  int live = 0;
+#pragma unroll
+  for (int i = 0; i < kNumBuckets; ++i)
+    if (s >= g.bucket_base[i] && s < g.bucket_base[i] + g.cap[i]) live = q.cnt[i] - (s - g.bucket_base[i]);
+  const int cur = q.has_cur ? q.cur_slot - s : -1;
+  const bool with_cur = cur >= 0 && cur < 4 && cur >= live;
+  const bool active = live > 0 || with_cur;
+  // most storage indices of a sequence are unused capacity: a block without a live key leaves at once
+  // (the publishing block of every sequence stays)
+  if (!__syncthreads_or(active || publish)) return;
+
   // final (max, sum) of every query head and the probability of the current token, as the combine
-  // step of this layer left them (issued early: independent of the EMA chain below)
-  float lse_l = 0.f, lse_m = 0.f, pcur = 0.f;
+  // step of this layer left them; the state the thread updates; the first logits
+  float lse_l = 0.f, lse_m = 0.f, pcur = 0.f, hs = 0.f;
+  const float* hs_old = p.head_state + ((long long)b * 2 + p.parity) * Hq;
+  float* hs_new = p.head_state + ((long long)b * 2 + (p.parity ^ 1)) * Hq;
   if (tid < Hq) {
     lse_l = p.lse_sum[(long long)b * Hq + tid];
     lse_m = p.lse_max[(long long)b * Hq + tid];
-    pcur = q.has_cur ? p.cur_prob[(long long)b * Hq + tid] * lse_l : 0.f;
+    pcur = q.has_cur ? p.cur_prob[(long long)b * Hq + tid] : 0.f;
+    hs = hs_old[tid];
   }
+  const long long ci = (long long)b * g.slots + s;
+  const long long li = ((long long)p.layer * g.num_seqs + b) * g.slots + s;
+  double cum[4];
+  float ema[4], mass[4] = {0.f, 0.f, 0.f, 0.f};
+  uint8_t seen[4];
+  if (active) {
+    load4<VEC>(p.cumulative + ci, cum);
+    load4<VEC>(p.layer_ema + li, ema);
+    load4<VEC>(p.touched + li, seen);
+  }
+  const float* lg = p.logits + (long long)b * Hq * g.slots + s;
+  float x[HEADS][4];
+  auto fetch = [&](int h0) {
+#pragma unroll
+    for (int h = 0; h < HEADS; ++h)
+      if (h0 + h < Hq) load4<VEC>(lg + (long long)(h0 + h) * g.slots, x[h]);
+  };
+  if (live > 0) fetch(0);
+
   // head-importance EMA (cache.py:242-248).  Every softmax row sums to one, so the
   // mean over keys of a head's probabilities is 1 / (number of keys).
-  const float* hs_old = p.head_state + ((long long)b * 2 + p.parity) * Hq;
-  float* hs_new = p.head_state + ((long long)b * 2 + (p.parity ^ 1)) * Hq;
   const float head_mean = total_keys > 0 ? 1.0f / (float)total_keys : 0.f;
   float hn = 0.f;
   if (tid < Hq) {
-    hn = hs_old[tid] * p.head_decay + head_mean * (1.0f - p.head_decay);
+    hn = hs * p.head_decay + head_mean * (1.0f - p.head_decay);
     sh.mx[tid] = hn;  // staged, replaced below
     if (publish) hs_new[tid] = hn;
   }
@@ -298,6 +376,7 @@ __device__ __forceinline__ void importance_prologue(const ImportanceParams& p, i
   float my_w = 0.f;
   if (tid < Hq) {
     float acc = 0.f;
+#pragma unroll 8
     for (int h = 0; h < Hq; ++h) acc += sh.mx[h];  // same order in every thread: one mean per block
     my_w = hn / (acc / (float)Hq + 1e-6f);
   }
@@ -305,191 +384,65 @@ __device__ __forceinline__ void importance_prologue(const ImportanceParams& p, i
   if (tid < Hq) {
     sh.w[tid] = lse_l > 0.f ? my_w / lse_l : 0.f;
     sh.mx[tid] = lse_m;
-    sh.cprob[tid] = pcur;
+    sh.cprob[tid] = pcur * lse_l;
   }
   __syncthreads();
-}
+  if (!active) return;
 
-// KPT chunks of 256 storage indices at once, one storage index of each per thread: the loads of all of them are in
-// flight together (the update of one key is two dependent round trips to memory and a handful of bytes; a large
-// batch is thousands of such blocks otherwise, each waiting out the same latencies).  chunks[k] < 0: nothing to do.
-// Per key the sum over the heads runs in head order whatever KPT is, so the results do not depend on it.
-template <int KPT>
-__device__ __forceinline__ void importance_chunks(const ImportanceParams& p, const int (&chunks)[KPT], int b,
-                                                  const ImportanceSeq& q, const ImportanceShared& sh) {
-  const StoreGeom& g = p.g;
-  const int Hq = p.num_q_heads;
-  int s[KPT];
-  bool valid[KPT], is_cur[KPT];
-  double cum[KPT];
-  float ema[KPT], mass[KPT];
-  uint8_t seen[KPT];
+  if (live > 0) {  // per key the sum over the heads runs in head order
+    for (int h0 = 0; h0 < Hq; h0 += HEADS) {
+      if (h0 > 0) fetch(h0);
 #pragma unroll
-  for (int k = 0; k < KPT; ++k) {
-    s[k] = chunks[k] * kPostThreads + threadIdx.x;  // storage index
-    valid[k] = false;
-    if (chunks[k] >= 0 && s[k] < g.slots) {
+      for (int h = 0; h < HEADS; ++h) {
+        if (h0 + h < Hq) {
+          const float wv = sh.w[h0 + h], mv = sh.mx[h0 + h];
 #pragma unroll
-      for (int i = 0; i < kNumBuckets; ++i) valid[k] |= (s[k] >= g.bucket_base[i] && s[k] < g.bucket_base[i] + q.cnt[i]);
-    }
-    is_cur[k] = chunks[k] >= 0 && !valid[k] && q.has_cur && s[k] == q.cur_slot;
-    mass[k] = 0.f;
-    cum[k] = 0.0;
-    ema[k] = 0.f;
-    seen[k] = 0;
-  }
-  const long long seq_base = (long long)b * g.slots;
-  const long long lay_base = ((long long)p.layer * g.num_seqs + b) * g.slots;
-  // the state these threads update is fetched before the logits so that the latencies overlap
-#pragma unroll
-  for (int k = 0; k < KPT; ++k) {
-    if (valid[k] || is_cur[k]) {
-      cum[k] = p.cumulative[seq_base + s[k]];
-      ema[k] = p.layer_ema[lay_base + s[k]];
-      seen[k] = p.touched[lay_base + s[k]];
-    }
-  }
-  const float* lg = p.logits + (long long)b * Hq * g.slots;
-  // The loads of the loop below carry no condition (a thread without a key reads index 0 and drops the result), so
-  // that the compiler can put a batch of them in flight before the first use.
-  int sv[KPT];
-  bool any_valid = false;
-#pragma unroll
-  for (int k = 0; k < KPT; ++k) {
-    sv[k] = valid[k] ? s[k] : 0;
-    any_valid |= valid[k];
-  }
-  if (any_valid) {
-    constexpr int kHeadsInFlight = 16 / KPT;  // 16 logit loads in flight per thread either way
-#pragma unroll kHeadsInFlight
-    for (int h = 0; h < Hq; ++h) {
-      const float wv = sh.w[h], mv = sh.mx[h];
-      const float* row = lg + (long long)h * g.slots;
-#pragma unroll
-      for (int k = 0; k < KPT; ++k) mass[k] += wv * ex2f(row[sv[k]] - mv);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < KPT; ++k) {
-    if (!valid[k]) mass[k] = 0.f;
-    if (is_cur[k]) {
-      // the newest token: it is stored at this storage index when the step's append commits
-      for (int h = 0; h < Hq; ++h) mass[k] += sh.w[h] * sh.cprob[h];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < KPT; ++k) {
-    if (valid[k] || is_cur[k]) {
-      p.cumulative[seq_base + s[k]] = cum[k] + (double)mass[k];
-      if (seen[k]) {
-        p.layer_ema[lay_base + s[k]] = p.decay * ema[k] + (1.0f - p.decay) * mass[k];
-      } else {
-        p.layer_ema[lay_base + s[k]] = mass[k];
-        p.touched[lay_base + s[k]] = 1;
+          for (int i = 0; i < 4; ++i) mass[i] += wv * ex2f(x[h][i] - mv);
+        }
       }
     }
   }
-}
-
-// One unit = 256 consecutive storage indices of one sequence; blockDim.x == kPostThreads.  (The common case, kept as one
-// straight-line function: the wide variant above costs this path a per cent when both go through the same code.)
-// `publish` marks the one block per sequence that writes the new head-importance EMA.
-__device__ __forceinline__ void importance_unit(const ImportanceParams& p, int chunk, int b, bool publish,
-                                                ImportanceShared& sh) {
-  const StoreGeom& g = p.g;
-  const int tid = threadIdx.x, Hq = p.num_q_heads;
-  int cnt[kNumBuckets];
-  int nkeys = 0;
-#pragma unroll
-  for (int i = 0; i < kNumBuckets; ++i) {
-    cnt[i] = p.counts[b * kNumBuckets + i];
-    nkeys += cnt[i];
-  }
-  const int cur_slot = (p.cur_prob != nullptr && p.cur_slot != nullptr) ? p.cur_slot[b] : -1;
-  const bool has_cur = cur_slot >= 0;
-  const int total_keys = nkeys + (has_cur ? 1 : 0);
-
-  // most storage indices of a sequence are unused capacity: a block without a live key leaves at once
-  // (the publishing block of every sequence stays)
-  const int s_lo = chunk * kPostThreads, s_hi = s_lo + kPostThreads;
-  bool block_live = publish || (has_cur && cur_slot >= s_lo && cur_slot < s_hi);
-#pragma unroll
-  for (int i = 0; i < kNumBuckets; ++i)
-    block_live |= cnt[i] > 0 && g.bucket_base[i] < s_hi && g.bucket_base[i] + cnt[i] > s_lo;
-  if (!block_live) return;
-
-  // final (max, sum) of every query head and the probability of the current token, as the combine
-  // step of this layer left them (issued early: independent of the EMA chain below)
-  float lse_l = 0.f, lse_m = 0.f, pcur = 0.f;
-  if (tid < Hq) {
-    lse_l = p.lse_sum[(long long)b * Hq + tid];
-    lse_m = p.lse_max[(long long)b * Hq + tid];
-    pcur = has_cur ? p.cur_prob[(long long)b * Hq + tid] * lse_l : 0.f;
-  }
-
-  // head-importance EMA (cache.py:242-248).  Every softmax row sums to one, so the
-  // mean over keys of a head's probabilities is 1 / (number of keys).
-  const float* hs_old = p.head_state + ((long long)b * 2 + p.parity) * Hq;
-  float* hs_new = p.head_state + ((long long)b * 2 + (p.parity ^ 1)) * Hq;
-  const float head_mean = total_keys > 0 ? 1.0f / (float)total_keys : 0.f;
-  float hn = 0.f;
-  if (tid < Hq) {
-    hn = hs_old[tid] * p.head_decay + head_mean * (1.0f - p.head_decay);
-    sh.mx[tid] = hn;  // staged, replaced below
-    if (publish) hs_new[tid] = hn;
-  }
-  __syncthreads();
-  float my_w = 0.f;
-  if (tid < Hq) {
-    float acc = 0.f;
-    for (int h = 0; h < Hq; ++h) acc += sh.mx[h];  // same order in every thread: one mean per block
-    my_w = hn / (acc / (float)Hq + 1e-6f);
-  }
-  __syncthreads();
-  if (tid < Hq) {
-    sh.w[tid] = lse_l > 0.f ? my_w / lse_l : 0.f;
-    sh.mx[tid] = lse_m;
-    sh.cprob[tid] = pcur;
-  }
-  __syncthreads();
-
-  const int s = s_lo + tid;  // storage index
-  bool valid = false;
-  if (s < g.slots) {
-#pragma unroll
-    for (int i = 0; i < kNumBuckets; ++i) valid |= (s >= g.bucket_base[i] && s < g.bucket_base[i] + cnt[i]);
-  }
-  float mass = 0.f;
-  const bool is_cur = !valid && has_cur && s == cur_slot;
-  const bool write = valid || is_cur;
-  const long long ci = (long long)b * g.slots + s;
-  const long long li = ((long long)p.layer * g.num_seqs + b) * g.slots + s;
-  // the state this thread updates is fetched before the logits so that the two latencies overlap
-  double cum = 0.0;
-  float ema = 0.f;
-  uint8_t seen = 0;
-  if (write) {
-    cum = p.cumulative[ci];
-    ema = p.layer_ema[li];
-    seen = p.touched[li];
-  }
-  if (valid) {
-    const float* lg = p.logits + (long long)b * Hq * g.slots + s;
-#pragma unroll 16
-    for (int h = 0; h < Hq; ++h) mass += sh.w[h] * ex2f(lg[(long long)h * g.slots] - sh.mx[h]);
-  } else if (is_cur) {
+  if (with_cur) {
     // the newest token: it is stored at this storage index when the step's append commits
-    for (int h = 0; h < Hq; ++h) mass += sh.w[h] * sh.cprob[h];
+    float m = 0.f;
+#pragma unroll 8
+    for (int h = 0; h < Hq; ++h) m += sh.w[h] * sh.cprob[h];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i == cur) mass[i] = m;
   }
-  if (write) {
-    p.cumulative[ci] = cum + (double)mass;
-    if (seen) {
-      p.layer_ema[li] = p.decay * ema + (1.0f - p.decay) * mass;
-    } else {
-      p.layer_ema[li] = mass;
-      p.touched[li] = 1;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    cum[i] += (double)mass[i];
+    ema[i] = seen[i] ? p.decay * ema[i] + (1.0f - p.decay) * mass[i] : mass[i];
+  }
+  if (VEC && live >= 4) {
+    *reinterpret_cast<double2*>(p.cumulative + ci) = make_double2(cum[0], cum[1]);
+    *reinterpret_cast<double2*>(p.cumulative + ci + 2) = make_double2(cum[2], cum[3]);
+    *reinterpret_cast<float4*>(p.layer_ema + li) = make_float4(ema[0], ema[1], ema[2], ema[3]);
+    if (!(seen[0] && seen[1] && seen[2] && seen[3])) *reinterpret_cast<uchar4*>(p.touched + li) = make_uchar4(1, 1, 1, 1);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (i < live || (with_cur && i == cur)) {
+      p.cumulative[ci + i] = cum[i];
+      p.layer_ema[li + i] = ema[i];
+      if (!seen[i]) p.touched[li + i] = 1;
     }
   }
+}
+
+// Heads in flight per thread.  Sixteen (118 registers, two blocks an SM) where there are more than eight and the launch still
+// fits one wave that way, else eight (80 registers, three blocks).  Steps, us, sixteen / eight: 8 x 770 keys, 32 heads
+// 303 / 313; 16 x 8192, 32 heads (448 blocks) 1705 / 1658.
+__host__ __device__ constexpr int imp_heads(bool few) { return few ? 8 : 16; }
+inline bool importance_few(int num_q_heads, long long blocks, int sms) { return num_q_heads <= 8 || blocks > 2LL * sms; }
+// Both forms of loads are there because the arrays are the caller's.
+inline bool importance_aligned(const ImportanceParams& p) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p.logits) | reinterpret_cast<uintptr_t>(p.cumulative) |
+                      reinterpret_cast<uintptr_t>(p.layer_ema);
+  return a % 16 == 0 && reinterpret_cast<uintptr_t>(p.touched) % 4 == 0;
 }
 
 // ---- append ---------------------------------------------------------------------------------------------
