@@ -36,7 +36,7 @@ __host__ __device__ constexpr int plan_tile_keys(int model) { return model == kP
 // these).  Model 1: the block's bytes in units of 256 B plus a fixed per-block term.  Only the ratios matter.
 __host__ __device__ constexpr int tile_cost_for(int head_dim, int bits, int model) {
   if (model == kPlanModelTc) return 128 * (2 * row_bytes_for(head_dim, bits) + 8) / 256 + 24;
-  return bits == 2 ? 95 : bits == 3 ? 107 : bits == 4 ? 100 : 115;
+  return bits == 2 ? 95 : bits == 3 ? 107 : bits == 4 ? 100 : 109;
 }
 
 struct SegLayout {

@@ -31,13 +31,17 @@ extern std::atomic<int> g_dependent_launch;  // decode_attention.cu
 
 namespace skv {
 
-constexpr int kWarps = 16;      // 128 registers a thread
 constexpr int kGroupRuns = kPlanFirstRuns;  // runs a CTA handles between two merges: 8 runs x 4 buckets = one lane each
 static_assert(kGroupRuns * kNumBuckets == 32, "one lane per (run, bucket)");
 constexpr float kLazyTau = 8.0f;  // the running maximum is raised when a score exceeds it by this much (log2 units)
 
+// Warps of a CTA.  head_dim 128: twelve, 168 registers each; sixteen at 128 end later for all their work in flight, because
+// every warp brings its start, its share of the merge and a rounding to whole tiles (steps of 16 x 8192 keys 1610 us
+// against 1658, 64 x 16384 1253 against 1288, 1 x 131072 the same; eight warps 1687, 1317 and 1487 against 1358).  head_dim 64, whose
+// contexts are short: sixteen (8 x 770 keys 303 us a step, twelve 316).
 template <int D>
 struct StreamShape {
+  static constexpr int WARPS = D == 128 ? 12 : 16;
   static constexpr int SLOT = 16 * (2 * D + 8);  // one 16-key tile at the widest: K rows, V rows, scales
   static constexpr int V_AT = 16 * D, S_AT = 32 * D;
   static constexpr int STAGES = D == 128 ? 3 : 6;
@@ -48,13 +52,14 @@ struct StreamShape {
 // What the CTA's warps share besides their rings.
 template <int D>
 struct __align__(16) StreamShared {
+  static constexpr int WARPS = StreamShape<D>::WARPS;
   int8_t limb[kGroupRuns][2][8][D];                    // query of a run: int8 limbs (radix 128), most significant first
   __half qh[D == 64 ? kGroupRuns : 1][D == 64 ? 8 : 1][D];  // fp16 rows, for the 3-bit keys of head_dim 64
   float sq[kGroupRuns][8];                             // limb step per head: q = sq * (128 * limb0 + limb1)
   int sum[kGroupRuns][8];                              // 128 * sum(limb0) + sum(limb1)
-  float tail_m[kWarps][8], tail_l[kWarps][8];          // (max, sum) of every warp's last piece
-  float weight[kWarps][8];                             // its weight in the merged partial
-  int tail_run[kWarps];                                // run (of the group) of that piece, -1: the warp had no tile
+  float tail_m[WARPS][8], tail_l[WARPS][8];          // (max, sum) of every warp's last piece
+  float weight[WARPS][8];                             // its weight in the merged partial
+  int tail_run[WARPS];                                // run (of the group) of that piece, -1: the warp had no tile
   int has_first[kGroupRuns], has_second[kGroupRuns];   // partials of a run written by a warp alone
 };
 
@@ -125,10 +130,11 @@ struct TileFeed {
 // HALF: at most four query heads per KV head.  The score rows of heads 4..7 then repeat heads 0..3, so that lanes g < 4 take
 // the first eight keys of a tile through the softmax and lanes g >= 4 the other eight, instead of idling.
 template <int D, bool MASKED, bool HALF>
-__global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(StreamShape<D>::WARPS * 32, 1) decode_attn_f16_kernel(const AttnParams p) {
   using S = StreamShape<D>;
+  constexpr int WARPS = S::WARPS;
   extern __shared__ __align__(128) uint8_t smem[];
-  StreamShared<D>& sh = *reinterpret_cast<StreamShared<D>*>(smem + kWarps * S::RING);
+  StreamShared<D>& sh = *reinterpret_cast<StreamShared<D>*>(smem + WARPS * S::RING);
   const StoreGeom& g = p.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lg = lane >> 2, t = lane & 3;
@@ -142,7 +148,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const A
     sh.sum[tid >> 3][tid & 7] = 0;
   }
   if constexpr (D == 64) {
-    for (int i = tid; i < kGroupRuns * 8 * D / 2; i += kWarps * 32) reinterpret_cast<uint32_t*>(&sh.qh[0][0][0])[i] = 0u;
+    for (int i = tid; i < kGroupRuns * 8 * D / 2; i += WARPS * 32) reinterpret_cast<uint32_t*>(&sh.qh[0][0][0])[i] = 0u;
   }
   __syncthreads();
   // What is read before pdl_wait() -- the plan and this layer's rows -- was written by kernels that completed long before a
@@ -185,7 +191,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const A
     }
     const unsigned total = __shfl_sync(0xffffffffu, end, 31), start = end - own;
     auto first_tile = [&](int w) -> int {  // first tile of this lane whose cost begins in slice w or a later one
-      const unsigned at = (unsigned)(((unsigned long long)total * w + kWarps - 1) / kWarps);
+      const unsigned at = (unsigned)(((unsigned long long)total * w + WARPS - 1) / WARPS);
       if (at <= start) return 0;
       if (at >= end) return n;
       return (int)(by_count ? at - start : tiles_in(at - start + cost - 1, D, bk));
@@ -262,7 +268,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const A
     int guard_flag = 0;  // the (layer, sequence) arena holds a V scale above kVScaleGuard
     if (rr < nr) guard_flag = *arena_flags(g, arena_ptr(g, p.store, p.layer, seq));
     if (tid < kGroupRuns) sh.has_first[tid] = sh.has_second[tid] = 0;
-    for (int i = warp; i < nr * G; i += kWarps) {
+    for (int i = warp; i < nr * G; i += WARPS) {
       const int qr = i / G, h = i - qr * G;
       const int qseq = __shfl_sync(0xffffffffu, seq, 4 * qr), qhead = __shfl_sync(0xffffffffu, head, 4 * qr);
       prep_query<D>(sh, qr, h, static_cast<const __half*>(p.query) + ((long long)qseq * p.num_q_heads + qhead * G + h) * D, lane);
@@ -522,18 +528,18 @@ __global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const A
     __syncthreads();
 
     // ---- merge: the warps whose last piece belongs to one run, in warp order ------------------------------------------------
-    if (tid < kWarps * 8) {
+    if (tid < WARPS * 8) {
       const int w = tid >> 3, h = tid & 7, run = sh.tail_run[w];
-      float mi[kWarps], M = -INFINITY, L = 0.f;
-      int leader = kWarps;
+      float mi[WARPS], M = -INFINITY, L = 0.f;
+      int leader = WARPS;
 #pragma unroll
-      for (int i = 0; i < kWarps; ++i) {
+      for (int i = 0; i < WARPS; ++i) {
         mi[i] = sh.tail_run[i] == run ? sh.tail_m[i][h] : -INFINITY;
         if (sh.tail_run[i] == run && i < leader) leader = i;
         M = fmaxf(M, mi[i]);
       }
 #pragma unroll
-      for (int i = 0; i < kWarps; ++i) {
+      for (int i = 0; i < WARPS; ++i) {
         const float f = mi[i] == -INFINITY ? 0.f : ex2f(mi[i] - M);
         if (i == w) sh.weight[w][h] = f;
         L += f == 0.f ? 0.f : sh.tail_l[i][h] * f;
@@ -543,23 +549,23 @@ __global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const A
             make_float2(M, L);
     }
     __syncthreads();
-    const int tr = lane < kWarps ? sh.tail_run[lane] : -1;
+    const int tr = lane < WARPS ? sh.tail_run[lane] : -1;
     for (int run = 0; run < nr; ++run) {
       const unsigned who = __ballot_sync(0xffffffffu, tr == run);
       float* out = p.partials + (long long)(r0 + run) * kF16PartialsPerRun * partial_stride(G, D);
       if (who != 0) {
-        for (int e = tid; e < G * D; e += kWarps * 32) {
+        for (int e = tid; e < G * D; e += WARPS * 32) {
           const int h = e / D, d = e - h * D;
           const float* acc_at = reinterpret_cast<const float*>(smem) + h * kAccStride<D> + d;
           float acc = 0.f;
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w)
+          for (int w = 0; w < WARPS; ++w)
             if ((who >> w) & 1u) acc = fmaf(sh.weight[w][h], acc_at[w * (S::RING / 4)], acc);
           out[h * (D + 2) + 2 + d] = acc;
         }
       }
       // partials nobody wrote are marked empty
-      for (int e = tid; e < kF16PartialsPerRun * G; e += kWarps * 32) {
+      for (int e = tid; e < kF16PartialsPerRun * G; e += WARPS * 32) {
         const int s = e / G, h = e - s * G;
         const bool written = s == 0 ? (who != 0 || sh.has_first[run]) : s == 1 ? sh.has_second[run] != 0 : false;
         if (!written) *reinterpret_cast<float2*>(out + (long long)s * partial_stride(G, D) + h * (D + 2)) = make_float2(-INFINITY, 0.f);
@@ -572,7 +578,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) decode_attn_f16_kernel(const A
 template <int D, bool MASKED, bool HALF>
 static int launch_f16(const AttnParams& p, cudaStream_t st) {
   static bool configured[64] = {};  // per template instance and device: the attribute belongs to the device's context
-  constexpr size_t smem = (size_t)kWarps * StreamShape<D>::RING + sizeof(StreamShared<D>);
+  constexpr int WARPS = StreamShape<D>::WARPS;
+  constexpr size_t smem = (size_t)WARPS * StreamShape<D>::RING + sizeof(StreamShared<D>);
   static_assert(smem <= 232448, "more shared memory than a CTA can have");
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return SKV_ERR_CUDA;
@@ -586,7 +593,7 @@ static int launch_f16(const AttnParams& p, cudaStream_t st) {
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   const int mode = g_dependent_launch.load();
-  launch_maybe_dependent(decode_attn_f16_kernel<D, MASKED, HALF>, dim3(p.num_ctas), dim3(kWarps * 32), smem, st, p,
+  launch_maybe_dependent(decode_attn_f16_kernel<D, MASKED, HALF>, dim3(p.num_ctas), dim3(WARPS * 32), smem, st, p,
                          p.dependent != 0 && (mode == 1 || mode == 2));
   const cudaError_t rc = cudaGetLastError();
   if (rc != cudaSuccess) {
