@@ -52,9 +52,10 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// fp16 queries (decode_attention_f16.cu).  A run has room for eleven partials, of which the kernel fills the first two --
-// what its warps merged, and the piece of a warp that went on to the next run -- and marks the rest empty.
-constexpr int kF16PartialsPerRun = 11, kF16LivePartials = 2;
+// fp16 queries (decode_attention_f16.cu).  A run has room for eleven partials, of which the kernel fills the first -- what its
+// warps merged -- and, of a run that ends inside a CTA (a segment's last), the second: the piece of a warp that went on to the
+// next run.  The rest is marked empty.
+constexpr int kF16PartialsPerRun = 11;
 int launch_attn_f16(const AttnParams& p, cudaStream_t stream);
 
 // The tensor-memory kernel (decode_attention_tc.cu): head_dim 128, fp16 queries, group <= 8.

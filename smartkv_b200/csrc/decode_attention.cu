@@ -737,9 +737,8 @@ extern "C" int skv_attn_partials_per_run(const SkvStoreDesc* desc, int query_dty
   if (use_tc_path(desc, query_dtype)) return attn_tc_partials_per_run();
   return query_dtype == SKV_DTYPE_F16 ? kF16PartialsPerRun : AttnCfgPrecise::NCONS;
 }
-int skv::attn_live_partials(const SkvStoreDesc* desc, int query_dtype) {
-  if (query_dtype == SKV_DTYPE_F16 && !use_tc_path(desc, query_dtype)) return kF16LivePartials;
-  return skv_attn_partials_per_run(desc, query_dtype);
+bool skv::attn_first_of_run(const SkvStoreDesc* desc, int query_dtype) {
+  return query_dtype == SKV_DTYPE_F16 && !use_tc_path(desc, query_dtype);
 }
 
 extern "C" int64_t skv_attn_plan_bytes(const SkvStoreDesc* desc, int num_ctas) {
@@ -880,7 +879,7 @@ extern "C" int skv_lse_combine_masked(const SkvStoreDesc* desc, const void* plan
   p.cur_prob = cur_prob;
   p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)desc->head_dim));
   p.per_run = skv_attn_partials_per_run(desc, query_dtype);
-  p.live = skv::attn_live_partials(desc, query_dtype);
+  p.first_of_run = skv::attn_first_of_run(desc, query_dtype);
   lse_combine_kernel<<<combine_units(p.g, group), kPostThreads, 0, as_stream(stream)>>>(p);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

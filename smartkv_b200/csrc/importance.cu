@@ -15,11 +15,17 @@
 
 namespace skv {
 
-// grid = (ceil(slots / kImpChunk), num_seqs)
-template <bool FEW, bool VEC>
+// grid = (ceil(slots / IMP::CHUNK), num_seqs)
+template <class IMP>
 __global__ void __launch_bounds__(kPostThreads) importance_update_kernel(const ImportanceParams p) {
   __shared__ ImportanceShared sh;
-  importance_block<imp_heads(FEW), VEC>(p, blockIdx.x, blockIdx.y, blockIdx.x == 0, sh);
+  importance_block<IMP>(p, blockIdx.x, blockIdx.y, blockIdx.x == 0, sh);
+}
+
+template <class IMP>
+static void launch_importance(const ImportanceParams& p, cudaStream_t st) {
+  const dim3 grid((p.g.slots + IMP::CHUNK - 1) / IMP::CHUNK, p.g.num_seqs);
+  importance_update_kernel<IMP><<<grid, kPostThreads, 0, st>>>(p);
 }
 
 }  // namespace skv
@@ -52,10 +58,10 @@ extern "C" int skv_importance_update(const SkvStoreDesc* desc, int layer, const 
   p.touched = touched;
   p.decay = decay;
   p.head_decay = head_decay;
-  const dim3 grid((desc->slots + kImpChunk - 1) / kImpChunk, desc->num_seqs);
-  const bool few = num_q_heads <= imp_heads(true), vec = importance_aligned(p);
-  auto* k = few ? (vec ? importance_update_kernel<true, true> : importance_update_kernel<true, false>)
-                : (vec ? importance_update_kernel<false, true> : importance_update_kernel<false, false>);
-  k<<<grid, kPostThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // as the launch after the attention chooses (post_attention.cuh); how many chunks are live is not known here
+  if ((long long)desc->slots * desc->num_seqs <= 4LL * 148 * ImpOne::CHUNK) launch_importance<ImpOne>(p, st);
+  else if (importance_aligned(p)) launch_importance<ImpFour8<true>>(p, st);
+  else launch_importance<ImpFour8<false>>(p, st);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

@@ -25,7 +25,7 @@ union PostShared {
   ImportanceShared i;
 };
 
-template <int EPL, bool FEW, bool VEC>
+template <int EPL, class IMP>
 __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const PostParams p) {
   __shared__ PostShared sh;
   // dependent launch: the next layer's attention kernel may be scheduled as soon as every block here has started (it
@@ -39,8 +39,8 @@ __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const Post
   if (blk < imp_blocks) {
     const int b = blk / p.imp_chunks, j = blk - b * p.imp_chunks;
     // a compact grid walks the live chunks only; the full grid visits every chunk
-    const int chunk = p.imp_compact ? live_chunk(p.c.g, p.imp.counts + b * kNumBuckets, j) : j;
-    if (chunk >= 0) importance_block<imp_heads(FEW), VEC>(p.imp, chunk, b, j == 0, sh.i);
+    const int chunk = p.imp_compact ? live_chunk<IMP::CHUNK>(p.c.g, p.imp.counts + b * kNumBuckets, j) : j;
+    if (chunk >= 0) importance_block<IMP>(p.imp, chunk, b, j == 0, sh.i);
     return;
   }
   blk -= imp_blocks;
@@ -53,11 +53,30 @@ __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const Post
   if (warp < (long long)p.app.rows * p.app.g.num_kv_heads * 2) append_row<EPL>(p.app, warp, threadIdx.x & 31);
 }
 
+// Chunks of CHUNK storage indices a sequence: all of them, or (compact) as many as can be live -- its tokens and a place behind
+// them spread over the buckets, and every bucket may begin and end inside a chunk.
+static int imp_chunks(const StoreGeom& g, int max_seq_tokens, int chunk, int* compact) {
+  const int all = (g.slots + chunk - 1) / chunk, live = (max_seq_tokens + kNumBuckets + chunk - 1) / chunk + 2 * kNumBuckets;
+  *compact = max_seq_tokens > 0 && live < all;
+  return *compact ? live : all;
+}
+
+template <int EPL, class IMP>
+static cudaError_t launch_post(PostParams& p, int max_seq_tokens, cudaStream_t st, bool dep) {
+  p.imp_chunks = p.imp.logits != nullptr ? imp_chunks(p.c.g, max_seq_tokens, IMP::CHUNK, &p.imp_compact) : 0;
+  const int grid = p.combine_blocks + p.imp_chunks * p.c.g.num_seqs + p.append_blocks;
+  return launch_maybe_dependent(post_attention_kernel<EPL, IMP>, dim3(grid), dim3(kPostThreads), 0, st, p, dep);
+}
 template <int EPL>
-static cudaError_t launch_post(const PostParams& p, bool few, bool vec, int grid, cudaStream_t st, bool dep) {
-  auto* k = few ? (vec ? post_attention_kernel<EPL, true, true> : post_attention_kernel<EPL, true, false>)
-                : (vec ? post_attention_kernel<EPL, false, true> : post_attention_kernel<EPL, false, false>);
-  return launch_maybe_dependent(k, dim3(grid), dim3(kPostThreads), 0, st, p, dep);
+static cudaError_t launch_post(PostParams& p, int max_seq_tokens, cudaStream_t st, bool dep) {
+  const long long other = p.combine_blocks + p.append_blocks, seqs = p.c.g.num_seqs, sms = p.c.num_ctas;
+  int compact;
+  if (p.imp.logits == nullptr || imp_chunks(p.c.g, max_seq_tokens, ImpOne::CHUNK, &compact) * seqs + other <= 4 * sms)
+    return launch_post<EPL, ImpOne>(p, max_seq_tokens, st, dep);
+  const bool sixteen = p.c.num_q_heads > 8 && imp_chunks(p.c.g, max_seq_tokens, ImpFour16<true>::CHUNK, &compact) * seqs + other <= 2 * sms;
+  if (importance_aligned(p.imp))
+    return sixteen ? launch_post<EPL, ImpFour16<true>>(p, max_seq_tokens, st, dep) : launch_post<EPL, ImpFour8<true>>(p, max_seq_tokens, st, dep);
+  return launch_post<EPL, ImpFour8<false>>(p, max_seq_tokens, st, dep);
 }
 
 }  // namespace skv
@@ -101,7 +120,7 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
   c.group = group;
   c.partials = static_cast<const float*>(partials);
   c.per_run = skv_attn_partials_per_run(desc, query_dtype);
-  c.live = attn_live_partials(desc, query_dtype);
+  c.first_of_run = attn_first_of_run(desc, query_dtype);
   c.num_ctas = num_ctas;
   c.cur_k = cur_k;
   c.cur_v = cur_v;
@@ -130,16 +149,6 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
     i.touched = touched;
     i.decay = decay;
     i.head_decay = head_decay;
-    p.imp_chunks = (desc->slots + kImpChunk - 1) / kImpChunk;
-    if (max_seq_tokens > 0) {
-      // live chunks of a sequence: its tokens (and a place behind them) spread over the buckets, every bucket may begin and
-      // end inside a chunk
-      const int compact = (max_seq_tokens + kNumBuckets + kImpChunk - 1) / kImpChunk + 2 * kNumBuckets;
-      if (compact < p.imp_chunks) {
-        p.imp_chunks = compact;
-        p.imp_compact = 1;
-      }
-    }
   }
   if (with_append) {
     AppendParams& a = p.app;
@@ -157,11 +166,9 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
     const long long warps = (long long)a.rows * desc->num_kv_heads * 2;
     p.append_blocks = (int)((warps + kPostThreads / 32 - 1) / (kPostThreads / 32));
   }
-  const int grid = p.combine_blocks + p.imp_chunks * desc->num_seqs + p.append_blocks;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool dep = g_dependent_launch.load() == 1 || g_dependent_launch.load() == 3;
-  const bool few = importance_few(num_q_heads, grid, num_ctas), vec = !with_importance || importance_aligned(p.imp);
-  if (desc->head_dim == 128) launch_post<4>(p, few, vec, grid, st, dep);
-  else launch_post<2>(p, few, vec, grid, st, dep);
+  if (desc->head_dim == 128) launch_post<4>(p, max_seq_tokens, st, dep);
+  else launch_post<2>(p, max_seq_tokens, st, dep);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

@@ -19,7 +19,7 @@ constexpr int kPostThreads = 256;
 constexpr int kCombineChunk = 256;
 constexpr int kMaxQHeads = 128;
 
-int attn_live_partials(const SkvStoreDesc* desc, int query_dtype);  // decode_attention.cu
+bool attn_first_of_run(const SkvStoreDesc* desc, int query_dtype);  // decode_attention.cu
 
 __host__ __device__ inline int partial_stride(int group, int head_dim) { return group * (head_dim + 2); }
 
@@ -39,7 +39,7 @@ struct CombineParams {
   int group;
   const float* partials;
   int per_run;  // partials a run has room for
-  int live;     // the first of them, which the attention launch fills (per_run or 2)
+  bool first_of_run;  // only the first of them is filled, and of a segment's last run the second (fp16 queries)
   int num_ctas;
   const void* cur_k;
   const void* cur_v;
@@ -89,20 +89,23 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
   const bool valid = gq < G;
   const int gqc = valid ? gq : G - 1;  // threads of a missing head go through the motions of the last one
   const PlanView pv = plan_view(const_cast<int*>(p.plan), p.num_ctas, g.num_seqs * Hkv);
-  const int nsplit = pv.seg_count[seg] * p.live;
-  const int r0 = nsplit > 0 ? pv.seg_begin[seg] * p.per_run : 0;
+  const int runs = pv.seg_count[seg];
+  const int nsplit = runs == 0 ? 0 : p.first_of_run ? runs + 1 : runs * p.per_run;
+  const int r0 = runs > 0 ? pv.seg_begin[seg] * p.per_run : 0;
   const int pstride = partial_stride(G, D);
-  const bool two = p.live == 2;
-  auto at = [&](int k) { return (long long)(two ? (k >> 1) * p.per_run + (k & 1) : k) * pstride; };  // k-th filled partial
+  // the k-th filled partial, in floats from the segment's first (its runs are at most one a CTA)
+  const int step = (p.first_of_run ? p.per_run : 1) * pstride, last = (runs - 1) * step + pstride;
+  auto at = [&](int k) { return p.first_of_run && k == runs ? last : k * step; };
   const float* base = p.partials + (long long)r0 * pstride + gqc * (D + 2);
   const bool has_cur = p.cur_k != nullptr && p.cur_v != nullptr;
   const long long hq = (long long)b * p.num_q_heads + h * G + gqc;
   const long long kv = ((long long)b * Hkv + h) * D + d;
 
-  // kRowsAhead rows at a time, their loads in flight together and the first of them beside the headers: a segment has two
-  // partials a run, and a loop over as many rows with a load each waits for every one (segments of 12 and of 40 partials: the
-  // last block ended 7.0 and 14.2 us after the attention launch, 4.5 and 9.3 with the rows in flight)
-  constexpr int kRowsAhead = 16;
+  // kRowsAhead rows at a time, their loads in flight together and the first of them beside the headers: a loop over the rows
+  // with a load each waits for every one (segments of 12 and of 40 partials: the last block ended 7.0 and 14.2 us after
+  // the attention launch, now 4.3 and 8 us).  Eight: sixteen and twenty-four cost more in code and registers than the
+  // round trips they save (steps of 8 x 770 keys 266 us, 274, 288).
+  constexpr int kRowsAhead = 8;
   float x[kRowsAhead];
   auto fetch = [&](int k0) {
 #pragma unroll
@@ -228,22 +231,20 @@ struct ImportanceShared {
   float cprob[kMaxQHeads];  // pc (unnormalised probability of the current token)
 };
 
-// An importance block updates kImpChunk consecutive storage indices of a sequence, four per thread.
-constexpr int kImpChunk = 4 * kPostThreads;
-
-// Maps the j-th *live* chunk of sequence b (chunks of kImpChunk storage indices that hold a cached
+// Maps the j-th *live* chunk of sequence b (chunks of CHUNK storage indices that hold a cached
 // key or the slot the current token will take) to its chunk index; -1 when j is past the last one.
 // Buckets lie at increasing storage indices, so their chunk ranges are increasing and only neighbours can
 // share a chunk.  j == 0 always maps to a chunk (chunk 0 if nothing is live): that block publishes the
 // head-importance EMA.
+template <int CHUNK>
 __device__ __forceinline__ int live_chunk(const StoreGeom& g, const int32_t* counts4, int j) {
   int prev_last = -1, seen = 0;
 #pragma unroll
   for (int i = 0; i < kNumBuckets; ++i) {
     const int cnt = counts4[i] + 1;  // + the slot a token appended this step would take
     if (g.cap[i] == 0) continue;
-    int first = g.bucket_base[i] / kImpChunk;
-    const int last = (g.bucket_base[i] + cnt - 1) / kImpChunk;
+    int first = g.bucket_base[i] / CHUNK;
+    const int last = (g.bucket_base[i] + cnt - 1) / CHUNK;
     if (first <= prev_last) first = prev_last + 1;
     if (last >= first) {
       const int n = last - first + 1;
@@ -271,47 +272,55 @@ __device__ __forceinline__ ImportanceSeq importance_seq(const ImportanceParams& 
   return q;
 }
 
-// `VEC` loads and stores of the four consecutive elements of a thread (the arrays are aligned for it), or one by one.
-template <bool VEC>
-__device__ __forceinline__ void load4(const float* p, float (&x)[4]) {
-  if constexpr (VEC) {
+// How an importance block works: KPT consecutive storage indices a thread, HEADS rows of logits in flight, and whether the
+// arrays are aligned for loads of four elements (they are the caller's).
+template <int KPT_, int HEADS_, bool VEC_>
+struct ImpShape {
+  static constexpr int KPT = KPT_, HEADS = HEADS_, CHUNK = KPT * kPostThreads;
+  static constexpr bool VEC = VEC_;
+  static_assert(KPT == 1 || KPT == 4, "one or four indices a thread");
+};
+template <class S>
+__device__ __forceinline__ void load_k(const float* p, float (&x)[S::KPT]) {
+  if constexpr (S::VEC && S::KPT == 4) {
     const float4 v = *reinterpret_cast<const float4*>(p);
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = p[i];
+    for (int i = 0; i < S::KPT; ++i) x[i] = p[i];
   }
 }
-template <bool VEC>
-__device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
-  if constexpr (VEC) {
+template <class S>
+__device__ __forceinline__ void load_k(const double* p, double (&x)[S::KPT]) {
+  if constexpr (S::VEC && S::KPT == 4) {
     const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
     x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = p[i];
+    for (int i = 0; i < S::KPT; ++i) x[i] = p[i];
   }
 }
-template <bool VEC>
-__device__ __forceinline__ void load4(const uint8_t* p, uint8_t (&x)[4]) {
-  if constexpr (VEC) {
+template <class S>
+__device__ __forceinline__ void load_k(const uint8_t* p, uint8_t (&x)[S::KPT]) {
+  if constexpr (S::VEC && S::KPT == 4) {
     const uchar4 v = *reinterpret_cast<const uchar4*>(p);
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = p[i];
+    for (int i = 0; i < S::KPT; ++i) x[i] = p[i];
   }
 }
 
 // One chunk of sequence b; blockDim.x == kPostThreads.  `publish` marks the one block per sequence that writes the new
-// head-importance EMA.  HEADS: logits rows in flight per thread.
+// head-importance EMA.
 //
 // Bound: round trips to memory, three one after the other (counts; state, (max, sum) and the first logits; the other logits)
-// for few bytes a thread.  So a thread takes four consecutive keys with 16-byte loads, every load that needs no weight is
-// issued before the weights are worked out, and the grid is one wave where a key a thread took several.  64 x 16384 keys, 8
-// heads: from the end of the attention launch to the last block's 29 us -> 19; 8 x 770, 32 heads 5.4 -> 5 (latency).
-template <int HEADS, bool VEC>
+// for few bytes a thread.  So every load that needs no weight is issued before the weights are worked out, and a launch of more
+// than a wave of single indices takes four consecutive ones a thread with 16-byte loads.  64 x 16384 keys, 8 heads: from
+// the end of the attention launch to the last block's 29 us -> 19.
+template <class S>
 __device__ __forceinline__ void importance_block(const ImportanceParams& p, int chunk, int b, bool publish, ImportanceShared& sh) {
+  constexpr int KPT = S::KPT, HEADS = S::HEADS;
   const StoreGeom& g = p.g;
   const int tid = threadIdx.x, Hq = p.num_q_heads;
   const ImportanceSeq q = importance_seq(p, b);
@@ -319,15 +328,15 @@ __device__ __forceinline__ void importance_block(const ImportanceParams& p, int 
 #pragma unroll
   for (int i = 0; i < kNumBuckets; ++i) total_keys += q.cnt[i];
 
-  // The thread's four storage indices s .. s + 3 lie in one bucket (capacities are multiples of 128): those before `live` hold
+  // The thread's storage indices s .. s + KPT - 1 lie in one bucket (capacities are multiples of 128): those before `live` hold
   // cached keys, `cur` is the one the current token will lie at.
-  const int s = chunk * kImpChunk + 4 * tid;
+  const int s = chunk * S::CHUNK + KPT * tid;
   int live = 0;
 #pragma unroll
   for (int i = 0; i < kNumBuckets; ++i)
     if (s >= g.bucket_base[i] && s < g.bucket_base[i] + g.cap[i]) live = q.cnt[i] - (s - g.bucket_base[i]);
   const int cur = q.has_cur ? q.cur_slot - s : -1;
-  const bool with_cur = cur >= 0 && cur < 4 && cur >= live;
+  const bool with_cur = cur >= 0 && cur < KPT && cur >= live;
   const bool active = live > 0 || with_cur;
   // most storage indices of a sequence are unused capacity: a block without a live key leaves at once
   // (the publishing block of every sequence stays)
@@ -346,20 +355,22 @@ __device__ __forceinline__ void importance_block(const ImportanceParams& p, int 
   }
   const long long ci = (long long)b * g.slots + s;
   const long long li = ((long long)p.layer * g.num_seqs + b) * g.slots + s;
-  double cum[4];
-  float ema[4], mass[4] = {0.f, 0.f, 0.f, 0.f};
-  uint8_t seen[4];
+  double cum[KPT];
+  float ema[KPT], mass[KPT];
+  uint8_t seen[KPT];
+#pragma unroll
+  for (int i = 0; i < KPT; ++i) mass[i] = 0.f;
   if (active) {
-    load4<VEC>(p.cumulative + ci, cum);
-    load4<VEC>(p.layer_ema + li, ema);
-    load4<VEC>(p.touched + li, seen);
+    load_k<S>(p.cumulative + ci, cum);
+    load_k<S>(p.layer_ema + li, ema);
+    load_k<S>(p.touched + li, seen);
   }
   const float* lg = p.logits + (long long)b * Hq * g.slots + s;
-  float x[HEADS][4];
+  float x[HEADS][KPT];
   auto fetch = [&](int h0) {
 #pragma unroll
     for (int h = 0; h < HEADS; ++h)
-      if (h0 + h < Hq) load4<VEC>(lg + (long long)(h0 + h) * g.slots, x[h]);
+      if (h0 + h < Hq) load_k<S>(lg + (long long)(h0 + h) * g.slots, x[h]);
   };
   if (live > 0) fetch(0);
 
@@ -397,7 +408,7 @@ __device__ __forceinline__ void importance_block(const ImportanceParams& p, int 
         if (h0 + h < Hq) {
           const float wv = sh.w[h0 + h], mv = sh.mx[h0 + h];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) mass[i] += wv * ex2f(x[h][i] - mv);
+          for (int i = 0; i < KPT; ++i) mass[i] += wv * ex2f(x[h][i] - mv);
         }
       }
     }
@@ -408,23 +419,25 @@ __device__ __forceinline__ void importance_block(const ImportanceParams& p, int 
 #pragma unroll 8
     for (int h = 0; h < Hq; ++h) m += sh.w[h] * sh.cprob[h];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < KPT; ++i)
       if (i == cur) mass[i] = m;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < KPT; ++i) {
     cum[i] += (double)mass[i];
     ema[i] = seen[i] ? p.decay * ema[i] + (1.0f - p.decay) * mass[i] : mass[i];
   }
-  if (VEC && live >= 4) {
-    *reinterpret_cast<double2*>(p.cumulative + ci) = make_double2(cum[0], cum[1]);
-    *reinterpret_cast<double2*>(p.cumulative + ci + 2) = make_double2(cum[2], cum[3]);
-    *reinterpret_cast<float4*>(p.layer_ema + li) = make_float4(ema[0], ema[1], ema[2], ema[3]);
-    if (!(seen[0] && seen[1] && seen[2] && seen[3])) *reinterpret_cast<uchar4*>(p.touched + li) = make_uchar4(1, 1, 1, 1);
-    return;
+  if constexpr (S::VEC && KPT == 4) {
+    if (live >= 4) {
+      *reinterpret_cast<double2*>(p.cumulative + ci) = make_double2(cum[0], cum[1]);
+      *reinterpret_cast<double2*>(p.cumulative + ci + 2) = make_double2(cum[2], cum[3]);
+      *reinterpret_cast<float4*>(p.layer_ema + li) = make_float4(ema[0], ema[1], ema[2], ema[3]);
+      if (!(seen[0] && seen[1] && seen[2] && seen[3])) *reinterpret_cast<uchar4*>(p.touched + li) = make_uchar4(1, 1, 1, 1);
+      return;
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < KPT; ++i) {
     if (i < live || (with_cur && i == cur)) {
       p.cumulative[ci + i] = cum[i];
       p.layer_ema[li + i] = ema[i];
@@ -433,17 +446,21 @@ __device__ __forceinline__ void importance_block(const ImportanceParams& p, int 
   }
 }
 
-// Heads in flight per thread.  Sixteen (118 registers, two blocks an SM) where there are more than eight and the launch still
-// fits one wave that way, else eight (80 registers, three blocks).  Steps, us, sixteen / eight: 8 x 770 keys, 32 heads
-// 303 / 313; 16 x 8192, 32 heads (448 blocks) 1705 / 1658.
-__host__ __device__ constexpr int imp_heads(bool few) { return few ? 8 : 16; }
-inline bool importance_few(int num_q_heads, long long blocks, int sms) { return num_q_heads <= 8 || blocks > 2LL * sms; }
-// Both forms of loads are there because the arrays are the caller's.
 inline bool importance_aligned(const ImportanceParams& p) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p.logits) | reinterpret_cast<uintptr_t>(p.cumulative) |
                       reinterpret_cast<uintptr_t>(p.layer_ema);
   return a % 16 == 0 && reinterpret_cast<uintptr_t>(p.touched) % 4 == 0;
 }
+// Single indices with all of 32 heads in flight where their blocks fit one wave of four an SM; else four indices a thread,
+// with sixteen heads in flight (118 registers, two blocks an SM) where there are more than eight and the launch fits one wave
+// that way, with eight (80 registers, three blocks) otherwise.  Steps, us: 8 x 770 keys, 32 heads, 22 layers: single 276, four
+// 317; 16 x 8192, 32 heads: four with eight heads 1603, with sixteen 1705, two with sixteen 1617; 64 x 16384, 8 heads:
+// four 1253, two 1402.
+using ImpOne = ImpShape<1, 32, false>;
+template <bool VEC>
+using ImpFour16 = ImpShape<4, 16, VEC>;
+template <bool VEC>
+using ImpFour8 = ImpShape<4, 8, VEC>;
 
 // ---- append ---------------------------------------------------------------------------------------------
 struct AppendParams {
