@@ -8,8 +8,8 @@
 
 namespace skv {
 
-// ---- eight consecutive elements per lane, head_dim / 8 lanes per row ---------------------------------------------------
-// The bulk paths (append of a prompt, rows moved by a reallocation) give a lane 8 consecutive elements, so that two or four rows
+// ---- groups of eight consecutive elements per lane -----------------------------------------------------------------------
+// The bulk paths give a lane one (rows moved by a reallocation) or two (append of a prompt) such groups, so that several rows
 // share a warp's instructions, and run everything per element on two elements at once (fma.rn.f32x2; element i is paired
 // with i + 4) and on the multiply-add pipe: those kernels are bound by issue slots and by the half-rate integer pipe that
 // compares, selects and byte permutes go through.
@@ -35,12 +35,12 @@ static __constant__ WidthConst kWidthConst[kNumBuckets] = {
     {127.f, 1.f / 127.f, 256.f, 8388736.f, 0u, 8},
 };
 
-// Quantises the row held by LPR lanes (8 elements each; `amax`: this lane's largest magnitude) at the width of `bucket`.  Returns
-// the row's scale, and this lane's packed field of 8 * bits bits: (lo, hi) at 8 bits, lo otherwise.  Bit-exact with
-// scale_of / quantize_vals; a lane with a near-tie, a NaN or a scale outside the normal range redoes its values with the
-// division, as those do.
-template <int LPR>
-__device__ __forceinline__ float quantize8(const float (&x)[8], float amax, int bucket, uint32_t& lo, uint32_t& hi) {
+// Quantises the row held by LPR lanes (G groups of 8 elements each; `amax`: this lane's largest magnitude) at the width of
+// `bucket`.  Returns the row's scale, and of each group the packed field of 8 * bits bits: (lo, hi) at 8 bits, lo otherwise.
+// Bit-exact with scale_of / quantize_vals; a lane with a near-tie, a NaN or a scale outside the normal range redoes its values
+// with the division, as those do.
+template <int LPR, int G>
+__device__ __forceinline__ float quantize_groups(const float (&x)[G][8], float amax, int bucket, uint32_t (&lo)[G], uint32_t (&hi)[G]) {
   const WidthConst& wc = kWidthConst[bucket];
 #pragma unroll
   for (int o = LPR / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -55,36 +55,54 @@ __device__ __forceinline__ float quantize8(const float (&x)[8], float amax, int 
   const float rc = rcp_approx(scale);
   const float up = rc * (1.f + 0x1p-20f), dn = rc * (1.f - 0x1p-20f);
   const uint64_t up2 = f32x2(up, up), dn2 = f32x2(dn, dn), magic2 = f32x2(kRoundMagic, kRoundMagic), neg2 = f32x2(-1.f, -1.f);
-  uint64_t nq[4], diff = 0ull;  // the negated codes of elements i and i + 4, as floats
+  uint64_t nq[G][4], diff = 0ull;  // the negated codes of elements i and i + 4, as floats
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint64_t x2 = f32x2(x[i], x[i + 4]);
-    const uint64_t m = f32x2_fma(x2, up2, magic2), d = f32x2_fma(f32x2_fma(x2, dn2, magic2), neg2, m);
-    diff = f32x2_fma(d, d, diff);
-    nq[i] = f32x2_fma(m, neg2, magic2);
+  for (int j = 0; j < G; ++j) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t x2 = f32x2(x[j][i], x[j][i + 4]);
+      const uint64_t m = f32x2_fma(x2, up2, magic2), d = f32x2_fma(f32x2_fma(x2, dn2, magic2), neg2, m);
+      diff = f32x2_fma(d, d, diff);
+      nq[j][i] = f32x2_fma(m, neg2, magic2);
+    }
   }
   const float2 dd = f32x2_parts(diff);
   const bool exact = !(scale >= 1e-30f && scale <= 1e30f && dd.x + dd.y == 0.f);
   if (exact) {
     const float fhi = wc.levels, flo = -fhi - 1.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      nq[i] = f32x2(-fminf(fmaxf(rintf(__fdiv_rn(x[i], scale)), flo), fhi),
-                    -fminf(fmaxf(rintf(__fdiv_rn(x[i + 4], scale)), flo), fhi));
+    for (int j = 0; j < G; ++j) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        nq[j][i] = f32x2(-fminf(fmaxf(rintf(__fdiv_rn(x[j][i], scale)), flo), fhi),
+                         -fminf(fmaxf(rintf(__fdiv_rn(x[j][i + 4], scale)), flo), fhi));
+    }
   }
   const uint64_t base2 = f32x2(wc.base, wc.base);
-  if (bucket == 3) {  // two's complement bytes: pairs of codes joined, offset so that no byte borrows from the next, flipped back
-    const float2 a = f32x2_parts(f32x2_add(f32x2_fma(nq[1], base2, nq[0]), magic2));
-    const float2 b = f32x2_parts(f32x2_add(f32x2_fma(nq[3], base2, nq[2]), magic2));
-    constexpr uint32_t m = 0x4B400000u, o = 0x80808080u;
-    lo = ((m + o - __float_as_uint(a.x)) + ((m - __float_as_uint(b.x)) << 16)) ^ o;
-    hi = ((m + o - __float_as_uint(a.y)) + ((m - __float_as_uint(b.y)) << 16)) ^ o;
-  } else {  // four codes each as a polynomial in 2^bits, made non-negative by the offset of every code, then joined
-    const float2 poly = f32x2_parts(f32x2_add(
-        f32x2_fma(f32x2_fma(f32x2_fma(nq[3], base2, nq[2]), base2, nq[1]), base2, nq[0]), magic2));
-    lo = (wc.off - __float_as_uint(poly.x)) + ((wc.off - __float_as_uint(poly.y)) << (4 * wc.bits));
-    hi = 0u;
+#pragma unroll
+  for (int j = 0; j < G; ++j) {
+    const uint64_t (&n)[4] = nq[j];
+    if (bucket == 3) {  // two's complement bytes: pairs of codes joined, offset so that no byte borrows from the next, flipped back
+      const float2 a = f32x2_parts(f32x2_add(f32x2_fma(n[1], base2, n[0]), magic2));
+      const float2 b = f32x2_parts(f32x2_add(f32x2_fma(n[3], base2, n[2]), magic2));
+      constexpr uint32_t m = 0x4B400000u, o = 0x80808080u;
+      lo[j] = ((m + o - __float_as_uint(a.x)) + ((m - __float_as_uint(b.x)) << 16)) ^ o;
+      hi[j] = ((m + o - __float_as_uint(a.y)) + ((m - __float_as_uint(b.y)) << 16)) ^ o;
+    } else {  // four codes each as a polynomial in 2^bits, made non-negative by the offset of every code, then joined
+      const float2 poly = f32x2_parts(f32x2_add(
+          f32x2_fma(f32x2_fma(f32x2_fma(n[3], base2, n[2]), base2, n[1]), base2, n[0]), magic2));
+      lo[j] = (wc.off - __float_as_uint(poly.x)) + ((wc.off - __float_as_uint(poly.y)) << (4 * wc.bits));
+      hi[j] = 0u;
+    }
   }
+  return scale;
+}
+template <int LPR>
+__device__ __forceinline__ float quantize8(const float (&x)[8], float amax, int bucket, uint32_t& lo, uint32_t& hi) {
+  uint32_t l[1], h[1];
+  const float scale = quantize_groups<LPR, 1>(reinterpret_cast<const float (&)[1][8]>(x), amax, bucket, l, h);
+  lo = l[0];
+  hi = h[0];
   return scale;
 }
 
@@ -101,6 +119,29 @@ __device__ __forceinline__ void store_field8(uint8_t* row, int bucket, int l, ui
     const int q = l & 3;
     const uint32_t word = q == 0 ? (lo | (next << 24)) : q == 1 ? ((lo >> 8) | (next << 16)) : ((lo >> 16) | (next << 8));
     if (q < 3) out[3 * (l >> 2) + q] = word;
+  }
+}
+
+// The same for a lane that holds two neighbouring groups (lane l of the row's head_dim / 16; `next` = lo[0] of the next lane).
+__device__ __forceinline__ void store_field16(uint8_t* row, int bucket, int l, const uint32_t (&lo)[2], const uint32_t (&hi)[2],
+                                              uint32_t next) {
+  uint32_t* out = reinterpret_cast<uint32_t*>(row);
+  if (bucket == 3) {
+    uint2* w = reinterpret_cast<uint2*>(out) + 2 * l;  // a store is asked for no more than 8-byte alignment here
+    w[0] = make_uint2(lo[0], hi[0]);
+    w[1] = make_uint2(lo[1], hi[1]);
+  } else if (bucket == 2) {
+    reinterpret_cast<uint2*>(out)[l] = make_uint2(lo[0], lo[1]);
+  } else if (bucket == 0) {
+    out[l] = lo[0] | (lo[1] << 16);
+  } else {  // 3 bits: two lanes' 48 bits make three words
+    uint32_t* w = out + 3 * (l >> 1);
+    if (l & 1) {
+      w[2] = (lo[0] >> 16) | (lo[1] << 8);
+    } else {
+      w[0] = lo[0] | (lo[1] << 24);
+      w[1] = (lo[1] >> 8) | (next << 16);
+    }
   }
 }
 

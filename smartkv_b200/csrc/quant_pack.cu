@@ -21,24 +21,26 @@ __global__ void quantize_pack_append_kernel(const AppendParams p) {
   append_row<EPL>(p, warp, lane);
 }
 
-// The same for inputs on a 16-byte boundary (whole rows are 128 bytes or more, so the base decides): a lane takes 8
-// consecutive elements in one or two 16-byte loads, head_dim / 8 lanes make a row, and the K and the V row of one
-// (token, KV head) go through the same instructions side by side, NPASS groups of them in flight per warp.
+// The same for inputs on a 16-byte boundary (whole rows are 128 bytes or more, so the base decides): a lane takes 16
+// consecutive elements in 16-byte loads, head_dim / 16 lanes make a row, and the K and the V rows of two or four
+// (token, KV head) pairs go through the same instructions side by side, NPASS groups of them in flight per warp.
 //
-// What bounds it is issue slots: with a row per warp, 282 warp instructions a row, 16 x 8192 x 8 rows of head_dim 128
-// took 638 us for 0.72 GB; now 260 us (quantize8; 64 registers, so that 32 warps fit an SM: a ninth slower with 24).  One or two
-// groups in flight per warp instead of four: a twentieth slower and more.
+// What bounds it is issue slots, so what is done once per lane or per row (row lookup, largest value, scale, stores) is spread
+// over more elements: 16 x 8192 x 8 rows of head_dim 128 (0.72 GB) took 638 us with a row per warp, 260 with 8 elements a
+// lane, 192 with 16.  Two groups in flight at 64 registers (four CTAs an SM); three CTAs 217, one group 235, four groups and
+// three CTAs 196.
 template <int D, bool HALF, int NPASS>
 __global__ void __launch_bounds__(256, 4) append_bulk_kernel(const AppendParams p) {
-  constexpr int LPR = D / 8;               // lanes per row
-  constexpr int PPP = 32 / (2 * LPR);      // (token, head) pairs per pass: 1 or 2
+  constexpr int LPR = D / 16;              // lanes per row
+  constexpr int PPP = 32 / (2 * LPR);      // (token, head) pairs per pass: 2 or 4
+  constexpr int LD = HALF ? 2 : 4;         // 16-byte loads per lane
   const StoreGeom& g = p.g;
   const int lane = threadIdx.x & 31, l = lane & (LPR - 1), which = (lane / LPR) & 1, sub = lane / (2 * LPR);
   const long long pairs = (long long)p.rows * g.num_kv_heads;
   const long long first = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (NPASS * PPP);
   if (first >= pairs) return;
 
-  uint4 raw[NPASS][HALF ? 1 : 2];
+  uint4 raw[NPASS][LD];
   int seq[NPASS], bucket[NPASS], pos[NPASS], head[NPASS];
   int r, h;
   if ((first + NPASS * PPP) >> 31) {  // 64-bit division is a long subroutine: only where the row count needs it
@@ -48,59 +50,59 @@ __global__ void __launch_bounds__(256, 4) append_bulk_kernel(const AppendParams 
     r = ((int)first + sub) / g.num_kv_heads;
     h = ((int)first + sub) - r * g.num_kv_heads;
   }
-  const uint8_t* src = static_cast<const uint8_t*>(which ? p.v : p.k) + ((first + sub) * D + l * 8) * (HALF ? 2 : 4);
+  const uint8_t* src = static_cast<const uint8_t*>(which ? p.v : p.k) + ((first + sub) * D + l * 16) * (HALF ? 2 : 4);
 #pragma unroll
   for (int u = 0; u < NPASS; ++u) {
     const bool in = first + u * PPP + sub < pairs;
     const uint4* s = reinterpret_cast<const uint4*>(src + (long long)u * PPP * D * (HALF ? 2 : 4));
 #pragma unroll
-    for (int i = 0; i < (HALF ? 1 : 2); ++i) raw[u][i] = in ? s[i] : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < LD; ++i) raw[u][i] = in ? s[i] : make_uint4(0u, 0u, 0u, 0u);
     seq[u] = in ? p.dst_seq[r] : -1;
     bucket[u] = in ? p.dst_bucket[r] : 0;
     pos[u] = in ? p.dst_pos[r] : 0;
     head[u] = h;
     h += PPP;
-    while (h >= g.num_kv_heads) {  // at most twice (one KV head, two pairs per pass)
+    while (h >= g.num_kv_heads) {  // at most four times (one KV head, four pairs per pass)
       h -= g.num_kv_heads;
       ++r;
     }
   }
 #pragma unroll
   for (int u = 0; u < NPASS; ++u) {
-    float x[8], amax = 0.f;
+    float x[2][8], amax = 0.f;
     if constexpr (HALF) {
-      const uint32_t w[4] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w};
+      const uint32_t w[8] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w, raw[u][1].x, raw[u][1].y, raw[u][1].z, raw[u][1].w};
       __half2 m2 = __habs2(bits_h2(w[0]));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 8; ++i) {
         if (i) m2 = __hmax2(m2, __habs2(bits_h2(w[i])));  // the number wins over a NaN, as in fmaxf
         const float2 f = __half22float2(bits_h2(w[i]));
-        x[2 * i] = f.x;
-        x[2 * i + 1] = f.y;
+        x[i / 4][2 * (i % 4)] = f.x;
+        x[i / 4][2 * (i % 4) + 1] = f.y;
       }
       const float2 f = __half22float2(m2);
       amax = fmaxf(fmaxf(amax, f.x), f.y);
     } else {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        x[4 * i] = __uint_as_float(raw[u][i].x);
-        x[4 * i + 1] = __uint_as_float(raw[u][i].y);
-        x[4 * i + 2] = __uint_as_float(raw[u][i].z);
-        x[4 * i + 3] = __uint_as_float(raw[u][i].w);
+      for (int i = 0; i < LD; ++i) {
+        x[i / 2][4 * (i % 2)] = __uint_as_float(raw[u][i].x);
+        x[i / 2][4 * (i % 2) + 1] = __uint_as_float(raw[u][i].y);
+        x[i / 2][4 * (i % 2) + 2] = __uint_as_float(raw[u][i].z);
+        x[i / 2][4 * (i % 2) + 3] = __uint_as_float(raw[u][i].w);
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
+      for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(x[i / 8][i % 8]));
     }
     const bool valid = seq[u] >= 0 && seq[u] < g.num_seqs && bucket[u] >= 0 && bucket[u] < kNumBuckets && pos[u] >= 0 &&
                        pos[u] < g.cap[bucket[u] & 3];
     const int bk = bucket[u] & 3;
-    uint32_t lo, up;
-    const float scale = quantize8<LPR>(x, amax, bk, lo, up);
+    uint32_t lo[2], up[2];
+    const float scale = quantize_groups<LPR, 2>(x, amax, bk, lo, up);
     uint8_t* arena = arena_ptr(g, p.store, p.layer, valid ? seq[u] : 0);
     const long long row = (long long)head[u] * g.cap[bk] + pos[u];
-    const uint32_t next = __shfl_down_sync(0xffffffffu, lo, 1);
+    const uint32_t next = __shfl_down_sync(0xffffffffu, lo[0], 1);
     if (valid) {
-      store_field8(arena + (which ? g.v_off[bk] : g.k_off[bk]) + row * g.row_bytes[bk], bk, l, lo, up, next);
+      store_field16(arena + (which ? g.v_off[bk] : g.k_off[bk]) + row * g.row_bytes[bk], bk, l, lo, up, next);
       if (l == 0) {
         reinterpret_cast<float*>(arena + g.sc_off[bk])[2 * row + which] = scale;
         if (which) note_v_scale(g, arena, scale);
@@ -113,13 +115,13 @@ __global__ void __launch_bounds__(256, 4) append_bulk_kernel(const AppendParams 
 
 template <int D, bool HALF>
 static void launch_append_bulk(const AppendParams& p, cudaStream_t st) {
-  constexpr int PPP = 128 / D, WPB = 8;
+  constexpr int PPP = 256 / D, WPB = 8;
   const long long pairs = (long long)p.rows * p.g.num_kv_heads;
-  // Four groups in flight per warp once that still leaves every SM several full blocks; below, one group per warp is the
+  // Two groups in flight per warp once that still leaves every SM several full blocks; below, one group per warp is the
   // shorter chain.
   if (pairs >= 65536) {
-    const long long per_block = (long long)WPB * 4 * PPP;
-    append_bulk_kernel<D, HALF, 4><<<(unsigned)((pairs + per_block - 1) / per_block), WPB * 32, 0, st>>>(p);
+    const long long per_block = (long long)WPB * 2 * PPP;
+    append_bulk_kernel<D, HALF, 2><<<(unsigned)((pairs + per_block - 1) / per_block), WPB * 32, 0, st>>>(p);
   } else {
     const long long per_block = (long long)WPB * PPP;
     append_bulk_kernel<D, HALF, 1><<<(unsigned)((pairs + per_block - 1) / per_block), WPB * 32, 0, st>>>(p);
