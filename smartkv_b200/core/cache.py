@@ -170,6 +170,7 @@ class SmartKVCache:
         self._layer_tokens: List[set] = [set() for _ in range(self.num_layers)]
         self._realloc_due = False
         self._dev_base = torch.zeros_like(self.store.cumulative)        # device importance already in the tracker
+        self._new_slots: List[Tuple[int, int, Optional[float]]] = []    # (storage index, token id, importance) not yet on the device
 
     def _pending_tokens(self) -> bool:
         return any(self._committed[b] < len(self._bucket_tokens[b]) for b in range(NUM_BUCKETS))
@@ -201,8 +202,25 @@ class SmartKVCache:
         self._layers_of[token_id] = set()
         return bucket, pos
 
+    def _enter_slots(self):
+        """Puts the tokens placed by _assign_slot on the device: one indexed write per array instead of
+        a launch per token."""
+        new, self._new_slots = self._new_slots, []
+        if not new:
+            return
+        st, dev = self.store, self._dev
+        at, tids = torch.tensor([[i for i, _, _ in new], [t for _, t, _ in new]], dtype=torch.int32).to(dev)
+        st.slot_token[0].index_put_((at.long(),), tids)
+        seeded = [(i, x) for i, _, x in new if x is not None]
+        if seeded:   # importance gathered before the token had a place in the store
+            idx = torch.tensor([i for i, _ in seeded], dtype=torch.int64).to(dev)
+            seed = torch.tensor([x for _, x in seeded], dtype=torch.float64).to(dev)
+            st.cumulative[0].index_put_((idx,), seed)
+            self._dev_base[0].index_put_((idx,), seed)
+
     def _grow(self):
         """Doubles the capacity: a new store, every stored row copied across as codes + scales."""
+        self._enter_slots()
         old = self.store
         old_slot, old_bucket_tokens = dict(self._slot), [list(t) for t in self._bucket_tokens]
         old_layers, old_committed = {t: set(s) for t, s in self._layers_of.items()}, list(self._committed)
@@ -275,32 +293,30 @@ class SmartKVCache:
         elif v.dtype != k.dtype:
             v = v.to(k.dtype)
         buckets, poss = [], []
-        for tid in ids:
-            if tid not in self._slot:
-                bits = self.precision_map.get(tid, 4)
-                if bits not in BITS_TO_BUCKET:
-                    raise ValueError(f"token {tid} has width {bits}; the store holds 2, 3, 4 or 8 bits")
-                self.precision_map.setdefault(tid, bits)
-                bucket, pos = self._assign_slot(tid, bits)
-                self.store.slot_token[0, self.store.bucket_base[bucket] + pos] = tid
-                seed = self.importance_tracker.token_importance.get(tid)
-                if seed is not None:   # importance gathered before the token had a place in the store
-                    idx = self.store.bucket_base[bucket] + pos
-                    self.store.cumulative[0, idx] = seed
-                    self._dev_base[0, idx] = seed
-            bucket, pos = self._slot[tid]
-            buckets.append(bucket)
-            poss.append(pos)
-        dev = self._dev
-        seq = torch.zeros(n, dtype=torch.int32, device=dev)
-        self.store.append(layer_idx, k, v, seq, torch.tensor(buckets, dtype=torch.int32, device=dev),
-                          torch.tensor(poss, dtype=torch.int32, device=dev))
+        slot, base = self._slot, self.store.bucket_base
+        try:
+            for tid in ids:
+                if tid not in slot:
+                    bits = self.precision_map.get(tid, 4)
+                    if bits not in BITS_TO_BUCKET:
+                        raise ValueError(f"token {tid} has width {bits}; the store holds 2, 3, 4 or 8 bits")
+                    self.precision_map.setdefault(tid, bits)
+                    bucket, pos = self._assign_slot(tid, bits)
+                    slot, base = self._slot, self.store.bucket_base      # of the new store, if there was no room
+                    self._new_slots.append((base[bucket] + pos, tid, self.importance_tracker.token_importance.get(tid)))
+                bucket, pos = slot[tid]
+                buckets.append(bucket)
+                poss.append(pos)
+        finally:
+            self._enter_slots()
+        seq, dst_bucket, dst_pos = torch.tensor([[0] * n, buckets, poss], dtype=torch.int32).to(self._dev)
+        self.store.append(layer_idx, k, v, seq, dst_bucket, dst_pos)
+        k_cache, v_cache, layers_of = self.k_cache, self.v_cache, self._layers_of
         for tid, bucket in zip(ids, buckets):
-            meta = {"bits": BUCKET_BITS[bucket], "token_id": tid, "layer": layer_idx}
-            self.k_cache[(layer_idx, tid)] = meta
-            self.v_cache[(layer_idx, tid)] = meta
-            self._layers_of[tid].add(layer_idx)
-            self._layer_tokens[layer_idx].add(tid)
+            k_cache[(layer_idx, tid)] = v_cache[(layer_idx, tid)] = {"bits": BUCKET_BITS[bucket], "token_id": tid,
+                                                                     "layer": layer_idx}
+            layers_of[tid].add(layer_idx)
+        self._layer_tokens[layer_idx].update(ids)
         self.total_tokens_stored += n
         self.token_counter += n
         self._advance_commits()
@@ -616,15 +632,16 @@ class SmartKVCache:
         self._realloc_due = False
         st = self.store
         self._pull_device_importance()
-        new_bits = torch.zeros(st.slots, dtype=torch.uint8)
-        moved = False
+        new_bits = bytearray(st.slots)
+        moved = []
         for tid, (bucket, pos) in self._slot.items():
             bits = self.precision_map.get(tid, BUCKET_BITS[bucket])
             new_bits[st.bucket_base[bucket] + pos] = bits
-            moved |= bits != BUCKET_BITS[bucket]
+            if bits != BUCKET_BITS[bucket]:
+                moved.append(tid)
         if not moved:
             return
-        st.repack(new_bits.view(1, -1).to(self._dev), max_moves=len(self._slot))
+        st.repack(torch.frombuffer(new_bits, dtype=torch.uint8).view(1, -1).to(self._dev), max_moves=len(self._slot))
         st.check_errors()
         counts = st.counts[0].tolist()
         slot_token = st.slot_token[0].cpu().tolist()
@@ -635,9 +652,11 @@ class SmartKVCache:
             self._committed[b] = counts[b]
             for pos, t in enumerate(toks):
                 self._slot[int(t)] = (b, pos)
-        for (layer, tid), meta in self.k_cache.items():
-            if tid in self._slot:
-                meta["bits"] = BUCKET_BITS[self._slot[tid][0]]
+        for tid in moved:
+            for layer in self._layers_of[tid]:
+                meta = self.k_cache.get((layer, tid))
+                if meta is not None and tid in self._slot:
+                    meta["bits"] = BUCKET_BITS[self._slot[tid][0]]
         self._dev_base = st.cumulative.clone()
 
     # ------------------------------------------------------------------ fused decode step (used by the Llama wrapper)
@@ -664,7 +683,8 @@ class SmartKVCache:
         kv_dtype = torch.float16 if cur_k.dtype == torch.float16 else torch.float32
         out = st.attention(layer_idx, q.contiguous(), cur_k.reshape(1, self.num_heads, self.head_dim).to(kv_dtype),
                            cur_v.reshape(1, self.num_heads, self.head_dim).to(kv_dtype),
-                           update_importance=update_importance, cur_storage=cur_storage)
+                           update_importance=update_importance, cur_storage=cur_storage,
+                           out=torch.empty((1, self.num_query_heads, self.head_dim), dtype=torch.float32, device=self._dev))
         if update_importance:
             self.global_step += 1
             self._fused_seen_step = self.global_step
@@ -676,7 +696,7 @@ class SmartKVCache:
                 for t in [t for t in self.forecast_pending if t in self._slot]:
                     self._record_forecast_target(t, self.importance_tracker.get_importance(t))
             self._maybe_reallocate(layer_idx, [tid])
-        return out[0].clone()
+        return out[0]
 
     # ------------------------------------------------------------------ stats and misc
     def get_memory_stats(self) -> Dict[str, Any]:
@@ -748,6 +768,7 @@ class SmartKVCache:
         self._layers_of.clear()
         self._layer_tokens = [set() for _ in range(self.num_layers)]
         self._realloc_due = False
+        self._new_slots = []
         self._dev_base.zero_()
 
     def reset(self) -> None:
