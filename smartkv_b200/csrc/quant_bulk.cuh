@@ -9,7 +9,7 @@
 namespace skv {
 
 // ---- groups of eight consecutive elements per lane -----------------------------------------------------------------------
-// The bulk paths give a lane one (rows moved by a reallocation) or two (append of a prompt) such groups, so that several rows
+// The bulk paths (append of a prompt, rows moved by a reallocation) give a lane two such groups, so that several rows
 // share a warp's instructions, and run everything per element on two elements at once (fma.rn.f32x2; element i is paired
 // with i + 4) and on the multiply-add pipe: those kernels are bound by issue slots and by the half-rate integer pipe that
 // compares, selects and byte permutes go through.
@@ -97,32 +97,8 @@ __device__ __forceinline__ float quantize_groups(const float (&x)[G][8], float a
   }
   return scale;
 }
-template <int LPR>
-__device__ __forceinline__ float quantize8(const float (&x)[8], float amax, int bucket, uint32_t& lo, uint32_t& hi) {
-  uint32_t l[1], h[1];
-  const float scale = quantize_groups<LPR, 1>(reinterpret_cast<const float (&)[1][8]>(x), amax, bucket, l, h);
-  lo = l[0];
-  hi = h[0];
-  return scale;
-}
-
-// Stores a lane's packed field (lane l of the row's LPR; whole warp, `next` = lo of the next lane) at the row's address.
-__device__ __forceinline__ void store_field8(uint8_t* row, int bucket, int l, uint32_t lo, uint32_t hi, uint32_t next) {
-  uint32_t* out = reinterpret_cast<uint32_t*>(row);
-  if (bucket == 3) {
-    reinterpret_cast<uint2*>(out)[l] = make_uint2(lo, hi);
-  } else if (bucket == 2) {
-    out[l] = lo;
-  } else if (bucket == 0) {
-    reinterpret_cast<uint16_t*>(out)[l] = (uint16_t)lo;
-  } else {  // 3 bits: four lanes' 24-bit fields make three words
-    const int q = l & 3;
-    const uint32_t word = q == 0 ? (lo | (next << 24)) : q == 1 ? ((lo >> 8) | (next << 16)) : ((lo >> 16) | (next << 8));
-    if (q < 3) out[3 * (l >> 2) + q] = word;
-  }
-}
-
-// The same for a lane that holds two neighbouring groups (lane l of the row's head_dim / 16; `next` = lo[0] of the next lane).
+// Stores the packed fields of a lane that holds two neighbouring groups (lane l of the row's head_dim / 16; whole warp, `next` =
+// lo[0] of the next lane) at the row's address.
 __device__ __forceinline__ void store_field16(uint8_t* row, int bucket, int l, const uint32_t (&lo)[2], const uint32_t (&hi)[2],
                                               uint32_t next) {
   uint32_t* out = reinterpret_cast<uint32_t*>(row);

@@ -31,7 +31,7 @@ namespace skv {
 namespace cg = cooperative_groups;
 
 constexpr int kPlanThreads = 1024;
-constexpr int kStageRowBytes = 136;  // 8 bytes for each of up to 16 lanes, the fp32 scale, padding
+constexpr int kStageRowBytes = 136;  // 16 bytes for each of up to 8 lanes, the fp32 scale, padding
 constexpr int kMaxSeqsRepack = 1024;
 
 __device__ __forceinline__ int bucket_of_slot(const StoreGeom& g, int s) {
@@ -213,7 +213,6 @@ __device__ __forceinline__ int find_seq(const int* s_prefix, int B, int m) {
 // CTAs of 512 threads that work at once: two per SM of a B200 (the staging size depends on it, so it is no question to a device).
 constexpr int kRowThreads = 512;
 constexpr int kRowCtas = 296;
-constexpr int kRowBatch = 4;  // row groups whose loads a warp has in flight
 
 // One item = the moves of one (layer, KV head, sequence).  Phase 0 reads the source rows, requantises where the width changes
 // and leaves every lane's packed field and the scale in staging; after the cluster's barrier phase 1 writes the
@@ -225,9 +224,11 @@ constexpr int kRowBatch = 4;  // row groups whose loads a warp has in flight
 // took 4377 us a reallocation, now 2720 us.
 //
 // What bounds it: the rows are scattered pieces of 32 to 128 bytes, so the memory system needs many of them in flight
-// (a warp issues the loads of kRowBatch groups of rows first), and the quantiser's instructions.  As two grid-wide kernels per
+// (a warp issues the loads of four moves first), and the quantiser's instructions.  As two grid-wide kernels per
 // layer range, each with one row per half-warp and a staging buffer in HBM, 16 sequences of 8192 tokens, 32 layers, 8 heads
-// took 2330 us for 13,000 moves (2.9 GB of DRAM traffic: a row is two or three 32-byte sectors and its scale one); now 1360 us.
+// took 2330 us for 13,000 moves (2.9 GB of DRAM traffic: a row is two or three 32-byte sectors and its scale one); with 8 elements
+// a lane 1360 us.  A lane holds 16 elements, so that twice as many rows share the instructions that are done once per lane or
+// row: a whole reallocation 1677 -> 1403 us (two moves in flight 1517).
 // A row's place inside its (arena, KV head): bucket and position in one word, so that a warp passes it round in one shuffle.
 // Positions stay below 2^30 (a store has fewer than 2^31 / 3 storage indices), so all ones is no place.
 constexpr uint32_t kNoPlace = 0xffffffffu;
@@ -238,9 +239,10 @@ __device__ __forceinline__ uint32_t row_place(const StoreGeom& g, int slot) {
 
 template <int D, int CS>
 __global__ void __launch_bounds__(kRowThreads, 2) repack_rows_kernel(const __grid_constant__ RowMoveParams p) {
-  constexpr int LPR = D / 8;              // lanes per row
+  constexpr int LPR = D / 16;             // lanes per row
   constexpr int PPP = 32 / (2 * LPR);     // moves side by side in a warp: the K and the V row of each
-  constexpr int MB = kRowBatch * PPP;     // moves whose rows a warp has in flight
+  constexpr int RB = 4 / PPP;        // row groups whose loads a warp has in flight
+  constexpr int MB = RB * PPP;            // moves whose rows a warp has in flight
   constexpr int MC = 8;                   // moves a warp looks up at a time: lanes 0-7 the sources, 8-15 the destinations
   const StoreGeom& g = p.g;
   __shared__ int s_prefix[kMaxSeqsRepack + 1];
@@ -308,47 +310,74 @@ __global__ void __launch_bounds__(kRowThreads, 2) repack_rows_kernel(const __gri
       const uint32_t mine = look_up(c0);
 #pragma unroll 1
       for (int m0 = 0; m0 < MC && c0 + m0 < moves; m0 += MB) {
-        uint32_t w0[kRowBatch], w1[kRowBatch];
-        float sc[kRowBatch];
-        int bs[kRowBatch];
+        uint4 w[RB];
+        float sc[RB];
+        int bs[RB];
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
+        for (int u = 0; u < RB; ++u) {
           const uint32_t at = __shfl_sync(0xffffffffu, mine, m0 + u * PPP + sub);
           bs[u] = at == kNoPlace ? 0 : (int)(at >> 30);
-          w0[u] = w1[u] = 0u;
+          w[u] = make_uint4(0u, 0u, 0u, 0u);
           sc[u] = 0.f;
           if (at == kNoPlace) continue;
-          const int bits = kWidthConst[bs[u]].bits;
-          const int wi = (l * bits) >> 2;  // a lane's 8 * bits bits lie in at most two aligned words
-          const uint32_t* rp = reinterpret_cast<const uint32_t*>(row_ptr(at));
-          w0[u] = rp[wi];
-          if (wi + 1 < D / 32 * bits) w1[u] = rp[wi + 1];
+          // a lane's 16 * bits bits: one word, at 3 bits two words of which every other lane's begins halfway, two, or four
+          const uint32_t* rp = reinterpret_cast<const uint32_t*>(row_ptr(at)) + ((l * kWidthConst[bs[u]].bits) >> 1);
+          if (bs[u] == 3) {
+            const uint2 a = reinterpret_cast<const uint2*>(rp)[0], b = reinterpret_cast<const uint2*>(rp)[1];
+            w[u] = make_uint4(a.x, a.y, b.x, b.y);
+          } else {
+            w[u].x = rp[0];
+            if (bs[u] != 0) w[u].y = rp[1];
+          }
           sc[u] = *scale_ptr(at);
         }
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
+        for (int u = 0; u < RB; ++u) {
           const uint32_t to = __shfl_sync(0xffffffffu, mine, MC + m0 + u * PPP + sub);
           if (__all_sync(0xffffffffu, to == kNoPlace)) break;
           const int b_from = bs[u], b_to = to == kNoPlace ? 0 : (int)(to >> 30);
-          uint32_t lo = __funnelshift_r(w0[u], w1[u], (l * 8 * kWidthConst[b_from].bits) & 31), hi = w1[u];
+          uint32_t lo[2], hi[2] = {w[u].y, w[u].w};  // of each group of 8 elements; hi at 8 bits only
+          if (b_from == 3) {
+            lo[0] = w[u].x;
+            lo[1] = w[u].z;
+          } else if (b_from == 2) {
+            lo[0] = w[u].x;
+            lo[1] = w[u].y;
+          } else if (b_from == 1) {
+            const int sh = (l & 1) * 16;
+            const uint32_t v = __funnelshift_r(w[u].x, w[u].y, sh);
+            lo[0] = v & 0x00ffffffu;
+            lo[1] = (v >> 24) | (((w[u].y >> sh) & 0xffffu) << 8);
+          } else {
+            lo[0] = w[u].x & 0xffffu;
+            lo[1] = w[u].x >> 16;
+          }
           float scale = sc[u];
           if (__any_sync(0xffffffffu, b_from != b_to)) {
-            float x[8], amax = 0.f;
-            dequantize8(lo, hi, b_from, scale, x);
+            float x[2][8], amax = 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
-            uint32_t nlo, nhi;
-            const float ns = quantize8<LPR>(x, amax, b_to, nlo, nhi);
+            for (int j = 0; j < 2; ++j) {
+              dequantize8(lo[j], hi[j], b_from, scale, x[j]);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[j][i]));
+            }
+            uint32_t nlo[2], nhi[2];
+            const float ns = quantize_groups<LPR, 2>(x, amax, b_to, nlo, nhi);
             if (b_from != b_to) {
-              lo = nlo;
-              hi = nhi;
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                lo[j] = nlo[j];
+                hi[j] = nhi[j];
+              }
               scale = ns;
             }
           }
           if (to != kNoPlace) {
             uint8_t* st = stage + (long long)(c0 + m0 + u * PPP + sub) * 2 * kStageRowBytes;
-            reinterpret_cast<uint2*>(st)[l] = make_uint2(lo, hi);
-            if (l == 0) *reinterpret_cast<float*>(st + 8 * LPR) = scale;
+            uint2* f = reinterpret_cast<uint2*>(st) + 2 * l;  // staged rows lie on 8-byte boundaries
+            f[0] = make_uint2(lo[0], hi[0]);
+            f[1] = make_uint2(lo[1], hi[1]);
+            if (l == 0) *reinterpret_cast<float*>(st + 16 * LPR) = scale;
           }
         }
       }
@@ -358,27 +387,27 @@ __global__ void __launch_bounds__(kRowThreads, 2) repack_rows_kernel(const __gri
       const uint32_t mine = look_up(c0);
 #pragma unroll 1
       for (int m0 = 0; m0 < MC && c0 + m0 < moves; m0 += MB) {
-        uint2 f[kRowBatch];
-        float sc[kRowBatch];
+        uint2 f[RB][2];
+        float sc[RB];
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
-          f[u] = make_uint2(0u, 0u);
+        for (int u = 0; u < RB; ++u) {
+          f[u][0] = f[u][1] = make_uint2(0u, 0u);
           sc[u] = 0.f;
           if (c0 + m0 + u * PPP + sub < moves) {
             const uint8_t* st = stage + (long long)(c0 + m0 + u * PPP + sub) * 2 * kStageRowBytes;
-            f[u] = reinterpret_cast<const uint2*>(st)[l];
-            if (l == 0) sc[u] = *reinterpret_cast<const float*>(st + 8 * LPR);
+            f[u][0] = reinterpret_cast<const uint2*>(st)[2 * l];
+            f[u][1] = reinterpret_cast<const uint2*>(st)[2 * l + 1];
+            if (l == 0) sc[u] = *reinterpret_cast<const float*>(st + 16 * LPR);
           }
         }
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
+        for (int u = 0; u < RB; ++u) {
           const uint32_t at = __shfl_sync(0xffffffffu, mine, MC + m0 + u * PPP + sub);
           const int b = (int)(at >> 30);
-          // the fields of a 3-bit row moved unchanged carry their neighbours' bits above the lane's 24
-          const uint32_t lo = b == 1 ? f[u].x & 0x00ffffffu : f[u].x;
-          const uint32_t next = __shfl_down_sync(0xffffffffu, lo, 1);
+          const uint32_t lo[2] = {f[u][0].x, f[u][1].x}, hi[2] = {f[u][0].y, f[u][1].y};
+          const uint32_t next = __shfl_down_sync(0xffffffffu, lo[0], 1);
           if (at == kNoPlace) continue;
-          store_field8(row_ptr(at), b, l, lo, f[u].y, next);
+          store_field16(row_ptr(at), b, l, lo, hi, next);
           if (l == 0) {
             *scale_ptr(at) = sc[u];
             if (which) note_v_scale(g, arena, sc[u]);
