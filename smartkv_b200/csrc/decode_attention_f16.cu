@@ -560,7 +560,11 @@ __global__ void __launch_bounds__(StreamShape<D>::WARPS * 32, 1) decode_attn_f16
           float acc = 0.f;
 #pragma unroll
           for (int w = 0; w < WARPS; ++w)
-            if ((who >> w) & 1u) acc = fmaf(sh.weight[w][h], acc_at[w * (S::RING / 4)], acc);
+            if ((who >> w) & 1u) {
+              // a piece that does not count may hold anything (masked keys with an infinite V scale): select, not multiply
+              const float f = sh.weight[w][h];
+              acc = f == 0.f ? acc : fmaf(f, acc_at[w * (S::RING / 4)], acc);
+            }
           out[h * (D + 2) + 2 + d] = acc;
         }
       }

@@ -56,3 +56,32 @@ def test_one_long_segment_over_all_ctas():
 def test_more_runs_than_a_merge_holds():
     # 1600 segments: eleven or so in each of 148 CTAs, eight between two merges
     check(32, 8, 128, 21, 200, (2, 3, 4, 8), seed=6, sequences=(0, 1, 73, 199))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("group", [4, 8])
+@pytest.mark.parametrize("masked_with", [float("-inf"), float(torch.finfo(torch.float32).min)])
+@pytest.mark.parametrize("width", [2, 8])
+def test_warps_that_hold_only_masked_infinite_values_do_not_count(d, group, masked_with, width):
+    """Three tiles for every CTA, one for each of three warps: every third tile's keys are masked and their V rows infinite.  The
+    warps are folded by weight, and those of weight 0 hold NaN."""
+    n = 16 * 148 * 3
+    gen = torch.Generator(device="cuda").manual_seed(d + group)
+    store = make_store(1, 1, 1, d, group, n)
+    k, v = (torch.randn((n, 1, d), generator=gen, device="cuda") for _ in range(2))
+    hidden = torch.arange(n, device="cuda") % 48 < 16
+    v[hidden, 0, 5] = float("inf")
+    dst = store.plan_bulk(torch.full((1, n), width, dtype=torch.int64, device="cuda"))
+    store.append(0, k, v, *dst[:3])
+    q = torch.randn((1, group, d), generator=gen, device="cuda").half()
+    mask = torch.zeros((1, n), device="cuda")
+    mask[0, hidden] = masked_with
+    out = store.attention(0, q, mask=mask).double()[0]
+    store.check_errors()
+    _, _, kc, vc, ks, vs = store.export_sequence(0, 0)
+    seen = ~hidden
+    kd, vd = kc[seen, 0].double() * ks[seen].double(), vc[seen, 0].double() * vs[seen].double()
+    p = torch.softmax(q[0].double() @ kd.T / math.sqrt(d), -1)
+    logit = q[0].double().abs().amax(1, keepdim=True) * 2.0 ** -15 * kd.abs().sum(1).max() / math.sqrt(d)
+    bound = (2.0 ** -11 + 2 * logit) * (p @ vd.abs()) + 1e-6    # as in check()
+    assert bool(((out - p @ vd).abs() <= bound).all())
