@@ -85,3 +85,31 @@ def test_warps_that_hold_only_masked_infinite_values_do_not_count(d, group, mask
     logit = q[0].double().abs().amax(1, keepdim=True) * 2.0 ** -15 * kd.abs().sum(1).max() / math.sqrt(d)
     bound = (2.0 ** -11 + 2 * logit) * (p @ vd.abs()) + 1e-6    # as in check()
     assert bool(((out - p @ vd).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("group", [4, 8])
+def test_the_weight_of_a_key_far_above_all_before_it_is_not_rounded(d, group):
+    """One CTA, four tiles a warp.  One key stands 2^4.5 to 2^7.5 above the others, in the last tile of the first warp; the
+    others have no value.  Its row is 2 bits wide, so its V scale is the fp16 number it was made from, and once it sets the
+    running maximum its weight times that scale is exact: what is left is 32-bit arithmetic.  Rounded to fp16 the weight would
+    be off by up to 2^-11."""
+    n = 16 * 4 * (16 if d == 64 else 12)
+    at = 16 * 3 + 5
+    store = make_store(1, 1, 1, d, group, n)
+    store.num_ctas = 1
+    k, v = torch.zeros((n, 1, d), device="cuda"), torch.zeros((n, 1, d), device="cuda")
+    k[at, 0, 7] = 1.0
+    v[at, 0] = torch.where(torch.arange(d, device="cuda") % 3 == 0, 0.7, -0.7).half().float()
+    dst = store.plan_bulk(torch.full((1, n), 2, dtype=torch.int64, device="cuda"))
+    store.append(0, k, v, *dst[:3])
+    above = torch.linspace(4.5, 7.5, group, device="cuda", dtype=torch.float64)
+    q = torch.zeros((1, group, d), device="cuda", dtype=torch.float16)
+    q[0, :, 7] = (above * math.sqrt(d) * math.log(2.0)).half()
+    out = store.attention(0, q).double()[0]
+    store.check_errors()
+    p = torch.softmax(torch.where(torch.arange(n, device="cuda") == at, q[0, :, 7:8].double() / math.sqrt(d), 0.0), -1)
+    ref = p[:, at:at + 1] * v[at, 0].double()
+    # the query's one element is a whole number of limb steps, so the logit (at most 7.5 log2 units) and the sum of up to 1024
+    # weights carry 32-bit roundings only: 2^-16 leaves room for 2^8 of them
+    assert bool(((out - ref).abs() <= 2.0 ** -16 * ref.abs()).all())
