@@ -679,9 +679,10 @@ __global__ void __launch_bounds__((CFG::NCONS + 1) * 32, 1) decode_attn_kernel(c
 }
 
 // ---- combine ----------------------------------------------------------------------
+template <bool FIRST>
 __global__ void __launch_bounds__(kPostThreads) lse_combine_kernel(const CombineParams p) {
   __shared__ CombineShared sh;
-  combine_unit(p, blockIdx.x, sh);
+  combine_unit<FIRST>(p, blockIdx.x, sh);
 }
 
 }  // namespace skv
@@ -879,8 +880,9 @@ extern "C" int skv_lse_combine_masked(const SkvStoreDesc* desc, const void* plan
   p.cur_prob = cur_prob;
   p.scale_log2 = (float)(1.4426950408889634 / sqrt((double)desc->head_dim));
   p.per_run = skv_attn_partials_per_run(desc, query_dtype);
-  p.first_of_run = skv::attn_first_of_run(desc, query_dtype);
-  lse_combine_kernel<<<combine_units(p.g, group), kPostThreads, 0, as_stream(stream)>>>(p);
+  const int units = combine_units(p.g, group);
+  if (skv::attn_first_of_run(desc, query_dtype)) lse_combine_kernel<true><<<units, kPostThreads, 0, as_stream(stream)>>>(p);
+  else lse_combine_kernel<false><<<units, kPostThreads, 0, as_stream(stream)>>>(p);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }
 

@@ -25,7 +25,7 @@ union PostShared {
   ImportanceShared i;
 };
 
-template <int EPL, class IMP>
+template <int EPL, class IMP, bool FIRST>
 __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const PostParams p) {
   __shared__ PostShared sh;
   // dependent launch: the next layer's attention kernel may be scheduled as soon as every block here has started (it
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kPostThreads) post_attention_kernel(const Post
   }
   blk -= imp_blocks;
   if (blk < p.combine_blocks) {
-    combine_unit(p.c, blk, sh.c);
+    combine_unit<FIRST>(p.c, blk, sh.c);
     return;
   }
   blk -= p.combine_blocks;
@@ -61,22 +61,23 @@ static int imp_chunks(const StoreGeom& g, int max_seq_tokens, int chunk, int* co
   return *compact ? live : all;
 }
 
-template <int EPL, class IMP>
+template <int EPL, bool FIRST, class IMP>
 static cudaError_t launch_post(PostParams& p, int max_seq_tokens, cudaStream_t st, bool dep) {
   p.imp_chunks = p.imp.logits != nullptr ? imp_chunks(p.c.g, max_seq_tokens, IMP::CHUNK, &p.imp_compact) : 0;
   const int grid = p.combine_blocks + p.imp_chunks * p.c.g.num_seqs + p.append_blocks;
-  return launch_maybe_dependent(post_attention_kernel<EPL, IMP>, dim3(grid), dim3(kPostThreads), 0, st, p, dep);
+  return launch_maybe_dependent(post_attention_kernel<EPL, IMP, FIRST>, dim3(grid), dim3(kPostThreads), 0, st, p, dep);
 }
-template <int EPL>
+template <int EPL, bool FIRST>
 static cudaError_t launch_post(PostParams& p, int max_seq_tokens, cudaStream_t st, bool dep) {
   const long long other = p.combine_blocks + p.append_blocks, seqs = p.c.g.num_seqs, sms = p.c.num_ctas;
   int compact;
   if (p.imp.logits == nullptr || imp_chunks(p.c.g, max_seq_tokens, ImpOne::CHUNK, &compact) * seqs + other <= 4 * sms)
-    return launch_post<EPL, ImpOne>(p, max_seq_tokens, st, dep);
+    return launch_post<EPL, FIRST, ImpOne>(p, max_seq_tokens, st, dep);
   const bool sixteen = p.c.num_q_heads > 8 && imp_chunks(p.c.g, max_seq_tokens, ImpFour16<true>::CHUNK, &compact) * seqs + other <= 2 * sms;
   if (importance_aligned(p.imp))
-    return sixteen ? launch_post<EPL, ImpFour16<true>>(p, max_seq_tokens, st, dep) : launch_post<EPL, ImpFour8<true>>(p, max_seq_tokens, st, dep);
-  return launch_post<EPL, ImpFour8<false>>(p, max_seq_tokens, st, dep);
+    return sixteen ? launch_post<EPL, FIRST, ImpFour16<true>>(p, max_seq_tokens, st, dep)
+                   : launch_post<EPL, FIRST, ImpFour8<true>>(p, max_seq_tokens, st, dep);
+  return launch_post<EPL, FIRST, ImpFour8<false>>(p, max_seq_tokens, st, dep);
 }
 
 }  // namespace skv
@@ -120,7 +121,7 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
   c.group = group;
   c.partials = static_cast<const float*>(partials);
   c.per_run = skv_attn_partials_per_run(desc, query_dtype);
-  c.first_of_run = attn_first_of_run(desc, query_dtype);
+  const bool first = attn_first_of_run(desc, query_dtype);
   c.num_ctas = num_ctas;
   c.cur_k = cur_k;
   c.cur_v = cur_v;
@@ -168,7 +169,7 @@ extern "C" int skv_post_attention(const SkvStoreDesc* desc, void* store, int lay
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool dep = g_dependent_launch.load() == 1 || g_dependent_launch.load() == 3;
-  if (desc->head_dim == 128) launch_post<4>(p, max_seq_tokens, st, dep);
-  else launch_post<2>(p, max_seq_tokens, st, dep);
+  if (desc->head_dim == 128) first ? launch_post<4, true>(p, max_seq_tokens, st, dep) : launch_post<4, false>(p, max_seq_tokens, st, dep);
+  else first ? launch_post<2, true>(p, max_seq_tokens, st, dep) : launch_post<2, false>(p, max_seq_tokens, st, dep);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

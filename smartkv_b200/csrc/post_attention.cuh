@@ -39,7 +39,6 @@ struct CombineParams {
   int group;
   const float* partials;
   int per_run;  // partials a run has room for
-  bool first_of_run;  // only the first of them is filled, and of a segment's last run the second (fp16 queries)
   int num_ctas;
   const void* cur_k;
   const void* cur_v;
@@ -78,6 +77,9 @@ __device__ __forceinline__ float head_dot(float prod, int sub, int d, int D, flo
 }
 
 // One unit = up to kPostThreads / D query heads of one (sequence, KV head); blockDim.x == kPostThreads.
+// FIRST: of a run's partials only the first is filled, and of a segment's last run the second (fp16 queries,
+// attn_first_of_run); otherwise all of them.
+template <bool FIRST>
 __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, CombineShared& sh) {
   const StoreGeom& g = p.g;
   const int D = g.head_dim, G = p.group, Hkv = g.num_kv_heads;
@@ -90,12 +92,12 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
   const int gqc = valid ? gq : G - 1;  // threads of a missing head go through the motions of the last one
   const PlanView pv = plan_view(const_cast<int*>(p.plan), p.num_ctas, g.num_seqs * Hkv);
   const int runs = pv.seg_count[seg];
-  const int nsplit = runs == 0 ? 0 : p.first_of_run ? runs + 1 : runs * p.per_run;
+  const int nsplit = runs == 0 ? 0 : FIRST ? runs + 1 : runs * p.per_run;
   const int r0 = runs > 0 ? pv.seg_begin[seg] * p.per_run : 0;
   const int pstride = partial_stride(G, D);
   // the k-th filled partial, in floats from the segment's first (its runs are at most one a CTA)
-  const int step = (p.first_of_run ? p.per_run : 1) * pstride, last = (runs - 1) * step + pstride;
-  auto at = [&](int k) { return p.first_of_run && k == runs ? last : k * step; };
+  const int step = (FIRST ? p.per_run : 1) * pstride, last = (runs - 1) * step + pstride;
+  auto at = [&](int k) { return FIRST && k == runs ? last : k * step; };
   const float* base = p.partials + (long long)r0 * pstride + gqc * (D + 2);
   const bool has_cur = p.cur_k != nullptr && p.cur_v != nullptr;
   const long long hq = (long long)b * p.num_q_heads + h * G + gqc;
@@ -103,9 +105,12 @@ __device__ __forceinline__ void combine_unit(const CombineParams& p, int unit, C
 
   // kRowsAhead rows at a time, their loads in flight together and the first of them beside the headers: a loop over the rows
   // with a load each waits for every one (segments of 12 and of 40 partials: the last block ended 7.0 and 14.2 us after
-  // the attention launch, now 4.3 and 8 us).  Eight: sixteen and twenty-four cost more in code and registers than the
-  // round trips they save (steps of 8 x 770 keys 266 us, 274, 288).
-  constexpr int kRowsAhead = 8;
+  // the attention launch, now 4.3 and 8 us).  Where a run leaves one partial the lists are short and eight do: sixteen and
+  // twenty-four cost more in code and registers than the round trips they save (8 x 770 keys, 22 layers: 276 us a step at eight,
+  // 8 and 22 us more at sixteen and twenty-four).  Where it leaves seven (fp32 queries) or four (tensor memory) a segment
+  // has up to a thousand and sixteen are needed (us for four layers, one KV head, eight / sixteen: 1 x 2048 keys fp32 337 / 221,
+  // 1 x 131072 fp32 439 / 304, tensor memory 308 / 232; eight KV heads: 1 x 2048 107 / 90, 16 x 8192 278 / 278).
+  constexpr int kRowsAhead = FIRST ? 8 : 16;
   float x[kRowsAhead];
   auto fetch = [&](int k0) {
 #pragma unroll
