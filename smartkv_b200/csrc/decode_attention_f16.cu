@@ -567,9 +567,10 @@ __global__ void __launch_bounds__(StreamShape<D>::WARPS * 32, 1) decode_attn_f16
 #pragma unroll
           for (int w = 0; w < WARPS; ++w)
             if ((who >> w) & 1u) {
-              // a piece that does not count may hold anything (masked keys with an infinite V scale): select, not multiply
-              const float f = sh.weight[w][h];
-              acc = f == 0.f ? acc : fmaf(f, acc_at[w * (S::RING / 4)], acc);
+              // a piece that does not count may hold anything (masked keys with an infinite V scale): select, not multiply,
+              // and select after both loads (a load that waits for the weight: 16 x 8192 keys 1588 -> 1612 us a step)
+              const float f = sh.weight[w][h], x = acc_at[w * (S::RING / 4)];
+              acc = fmaf(f, f == 0.f ? 0.f : x, acc);
             }
           out[h * (D + 2) + 2 + d] = acc;
         }
