@@ -297,6 +297,8 @@ class SmartKVCache:
         try:
             for tid in ids:
                 if tid not in slot:
+                    if not -2 ** 31 <= tid < 2 ** 31:
+                        raise ValueError(f"token id {tid} does not fit the 32 bits the store keeps it in")
                     bits = self.precision_map.get(tid, 4)
                     if bits not in BITS_TO_BUCKET:
                         raise ValueError(f"token {tid} has width {bits}; the store holds 2, 3, 4 or 8 bits")

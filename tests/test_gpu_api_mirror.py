@@ -330,3 +330,25 @@ def test_cache_grows_past_its_initial_capacity():
     vq, vs = orc.quantize_rows(kv[0][1], 4)
     ref, _ = orc.streaming_attention(q[None, :, None, :], kq, ks, vq, vs, tile_size=512, current_k=ck[None], current_v=cv[None])
     assert_close(out.cpu().numpy(), ref[0, :, 0], what="attention after growth")
+
+
+@pytest.mark.parametrize("bad", ["id", "width"])
+def test_a_refused_token_does_not_lose_the_ones_before_it(bad):
+    """A batch whose third token cannot be stored raises; the first two have their places, on the device as on the host, and
+    everything stored afterwards works."""
+    from smartkv_b200 import SmartKVCache
+    cache = SmartKVCache(num_layers=1, num_heads=2, head_dim=64, memory_budget=0.5, max_tokens=100)
+    cache.token_counter = 1
+    kv = torch.randn((4, 2, 64), device="cuda")
+    refused = 2 ** 31 if bad == "id" else 2
+    if bad == "width":
+        cache.precision_map[2] = 5
+    with pytest.raises(Exception):
+        cache.quantize_and_store_batch(0, [0, 1, refused, 3], kv, kv)
+    cache.precision_map.pop(2, None)
+    ids = [0, 1, 3, 4]
+    cache.quantize_and_store_batch(0, ids, kv, kv)
+    assert sorted(cache._slot) == ids and cache.store.counts.sum().item() == 4
+    tokens = cache.store.slot_token[0].cpu().tolist()
+    for t, (bucket, pos) in cache._slot.items():
+        assert tokens[cache.store.bucket_base[bucket] + pos] == t
