@@ -202,8 +202,20 @@ class SmartKVCache:
         self._layers_of[token_id] = set()
         return bucket, pos
 
+    def _place(self, token_id: int) -> None:
+        """Gives a new token its place (the store may be replaced by a larger one); _enter_slots puts it on the device."""
+        if not -2 ** 31 <= token_id < 2 ** 31:
+            raise ValueError(f"token id {token_id} does not fit the 32 bits the store keeps it in")
+        bits = self.precision_map.get(token_id, 4)
+        if bits not in BITS_TO_BUCKET:
+            raise ValueError(f"token {token_id} has width {bits}; the store holds 2, 3, 4 or 8 bits")
+        self.precision_map.setdefault(token_id, bits)
+        bucket, pos = self._assign_slot(token_id, bits)
+        self._new_slots.append((self.store.bucket_base[bucket] + pos, token_id,
+                                self.importance_tracker.token_importance.get(token_id)))
+
     def _enter_slots(self):
-        """Puts the tokens placed by _assign_slot on the device: one indexed write per array instead of
+        """Puts the tokens placed by _place on the device: one indexed write per array instead of
         a launch per token."""
         new, self._new_slots = self._new_slots, []
         if not new:
@@ -293,20 +305,11 @@ class SmartKVCache:
         elif v.dtype != k.dtype:
             v = v.to(k.dtype)
         buckets, poss = [], []
-        slot, base = self._slot, self.store.bucket_base
         try:
             for tid in ids:
-                if tid not in slot:
-                    if not -2 ** 31 <= tid < 2 ** 31:
-                        raise ValueError(f"token id {tid} does not fit the 32 bits the store keeps it in")
-                    bits = self.precision_map.get(tid, 4)
-                    if bits not in BITS_TO_BUCKET:
-                        raise ValueError(f"token {tid} has width {bits}; the store holds 2, 3, 4 or 8 bits")
-                    self.precision_map.setdefault(tid, bits)
-                    bucket, pos = self._assign_slot(tid, bits)
-                    slot, base = self._slot, self.store.bucket_base      # of the new store, if there was no room
-                    self._new_slots.append((base[bucket] + pos, tid, self.importance_tracker.token_importance.get(tid)))
-                bucket, pos = slot[tid]
+                if tid not in self._slot:
+                    self._place(tid)
+                bucket, pos = self._slot[tid]
                 buckets.append(bucket)
                 poss.append(pos)
         finally:
@@ -671,12 +674,10 @@ class SmartKVCache:
         token and of the current one is folded into the importance arrays on the device (the
         cache-level contract of update_attention: token_ids are the ids of the keys)."""
         tid = int(token_id)
-        st = self.store
         if tid not in self._slot:
-            bits = self.precision_map.get(tid, 4)
-            self.precision_map.setdefault(tid, bits)
-            bucket, pos = self._assign_slot(tid, bits)
-            st.slot_token[0, st.bucket_base[bucket] + pos] = tid
+            self._place(tid)
+            self._enter_slots()
+        st = self.store                         # after _place, which may have replaced it
         bucket, pos = self._slot[tid]
         cur_storage = torch.tensor([st.bucket_base[bucket] + pos], dtype=torch.int32, device=self._dev)
         q = query.reshape(1, self.num_query_heads, self.head_dim)

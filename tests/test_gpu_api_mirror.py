@@ -352,3 +352,46 @@ def test_a_refused_token_does_not_lose_the_ones_before_it(bad):
     tokens = cache.store.slot_token[0].cpu().tolist()
     for t, (bucket, pos) in cache._slot.items():
         assert tokens[cache.store.bucket_base[bucket] + pos] == t
+
+
+def test_cache_grows_inside_a_decode_step():
+    """A step's token that finds its bucket full makes the store grow inside fused_decode_attention.  From there on the cache must
+    hold what one that was large enough from the start holds: outputs, tokens, importance, and widths after a reallocation."""
+    from smartkv_b200 import SmartKVCache
+    L, Hq, H, d, steps = 2, 4, 2, 64, 6
+    small, large = (SmartKVCache(num_layers=L, num_heads=H, head_dim=d, memory_budget=0.5, max_tokens=m, num_query_heads=Hq)
+                    for m in (100, 400))
+    n = small.store.caps[2] - 4             # the bucket of 4 bits is full after three steps
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    rand = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    prompt = [(rand(n, H, d), rand(n, H, d)) for _ in range(L)]
+    for c in (small, large):
+        c.token_counter = 1
+        c.importance_tracker.token_importance[n + 3] = 0.25     # gathered before the token had a place
+        for layer, (k, v) in enumerate(prompt):
+            c.quantize_and_store_batch(layer, list(range(n)), k, v)
+    for i in range(steps):
+        for layer in range(L):
+            q, k, v = rand(Hq, d), rand(H, d), rand(H, d)
+            outs = []
+            for c in (small, large):
+                c.token_counter = 1         # no reallocation yet
+                outs.append(c.fused_decode_attention(layer, q, k, v, n + i))
+                c.quantize_and_store_batch(layer, [n + i], k[None], v[None])
+            assert torch.allclose(*outs, rtol=1e-5, atol=1e-6), (i, layer)
+    assert small.store.caps[2] > n + 4
+
+    def by_token(c, values):
+        values = values.cpu()
+        return torch.stack([values[c.store.bucket_base[b] + p] for b, p in (c._slot[t] for t in range(n + steps))])
+
+    for _ in range(2):
+        for c in (small, large):
+            assert sorted(c._slot) == list(range(n + steps))
+            assert by_token(c, c.store.slot_token[0]).tolist() == list(range(n + steps))
+        assert torch.allclose(by_token(small, small.store.cumulative[0]), by_token(large, large.store.cumulative[0]), rtol=1e-5)
+        a, b = ([c.get_importance(t) for t in range(n + steps)] for c in (small, large))
+        assert np.allclose(a, b, rtol=1e-5)
+        for c in (small, large):            # second time round: after a reallocation that moves tokens
+            c.allocate_precision(0, list(range(n + steps)))
+    assert small.precision_map == large.precision_map and len(set(small.precision_map.values())) > 1
