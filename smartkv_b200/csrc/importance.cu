@@ -61,7 +61,7 @@ extern "C" int skv_importance_update(const SkvStoreDesc* desc, int layer, const 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // as the launch after the attention chooses (post_attention.cuh); how many chunks are live is not known here
   if ((long long)desc->slots * desc->num_seqs <= 4LL * 148 * ImpOne::CHUNK) launch_importance<ImpOne>(p, st);
-  else if (importance_aligned(p)) launch_importance<ImpFour8<true>>(p, st);
-  else launch_importance<ImpFour8<false>>(p, st);
+  else if (importance_aligned(p)) launch_importance<ImpFour<true>>(p, st);
+  else launch_importance<ImpFour<false>>(p, st);
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_CUDA;
 }

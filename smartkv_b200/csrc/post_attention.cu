@@ -73,11 +73,8 @@ static cudaError_t launch_post(PostParams& p, int max_seq_tokens, cudaStream_t s
   int compact;
   if (p.imp.logits == nullptr || imp_chunks(p.c.g, max_seq_tokens, ImpOne::CHUNK, &compact) * seqs + other <= 4 * sms)
     return launch_post<EPL, FIRST, ImpOne>(p, max_seq_tokens, st, dep);
-  const bool sixteen = p.c.num_q_heads > 8 && imp_chunks(p.c.g, max_seq_tokens, ImpFour16<true>::CHUNK, &compact) * seqs + other <= 2 * sms;
-  if (importance_aligned(p.imp))
-    return sixteen ? launch_post<EPL, FIRST, ImpFour16<true>>(p, max_seq_tokens, st, dep)
-                   : launch_post<EPL, FIRST, ImpFour8<true>>(p, max_seq_tokens, st, dep);
-  return launch_post<EPL, FIRST, ImpFour8<false>>(p, max_seq_tokens, st, dep);
+  return importance_aligned(p.imp) ? launch_post<EPL, FIRST, ImpFour<true>>(p, max_seq_tokens, st, dep)
+                                   : launch_post<EPL, FIRST, ImpFour<false>>(p, max_seq_tokens, st, dep);
 }
 
 }  // namespace skv

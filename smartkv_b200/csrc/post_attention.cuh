@@ -456,16 +456,14 @@ inline bool importance_aligned(const ImportanceParams& p) {
                       reinterpret_cast<uintptr_t>(p.layer_ema);
   return a % 16 == 0 && reinterpret_cast<uintptr_t>(p.touched) % 4 == 0;
 }
-// Single indices with all of 32 heads in flight where their blocks fit one wave of four an SM; else four indices a thread,
-// with sixteen heads in flight (118 registers, two blocks an SM) where there are more than eight and the launch fits one wave
-// that way, with eight (80 registers, three blocks) otherwise.  Steps, us: 8 x 770 keys, 32 heads, 22 layers: single 276, four
-// 317; 16 x 8192, 32 heads: four with eight heads 1603, with sixteen 1705, two with sixteen 1617; 64 x 16384, 8 heads:
-// four 1253, two 1402.
+// Single indices with all of 32 heads in flight where their blocks fit one wave of four an SM; else four indices a thread with
+// eight heads in flight (80 registers, three blocks an SM).  Steps, us: 8 x 770 keys, 32 heads, 22 layers: single 276, four
+// 317; 16 x 8192, 32 heads: four 1603, two with sixteen heads 1617; 64 x 16384, 8 heads: four 1253, two 1402.  Between them (four
+// layers; a form with sixteen heads in flight had been kept for these), single / four with sixteen / four with eight:
+// 4 x 32768, 32 heads 210 / 214 / 214; 2 x 65536, 64 heads 243 / 251 / 252; 2 x 100000, 16 heads (two layers) 106 / 102 / 101.
 using ImpOne = ImpShape<1, 32, false>;
 template <bool VEC>
-using ImpFour16 = ImpShape<4, 16, VEC>;
-template <bool VEC>
-using ImpFour8 = ImpShape<4, 8, VEC>;
+using ImpFour = ImpShape<4, 8, VEC>;
 
 // ---- append ---------------------------------------------------------------------------------------------
 struct AppendParams {
