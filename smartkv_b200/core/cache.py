@@ -221,6 +221,13 @@ class SmartKVCache:
         if not new:
             return
         st, dev = self.store, self._dev
+        if len(new) == 1:   # a fill each: less host time than tensors made for one element (98 -> 72 us a stored token of one layer)
+            at, tid, seed = new[0]
+            st.slot_token[0, at] = tid
+            if seed is not None:
+                st.cumulative[0, at] = seed
+                self._dev_base[0, at] = seed
+            return
         at, tids = torch.tensor([[i for i, _, _ in new], [t for _, t, _ in new]], dtype=torch.int32).to(dev)
         st.slot_token[0].index_put_((at.long(),), tids)
         seeded = [(i, x) for i, _, x in new if x is not None]
