@@ -7,27 +7,43 @@ import pytest
 import torch
 
 from oracle import smartkv_oracle as orc
+from smartkv_b200 import _lib
 from tests.gpu_util import fill_store, make_store
 
 pytestmark = pytest.mark.gpu
 
 
-def check(hq, hkv, d, n, batch, widths, seed, sequences=None):
+def check(hq, hkv, d, n, batch, widths, seed, sequences=None, masked=False, value_gain=None, plan_of_128=False):
     rng = np.random.default_rng(seed)
     k, v = orc.synth_kv(batch * n, hkv, d, seed=seed)
+    if value_gain is not None:
+        v = (v * rng.uniform(*value_gain, size=(batch * n, hkv, 1))).astype(np.float32)
     bits = rng.choice(widths, size=(batch, n))
     store = make_store(1, batch, hkv, d, hq, n)
     fill_store(store, [(k.reshape(batch, n, hkv, d), v.reshape(batch, n, hkv, d))], bits)
     q = torch.from_numpy(rng.standard_normal((batch, hq, d)).astype(np.float16)).cuda()
-    out = store.attention(0, q).double()
+    mask = None
+    if masked:      # single keys, whole tiles of 16 and beyond, and ordinary values
+        mask = torch.from_numpy(rng.standard_normal((batch, n)).astype(np.float32)).cuda()
+        mask[:, 5::11] = -1e4
+        mask[:, n // 3:n // 2] = float("-inf")
+    if plan_of_128:
+        _lib.lib().skv_set_attention_path(2)
+        try:
+            store.build_plan()
+        finally:
+            _lib.lib().skv_set_attention_path(0)
+        assert int(store.plan[3]) == 128 and store._plan_valid
+    out = store.attention(0, q, mask=mask).double()
     store.check_errors()
     group = hq // hkv
     for b in sequences or range(batch):
-        _, _, kc, vc, ks, vs = store.export_sequence(0, b)
+        ids, _, kc, vc, ks, vs = store.export_sequence(0, b)
+        bias = 0.0 if mask is None else mask[b, ids.long()].double()
         for h in range(hkv):
             kd, vd = kc[:, h].double() * ks[:, h, None].double(), vc[:, h].double() * vs[:, h, None].double()
             qd = q[b, h * group:(h + 1) * group].double()
-            p = torch.softmax(qd @ kd.T / math.sqrt(d), -1)
+            p = torch.softmax(qd @ kd.T / math.sqrt(d) + bias, -1)
             # p * v_scale is rounded to fp16 (2^-11 of each term); the query to 2^-15 of its row's largest element, which moves
             # a logit by at most that times sum |k| / sqrt(d) and a probability by twice as much of itself
             logit = qd.abs().amax(1, keepdim=True) * 2.0 ** -15 * kd.abs().sum(1).max() / math.sqrt(d)
@@ -47,6 +63,30 @@ def test_group_sizes(d, group):
 @pytest.mark.parametrize("n", [1, 17, 4096 + 5])
 def test_one_width(d, width, n):
     check(8, 2, d, n, 1, (width,), seed=n + width)
+
+
+# 2 x 2 x 331 keys are a tile or less a warp; one sequence of 40007 keys gives every warp several, with a ragged last one
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("group", [4, 5, 8])
+@pytest.mark.parametrize("hkv,n,batch", [(2, 331, 2), (1, 40007, 1)])
+def test_masked(d, group, hkv, n, batch):
+    check(group * hkv, hkv, d, n, batch, (2, 3, 4, 8), seed=group + n, masked=True)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("group", [4, 8])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("hkv,n,batch", [(2, 331, 2), (1, 40007, 1)])
+def test_value_scales_beyond_the_fp16_guard(d, group, masked, hkv, n, batch):
+    # scales of 10 to 1e5: some below the limit of 64 and most above it, so the running maximum is raised for some tiles
+    check(group * hkv, hkv, d, n, batch, (2, 3, 4, 8), seed=group + n, masked=masked, value_gain=(10, 1e5))
+
+
+@pytest.mark.parametrize("group", [4, 8])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("hkv,n,batch", [(2, 331, 2), (1, 40007, 1)])
+def test_plan_in_tiles_of_128_keys(group, masked, hkv, n, batch):
+    check(group * hkv, hkv, 128, n, batch, (2, 3, 4, 8), seed=group + n, masked=masked, plan_of_128=True)
 
 
 def test_one_long_segment_over_all_ctas():

@@ -1,8 +1,7 @@
-"""skv_importance_update over head counts, bucket fills and array alignments: the same bits whether the arrays can be read four
-elements at a time or not, and the 64-bit sums within the rounding of 32-bit ones."""
+"""skv_importance_update over head counts, bucket fills, array alignments and sizes on both sides of the limit between one and four
+storage indices a thread: the same bits in every form, and the 64-bit sums within the rounding of 32-bit ones."""
 import ctypes
 
-import numpy as np
 import pytest
 import torch
 
@@ -23,29 +22,43 @@ def shifted(t, elements):
 
 @pytest.mark.parametrize("heads", [1, 8, 9, 32, 128])
 @pytest.mark.parametrize("counts", [(0, 0, 0, 0), (1, 3, 127, 5), (128, 0, 126, 1023), (1021, 130, 2, 64)])
-def test_importance_update(heads, counts):
-    batch, layers, layer = 3, 2, 1
+@pytest.mark.parametrize("batch", [3, 66])
+def test_importance_update(heads, counts, batch):
+    # 2688 storage indices a sequence; up to 4 x 148 blocks of 256 take one a thread, 66 sequences are more
+    layers, layer = 2, 1
     store = PackedKVStore(layers, batch, 1, 64, 8, (1152, 256, 128, 1152))
-    slots, rng = store.slots, np.random.default_rng(heads + counts[0])
+    slots = store.slots
+    assert (batch * slots <= 4 * 148 * 256) == (batch == 3)
     gen = torch.Generator(device="cuda").manual_seed(heads)
     rand = lambda *s: torch.rand(s, generator=gen, device="cuda")
-    filled = torch.tensor([counts, (0, 0, 0, 0), counts], dtype=torch.int32, device="cuda")
+    filled = torch.tensor([counts, (0, 0, 0, 0), counts] * (batch // 3), dtype=torch.int32, device="cuda")
     base = store.bucket_base
-    cur_slot = torch.tensor([base[2] + counts[2] if counts[2] < 128 else base[0] + counts[0], base[3], -1], dtype=torch.int32, device="cuda")
+    cur_slot = torch.tensor([base[2] + counts[2] if counts[2] < 128 else base[0] + counts[0], base[3], -1] * (batch // 3),
+                            dtype=torch.int32, device="cuda")
     logits, lse_max, lse_sum = -8 * rand(batch, heads, slots), rand(batch, heads), 1 + 9 * rand(batch, heads)
     cur_prob, head_state = rand(batch, heads), 0.5 + rand(batch, 2, heads)
     cumulative, ema = torch.rand((batch, slots), generator=gen, device="cuda", dtype=torch.float64), rand(layers, batch, slots)
     touched = (rand(layers, batch, slots) < 0.5).to(torch.uint8)
     decay, head_decay = 0.9, 0.8
-    results = []
-    for offset in (0, 1):
-        lg, cm, em, tc, hs = (shifted(t, offset) for t in (logits, cumulative, ema, touched, head_state))
-        check(store.lib.skv_importance_update(ctypes.byref(store.desc), layer, ptr(filled), heads, ptr(lg), ptr(lse_max), ptr(lse_sum),
+
+    def update(desc, offset, *arrays):
+        filled, lg, lse_max, lse_sum, cur_prob, cur_slot, hs, cm, em, tc = arrays
+        lg, cm, em, tc, hs = (shifted(t, offset) for t in (lg, cm, em, tc, hs))
+        check(store.lib.skv_importance_update(ctypes.byref(desc), layer, ptr(filled), heads, ptr(lg), ptr(lse_max), ptr(lse_sum),
                                               ptr(cur_prob), ptr(cur_slot), ptr(hs), 0, ptr(cm), ptr(em), ptr(tc), decay, head_decay,
                                               _lib.stream_ptr()))
-        results.append((cm, em, tc, hs))
+        return cm, em, tc, hs
+
+    arrays = (filled, logits, lse_max, lse_sum, cur_prob, cur_slot, head_state, cumulative, ema, touched)
+    results = [update(store.desc, offset, *arrays) for offset in (0, 1)]
     for a, b in zip(*results):
         assert torch.equal(a, b)
+    alone = PackedKVStore(layers, 1, 1, 64, 8, (1152, 256, 128, 1152)).desc
+    for b in range(3):      # a sequence by itself takes one index a thread
+        one = update(alone, 0, *(t[:, b:b + 1].contiguous() if t is ema or t is touched else t[b:b + 1].contiguous() for t in arrays))
+        cm, em, tc, hs = results[0]
+        for x, y in zip(one, (cm[b:b + 1], em[:, b:b + 1], tc[:, b:b + 1], hs[b:b + 1])):
+            assert torch.equal(x, y)
     cm, em, tc, hs = results[0]
     want_c, want_e, want_t = cumulative.clone(), ema.double(), touched.clone()
     for b in range(batch):

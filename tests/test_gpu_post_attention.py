@@ -30,16 +30,20 @@ def test_fused_post_attention_equals_separate_calls(hq, hkv, d, q_dtype):
     _fused_equals_separate(3, hq, hkv, d, 700, q_dtype)
 
 
-def test_fused_post_attention_large_batch_takes_the_wide_importance_blocks():
-    """80 sequences x 18 live chunks exceed two waves of importance blocks, so the fused launch switches to blocks of four
-    chunks (four keys per thread, their loads in flight together); the stand-alone importance kernel keeps one.  The
-    per-key sums run in the same order either way, so every importance array must come out the same."""
-    _fused_equals_separate(80, 4, 1, 64, 2000, np.float16)
+@pytest.mark.parametrize("aligned", [True, False])
+def test_fused_post_attention_large_batch_takes_the_wide_importance_blocks(aligned):
+    """80 sequences x 2000 keys are more than a wave of blocks with one key a thread, so the fused launch takes four a thread; so
+    does the stand-alone kernel (test_gpu_importance_blocks.py compares the forms).  With arrays that are not aligned for loads
+    of four elements both read one at a time."""
+    _fused_equals_separate(80, 4, 1, 64, 2000, np.float16, aligned)
 
 
-def _fused_equals_separate(B, hq, hkv, d, n, q_dtype):
+def _fused_equals_separate(B, hq, hkv, d, n, q_dtype, aligned=True):
     L = 2
     (a, b, c), rng = _pair(B, hq, hkv, d, n, L, seed=hq + d)
+    if not aligned:
+        for s in (a, b, c):
+            s.layer_ema = torch.zeros(s.layer_ema.numel() + 1, device="cuda")[1:].view(s.layer_ema.shape)
     for step in range(3):
         plan_a, plan_b, plan_c = a.plan_step(), b.plan_step(), c.plan_step()
         outs_a, outs_c = [], [torch.empty((B, hq, d), dtype=torch.float32, device="cuda") for _ in range(L)]
