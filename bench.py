@@ -491,7 +491,7 @@ def run_ours(args):
     else:
         skv_lib.lib().skv_set_attention_path(2 if args.attn_kernel == "tensor_memory" else 1)
         store._plan_valid = False
-    kernel_name = "decode_attn_tc_kernel" if skv_lib.lib().skv_get_attention_path() == 2 else "decode_attn_kernel"
+    kernel_name = "decode_attn_tc_kernel" if skv_lib.lib().skv_get_attention_path() == 2 else "decode_attn_f16_kernel"
 
     attn_events = []
     launches = [0]
@@ -800,7 +800,7 @@ def run_ours(args):
         "metric": "packed_kv_decode_attention_throughput", "value": round(value, 2), "unit": "GB/s",
         "n_gpus": world, "steps": steps, "warmup": warmup, "ms_per_step": round(ms / steps, 4),
         "higher_is_better": True, "scaling": "weak" if (shard == "replicas" and world > 1) else "strong", "vs_baseline": None,
-        "dtype": "int8 tensor-core scores, f16 P.V, f32 accumulate" if kernel_name == "decode_attn_kernel" else "int8 tensor-core scores and P.V (tcgen05), f32 accumulate",
+        "dtype": "int8 tensor-core scores, f16 P.V, f32 accumulate" if kernel_name == "decode_attn_f16_kernel" else "int8 tensor-core scores and P.V (tcgen05), f32 accumulate",
         "data": f"synthetic (seeded N(0,1) K/V, 4 outlier channels x8 per head, Zipf({cfg['zipf_s']}) importance)",
         "config": {"workload": workload_string(cfg),
                    "sharding": shard_txt if world > 1 else "one GPU", "kv_heads_per_gpu": Hkv_r,

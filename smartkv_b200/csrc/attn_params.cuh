@@ -1,5 +1,5 @@
-// Launch parameters and helpers shared by the two decode-attention kernels (the mma.sync fragment
-// kernel in decode_attention.cu and the tensor-memory kernel in decode_attention_tc.cu).
+// Launch parameters and helpers shared by the decode-attention kernels (mma.sync: decode_attention_f16.cu for fp16 queries,
+// decode_attention.cu for fp32; tensor memory: decode_attention_tc.cu).
 #pragma once
 
 #include "attn_sched.cuh"
@@ -52,10 +52,13 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// fp16 queries (decode_attention_f16.cu).  A run has room for eleven partials, of which the kernel fills the first -- what its
-// warps merged -- and, of a run that ends inside a CTA (a segment's last), the second: the piece of a warp that went on to the
-// next run.  The rest is marked empty.
+// Partials of a run.  The caller's buffer has room for kMaxPartialsPerRun of them whatever the path; each kernel asserts that it
+// leaves no more.  fp16 queries (decode_attention_f16.cu): of the eleven places the kernel fills the first -- what its warps
+// merged -- and, of a run that ends inside a CTA (a segment's last), the second: the piece of a warp that went on to the next run.
+// The rest is marked empty.
+constexpr int kMaxPartialsPerRun = 11;
 constexpr int kF16PartialsPerRun = 11;
+static_assert(kF16PartialsPerRun <= kMaxPartialsPerRun, "the partials buffer is sized for kMaxPartialsPerRun");
 int launch_attn_f16(const AttnParams& p, cudaStream_t stream);
 
 // The tensor-memory kernel (decode_attention_tc.cu): head_dim 128, fp16 queries, group <= 8.

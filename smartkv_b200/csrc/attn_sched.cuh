@@ -30,10 +30,11 @@ constexpr int kPlanModelTc = 1;    // 128-key tiles, tensor-memory kernel
 __host__ __device__ constexpr int plan_tile_keys(int model) { return model == kPlanModelTc ? 128 : 16; }
 
 // Relative cost of one tile.  Model 0: what a warp of the fp16-query kernel spends on a 16-key tile of each width while its
-// SM works on all of them (B200, head_dim 128, cycles per tile at 2 / 3 / 4 / 8 bits: 16 x 8192 keys at a budget of 0.35
-// 1770 / 1810 / 1890 / 2070, one sequence of 131072 at 0.25 1400 / 1720 / 1540 / 1730); the costs it replaces, 105 / 116 / 110 /
-// 143, had been measured width by width on whole launches (one sequence of 131072: 37.6 us a launch with those, 35.6 with
-// these).  Model 1: the block's bytes in units of 256 B plus a fixed per-block term.  Only the ratios matter.
+// SM works on all of them, at head_dim 128; the costs it replaces, 105 / 116 / 110 / 143, had been measured width by width on
+// whole launches.  One plan serves fp32 queries and head_dim 64 too.  Steps of four layers, us, with those / with these: fp16
+// queries, head_dim 128, 16 x 8192 keys 226 / 222, 1 x 32768 at a budget of 0.35 103 / 101, at 0.25 96 / 97; head_dim 64, 64 x 4096
+// 219 / 215, 8 x 770 67 / 67; fp32 queries, 16 x 8192 279 / 278, head_dim 64 154 / 151, 64 x 4096 262 / 260.  Model 1: the block's bytes
+// in units of 256 B plus a fixed per-block term.  Only the ratios matter.
 __host__ __device__ constexpr int tile_cost_for(int head_dim, int bits, int model) {
   if (model == kPlanModelTc) return 128 * (2 * row_bytes_for(head_dim, bits) + 8) / 256 + 24;
   return bits == 2 ? 95 : bits == 3 ? 107 : bits == 4 ? 100 : 109;

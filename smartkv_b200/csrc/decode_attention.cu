@@ -37,8 +37,8 @@ template <int NCONS_, int STAGES_, int STAGE_BYTES_>
 struct AttnCfg {
   static constexpr int NCONS = NCONS_, STAGES = STAGES_, STAGE_BYTES = STAGE_BYTES_;
 };
-constexpr int kMaxPartialsPerRun = kF16PartialsPerRun;
 using AttnCfgPrecise = AttnCfg<7, 3, 42240>;   // three query limbs and P in two halves: 8 warps, up to 255 registers a thread
+static_assert(AttnCfgPrecise::NCONS <= kMaxPartialsPerRun, "the partials buffer is sized for kMaxPartialsPerRun");
 
 // tiles per block for a bit-width: as many 16-key tiles as fit one stage
 __host__ __device__ constexpr int block_tiles(int stage_bytes, int head_dim, int bits) {

@@ -13,12 +13,12 @@
 // Replaces smartkv/csrc/quantized_attention.cu:460-828 (per-bucket kernel, one CTA per head walking the whole context);
 // numerics follow the CPU streaming path smartkv/core/fused_cpu.py:70-113 (dequantise, q.k/sqrt(d), online softmax).
 //
-// Bound: HBM while streaming (16 x 8192 keys at a budget of 0.35: 190 MB in 30 of the launch's 46 us, 6.3 TB/s); the rest is the
-// start (plan, first copies, query: 5 us), the merge and the spread of the warps' ends.  Before (one producer warp with bulk
-// copies, 11 consumer warps on shared blocks, partials per warp; see decode_attention.cu, which keeps that form for fp32
-// queries), us a launch: 45.8 (16 x 8192) -> 45.9, 41.2 (1 x 131072) -> 35.6, 53.5 (64 x 16384, one KV head) -> 50.1, 13.0 (8 x
-// 770, head_dim 64) -> 11.3; a decode step, whose combine now folds two partials a run: 1763 -> 1714, 1740 -> 1448, 1640 -> 1463,
-// 418 -> 331.
+// Bound: HBM while streaming (16 x 8192 keys at a budget of 0.35: 188 MB in 41.4 us a launch back to back, some 30 of them at
+// 6.3 TB/s); the rest is the start (plan, first copies, query: 5 us), the merge and the spread of the warps' ends.  Before (one
+// producer warp with bulk copies, 11 consumer warps on shared blocks, partials per warp; see decode_attention.cu, which keeps
+// that form for fp32 queries) and now, us a launch back to back: 43.5 / 41.4 (16 x 8192), 38.2 / 33.3 (1 x 131072), 50.8 / 46.1
+// (64 x 16384, one KV head), 11.1 / 7.6 (8 x 770, head_dim 64); a decode step, whose combine now folds one partial a run:
+// 1763 / 1589, 1740 / 1304, 1640 / 1249, 418 / 274.
 #include <atomic>
 #include <cstdio>
 #include <type_traits>
@@ -43,8 +43,8 @@ constexpr float kLazyTau = 4.0f;
 
 // Warps of a CTA.  head_dim 128: twelve, 168 registers each; sixteen at 128 end later for all their work in flight, because
 // every warp brings its start, its share of the merge and a rounding to whole tiles (steps of 16 x 8192 keys 1610 us
-// against 1658, 64 x 16384 1253 against 1288, 1 x 131072 the same; eight warps 1687, 1317 and 1487 against 1358).  head_dim 64, whose
-// contexts are short: sixteen (8 x 770 keys 303 us a step, twelve 316).
+// against 1658, 64 x 16384 1253 against 1288, 1 x 131072 the same; eight warps 1687, 1317 and 1487 against 1358; all with the
+// combine of two partials a run).  head_dim 64, whose contexts are short: sixteen (8 x 770 keys 303 us a step, twelve 316).
 template <int D>
 struct StreamShape {
   static constexpr int WARPS = D == 128 ? 12 : 16;

@@ -898,6 +898,7 @@ int launch_tc(const AttnParams& p, const CUtensorMap& kmap, const CUtensorMap& v
 
 namespace skv {
 
+static_assert(kTcPartialsPerRun <= kMaxPartialsPerRun, "the partials buffer is sized for kMaxPartialsPerRun");
 int attn_tc_partials_per_run() { return kTcPartialsPerRun; }
 
 int launch_attn_tc(const AttnParams& p, const SkvStoreDesc& desc, cudaStream_t stream) {

@@ -59,7 +59,8 @@ extern "C" int skv_importance_update(const SkvStoreDesc* desc, int layer, const 
   p.decay = decay;
   p.head_decay = head_decay;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // as the launch after the attention chooses (post_attention.cuh); how many chunks are live is not known here
+  // as the launch after the attention chooses (post_attention.cuh), on a B200's 148 SMs; how many chunks are live and how many
+  // SMs the attention has is not known here
   if ((long long)desc->slots * desc->num_seqs <= 4LL * 148 * ImpOne::CHUNK) launch_importance<ImpOne>(p, st);
   else if (importance_aligned(p)) launch_importance<ImpFour<true>>(p, st);
   else launch_importance<ImpFour<false>>(p, st);

@@ -238,8 +238,8 @@ struct ImportanceShared {
 
 // Maps the j-th *live* chunk of sequence b (chunks of CHUNK storage indices that hold a cached
 // key or the slot the current token will take) to its chunk index; -1 when j is past the last one.
-// Buckets lie at increasing storage indices, so their chunk ranges are increasing and only neighbours can
-// share a chunk.  j == 0 always maps to a chunk (chunk 0 if nothing is live): that block publishes the
+// Buckets lie at increasing storage indices, so their chunk ranges are increasing; a chunk that several buckets share belongs to
+// the first of them.  j == 0 always maps to a chunk (chunk 0 if nothing is live): that block publishes the
 // head-importance EMA.
 template <int CHUNK>
 __device__ __forceinline__ int live_chunk(const StoreGeom& g, const int32_t* counts4, int j) {
